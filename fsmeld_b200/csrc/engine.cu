@@ -420,9 +420,10 @@ static int run_stats(fsmeld_ctx* c, const Geom& g, Stats* st, const std::string&
     if ((r = bufT(c, "sig" + tag, (size_t)g.S * g.kml, &st->SIG))) return r;
     const size_t smem = mvmean_smem_bytes();
     if ((r = allow_smem(c, k_mvmean, smem))) return r;
-    const unsigned blocks = (unsigned)((g.S + 31) / 32);
+    const int seg = mvmean_segments(g.S, c->sm_count);
+    const unsigned blocks = (unsigned)((g.S + seg - 1) / seg);
     prof_begin(c, ST_STATS);
-    k_mvmean<<<blocks, kMvmeanThreads, smem, c->stream>>>(c->d_target, g, st->MU, st->SIG);
+    k_mvmean<<<blocks, kMvmeanThreads, smem, c->stream>>>(c->d_target, g, st->MU, st->SIG, seg);
     LAUNCH_CHECK(c);
     return FSMELD_OK;
 }

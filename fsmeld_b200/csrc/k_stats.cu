@@ -6,24 +6,31 @@
 // a window containing a non-finite point gets NaN statistics.  The sums are
 // a serial recurrence whose rounding decides validity (sigma <= 1e-12) and
 // every z-normalised candidate, so each segment is one sequential chain: one
-// lane per segment, 32 segments per warp.
+// lane per segment, up to 16 segments per block.
 //
-// Memory: lanes of a warp walk 32 different segments in lock step.  The raw
-// stream is staged through shared memory in tiles of kTile points (32
-// coalesced 256-byte loads per tile and stream, prefetched into registers a
-// tile ahead), so global traffic is one read of the target (plus the m-1 halo
-// per segment) and one coalesced write of mu and sigma.
+// What bounds it: the chain, two dependent FP64 adds (16 cycles) per point and
+// segment, m_k points long whatever the target's length (24 cycles a point
+// with its shared-memory accesses), next to about 35 FP64 operations per window
+// for mean and sigma; from a few hundred blocks on also
+// the HBM traffic (one read of the target with the m-1 halo per segment, the
+// outgoing points again from L2, 16 bytes written per window).  So one warp of
+// the block does nothing but the chain: its operands lie ready in shared
+// memory and its loop is 32 unrolled steps without a branch, and the other
+// eight warps do the rest a tile of 32 points ahead or behind:
+//   * the incoming points t[k] and the outgoing points t[k-m] (0 before the
+//     first full window) of tile t + 3 into registers, those of tile t + 1
+//     from registers into shared memory, non-finite points as 0.0 and one bit
+//     in a mask per segment (x - 0.0 and x + 0.0 leave every sum as it is, so
+//     the first m points and the skipped ones need no case of their own);
+//   * mean and sigma of the windows that end in tile t - 1 (two divisions by
+//     m, each a multiply by RN(1/m) and FMA corrections that give the
+//     correctly rounded quotient, and a square root), written coalesced.
+// One block barrier per tile.  Short targets take fewer segments per block
+// (mvmean_segments), so that their windows' divisions spread over more SMs.
 //
 // Raw (non-normalised) mode (g.raw): a window is valid iff its points are all
 // finite, and its statistics are mean 0 and sigma 1, so every later stage
 // sees the raw values ((t - 0) / 1 = t exactly) with the same code.
-//
-// Work split: warp 0 of the block runs the 32 running-sum chains (the serial
-// part) and stages each emitted window's sums and non-finite flag in a
-// double-buffered tile; warps 1-3 turn the previous tile's sums into mean
-// and sigma (two divisions by m, each a multiply by RN(1/m) and FMA
-// corrections that give the correctly rounded quotient, and a square root
-// per window) and write them out, so the chains never wait for them.
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -32,123 +39,168 @@ namespace fsm {
 namespace {
 constexpr int kTile = 32;
 constexpr int kPitch = kTile + 1;  // padded rows: lane-strided smem reads hit distinct banks
-constexpr int kTileDoubles = 32 * kPitch;
+constexpr int kRows = 16;          // segments per block at most
+constexpr int kTileDoubles = kRows * kPitch;
+constexpr int kMaskTiles = 4;      // tiles whose non-finite masks are kept (tile t - 1 .. t + 1)
+constexpr int kHelpers = kMvmeanThreads / 32 - 1;  // two rows of a tile each
+static_assert(2 * kHelpers == kRows, "helpers take rows h and h + kHelpers");
 }
 
-__global__ void __launch_bounds__(kMvmeanThreads) k_mvmean(const double* __restrict__ target, Geom g,
-                                                           double* __restrict__ mu, double* __restrict__ sig) {
-    extern __shared__ double sm[];
-    double* tin = sm;                        // [32][kPitch] incoming points t[k] (warp 0)
-    double* tout = sm + kTileDoubles;        // [32][kPitch] outgoing points t[k-m] (warp 0)
-    double* S1 = sm + 2 * kTileDoubles;      // [2][32][kPitch] staged sums, by tile parity
-    double* S2 = sm + 4 * kTileDoubles;      // [2][32][kPitch] staged sums of squares
-    int* FL = (int*)(sm + 6 * kTileDoubles); // [2][32][kPitch] staged non-finite flags
-    const int tid = threadIdx.x;
-    const int lane = tid & 31;
-    const long long s0 = (long long)blockIdx.x * 32;
+__global__ void __launch_bounds__(kMvmeanThreads, 4) k_mvmean(const double* __restrict__ target, Geom g,
+                                                              double* __restrict__ mu, double* __restrict__ sig,
+                                                              int seg) {
+    extern __shared__ __align__(16) double sm[];
+    double* tin = sm;                                     // [2][kRows][kPitch] incoming points t[k], by tile parity
+    double* tout = tin + 2 * kTileDoubles;                // [2][kRows][kPitch] outgoing points t[k-m]
+    double* S1 = tout + 2 * kTileDoubles;                 // [2][kRows][kPitch] sums after each point
+    double* S2 = S1 + 2 * kTileDoubles;                   // [2][kRows][kPitch] sums of squares
+    unsigned* IM = (unsigned*)(S2 + 2 * kTileDoubles);    // [kMaskTiles][kRows] non-finite incoming points of a row
+    unsigned* OM = IM + kMaskTiles * kRows;                  // [kMaskTiles][kRows] the same of the outgoing points
+    int* NF = (int*)(OM + kMaskTiles * kRows);               // [2][kRows] non-finite points in the window before the tile
+    const int lane = threadIdx.x & 31;
+    // the chain warps of the blocks resident on one SM sit on different
+    // sub-partitions (blocks are handed out to the SMs in turn)
+    const int id = threadIdx.x >> 5, cw = (int)(blockIdx.x / 148) & 3;
+    const bool chain = id == cw;
+    const int h = id - (id > cw ? 1 : 0);  // helper: rows h and h + kHelpers
+    const long long s0 = (long long)blockIdx.x * seg;  // seg <= kRows segments
     const int m = g.m, mk = g.m_k, kml = g.kml;
     const int ntiles = (mk + kTile - 1) / kTile;
+    const bool row[2] = {h < seg && s0 + h < g.S, h + kHelpers < seg && s0 + h + kHelpers < g.S};
+    const double* tp[2] = {target + g.off(row[0] ? s0 + h : 0) + lane, target + g.off(row[1] ? s0 + h + kHelpers : 0) + lane};
 
-    // consumers (warps 1-3): mean and sigma of the emitted windows of tile t
-    auto finish_tile = [&](int t) {
-        const int k0 = t * kTile, cnt = min(kTile, mk - k0);
-        const int b = t & 1;
-        const double dm = (double)m;
-        const double invm = ddiv(1.0, dm);  // S / m by the reciprocal method (correctly rounded)
-        const double qnan = dnan();
-        for (int idx = tid - 32; idx < 32 * kTile; idx += kMvmeanThreads - 32) {
-            const int r = idx / kTile, x = idx % kTile;  // segment s0 + r, point k0 + x
-            const long long sr = s0 + r;
-            if (x < cnt && k0 + x >= m - 1 && sr < g.S) {
-                const int o = b * kTileDoubles + r * kPitch + x;
-                const bool bad = FL[o] != 0;
-                double mean, sd;
-                if (g.raw) {  // raw mode: valid iff every point is finite
-                    mean = bad ? qnan : 0.0;
-                    sd = bad ? qnan : 1.0;
-                } else {
-                    mean = bad ? qnan : zdiv_i(S1[o], dm, invm, true);
-                    sd = bad ? qnan : dsqrt(dsub(zdiv_i(S2[o], dm, invm, true), dmul(mean, mean)));
-                }
-                const long long w = sr * kml + (k0 + x - m + 1);
-                mu[w] = mean;
-                sig[w] = sd;
+    // helpers: this thread's points of tile t (row h + kHelpers u, point lane)
+    struct Points { double in[2], out[2]; };
+    auto load_tile = [&](int t, Points& p) {
+        if (h >= seg) return;
+        const int k0 = t * kTile, k = k0 + lane;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const bool in = row[u] && k < mk;
+            p.in[u] = in ? tp[u][k0] : 0.0;
+            p.out[u] = in && k >= m ? tp[u][k0 - m] : 0.0;
+        }
+    };
+    auto stage_tile = [&](int t, const Points& p) {
+        if (h >= seg) return;
+        const int b = (t & (kMaskTiles - 1)) * kRows, st = (t & 1) * kTileDoubles;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int r = h + kHelpers * u, o = st + r * kPitch + lane;
+            const bool bi = !isfinite(p.in[u]), bo = !isfinite(p.out[u]);
+            const unsigned mi = __ballot_sync(0xffffffffu, bi), mo = __ballot_sync(0xffffffffu, bo);
+            if (r >= seg) continue;
+            tin[o] = bi ? 0.0 : p.in[u];
+            tout[o] = bo ? 0.0 : p.out[u];
+            if (lane == 0) {
+                IM[b + r] = mi;
+                OM[b + r] = mo;
             }
         }
     };
+    // helpers: mean and sigma of the windows that end in tile t
+    const double dm = (double)m;
+    const double invm = ddiv(1.0, dm);  // S / m by the reciprocal method (correctly rounded)
+    auto finish_tile = [&](int t) {
+        const int k = t * kTile + lane;
+        const int b = t & 1, ms = (t & (kMaskTiles - 1)) * kRows;
+        if (k < m - 1 || k >= mk) return;
+        const unsigned upto = 0xffffffffu >> (31 - lane);
+        double mean[2] = {}, sd[2] = {};
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int r = h + kHelpers * u, o = b * kTileDoubles + r * kPitch + lane;
+            if (!row[u]) continue;
+            const bool bad = NF[b * kRows + r] + __popc(IM[ms + r] & upto) - __popc(OM[ms + r] & upto) != 0;
+            mean[u] = 0.0;
+            sd[u] = 1.0;  // raw mode: valid iff every point is finite
+            if (!g.raw) {
+                // both quotients by the reciprocal method with one range test
+                const double a1 = S1[o], a2 = S2[o];
+                const double e1 = rcp_div_estimate(a1, invm), e2 = rcp_div_estimate(a2, invm);
+                double z1 = rcp_div_finish(a1, dm, invm, e1), z2 = rcp_div_finish(a2, dm, invm, e2);
+                if (!(rcp_div_in_range_bits(e1) & rcp_div_in_range_bits(e2))) {
+                    z1 = ddiv(a1, dm);
+                    z2 = ddiv(a2, dm);
+                }
+                mean[u] = z1;
+                sd[u] = dsqrt(dsub(z2, dmul(z1, z1)));
+            }
+            if (bad) mean[u] = sd[u] = dnan();
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            if (!row[u]) continue;
+            const long long w = (s0 + h + kHelpers * u) * kml + (k - m + 1);
+            mu[w] = mean[u];
+            sig[w] = sd[u];
+        }
+    };
 
-    // producer (warp 0): the running sums of segment s0 + lane
     double s1 = 0.0, s2 = 0.0;
     int nonfinite = 0;
-    double pin[32], pout[32];  // the next tile (row r = segment s0 + r, column = lane)
-    auto load_tile = [&](int k0) {
-        const int cnt = min(kTile, mk - k0);
-#pragma unroll
-        for (int r = 0; r < 32; ++r) {
-            const long long sr = s0 + r;
-            double vi = 0.0, vo = 0.0;
-            if (sr < g.S && lane < cnt) {
-                const double* tp = target + g.off(sr);
-                vi = tp[k0 + lane];
-                const int ko = k0 + lane - m;
-                if (ko >= 0) vo = tp[ko];
-            }
-            pin[r] = vi;
-            pout[r] = vo;
-        }
-    };
-    if (tid < 32) load_tile(0);
+    Points p1{}, p2{};
+    if (!chain) {
+        load_tile(0, p1);
+        stage_tile(0, p1);
+        load_tile(1, p1);
+        load_tile(2, p2);
+    }
+    __syncthreads();
+    const int first = (m - 1) / kTile;  // the first tile that a window ends in
     for (int t = 0; t <= ntiles; ++t) {
-        if (tid < 32) {
-            if (t < ntiles) {
-                const int k0 = t * kTile, cnt = min(kTile, mk - k0);
-                const int b = t & 1;
+        if (chain) {
+            if (t < ntiles && lane < seg) {
+                const int b = t & 1, ms = (t & (kMaskTiles - 1)) * kRows, o = b * kTileDoubles + lane * kPitch;
+                const double *in = tin + o, *out = tout + o;
+                double *q1 = S1 + o, *q2 = S2 + o;
+                NF[b * kRows + lane] = nonfinite;
+                nonfinite += __popc(IM[ms + lane]) - __popc(OM[ms + lane]);
+                // src/mvmean.cpp:16-27 (outgoing 0.0) and 32-44; operands in
+                // registers four steps ahead of the adds
+                double vi[4], vo[4];
 #pragma unroll
-                for (int r = 0; r < 32; ++r) {
-                    tin[r * kPitch + lane] = pin[r];
-                    tout[r * kPitch + lane] = pout[r];
-                }
-                __syncwarp();
-                if (k0 + kTile < mk) load_tile(k0 + kTile);
-                for (int x = 0; x < cnt; ++x) {
-                    const int k = k0 + x;
-                    const double incoming_raw = tin[lane * kPitch + x];
-                    if (k < m) {
-                        // initial window (src/mvmean.cpp:16-27)
-                        if (isfinite(incoming_raw)) {
-                            s1 = dadd(s1, incoming_raw);
-                            s2 = dadd(s2, dmul(incoming_raw, incoming_raw));
-                        } else {
-                            ++nonfinite;
-                        }
-                    } else {
-                        // slide by one (src/mvmean.cpp:32-44)
-                        const double outgoing_raw = tout[lane * kPitch + x];
-                        const bool of = isfinite(outgoing_raw), inf = isfinite(incoming_raw);
-                        const double outgoing = of ? outgoing_raw : 0.0;
-                        const double incoming = inf ? incoming_raw : 0.0;
-                        nonfinite += (int)!inf - (int)!of;
-                        s1 = dadd(dsub(s1, outgoing), incoming);
-                        s2 = dadd(dsub(s2, dmul(outgoing, outgoing)), dmul(incoming, incoming));
+                for (int u = 0; u < 4; ++u) { vi[u] = in[u]; vo[u] = out[u]; }
+#pragma unroll
+                for (int x0 = 0; x0 < kTile; x0 += 4) {
+                    double ni[4] = {}, no[4] = {};
+                    if (x0 + 4 < kTile) {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) { ni[u] = in[x0 + 4 + u]; no[u] = out[x0 + 4 + u]; }
                     }
-                    if (k >= m - 1) {  // a window ends here
-                        const int o = b * kTileDoubles + lane * kPitch + x;
-                        S1[o] = s1;
-                        S2[o] = s2;
-                        FL[o] = nonfinite;
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        s1 = dadd(dsub(s1, vo[u]), vi[u]);
+                        s2 = dadd(dsub(s2, dmul(vo[u], vo[u])), dmul(vi[u], vi[u]));
+                        q1[x0 + u] = s1;
+                        q2[x0 + u] = s2;
                     }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) { vi[u] = ni[u]; vo[u] = no[u]; }
                 }
-                __syncwarp();
             }
-        } else if (t > 0) {
-            finish_tile(t - 1);
+        } else {
+            if (t + 1 < ntiles) stage_tile(t + 1, p1);
+            p1 = p2;
+            load_tile(t + 3, p2);
+            if (t > first) finish_tile(t - 1);
         }
-        // tile t is staged and tile t-1 consumed: the producer may overwrite
-        // buffer (t-1) & 1 with tile t+1
+        // tile t's sums are staged, tile t-1's consumed, tile t+1's points are there
         __syncthreads();
     }
 }
 
-size_t mvmean_smem_bytes() { return sizeof(double) * 6 * kTileDoubles + sizeof(int) * 2 * kTileDoubles; }
+size_t mvmean_smem_bytes() {
+    return sizeof(double) * 8 * kTileDoubles + sizeof(unsigned) * (2 * kMaskTiles + 2) * kRows;
+}
+
+// Segments per block: the fewest for which all blocks are resident at once,
+// one chain on every sub-partition of an SM at most (the chain of a block takes
+// the same time for one segment as for kRows)
+int mvmean_segments(long long S, int sm_count) {
+    int seg = 2;
+    while (seg < kRows && (S + seg - 1) / seg > 4LL * sm_count) seg *= 2;
+    return seg;
+}
 
 }  // namespace fsm

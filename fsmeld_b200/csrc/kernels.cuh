@@ -115,11 +115,12 @@ size_t lbgemm_smem_bytes(int nq_pad, int m);
 constexpr int kLbGemmThreads = 128;
 constexpr int kLbGemmKChunk = 64;
 
-// window statistics: one block per 32 segments, warp 0 runs the running sums
-// and warps 1-3 derive mean and sigma
-constexpr int kMvmeanThreads = 128;
+// window statistics: one block per seg (mvmean_segments) segments, one warp runs the running sums
+// and eight load the points and derive mean and sigma
+constexpr int kMvmeanThreads = 288;
 __global__ void k_mvmean(const double* __restrict__ target, Geom g, double* __restrict__ mu,
-                         double* __restrict__ sig);
+                         double* __restrict__ sig, int seg);
+int mvmean_segments(long long S, int sm_count);
 template <int T, int OPT, bool GW>
 __global__ void k_envelope(const double* __restrict__ target, const double* __restrict__ MU,
                            const double* __restrict__ SIG, Geom g, int w, double* __restrict__ Un,

@@ -202,7 +202,8 @@ static int exact_noalloc(int device, const double* device_target, int64_t n, con
     const size_t sm_stats = mvmean_smem_bytes();
     if ((e = raise_smem_limit((const void*)k_mvmean, device, sm_stats)) != cudaSuccess)
         return cuda_fail(e, "cudaFuncSetAttribute", __FILE__, __LINE__);
-    k_mvmean<<<(unsigned)((g.S + 31) / 32), kMvmeanThreads, sm_stats, st>>>(device_target, g, MU, SIG);
+    const int seg = mvmean_segments(g.S, sms);
+    k_mvmean<<<(unsigned)((g.S + seg - 1) / seg), kMvmeanThreads, sm_stats, st>>>(device_target, g, MU, SIG, seg);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_mvmean", __FILE__, __LINE__);
 
     QueryDev qd{};
