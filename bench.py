@@ -174,6 +174,8 @@ def roofline(stages, cells, peaks):
     if launches == 0 or ms <= 0.0:
         return None
     kernel = "k_dp" if n_wave == 0 else ("k_dpw" if n_lane == 0 else "k_dp+k_dpw")
+    # EDR and LCSS run as bit vectors (k_bitdp): no FP64 cells
+    cells = {mt: c for mt, c in cells.items() if mt not in ("edr", "lcss")}
     flops = sum(cells[mt] * FLOPS_PER_CELL[mt] for mt in cells)
     avg_s = ms / launches / 1e3
     achieved = flops / launches / avg_s / 1e12

@@ -195,6 +195,20 @@ __device__ __forceinline__ double qt_term(int metric, double x, int k, int m, in
     return qt_term_env(metric, x, (a1 < a0) ? a1 : a0, (b0 < b1) ? b1 : b0, mu, sg, inv, ok, arg);
 }
 
+// The matching table of an EDR or LCSS query (k_bitdp): E holds the 2m ends of
+// the intervals of candidate values that match a query point, ascending, then
+// +inf; grid[b] is the number of ends in buckets below b; table has a row of
+// rs words for each of the 2m + 1 ranges between ends.
+constexpr int kBitBuckets = 2048;
+struct BitTab {
+    const double* E = nullptr;
+    const unsigned short* grid = nullptr;
+    const unsigned* table = nullptr;
+    int rs = 0, pad = 0;  // words per row, zero words in front of query point 0
+    int in_smem = 0;
+    double e0 = 0.0, elast = 0.0, scale = 0.0;
+};
+
 // Per-query tables prepared on the host (query z-normalisation as
 // src/fsmeld.cpp:622-643, powers with the C library's pow as
 // src/find_t_lp.cpp:253 etc.).
@@ -219,6 +233,7 @@ struct QueryDev {
     const int* ordB_l;     // H1 pop order, lower side: q desc
     const int* ordA_u;     // H2 pop order, upper side: t_u asc, index asc
     const int* ordB_u;     // H1 pop order, upper side: q asc
+    BitTab bit;            // EDR, LCSS (E null: none)
 };
 
 }  // namespace fsm

@@ -116,6 +116,83 @@ static double fn_tl(double q, double C, int metric) {
     return q;
 }
 
+// doubles in ascending order as integers
+static long long order_int(double v) {
+    long long u;
+    memcpy(&u, &v, 8);
+    return u < 0 ? (long long)0x8000000000000000ull - u : u;
+}
+static double from_order_int(long long k) {
+    if (k < 0) k = (long long)0x8000000000000000ull - k;
+    double v;
+    memcpy(&v, &k, 8);
+    return v;
+}
+
+// the largest finite y with fl(|x - y|) <= eps; the test is true up to it
+// (rounding is monotone), so it is bracketed around x + eps and bisected
+static double match_end(double x, double eps) {
+    auto hit = [&](long long k) { return std::fabs(x - from_order_int(k)) <= eps; };
+    const long long kmax = order_int(DBL_MAX);
+    const double y0 = x + eps;
+    long long lo = order_int(x), hi = std::min(kmax, std::isfinite(y0) ? order_int(y0) + 2 : kmax);
+    for (long long step = 4; hi < kmax && hit(hi); step *= 2) {
+        lo = hi;
+        hi = hi > kmax - step ? kmax : hi + step;
+    }
+    if (hit(hi)) return DBL_MAX;
+    for (long long step = 4; hi - step > lo; step *= 2)
+        if (hit(hi - step)) { lo = hi - step; break; }
+    while (hi - lo > 1) {
+        const long long mid = lo + (hi - lo) / 2;
+        if (hit(mid)) lo = mid;
+        else hi = mid;
+    }
+    return from_order_int(lo);
+}
+
+// The matching intervals of the query's points (BitTab): point i matches the
+// candidate values y with A_i <= y < B_i.  The bucket of an end comes from the
+// operations of the device's lookup (bit_rank), so equal values fall in equal
+// buckets and the buckets ascend with the values.
+static void match_table(HostQuery* hq) {
+    const int m = hq->m, ne = 2 * m;
+    std::vector<std::pair<double, int>> ev(ne);
+    for (int i = 0; i < m; ++i) {
+        const double x = hq->qn[i];
+        ev[i] = {-match_end(-x, hq->arg), i};
+        ev[m + i] = {std::nextafter(match_end(x, hq->arg), INFINITY), m + i};
+    }
+    std::sort(ev.begin(), ev.end());
+    hq->bitE.resize(ne + 1);
+    hq->bitA.resize(m);
+    hq->bitB.resize(m);
+    for (int k = 0; k < ne; ++k) {
+        hq->bitE[k] = ev[k].first;
+        (ev[k].second < m ? hq->bitA[ev[k].second] : hq->bitB[ev[k].second - m]) = k;
+    }
+    hq->bitE[ne] = INFINITY;
+    double e0 = ev[0].first, el = e0;  // ev[0] is finite: an interval's lower end
+    for (int k = 0; k < ne; ++k)
+        if (std::isfinite(ev[k].first)) el = ev[k].first;
+    double scale = el > e0 ? kBitBuckets / (el - e0) : 0.0;
+    if (!std::isfinite(el - e0) || !std::isfinite(scale)) { el = e0; scale = 0.0; }
+    hq->bit_e0 = e0;
+    hq->bit_elast = el;
+    hq->bit_scale = scale;
+    hq->bitGrid.assign(kBitBuckets + 1, 0);
+    std::vector<int> cnt(kBitBuckets + 2, 0);
+    for (int k = 0; k < ne; ++k) {
+        const double y = ev[k].first, c = y < e0 ? e0 : (y > el ? el : y);
+        const double v = (c - e0) * scale + 6755399441055744.0;
+        long long u;
+        memcpy(&u, &v, 8);
+        ++cnt[(int)(u & 0xffffffff) + 1];
+    }
+    for (int b = 1; b <= kBitBuckets; ++b) cnt[b] += cnt[b - 1];
+    for (int b = 0; b <= kBitBuckets; ++b) hq->bitGrid[b] = (unsigned short)cnt[b];
+}
+
 int prepare_query(const double* q, int m, int metric, int w, double arg, HostQuery* hq, bool raw) {
     if (m < 2) return fail(FSMELD_E_ARG, "m must be at least 2.");
     if (w < 0 || w >= m) return fail(FSMELD_E_ARG, "w must satisfy 0 <= w < m.");
@@ -179,6 +256,7 @@ int prepare_query(const double* q, int m, int metric, int w, double arg, HostQue
     hq->ordB_l = order(qn, true);
     hq->ordA_u = order(hq->otu, false);
     hq->ordB_u = order(qn, false);
+    if ((metric == EDR || metric == LCSS) && m <= kBitMaxM && bit_words(w) > 0) match_table(hq);
     return FSMELD_OK;
 }
 
@@ -311,10 +389,10 @@ static int allow_smem(fsmeld_ctx* c, K kernel, size_t bytes) {
     return FSMELD_OK;
 }
 
-enum Stage { ST_STATS, ST_ENV, ST_THR, ST_LBIP, ST_GLB1, ST_GLB2, ST_DP, ST_SELECT, ST_FWD, ST_DPW, ST_GEMM, ST_N };
+enum Stage { ST_STATS, ST_ENV, ST_THR, ST_LBIP, ST_GLB1, ST_GLB2, ST_DP, ST_SELECT, ST_FWD, ST_DPW, ST_GEMM, ST_BIT, ST_N };
 static const char* kStageNames[ST_N] = {"k_mvmean", "k_envelope", "k_threshold", "k_lbip",
                                         "k_glb_tq", "k_glb_qt", "k_dp", "k_select",
-                                        "k_fwd_env", "k_dpw", "k_lbgemm"};
+                                        "k_fwd_env", "k_dpw", "k_lbgemm", "k_bitdp"};
 
 static cudaEvent_t prof_event(fsmeld_ctx* c) {
     if (!c->pool.empty()) { cudaEvent_t e = c->pool.back(); c->pool.pop_back(); return e; }
@@ -375,7 +453,11 @@ static int twiddle_table(fsmeld_ctx* c, int P, const double2** out) {
 static int upload_query(fsmeld_ctx* c, const HostQuery& hq, const std::string& slot, QueryDev* qd) {
     const int m = hq.m;
     const size_t nd = (size_t)m * (3 + 4 + 3 + 3 + 3 + 3), ni = (size_t)m * 4;
-    std::vector<unsigned char> host(nd * 8 + ni * 4);
+    // the matching table's inputs (EDR, LCSS) follow: ends, ranks, grid
+    const bool bits = !hq.bitE.empty();
+    const size_t bytes0 = nd * 8 + ni * 4;
+    const size_t nbit = bits ? hq.bitE.size() * 8 + 2 * (size_t)m * 4 + hq.bitGrid.size() * 2 : 0;
+    std::vector<unsigned char> host(bytes0 + nbit);
     double* d = (double*)host.data();
     size_t o = 0;
     auto put = [&](const std::vector<double>& v) { memcpy(d + o, v.data(), v.size() * 8); size_t at = o; o += v.size(); return at; };
@@ -387,10 +469,39 @@ static int upload_query(fsmeld_ctx* c, const HostQuery& hq, const std::string& s
     memcpy(ip + m, hq.ordB_l.data(), m * 4);
     memcpy(ip + 2 * m, hq.ordA_u.data(), m * 4);
     memcpy(ip + 3 * m, hq.ordB_u.data(), m * 4);
+    if (bits) {
+        unsigned char* b = host.data() + bytes0;
+        memcpy(b, hq.bitE.data(), hq.bitE.size() * 8);
+        b += hq.bitE.size() * 8;
+        memcpy(b, hq.bitA.data(), (size_t)m * 4);
+        memcpy(b + (size_t)m * 4, hq.bitB.data(), (size_t)m * 4);
+        memcpy(b + 2 * (size_t)m * 4, hq.bitGrid.data(), hq.bitGrid.size() * 2);
+    }
     void* dev;
     int r = buf(c, slot, host.size(), &dev);
     if (r) return r;
     FSM_CUDA_TRY(cudaMemcpyAsync(dev, host.data(), host.size(), cudaMemcpyHostToDevice, c->stream));
+    qd->bit = BitTab{};
+    if (bits) {
+        BitTab& bt = qd->bit;
+        const int nw = bit_words(hq.w);
+        bt.pad = (hq.w + 31) / 32;
+        bt.rs = (bt.pad + (m + 31) / 32 + nw + 1) | 1;  // odd: rows start on different banks
+        bt.e0 = hq.bit_e0;
+        bt.elast = hq.bit_elast;
+        bt.scale = hq.bit_scale;
+        const unsigned char* b = (const unsigned char*)dev + bytes0;
+        bt.E = (const double*)b;
+        const int* pa = (const int*)(b + hq.bitE.size() * 8);
+        bt.grid = (const unsigned short*)(pa + 2 * m);
+        unsigned* tab;
+        const size_t words = (size_t)(2 * m + 1) * bt.rs;
+        if ((r = bufT(c, "bit" + slot, words, &tab))) return r;
+        bt.table = tab;
+        const unsigned grid = (unsigned)std::min<size_t>((words + 255) / 256, (size_t)c->sm_count * 8);
+        k_bit_table<<<grid, 256, 0, c->stream>>>(pa, pa + m, m, bt.pad, bt.rs, tab);
+        LAUNCH_CHECK(c);
+    }
     FSM_CUDA_TRY(cudaStreamSynchronize(c->stream));  // host staging buffer is released on return
     const double* D = (const double*)dev;
     const int* I = (const int*)(D + nd);
@@ -582,9 +693,11 @@ static int run_lbip(fsmeld_ctx* c, const Geom& g, LbJob job) {
 // counters slot layout
 enum { C_SURV, C_G1, C_G2, C_OUT, C_VALID, C_SEED, C_SEEDOUT, C_DPNEXT, C_CELLS, C_N };
 
+static bool use_bitdp(const fsmeld_ctx* c, const QueryDev& q) { return q.bit.E && c->dp_form == 0 && !c->dp_exact; }
+
 static int run_glb(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const Stats& st, const long long* in,
                    unsigned long long* cnt, long long cap, long long* segc, long long** out_list,
-                   double** out_qt = nullptr, const double* cutoff_ptr = nullptr) {
+                   double** out_qt, double** out_tq, const double* cutoff_ptr = nullptr) {
     long long *g1, *g2;
     double *g1b, *g1t;
     int r;
@@ -619,6 +732,10 @@ static int run_glb(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const Stats
     if ((r = bufT(c, "g2t", (size_t)cap, &g2t))) return r;
     j2.in = g1; j2.in_b = g1b; j2.in_t = g1t; j2.n_in = cnt + C_G1;
     j2.out = g2; j2.out_b = nullptr; j2.out_t = g2t; j2.n_out = cnt + C_G2;
+    // the bit-vector DP bounds what is to come by the T->Q sums, the others by
+    // the Q->T sums
+    const bool bits = use_bitdp(c, qd);
+    if (bits) std::swap(j2.out_b, j2.out_t);
     const size_t sm2 = sizeof(double) * (((size_t)qd.m + 1) & ~(size_t)1);
     const void* qtf = qd.metric == DTW ? (const void*)k_glb_qt<DTW>
                     : qd.metric == ERP ? (const void*)k_glb_qt<ERP>
@@ -637,7 +754,8 @@ static int run_glb(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const Stats
         default: k_glb_qt<MSM><<<g2grid, 128, sm2, c->stream>>>(g, j2); break;
     }
     LAUNCH_CHECK(c);
-    if (out_qt) *out_qt = g2t;
+    *out_qt = bits ? nullptr : g2t;
+    *out_tq = bits ? g2t : nullptr;
     *out_list = g2;
     return FSMELD_OK;
 }
@@ -654,6 +772,33 @@ static int tuned(const fsmeld_ctx* c, int kind, int metric, int m_k, int v) {
     return 0;
 }
 
+// EDR and LCSS: the bit-vector DP.  The matching table goes to shared memory
+// while that leaves at least four blocks per SM, else it is read through the
+// caches.
+static int run_bitdp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
+    BitTab bt = job.q.bit;
+    const int m = job.q.m;
+    const void* kf = bitdp_kernel(job.q.metric, job.q.w);
+    const size_t tab = (size_t)(2 * m + 1) * bt.rs * 4;
+    size_t smem = bit_table_offset(m);
+    bt.in_smem = smem + tab <= 54 * 1024;
+    if (bt.in_smem) smem += tab;
+    int r;
+    if ((r = allow_smem(c, kf, smem))) return r;
+    int per_sm = 0;
+    FSM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kf, kBitThreads, smem));
+    const long long want = (expected + kBitThreads - 1) / kBitThreads;
+    const unsigned grid =
+        (unsigned)std::max<long long>(1, std::min<long long>(want, (long long)std::max(1, per_sm) * c->sm_count));
+    prof_begin(c, ST_BIT);
+    Geom ga = g;
+    void* args[] = {&ga, &job, &bt};
+    const cudaError_t le = cudaLaunchKernel(kf, dim3(grid), dim3(kBitThreads), args, smem, c->stream);
+    if (le != cudaSuccess) return cuda_fail(le, "k_bitdp launch", __FILE__, __LINE__);
+    LAUNCH_CHECK(c);
+    return FSMELD_OK;
+}
+
 static int run_dp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
     const int w = job.q.w;
     const int warps = kDpThreads / 32;
@@ -667,6 +812,7 @@ static int run_dp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
     job.gwork = nullptr;
     job.force_exact = c->dp_exact ? 1 : 0;
     unsigned grid;
+    if (use_bitdp(c, job.q)) return run_bitdp(c, g, job, expected);
     const bool gw_path = smem > (size_t)c->smem_optin - 4096;
     // wide bands (and FSMELD_DP_FORM=wave): one warp per candidate, band in registers
     int form = c->dp_form;
@@ -777,8 +923,8 @@ static int search_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     out.segments = g.forsize;
     out.tail = g.tsn % g.kml;
     long long* g2;
-    double* g2t;
-    if ((r = run_glb(c, g, qd, st, surv, cnt, cap, segc, &g2, &g2t))) return r;
+    double *g2t, *g2q;
+    if ((r = run_glb(c, g, qd, st, surv, cnt, cap, segc, &g2, &g2t, &g2q))) return r;
     long long* oi;
     double* od;
     if ((r = bufT(c, "outi", (size_t)cap, &oi))) return r;
@@ -786,7 +932,7 @@ static int search_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     DpJob dj{};
     dj.q = qd; dj.target = c->d_target; dj.MU = st.MU; dj.SIG = st.SIG;
     dj.lraw = st.Lraw; dj.uraw = st.Uraw;
-    dj.list = g2; dj.list_s = g2t; dj.n_list = cnt + C_G2; dj.list_cap = cap; dj.mode = 0; dj.cutoff = qr.cutoff;
+    dj.list = g2; dj.list_s = g2t; dj.list_t = g2q; dj.n_list = cnt + C_G2; dj.list_cap = cap; dj.mode = 0; dj.cutoff = qr.cutoff;
     dj.out_idx = oi; dj.out_dist = od; dj.n_out = cnt + C_OUT; dj.n_cells = cnt + C_CELLS; dj.out_cap = cap; dj.n_valid = nullptr;
     if ((r = run_dp(c, g, dj, (long long)c->sm_count * 16 * 128))) return r;
     FSM_CUDA_TRY(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
@@ -873,8 +1019,8 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     QueryDev qt = qd;
     qt.cutoff = DBL_MAX;  // the GLB kernels read tau from device memory
     long long* g2;
-    double* g2t;
-    if ((r = run_glb(c, g, qt, st, f1, cnt, cap, nullptr, &g2, &g2t, tau_dev))) return r;
+    double *g2t, *g2q;
+    if ((r = run_glb(c, g, qt, st, f1, cnt, cap, nullptr, &g2, &g2t, &g2q, tau_dev))) return r;
     long long* oi;
     double* od;
     if ((r = bufT(c, "outi", (size_t)cap, &oi))) return r;
@@ -882,7 +1028,7 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     DpJob dj{};
     dj.q = qt; dj.target = c->d_target; dj.MU = st.MU; dj.SIG = st.SIG;
     dj.lraw = st.Lraw; dj.uraw = st.Uraw;
-    dj.list = g2; dj.list_s = g2t; dj.n_list = cnt + C_G2; dj.list_cap = cap; dj.mode = 1; dj.cutoff = DBL_MAX;
+    dj.list = g2; dj.list_s = g2t; dj.list_t = g2q; dj.n_list = cnt + C_G2; dj.list_cap = cap; dj.mode = 1; dj.cutoff = DBL_MAX;
     dj.cutoff_ptr = tau_dev;
     dj.out_idx = oi; dj.out_dist = od; dj.n_out = cnt + C_OUT; dj.n_cells = cnt + C_CELLS; dj.out_cap = cap;
     if ((r = run_dp(c, g, dj, (long long)c->sm_count * 16 * 128))) return r;

@@ -14,6 +14,11 @@ struct HostQuery {
     double arg = 0.0;
     std::vector<double> qn, LQ, UQ, qs, pw, Dq, tlq, tuq, opw, oD, otl, otu;
     std::vector<int> ordA_l, ordB_l, ordA_u, ordB_u;
+    // EDR, LCSS: the ends of the matching intervals and their ranks (BitTab)
+    std::vector<double> bitE;
+    std::vector<unsigned short> bitGrid;
+    std::vector<int> bitA, bitB;
+    double bit_e0 = 0.0, bit_elast = 0.0, bit_scale = 0.0;
 };
 
 // raw: the query is used as given (no z-normalisation; raw mode)

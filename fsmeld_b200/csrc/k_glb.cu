@@ -337,6 +337,7 @@ __global__ void __launch_bounds__(128) k_glb_qt(Geom g, GlbJob job) {
             if (o < (unsigned long long)job.out_cap) {
                 job.out[o] = gi;
                 if (job.out_t) job.out_t[o] = (boundary == -1.0) ? -1.0 : qt;
+                if (job.out_b) job.out_b[o] = (boundary == -1.0) ? -1.0 : tq;
             }
             if (job.segc && s < g.forsize) atomicAdd((unsigned long long*)&job.segc[3 * s + 2], 1ull);
         }

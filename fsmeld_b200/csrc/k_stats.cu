@@ -27,6 +27,9 @@
 //     correctly rounded quotient, and a square root), written coalesced.
 // One block barrier per tile.  Short targets take fewer segments per block
 // (mvmean_segments), so that their windows' divisions spread over more SMs.
+// Measured against one warp that loads, chains and stages: m_k = 16384 2.39 ->
+// 0.33 ms, 2^20 points with m_k = 1024 0.162 -> 0.046 ms, 2^24 points with
+// m_k = 2048 (585 blocks) 0.320 -> 0.165 ms = 2.6 TB/s.
 //
 // Raw (non-normalised) mode (g.raw): a window is valid iff its points are all
 // finite, and its statistics are mean 0 and sigma 1, so every later stage

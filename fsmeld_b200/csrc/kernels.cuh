@@ -58,6 +58,7 @@ struct DpJob {
     const double* SIG;
     const long long* list;      // candidates, or null for windows [0, n_windows)
     const double* list_s;       // optional: GLB Q->T sum per candidate (cascading abandon)
+    const double* list_t;       // optional: GLB T->Q sum per candidate (k_bitdp)
     const unsigned long long* n_list;
     long long list_cap;
     long long n_windows;
@@ -157,6 +158,22 @@ const void* dpw_kernel(int metric, int w);
 // suffix sums of the abandon bound
 __host__ __device__ size_t dpw_warp_doubles(int m);
 size_t dpw_smem_bytes(int m, int warps);
+// EDR and LCSS as bit vectors: the query's matching table (BitTab in
+// common.cuh), one lane per candidate
+constexpr int kBitThreads = 256;
+constexpr int kBitMaxM = 2048;
+// row r of the table: the query points that match candidate points of rank r
+__global__ void k_bit_table(const int* __restrict__ pa, const int* __restrict__ pb, int m, int pad, int rs,
+                            unsigned* __restrict__ table);
+template <int METRIC, int NW>
+__global__ void k_bitdp(Geom g, DpJob job, BitTab bt);
+// the kernel for (metric, w), or null when the band is wider than 16 words
+const void* bitdp_kernel(int metric, int w);
+int bit_words(int w);
+// byte offset of the table in shared memory, after the ends and the grid
+__host__ __device__ inline size_t bit_table_offset(int m) {
+    return ((size_t)(2 * m + 1) * 8 + (kBitBuckets + 1) * 2 + 15) & ~size_t(15);
+}
 __global__ void k_lb_filter(Geom g, const double* __restrict__ z, const double* __restrict__ SIG,
                             const double* __restrict__ cutoff, int metric, long long* out,
                             unsigned long long* n_out, long long cap);

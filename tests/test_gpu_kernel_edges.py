@@ -32,3 +32,28 @@ def test_window_stats_tiles(api, oracle, n, m):  # noqa: F811
         omu, osg = oracle.mvmean(ts, m)
         assert bits_equal(mu[s], omu), s
         assert bits_equal(sg[s], osg), s
+
+
+# k_bitdp (EDR, LCSS): band widths around the word borders (2w+1 bits in 1..16
+# words), lengths not a multiple of the four points of a step, ties (integer
+# targets), tolerances that match nothing, little and everything
+@pytest.mark.parametrize("m,w", [(2, 0), (3, 2), (33, 15), (34, 16), (66, 31), (65, 32), (101, 47), (130, 64),
+                                 (299, 255)])
+@pytest.mark.parametrize("metric", ["edr", "lcss"])
+def test_bit_vector_distances(api, oracle, metric, m, w):  # noqa: F811
+    t = random_walk(3 * m + 200, [7, m])
+    t[m:2 * m] = np.round(t[m:2 * m])
+    q, _ = query_from(t, m, np.random.default_rng([8, m]))
+    with api.Engine(t) as e:
+        for arg in (0.0, 0.25, 1.7, 1e300):
+            gi, gd, gc = e.exact(q, m, 1e300, metric, w, arg)
+            oi, od, oc = oracle.exact(t, q, m, 1e300, metric, w, arg)
+            assert list(gi) == list(oi) and gc["valid"] == oc["valid"]
+            assert bits_equal(gd, od), arg
+            k = min(9, len(oi))
+            ci, cd, _ = e.cutoff(q, m, k, metric, w, arg)
+            xi, xd, _ = oracle.cutoff(t, q, m, k, metric, w, arg)
+            assert list(ci) == list(xi) and bits_equal(cd, xd), arg
+            si, sc = e.search(q, m, float(xd[-1]), metric, w, arg)
+            yi, yc = oracle.search(t, q, m, float(xd[-1]), metric, w, arg)
+            assert list(si) == list(yi) and sc["after_glb"] == yc["after_glb"], arg
