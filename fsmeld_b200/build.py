@@ -51,7 +51,7 @@ CUTLASS_INC = None
 NVFLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-static-global-template-stub=false",
                   "-Xcompiler", "-fPIC,-ffp-contract=off", f"-I{INCLUDE}"]
 
-CU = ["k_stats", "k_envelope", "k_threshold", "k_lbip", "k_glb", "k_dp", "k_dpw", "k_bitdp", "k_lbgemm", "k_select", "engine", "noalloc"]
+CU = ["k_stats", "k_envelope", "k_threshold", "k_lbip", "k_glb", "k_dp", "k_dpw", "k_bitdp", "k_screen", "k_lbgemm", "k_select", "engine", "noalloc"]
 
 
 def _newer(src_files, out):

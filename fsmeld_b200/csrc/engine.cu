@@ -389,10 +389,10 @@ static int allow_smem(fsmeld_ctx* c, K kernel, size_t bytes) {
     return FSMELD_OK;
 }
 
-enum Stage { ST_STATS, ST_ENV, ST_THR, ST_LBIP, ST_GLB1, ST_GLB2, ST_DP, ST_SELECT, ST_FWD, ST_DPW, ST_GEMM, ST_BIT, ST_N };
+enum Stage { ST_STATS, ST_ENV, ST_THR, ST_LBIP, ST_GLB1, ST_GLB2, ST_DP, ST_SELECT, ST_FWD, ST_DPW, ST_GEMM, ST_BIT, ST_SCREEN, ST_N };
 static const char* kStageNames[ST_N] = {"k_mvmean", "k_envelope", "k_threshold", "k_lbip",
                                         "k_glb_tq", "k_glb_qt", "k_dp", "k_select",
-                                        "k_fwd_env", "k_dpw", "k_lbgemm", "k_bitdp"};
+                                        "k_fwd_env", "k_dpw", "k_lbgemm", "k_bitdp", "k_screen"};
 
 static cudaEvent_t prof_event(fsmeld_ctx* c) {
     if (!c->pool.empty()) { cudaEvent_t e = c->pool.back(); c->pool.pop_back(); return e; }
@@ -691,7 +691,7 @@ static int run_lbip(fsmeld_ctx* c, const Geom& g, LbJob job) {
 }
 
 // counters slot layout
-enum { C_SURV, C_G1, C_G2, C_OUT, C_VALID, C_SEED, C_SEEDOUT, C_DPNEXT, C_CELLS, C_N };
+enum { C_SURV, C_G1, C_G2, C_OUT, C_VALID, C_SEED, C_SEEDOUT, C_DPNEXT, C_CELLS, C_SCREEN, C_N };
 
 static bool use_bitdp(const fsmeld_ctx* c, const QueryDev& q) { return q.bit.E && c->dp_form == 0 && !c->dp_exact; }
 
@@ -799,6 +799,42 @@ static int run_bitdp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected
     return FSMELD_OK;
 }
 
+// DTW, ERP, MSM: the FP32 screen, then `job` is the exact DP over what it left.
+// Bands from w = 2 (the kernel's row -2 lies inside the band) while a warp's
+// band and points take at most a third of an SM's shared memory; a cutoff no
+// bound can reach (every window is asked for) is not screened.
+static bool use_screen(const fsmeld_ctx* c, const DpJob& job) {
+    return job.screened && c->dp_form == 0 && !c->dp_exact && screen_kernel(job.q.metric) && job.q.w >= 2 &&
+           3 * screen_warp_bytes(job.q.w) <= (size_t)c->smem_optin && (job.cutoff_ptr || job.cutoff < 1e12) &&
+           dpw_kernel(job.q.metric, job.q.w);
+}
+
+static int run_screen(fsmeld_ctx* c, const Geom& g, DpJob* job) {
+    const void* kf = screen_kernel(job->q.metric);
+    const size_t per_warp = screen_warp_bytes(job->q.w);
+    const int warps = per_warp * 4 <= 64 * 1024 ? 4 : per_warp * 2 <= 96 * 1024 ? 2 : 1;
+    const size_t smem = per_warp * warps;
+    int r;
+    if ((r = allow_smem(c, kf, smem))) return r;
+    int per_sm = 0;
+    FSM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kf, warps * 32, smem));
+    const unsigned grid = (unsigned)(std::max(1, per_sm) * c->sm_count);
+    // the exact DP runs this many candidates in one wave of warps
+    long long few = 32LL * c->sm_count;
+    Geom ga = g;
+    void* args[] = {&ga, job, &job->screened, &job->n_screened, &few};
+    prof_begin(c, ST_SCREEN);
+    const cudaError_t le = cudaLaunchKernel(kf, dim3(grid), dim3(warps * 32), args, smem, c->stream);
+    if (le != cudaSuccess) return cuda_fail(le, "k_screen launch", __FILE__, __LINE__);
+    LAUNCH_CHECK(c);
+    job->list = job->screened;
+    job->n_list = job->n_screened;
+    job->list_s = nullptr;
+    job->n_valid = nullptr;
+    FSM_CUDA_TRY(cudaMemsetAsync(job->next, 0, sizeof(unsigned long long), c->stream));
+    return FSMELD_OK;
+}
+
 static int run_dp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
     const int w = job.q.w;
     const int warps = kDpThreads / 32;
@@ -813,10 +849,16 @@ static int run_dp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
     job.force_exact = c->dp_exact ? 1 : 0;
     unsigned grid;
     if (use_bitdp(c, job.q)) return run_bitdp(c, g, job, expected);
+    const bool screened = use_screen(c, job);
+    if (screened) {
+        if ((r = run_screen(c, g, &job))) return r;
+        expected = (long long)c->sm_count * 16 * 128;
+    }
     const bool gw_path = smem > (size_t)c->smem_optin - 4096;
     // wide bands (and FSMELD_DP_FORM=wave): one warp per candidate, band in registers
     int form = c->dp_form;
-    if (form == 0) form = tuned(c, job.list ? 0 : 3, job.q.metric, g.m_k, w);
+    if (screened) form = 2;  // few candidates: a warp each
+    else if (form == 0) form = tuned(c, job.list ? 0 : 3, job.q.metric, g.m_k, w);
     const void* wk = form == 1 ? nullptr : dpw_kernel(job.q.metric, w);
     const size_t wsm = dpw_smem_bytes(job.q.m, kDpwThreads / 32);
     if (wk && wsm + 1024 <= (size_t)c->smem_optin && (form == 2 || gw_path)) {
@@ -933,6 +975,7 @@ static int search_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     dj.q = qd; dj.target = c->d_target; dj.MU = st.MU; dj.SIG = st.SIG;
     dj.lraw = st.Lraw; dj.uraw = st.Uraw;
     dj.list = g2; dj.list_s = g2t; dj.list_t = g2q; dj.n_list = cnt + C_G2; dj.list_cap = cap; dj.mode = 0; dj.cutoff = qr.cutoff;
+    dj.screened = surv; dj.n_screened = cnt + C_SCREEN;  // the LB_IP survivors are done with
     dj.out_idx = oi; dj.out_dist = od; dj.n_out = cnt + C_OUT; dj.n_cells = cnt + C_CELLS; dj.out_cap = cap; dj.n_valid = nullptr;
     if ((r = run_dp(c, g, dj, (long long)c->sm_count * 16 * 128))) return r;
     FSM_CUDA_TRY(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
@@ -1030,6 +1073,7 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     dj.lraw = st.Lraw; dj.uraw = st.Uraw;
     dj.list = g2; dj.list_s = g2t; dj.list_t = g2q; dj.n_list = cnt + C_G2; dj.list_cap = cap; dj.mode = 1; dj.cutoff = DBL_MAX;
     dj.cutoff_ptr = tau_dev;
+    if (nslot >= qr.k) { dj.screened = f1; dj.n_screened = cnt + C_SCREEN; }  // fewer seeds than k: tau is no bound
     dj.out_idx = oi; dj.out_dist = od; dj.n_out = cnt + C_OUT; dj.n_cells = cnt + C_CELLS; dj.out_cap = cap;
     if ((r = run_dp(c, g, dj, (long long)c->sm_count * 16 * 128))) return r;
     FSM_CUDA_TRY(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
@@ -1084,7 +1128,9 @@ static int run_query(fsmeld_ctx* c, const QueryRun& qr, const Geom& g0, Stats& s
         qd.cutoff = qr.cutoff;
         DpJob dj{};
         dj.q = qd; dj.target = c->d_target; dj.MU = st.MU; dj.SIG = st.SIG;
-        dj.list = nullptr; dj.n_windows = g.tsn; dj.mode = 0; dj.cutoff = qr.cutoff;
+        dj.list = nullptr; dj.n_windows = g.tsn; dj.list_cap = cap; dj.mode = 0; dj.cutoff = qr.cutoff;
+        if ((r = bufT(c, "surv", (size_t)cap, &dj.screened))) return r;
+        dj.n_screened = cnt + C_SCREEN;
         dj.out_idx = oi; dj.out_dist = od; dj.n_out = cnt + C_OUT; dj.n_cells = cnt + C_CELLS; dj.out_cap = cap; dj.n_valid = cnt + C_VALID;
         if ((r = run_dp(c, g, dj, g.tsn))) return r;
         FSM_CUDA_TRY(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, c->stream));

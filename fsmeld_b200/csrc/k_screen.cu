@@ -1,0 +1,352 @@
+// FP32 screen before the exact FP64 DP (DTW, ERP, MSM): drops candidates whose
+// banded distance provably exceeds the cutoff and hands the others on.  No
+// result is computed here: every kept candidate is evaluated by the exact DP,
+// and a dropped one is one that the exact DP would discard.
+//
+// The proof per candidate.  x, y, g are rounded to FP32; a point difference
+// computed in FP32 is off by at most delta = 2^-22 (A + Y + |g|), A = max|x|,
+// Y the limit on |y| below (two roundings of the operands, one of the
+// difference; MSM's distance of a point to an interval is 1-Lipschitz in each
+// argument, which delta covers twice over).  Sums of non-negative terms and
+// minima of them carry a relative error of 2^-24 per operation, at most 4m + 4
+// on a path of at most 2m + 2 cells: the factor G.
+//   MSM: a path of true cost D costs at most (D + (2m+2) delta_c) G here
+//     (delta_c = delta + 2^-23 c).
+//   DTW, ERP: at most (sqrt(D) + delta sqrt(2m+2))^2 G (Cauchy-Schwarz over
+//     the path's differences); for D <= R <= s^2 that is at most
+//     (R + 2 e s + e^2) G with e = delta sqrt(2m+2).
+// So the computed minimum V over a row proves D > R when V > (R + E) G.  R is
+// the cutoff (squared for DTW, ERP; with the 1e-9 slack of the exact DP's
+// abandon test) less what the rows to come must still add: GLB's Q->T sum
+// less an upper bound of the terms of the rows done (FP32 on an envelope
+// narrowed by 2^-21 Y).  A candidate with a point beyond Y = 2A + 8 is kept.
+// Points outside the matrix are +-1e15: every path through them costs at least
+// about 1e15, and the screen is skipped unless (R + E) G < 1e12.
+//
+// One lane per candidate, the band row and the candidate points in shared
+// memory [slot][lane].  A warp takes 32 consecutive list entries and steps
+// them together, so every index is uniform and neighbours read neighbouring
+// points.  Two rows are computed per pass: cell d of the first and cell d-1 of
+// the second row lie in the same column, so a pass reads each band cell and
+// each point once and writes one cell for two computed, and two chains of
+// dependent operations interleave.
+//
+// What bounds it: instruction issue (DTW about 6, MSM 13 instructions per
+// cell; the exact DP spends 30 to 110 on FP64 selects and compares).
+#include "common.cuh"
+#include "kernels.cuh"
+
+namespace fsm {
+
+namespace {
+
+constexpr float kOut = 1e15f;    // candidate points outside the matrix
+constexpr float kBlock = 1e30f;  // band cells outside the band
+
+__device__ __forceinline__ float min3(float a, float b, float c) { return fminf(fminf(a, b), c); }
+
+struct Row {
+    float x, c0, s;  // ERP: c0 = (x-g)^2; MSM: c0 = |x-x'| + c, s = sign(x-x')
+};
+
+struct Col {
+    float y, gy, ady;  // ERP: gy = (y-g)^2; MSM: ady = |y-y'|
+    unsigned flip;     // MSM: sign bit that turns x-y into the side of the step
+};
+
+template <int METRIC>
+__device__ __forceinline__ Col make_col(float y, float yprev, float arg) {
+    Col c;
+    c.y = y;
+    c.gy = c.ady = 0.f;
+    c.flip = 0u;
+    if (METRIC == ERP) {
+        const float d = y - arg;
+        c.gy = d * d;
+    }
+    if (METRIC == MSM) {
+        const float dy = y - yprev;
+        c.ady = fabsf(dy);
+        c.flip = ~__float_as_uint(dy) & 0x80000000u;
+    }
+    return c;
+}
+
+// one cell from the cells above (up), diagonal and left
+template <int METRIC>
+__device__ __forceinline__ float cell(float up, float diag, float left, const Row& r, const Col& c, float arg) {
+    const float d = r.x - c.y;
+    if (METRIC == DTW) return fmaf(d, d, min3(up, diag, left));
+    if (METRIC == ERP) return min3(fmaf(d, d, diag), left + c.gy, up + r.c0);
+    // MSM: C(x, x', y) = c + the distance of x to [x', y], C(y, x, y') likewise
+    const float e2 = fmaxf(arg, fminf(r.c0, fmaf(r.s, d, arg)));
+    const float e3 = fmaxf(0.f, fminf(c.ady, __uint_as_float(__float_as_uint(d) ^ c.flip)));
+    return min3(up + e2, (left + arg) + e3, diag + fabsf(d));
+}
+
+}  // namespace
+
+size_t screen_warp_bytes(int w) { return (size_t)(2 * w + 2 + 2 * w + 2) * 32 * sizeof(float); }
+
+template <int METRIC>
+__global__ void __launch_bounds__(kScreenThreads) k_screen(Geom g, DpJob job, long long* __restrict__ out,
+                                                           unsigned long long* __restrict__ n_out, long long few) {
+    extern __shared__ __align__(16) float scr_smem[];
+    const QueryDev& q = job.q;
+    const int m = q.m, w = q.w, NR = 2 * w + 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr unsigned kAll = 0xffffffffu;
+    float* const A = scr_smem + (size_t)warp * 2 * NR * 32 + lane;  // band row A[d * 32], d in [0, 2w+1]
+    float* const Yr = A + NR * 32;                                  // points, slot p - (k0-w) + 1 (mod NR)
+    const double* __restrict__ X = q.qn;
+    const unsigned long long n_all = job.list ? *job.n_list : (unsigned long long)job.n_windows;
+    const unsigned long long n =
+        (job.list && n_all > (unsigned long long)job.list_cap) ? job.list_cap : n_all;
+    const double cut = job.cutoff_ptr ? *job.cutoff_ptr : job.cutoff;
+    const float arg = (float)q.arg;
+
+    double xm = 0.0;
+    for (int k = lane; k < m; k += 32) xm = fmax(xm, fabs(X[k]));
+    for (int o = 16; o; o >>= 1) xm = fmax(xm, __shfl_xor_sync(kAll, xm, o));
+    const double ymax = 2.0 * xm + 8.0;
+    const double cut_s = cut + 1e-9 * (1.0 + fabs(cut));
+    const double delta = 0x1p-22 * (xm + ymax + fabs(q.arg)) * 1.01;
+    const double G = 1.0 + (2.0 * m + 16.0) * 0x1p-23 * 1.01;
+    double R, Eb;
+    if (METRIC == MSM) {
+        R = cut_s;
+        Eb = (2.0 * m + 2.0) * (delta + 0x1p-23 * fabs(q.arg));
+    } else {
+        const double e = delta * sqrt(2.0 * m + 2.0);
+        R = cut_s * cut_s * (1.0 + 0x1p-50);
+        Eb = 2.0 * e * cut_s + e * e;
+    }
+    const double lim_all = (R + Eb) * G * (1.0 + 0x1p-20);
+    // nothing to gain (a short list: the exact DP runs it in one wave) or no
+    // proof possible: every valid candidate goes on
+    const bool pass = n <= (unsigned long long)few || !(lim_all < 1e12) || !(xm + ymax + fabs(q.arg) < 1e9);
+    const float ylim = (float)ymax, narrow = (float)(0x1p-21 * ymax);
+    const float grow = (float)(1.0 + (m + 16.0) * 0x1p-23);
+
+    unsigned long long valid_count = 0, cells = 0;
+    const int erp = METRIC == ERP ? 1 : 0;
+    // first row of the first pair: row 0 (ERP: -1, the empty prefix), one
+    // earlier when that makes the number of rows even
+    const int k0 = ((m + erp) & 1) ? -1 - erp : -erp;
+    for (;;) {
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(job.next, 32ull);
+        base = __shfl_sync(kAll, base, 0);
+        if (base >= n) break;
+        const unsigned long long item = base + lane;
+        bool active = item < n;
+        long long gi = 0;
+        double mu = 0.0, sg = 1.0, S = 0.0;
+        bool casc = false;
+        if (active) {
+            gi = job.list ? job.list[item] : (long long)item;
+            long long s;
+            int j;
+            g.locate(gi, &s, &j);
+            mu = job.MU[s * g.kml + j];
+            sg = job.SIG[s * g.kml + j];
+            active = !window_invalid(sg, g, gi);
+            if (active) ++valid_count;
+            if (active && job.list_s && job.lraw) {
+                S = job.list_s[item];
+                casc = S >= 0.0;
+            }
+        }
+        if (!active) gi = 0;
+        bool keep = active;
+        if (!pass && __any_sync(kAll, active)) {
+            const double inv = 1.0 / sg;
+            const double* __restrict__ tp = job.target + gi;
+            const double* __restrict__ lr = job.lraw + gi;
+            const double* __restrict__ ur = job.uraw + gi;
+            const bool warp_casc = __any_sync(kAll, casc);
+            // (R - S + Pre + E) G: the part known before the first row, rounded up
+            const float lim0 = (float)((R - (casc ? S : 0.0) + Eb) * G + 0x1p-20 * lim_all);
+            const float limg = (float)(G * (1.0 + 0x1p-22)) * grow;
+            bool over = false;
+            float pre = 0.f;
+            // ring: point k0 - w in slot 1, so a pair's columns d = 1, 2 start on an even slot
+            auto point = [&](int p, double raw) {
+                float y = p < 0 ? -kOut : kOut;
+                if (p >= 0 && p < m) {
+                    y = (float)((raw - mu) * inv);
+                    over = over || !(fabsf(y) <= ylim);
+                }
+                return y;
+            };
+            for (int d = 0; d < NR; ++d) A[d * 32] = kBlock;
+            // the cell that the first row grows from (see the rows above the matrix below)
+            A[(w + (erp ? -k0 : 0)) * 32] = 0.f;
+            for (int i = 0; i < NR; ++i) {
+                const int p = k0 - w + i;
+                const double raw = (active && p >= 0 && p < m) ? tp[p] : 0.0;
+                Yr[((i + 1) % NR) * 32] = point(p, raw);
+            }
+            int b = 1;  // slot of the pair's first column
+            // inputs of the next pair, loaded a pair ahead
+            double n0 = 0.0, n1 = 0.0, ea[4], eb[4];
+            auto load = [&](int k) {  // the last two points of the pair (k, k+1)
+                const int p = k + w;
+                n0 = (active && p >= 0 && p < m) ? tp[p] : 0.0;
+                n1 = (active && p + 1 >= 0 && p + 1 < m) ? tp[p + 1] : 0.0;
+            };
+            auto load_env = [&](int k) {  // its rows' forward windows
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int kk = k + u;
+                    const bool in = casc && active && kk >= 1 && kk <= m - 2;
+                    const int p0 = in ? qt_p0(kk, w) : 0, p1 = in ? qt_p1(kk, m, w) : 0;
+                    ea[2 * u] = in ? lr[p0] : 0.0;
+                    ea[2 * u + 1] = in ? lr[p1] : 0.0;
+                    eb[2 * u] = in ? ur[p0] : 0.0;
+                    eb[2 * u + 1] = in ? ur[p1] : 0.0;
+                }
+            };
+            float yl0 = -kOut;  // the point left of the pair's first column (MSM)
+            if (warp_casc) load_env(k0);
+            for (int k = k0; k < m; k += 2) {
+                // rows above the matrix: x = -1e15 matches the padding left of it
+                // at no cost and nothing else, so the zero travels down the
+                // diagonal (DTW, MSM) or straight down (ERP, whose row -1 then
+                // gathers the deletions of the prefix) to the first real row
+                Row r1, r2;
+                r1.x = k >= 0 ? (float)X[k] : -kOut;
+                r2.x = k + 1 >= 0 ? (float)X[k + 1] : -kOut;
+                if (METRIC == ERP) {
+                    r1.c0 = k >= 0 ? (r1.x - arg) * (r1.x - arg) : 0.f;
+                    r2.c0 = k + 1 >= 0 ? (r2.x - arg) * (r2.x - arg) : 0.f;
+                    r1.s = r2.s = 0.f;
+                } else if (METRIC == MSM) {
+                    const float xp = k >= 1 ? (float)X[k - 1] : -kOut;
+                    r1.c0 = fabsf(r1.x - xp) + arg;
+                    r1.s = r1.x >= xp ? 1.f : -1.f;
+                    r2.c0 = fabsf(r2.x - r1.x) + arg;
+                    r2.s = r2.x >= r1.x ? 1.f : -1.f;
+                } else {
+                    r1.c0 = r2.c0 = r1.s = r2.s = 0.f;
+                }
+                if (k + 2 < m) load(k + 2);
+                // terms of the pair's rows on the narrowed envelope
+                if (warp_casc) {
+                    float e2[2];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const double a = ea[2 * u] < ea[2 * u + 1] ? ea[2 * u] : ea[2 * u + 1];
+                        const double c = eb[2 * u] > eb[2 * u + 1] ? eb[2 * u] : eb[2 * u + 1];
+                        const float lo = (float)((a - mu) * inv) + narrow, up = (float)((c - mu) * inv) - narrow;
+                        const float x = u ? r2.x : r1.x;
+                        const float e = fmaxf(fmaxf(lo - x, x - up), 0.f);
+                        float t;
+                        if (METRIC == MSM) t = fminf(e, arg * (1.f + 0x1p-22f));
+                        else if (METRIC == ERP) t = fminf(e * e, (fabsf(x - arg) + narrow) * (fabsf(x - arg) + narrow));
+                        else t = e * e;
+                        e2[u] = (casc && k + u >= 1 && k + u <= m - 2) ? t : 0.f;
+                    }
+                    pre += e2[0];
+                    pre += e2[1];
+                    if (k + 2 < m) load_env(k + 2);
+                }
+                // the pair
+                float ext = kBlock, left2 = kBlock;
+                Col c = make_col<METRIC>(Yr[b * 32], yl0, arg);
+                float pd = A[0], pn = A[32];
+                float v1 = cell<METRIC>(pn, pd, kBlock, r1, c, arg);
+                float yp = c.y;
+                int slot = b + 1 == NR ? 0 : b + 1, d = 1;
+                // columns d = 1 .. 2w, two at a time (even slots: no wrap inside a two)
+                const int first = min(w, (NR - slot) >> 1);
+#pragma unroll 1
+                for (int part = 0; part < 2; ++part) {
+                    const int cnt = part ? w - first : first;
+                    const float* yptr = Yr + slot * 32;
+                    float* aptr = A + d * 32;
+#pragma unroll 2
+                    for (int t = 0; t < cnt; ++t) {
+                        const float ya = yptr[0], yb = yptr[32];
+                        const float pna = aptr[32], pnb = aptr[64];
+                        Col ca = make_col<METRIC>(ya, yp, arg);
+                        const float va = cell<METRIC>(pna, pn, v1, r1, ca, arg);
+                        left2 = cell<METRIC>(va, v1, left2, r2, ca, arg);
+                        aptr[-32] = left2;
+                        const float l1 = left2;
+                        Col cb = make_col<METRIC>(yb, ya, arg);
+                        v1 = cell<METRIC>(pnb, pna, va, r1, cb, arg);
+                        left2 = cell<METRIC>(v1, va, left2, r2, cb, arg);
+                        aptr[0] = left2;
+                        ext = min3(ext, l1, left2);
+                        pn = pnb;
+                        yp = yb;
+                        yptr += 64;
+                        aptr += 64;
+                    }
+                    slot = 0;
+                    d += 2 * cnt;
+                }
+                // column 2w+1: the second row's last cell only
+                {
+                    int ls = b + 2 * w + 1;
+                    if (ls >= NR) ls -= NR;
+                    c = make_col<METRIC>(Yr[ls * 32], yp, arg);
+                    left2 = cell<METRIC>(kBlock, v1, left2, r2, c, arg);
+                    A[2 * w * 32] = left2;
+                    ext = fminf(ext, left2);
+                }
+                cells += active ? (unsigned long long)(2 * w + 1) * 2 : 0ull;
+                // the next pair starts two columns on: the slots of this pair's
+                // first two columns take its last two points
+                if (METRIC == MSM) yl0 = Yr[(b + 1 == NR ? 0 : b + 1) * 32];
+                if (k + 2 < m) {
+                    const int p = k + 2 + w;
+                    Yr[b * 32] = point(p, n0);
+                    Yr[(b + 1 == NR ? 0 : b + 1) * 32] = point(p + 1, n1);
+                    b += 2;
+                    if (b >= NR) b -= NR;
+                }
+                if (over) {  // keep: the bound does not cover it
+                    active = false;
+                } else if (active && ext > fmaf(pre, limg, lim0)) {
+                    active = keep = false;
+                }
+                if (!__any_sync(kAll, active)) break;
+            }
+            // the last row's cell (m-1, m-1)
+            if (active && A[w * 32] > (float)lim_all) keep = false;
+        }
+        const unsigned mask = __ballot_sync(kAll, keep);
+        if (mask) {
+            unsigned long long o = 0;
+            if (lane == 0) o = atomicAdd(n_out, (unsigned long long)__popc(mask));
+            o = __shfl_sync(kAll, o, 0) + __popc(mask & ((1u << lane) - 1));
+            if (keep) out[o] = gi;
+        }
+        __syncwarp();
+    }
+    for (int o = 16; o; o >>= 1) {
+        valid_count += __shfl_xor_sync(kAll, valid_count, o);
+        cells += __shfl_xor_sync(kAll, cells, o);
+    }
+    if (lane == 0) {
+        if (job.n_valid && valid_count) atomicAdd(job.n_valid, valid_count);
+        if (job.n_cells && cells) atomicAdd(job.n_cells, cells);
+    }
+}
+
+template __global__ void k_screen<DTW>(Geom, DpJob, long long*, unsigned long long*, long long);
+template __global__ void k_screen<ERP>(Geom, DpJob, long long*, unsigned long long*, long long);
+template __global__ void k_screen<MSM>(Geom, DpJob, long long*, unsigned long long*, long long);
+
+const void* screen_kernel(int metric) {
+    switch (metric) {
+        case DTW: return (const void*)k_screen<DTW>;
+        case ERP: return (const void*)k_screen<ERP>;
+        case MSM: return (const void*)k_screen<MSM>;
+        default: return nullptr;
+    }
+}
+
+}  // namespace fsm

@@ -74,6 +74,8 @@ struct DpJob {
     int force_exact;            // every candidate in the DP's exact boundary mode
     unsigned long long* n_cells;  // band cells computed (optional)
     const double* cutoff_ptr;   // when set: the cutoff in device memory (read at kernel start)
+    long long* screened;        // when set: room for the candidates an FP32 screen leaves
+    unsigned long long* n_screened;
 };
 
 // LB_IP of a group of queries of equal (m, w) with shared thresholds as one
@@ -174,6 +176,14 @@ int bit_words(int w);
 __host__ __device__ inline size_t bit_table_offset(int m) {
     return ((size_t)(2 * m + 1) * 8 + (kBitBuckets + 1) * 2 + 15) & ~size_t(15);
 }
+// FP32 screen before the exact DP (DTW, ERP, MSM): the candidates it cannot
+// drop, to out; lists of at most `few` entries go on whole
+constexpr int kScreenThreads = 128;
+template <int METRIC>
+__global__ void k_screen(Geom g, DpJob job, long long* __restrict__ out, unsigned long long* __restrict__ n_out,
+                         long long few);
+const void* screen_kernel(int metric);
+size_t screen_warp_bytes(int w);
 __global__ void k_lb_filter(Geom g, const double* __restrict__ z, const double* __restrict__ SIG,
                             const double* __restrict__ cutoff, int metric, long long* out,
                             unsigned long long* n_out, long long cap);

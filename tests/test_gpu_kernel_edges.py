@@ -57,3 +57,37 @@ def test_bit_vector_distances(api, oracle, metric, m, w):  # noqa: F811
             si, sc = e.search(q, m, float(xd[-1]), metric, w, arg)
             yi, yc = oracle.search(t, q, m, float(xd[-1]), metric, w, arg)
             assert list(si) == list(yi) and sc["after_glb"] == yc["after_glb"], arg
+
+
+# k_screen (DTW, ERP, MSM): odd and even row counts, narrow and wide bands (one,
+# two and four warps a block), cutoffs equal to a distance, between two, below
+# all; lists long enough to be screened (over 32 per SM); raw mode with large
+# values; points beyond the bound's limit.  Every decision is the oracle's.
+@pytest.mark.parametrize("m,w,raw", [(3, 2, False), (16, 2, False), (17, 3, False), (40, 39, False), (63, 15, False),
+                                     (64, 16, True), (90, 70, False), (150, 140, False)])
+@pytest.mark.parametrize("metric,arg", [("dtw", 0.0), ("erp", 0.0), ("erp", 0.4), ("msm", 0.5)])
+def test_screened_distances(api, oracle, metric, arg, m, w, raw):  # noqa: F811
+    n = 6000 + m
+    t = random_walk(n, [9, m])
+    t[2000:2010] += 500.0  # spikes: normalised points near sqrt(m)
+    t[4000] = np.nan
+    if raw:
+        t = t * 50.0 + 1e4
+    q, _ = query_from(t, m, np.random.default_rng([10, m]))
+    try:
+        oracle.set_normalization("raw" if raw else "zscore")
+        with api.Engine(t) as e:
+            e.set_normalization("raw" if raw else "zscore")
+            oi, od, oc = oracle.exact(t, q, m, 1e300, metric, w, arg)
+            ranked = np.sort(od)
+            for cut in (ranked[0], ranked[20], 0.5 * (ranked[50] + ranked[51]), ranked[len(ranked) // 2],
+                        ranked[-1], 0.5 * ranked[0]):
+                keep = od <= cut
+                gi, gd, gc = e.exact(q, m, float(cut), metric, w, arg)
+                assert list(gi) == list(oi[keep]) and gc["valid"] == oc["valid"], cut
+                assert bits_equal(gd, od[keep]), cut
+                si, sc = e.search(q, m, float(cut), metric, w, arg)
+                yi, yc = oracle.search(t, q, m, float(cut), metric, w, arg)
+                assert list(si) == list(yi) and sc["after_glb"] == yc["after_glb"], cut
+    finally:
+        oracle.set_normalization("zscore")
