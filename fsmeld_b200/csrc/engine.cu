@@ -305,6 +305,8 @@ struct fsmeld_ctx {
     // normalisation mode (the reference's set_normalization_mode, include/funcs.h:20-28):
     // false z-score (the reference CLI's only mode), true raw
     bool raw = false;
+    // workspace is short: envelopes without the buffers a query can do without
+    bool lean = false;
     double last_ms = 0.0;
     std::string err;
     struct Buf { void* p = nullptr; size_t bytes = 0; };
@@ -371,6 +373,25 @@ static int buf(fsmeld_ctx* c, const std::string& name, size_t bytes, void** out)
     }
     *out = b.p;
     return FSMELD_OK;
+}
+
+// a buffer the caller can do without: false (and no error) when it does not fit
+static bool buf_optional(fsmeld_ctx* c, const std::string& name, size_t bytes, double** out) {
+    void* p = nullptr;
+    if (buf(c, name, bytes, &p) == FSMELD_OK) { *out = (double*)p; return true; }
+    cudaGetLastError();
+    g_last_error.clear();
+    return false;
+}
+
+// frees one buffer after the stream's work is done
+static void release_buf(fsmeld_ctx* c, const std::string& name) {
+    cudaStreamSynchronize(c->stream);
+    std::lock_guard<std::mutex> lk(ws_root(c)->ws_mu);
+    auto it = c->bufs.find(name);
+    if (it == c->bufs.end()) return;
+    if (it->second.p) cudaFree(it->second.p);
+    c->bufs.erase(it);
 }
 
 template <typename T>
@@ -523,6 +544,8 @@ struct Stats {
     double* Ln = nullptr;
     double* Lraw = nullptr;  // forward windows min / max(t[p .. p+w]) of the raw target
     double* Uraw = nullptr;
+    double* Clo = nullptr;   // centred windows (GLB's Q->T terms); null when the workspace has no room for them
+    double* Cup = nullptr;
 };
 
 static int run_stats(fsmeld_ctx* c, const Geom& g, Stats* st, const std::string& tag) {
@@ -578,15 +601,21 @@ static int run_env(fsmeld_ctx* c, const Geom& g, int w, Stats* st, const std::st
     if ((r = bufT(c, "ln" + tag, (size_t)g.S * g.m_k, &st->Ln))) return r;
     if ((r = bufT(c, "lraw" + tag, (size_t)g.n, &st->Lraw))) return r;
     if ((r = bufT(c, "uraw" + tag, (size_t)g.n, &st->Uraw))) return r;
+    st->Clo = st->Cup = nullptr;
+    if (!c->lean) {
+        if (buf_optional(c, "clo" + tag, sizeof(double) * (size_t)g.n, &st->Clo) &&
+            !buf_optional(c, "cup" + tag, sizeof(double) * (size_t)g.n, &st->Cup))
+            st->Clo = nullptr;
+    }
     {
-        const size_t fsm = fwd_env_smem_bytes(w);
+        const size_t fsm = fwd_env_smem_bytes(w, st->Clo != nullptr);
         if ((r = allow_smem(c, k_fwd_env, fsm))) return r;
         int per_sm = 0;
         FSM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fwd_env, kFwdThreads, fsm));
         const unsigned fgrid = (unsigned)std::max<long long>(
             1, std::min<long long>((g.n + kFwdTile - 1) / kFwdTile, (long long)std::max(1, per_sm) * c->sm_count));
         prof_begin(c, ST_FWD);
-        k_fwd_env<<<fgrid, kFwdThreads, fsm, c->stream>>>(c->d_target, g.n, w, st->Lraw, st->Uraw);
+        k_fwd_env<<<fgrid, kFwdThreads, fsm, c->stream>>>(c->d_target, g.n, w, st->Lraw, st->Uraw, st->Clo, st->Cup);
         LAUNCH_CHECK(c);
     }
     const int mk = g.m_k;
@@ -707,12 +736,12 @@ static int run_glb(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const Stats
     if ((r = bufT(c, "g2", (size_t)cap, &g2))) return r;
     GlbJob j1{};
     j1.q = qd; j1.target = c->d_target; j1.MU = st.MU; j1.SIG = st.SIG;
-    j1.lraw = st.Lraw; j1.uraw = st.Uraw;
+    j1.lraw = st.Lraw; j1.uraw = st.Uraw; j1.clo = st.Clo; j1.cup = st.Cup;
     j1.in = in; j1.n_in = cnt + C_SURV; j1.in_cap = cap;
     j1.out = g1; j1.out_b = g1b; j1.out_t = g1t; j1.n_out = cnt + C_G1; j1.out_cap = cap;
     j1.segc = segc;
     j1.cutoff_ptr = cutoff_ptr;
-    const size_t sm1 = sizeof(double) * 3 * qd.m;
+    const size_t sm1 = sizeof(float2) * 2 * qd.m;
     const void* tqf = qd.metric == DTW ? (const void*)k_glb_tq<DTW>
                     : qd.metric == ERP ? (const void*)k_glb_tq<ERP>
                     : qd.metric == EDR ? (const void*)k_glb_tq<EDR>
@@ -736,22 +765,22 @@ static int run_glb(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const Stats
     // the Q->T sums
     const bool bits = use_bitdp(c, qd);
     if (bits) std::swap(j2.out_b, j2.out_t);
-    const size_t sm2 = sizeof(double) * (((size_t)qd.m + 1) & ~(size_t)1);
+    const size_t sm2 = sizeof(float2) * qd.m;
     const void* qtf = qd.metric == DTW ? (const void*)k_glb_qt<DTW>
                     : qd.metric == ERP ? (const void*)k_glb_qt<ERP>
                     : qd.metric == EDR ? (const void*)k_glb_qt<EDR>
                     : qd.metric == LCSS ? (const void*)k_glb_qt<LCSS> : (const void*)k_glb_qt<MSM>;
     if ((r = allow_smem(c, qtf, sm2))) return r;
     int per_sm = 0;
-    FSM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, qtf, 128, sm2));
+    FSM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, qtf, 256, sm2));
     const unsigned g2grid = (unsigned)(std::max(1, per_sm) * c->sm_count);
     prof_begin(c, ST_GLB2);
     switch (qd.metric) {
-        case DTW: k_glb_qt<DTW><<<g2grid, 128, sm2, c->stream>>>(g, j2); break;
-        case ERP: k_glb_qt<ERP><<<g2grid, 128, sm2, c->stream>>>(g, j2); break;
-        case EDR: k_glb_qt<EDR><<<g2grid, 128, sm2, c->stream>>>(g, j2); break;
-        case LCSS: k_glb_qt<LCSS><<<g2grid, 128, sm2, c->stream>>>(g, j2); break;
-        default: k_glb_qt<MSM><<<g2grid, 128, sm2, c->stream>>>(g, j2); break;
+        case DTW: k_glb_qt<DTW><<<g2grid, 256, sm2, c->stream>>>(g, j2); break;
+        case ERP: k_glb_qt<ERP><<<g2grid, 256, sm2, c->stream>>>(g, j2); break;
+        case EDR: k_glb_qt<EDR><<<g2grid, 256, sm2, c->stream>>>(g, j2); break;
+        case LCSS: k_glb_qt<LCSS><<<g2grid, 256, sm2, c->stream>>>(g, j2); break;
+        default: k_glb_qt<MSM><<<g2grid, 256, sm2, c->stream>>>(g, j2); break;
     }
     LAUNCH_CHECK(c);
     *out_qt = bits ? nullptr : g2t;
@@ -1646,6 +1675,7 @@ static int run_tasks_parallel(fsmeld_ctx* c, std::vector<QueryRun>& runs, const 
         // context itself holds is needed here either
         release_bufs(c);
         for (fsmeld_ctx* w : c->workers) release_bufs(w);
+        ws[0]->lean = true;
         for (size_t ti = 0; ti < tasks.size() && !cuda_dead.load(); ++ti) {
             bool any = false;
             for (size_t k = tasks[ti].first; k < tasks[ti].second; ++k)
@@ -1654,6 +1684,7 @@ static int run_tasks_parallel(fsmeld_ctx* c, std::vector<QueryRun>& runs, const 
             errs[0].clear();
             run_task(ws[0], ti, true, errs[0]);
         }
+        ws[0]->lean = false;
         absorb_worker(c, ws[0]);
     }
     int first_err = FSMELD_OK;
@@ -1661,6 +1692,14 @@ static int run_tasks_parallel(fsmeld_ctx* c, std::vector<QueryRun>& runs, const 
     if (first_err)
         for (auto& e : errs) if (!e.empty()) { g_last_error = e; break; }
     return first_err;
+}
+
+// gives the centred windows back (GLB then reads two forward windows per point)
+static void drop_centred(fsmeld_ctx* c, Stats& st) {
+    if (!st.Clo) return;
+    st.Clo = st.Cup = nullptr;
+    release_buf(c, "clo");
+    release_buf(c, "cup");
 }
 
 // One call over many queries: statistics per distinct m, envelopes per distinct
@@ -1724,6 +1763,15 @@ int run_batch(fsmeld_ctx* c, std::vector<QueryRun>& runs, std::vector<int>* stat
         // searches through the tensor-core LB_IP (when selected), then the rest
         std::vector<char> done(oj, 0);
         if ((r = group_gemm(c, g, st, runs, order, oi, oj, status, &done, true)) == FSMELD_E_CUDA) return r;
+        // a grouped query refused for workspace runs again by itself, without
+        // the centred windows
+        for (size_t k = oi; k < oj; ++k)
+            if (done[k] && (*status)[order[k]] == FSMELD_E_NOMEM && st.Clo) done[k] = 2;
+        if (std::count(done.begin(), done.end(), 2)) {
+            for (fsmeld_ctx* w : c->workers) release_bufs(w);
+            drop_centred(c, st);
+            for (char& d : done) if (d == 2) d = 0;
+        }
         std::vector<size_t> rest;
         for (size_t k = oi; k < oj; ++k)
             if (!done[k]) rest.push_back(order[k]);
@@ -1738,6 +1786,10 @@ int run_batch(fsmeld_ctx* c, std::vector<QueryRun>& runs, std::vector<int>* stat
                     // the buffers an earlier batch's workers kept may be what is
                     // missing: release them and run the query again
                     for (fsmeld_ctx* w : c->workers) release_bufs(w);
+                    q = run_query(c, runs[k], g, st, have_env);
+                }
+                if (q == FSMELD_E_NOMEM && st.Clo) {
+                    drop_centred(c, st);
                     q = run_query(c, runs[k], g, st, have_env);
                 }
                 (*status)[k] = q;
@@ -1781,6 +1833,7 @@ int run_batch(fsmeld_ctx* c, std::vector<QueryRun>& runs, std::vector<int>* stat
             }
             if (nomem && !dead) {
                 for (fsmeld_ctx* w : c->workers) release_bufs(w);
+                drop_centred(c, st);
                 for (size_t k : rest) {
                     if ((*status)[k] != FSMELD_E_NOMEM) continue;
                     const int q = run_query(c, runs[k], g, st, have_env);

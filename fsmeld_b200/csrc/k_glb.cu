@@ -1,20 +1,48 @@
 // GLB second filter (src/glb.cpp:200-373), split in the reference's own two
 // directions:
-//  * k_glb_tq: one lane per LB_IP survivor computes the boundary term and the
-//    T->Q sum with early abandon, z-normalising candidate points lazily
-//    (t - mu) / sigma exactly as src/fsmeld.cpp:823-826 does (one correctly
-//    rounded division, taken from the window's reciprocal by FMA corrections),
-//    so abandoned candidates never pay for the whole window;
-//  * k_glb_qt: one lane per T->Q survivor adds the Q->T terms in the
-//    reference's order.  The candidate envelope (lower_upper_lemire of the
-//    z-normalised window, src/glb.cpp:302-304) is never materialised:
-//    z-normalisation x -> (x - mu) / sigma is monotone even after rounding,
-//    so the minimum of the normalised points equals the normalised minimum of
-//    the raw points, bit for bit; every envelope point, edge or interior, is
-//    the min/max of two forward windows of the target (k_fwd_env).
-// Early abandon compares a running sum of non-negative terms with the
-// cutoff; running sums never decrease, so testing the final sum once is the
-// same decision as testing after every term.
+//  * k_glb_tq: one lane per LB_IP survivor, the boundary term and the T->Q sum
+//    (candidate points against the query's envelope);
+//  * k_glb_qt: one lane per T->Q survivor, the Q->T sum (query points against
+//    the candidate's envelope).  The candidate envelope (lower_upper_lemire of
+//    the z-normalised window, src/glb.cpp:302-304) is never materialised:
+//    z-normalisation x -> (x - mu) / sigma is monotone even after rounding, so
+//    the minimum of the normalised points equals the normalised minimum of the
+//    raw points, bit for bit; every envelope point is the min/max of two
+//    forward windows of the target, an interior one (w <= k <= m-1-w) a value
+//    of the centred windows (k_fwd_env).
+// What GLB decides is whether boundary + T->Q and boundary + Q->T stay within
+// the cutoff (LCSS: whether both counts reach it): running sums never decrease
+// and rounding is monotone, so glb <= cutoff exactly when both hold, and when
+// a sum is abandoned makes no difference.
+//
+// So the sums are taken in fixed point and single precision with a proven
+// margin, and only a candidate whose sum falls within the margin of the limit
+// is decided by the reference's FP64 operations (exact_tq, exact_qt).
+//   * One FP64 fused multiply-add turns a raw point into a fixed-point number
+//     and an FP32 one at once: v = fl(t A + B), A = 2^K / sigma, B = M - mu A,
+//     with M = 1.5 2^52 + 0x4b400000.  The low word of v is then the bit
+//     pattern of the float F = 1.5 2^23 + n, n the integer next to y 2^K, off
+//     the reference's normalised point by at most 1.01 units of 2^-K (0.5 from
+//     B, 0.5 from v).  No conversion instruction (14 a cycle and SM against 64
+//     for the multiply-add).  K is the largest with |y| 2^K < 2^22 for
+//     |y| <= sqrt(m) (raw mode: four times the query's half range around its
+//     middle, which M then carries); a point outside shows in the upper bits,
+//     and its candidate is decided in FP64.
+//   * Differences of such floats are exact integers; with the query's side
+//     rounded to units too, each is off by less than 2 units (ERP with a gap
+//     far outside: by its FP32 rounding more).
+//   * DTW, ERP: the sum of squares is the squared norm of the differences
+//     (boundary terms among them), so its root is off by at most 2 sqrt(m+2)
+//     units (triangle inequality); MSM: the sum by 2 (m+4) units (its boundary
+//     is continuous in its arguments); the FP32 sums by a relative (m+16) 2^-23.
+//   * EDR, LCSS: terms are 0 or 1; those within 2 units of the tolerance count
+//     as 0 in one total and as 1 in the other.
+// What bounds it: instruction issue, about 14 instructions a point (T->Q) and
+// 18 (Q->T, with two unaligned 8-byte loads that keep the L1 path 84% busy)
+// where the FP64 sums took 45 and 90 issue slots.  Measured on the five-metric
+// workload (2^24 points, m = 256, w = 13), T->Q and Q->T of all five queries:
+// 19.3 and 14.6 ms with FP64 sums, 9.3 and 7.4 ms here; 8 top-k queries (m =
+// 512, 2^23 points) 18.6 and 7.6 ms -> 9.6 and 5.0 ms.
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -62,8 +90,6 @@ __device__ __forceinline__ void zdiv_group(F dividend, double sg, double inv, bo
     }
 }
 
-}  // namespace
-
 // T->Q term of normalised candidate point t against the query envelope
 // [lo, hi] at the same index (src/glb.cpp:230-300), written with selects so
 // lanes never split on the data.  lo <= hi, so at most one of t < lo, t > hi
@@ -90,20 +116,312 @@ __device__ __forceinline__ double tq_term(double t, double lo, double hi, double
     }
 }
 
+// boundary term and T->Q sum in the reference's operations; false: abandoned
+template <int METRIC>
+__device__ __noinline__ bool exact_tq(const double* __restrict__ Q, const double* __restrict__ LQ,
+                                      const double* __restrict__ UQ, int m, double arg,
+                                      const double* __restrict__ tp, double mu, double sg, double bsf,
+                                      double& boundary_out, double& tq_out) {
+    double boundary, tq;
+    const double inv = __drcp_rn(sg);
+    const bool rok = rcp_div_in_range(sg);
+    const double lim = (METRIC == DTW || METRIC == ERP) ? dmul(bsf, bsf) : bsf;  // src/glb.cpp:28-31
+    bool alive = true;
+    boundary = tq = 0.0;
+#define TN(k) zdiv_i(dsub(tp[(k)], mu), sg, inv, rok)
+    const double T0 = TN(0), TL = TN(m - 1);
+    if (METRIC == DTW) {
+        boundary = dadd(dsq(T0, Q[0]), dsq(TL, Q[m - 1]));
+    } else if (METRIC == ERP) {
+        boundary = dmin3(dsq(Q[m - 1], TL), dsq(Q[m - 1], arg), dsq(TL, arg));
+    } else if (METRIC == EDR) {
+        boundary = dminv(edr_sub(Q[m - 1], TL, arg), 1.0);
+    } else if (METRIC == MSM) {
+        const double T2 = TN(m - 2);
+        const double q0 = Q[0], ql = Q[m - 1], ql2 = Q[m - 2];
+        if ((T2 >= TL && TL >= ql) || (T2 <= TL && TL <= ql) || (ql2 <= ql && ql <= TL) ||
+            (ql2 >= ql && ql >= TL)) {
+            boundary = dadd(fabs(dsub(q0, T0)), dminv(fabs(dsub(ql, TL)), arg));
+        } else {
+            boundary = dadd(fabs(dsub(q0, T0)),
+                            dmin3(fabs(dsub(ql, TL)), dadd(arg, fabs(dsub(TL, T2))),
+                                  dadd(arg, fabs(dsub(ql, ql2)))));
+        }
+    }
+    if (METRIC == LCSS) {
+        // every point, no abandon (src/glb.cpp:238-252)
+        const double min_len = (double)m;
+        int k = 0;
+        for (; k + 4 <= m; k += 4) {
+            double z4[4], t4[4];
+            zdiv_group([&](int u) { return dsub(tp[k + u], mu); }, sg, inv, rok, z4);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) t4[u] = tq_term<LCSS>(z4[u], LQ[k + u], UQ[k + u], arg);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) tq = dadd(tq, t4[u]);
+        }
+        for (; k < m; ++k) tq = dadd(tq, tq_term<LCSS>(TN(k), LQ[k], UQ[k], arg));
+        if (dmax0(dsub(1.0, ddiv(tq, min_len))) > bsf) alive = false;
+    } else {
+        // points 1..m-2 four at a time: the four normalisations are
+        // independent, the sum takes them in the reference's order, and
+        // the abandon test runs once per group -- the sum never
+        // decreases, so a sum past the limit anywhere in the group is
+        // past it at the group's end (the same decision)
+        int k = 1;
+        for (; k + 4 <= m - 1; k += 4) {
+            double z4[4], t4[4];
+            zdiv_group([&](int u) { return dsub(tp[k + u], mu); }, sg, inv, rok, z4);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) t4[u] = tq_term<METRIC>(z4[u], LQ[k + u], UQ[k + u], arg);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) tq = dadd(tq, t4[u]);
+            if (dadd(boundary, tq) > lim) { alive = false; break; }
+        }
+        if (alive) {
+            for (; k < m - 1; ++k) tq = dadd(tq, tq_term<METRIC>(TN(k), LQ[k], UQ[k], arg));
+            if (dadd(boundary, tq) > lim) alive = false;
+        }
+    }
+#undef TN
+    boundary_out = boundary;
+    tq_out = tq;
+    return alive;
+}
+
+// the Q->T sum in the reference's operations and order
+template <int METRIC>
+__device__ __noinline__ double exact_qt(const double* __restrict__ Q, int m, int w, double arg,
+                                        const double* __restrict__ lf, const double* __restrict__ uf, double mu,
+                                        double sg) {
+    const double inv = __drcp_rn(sg);
+    const bool rok = rcp_div_in_range(sg);
+    double qt = 0.0;
+    const int k0 = (METRIC == LCSS) ? 0 : 1, k1 = (METRIC == LCSS) ? m - 1 : m - 2;
+    // the terms are independent (unrolled so their loads and divisions
+    // overlap); only the sum is sequential, in the reference's order.
+    // Interior points (w <= k <= m-1-w) read the windows at k-w and k
+    // directly; the edges take the clamped indices.
+    const int i0 = max(k0, w), i1 = min(k1, m - 1 - w);
+    int k = k0;
+    for (; k <= k1 && k < i0; ++k) qt = dadd(qt, qt_term(METRIC, Q[k], k, m, w, lf, uf, mu, sg, inv, rok, arg));
+    for (; k + 1 <= i1; k += 2) {  // two points, four quotients, one range test
+        double z4[4];
+        zdiv_group(
+            [&](int u) {
+                const int kk = k + (u & 1);
+                if (u < 2) { const double a0 = lf[kk - w], a1 = lf[kk]; return dsub((a1 < a0) ? a1 : a0, mu); }
+                const double b0 = uf[kk - w], b1 = uf[kk];
+                return dsub((b0 < b1) ? b1 : b0, mu);
+            },
+            sg, inv, rok, z4);
+        qt = dadd(qt, qt_term_norm(METRIC, Q[k], z4[0], z4[2], arg));
+        qt = dadd(qt, qt_term_norm(METRIC, Q[k + 1], z4[1], z4[3], arg));
+    }
+    for (; k <= i1; ++k) {
+        const double a0 = lf[k - w], a1 = lf[k], b0 = uf[k - w], b1 = uf[k];
+        qt = dadd(qt, qt_term_env(METRIC, Q[k], (a1 < a0) ? a1 : a0, (b0 < b1) ? b1 : b0, mu, sg, inv, rok,
+                                  arg));
+    }
+    for (; k <= k1; ++k) qt = dadd(qt, qt_term(METRIC, Q[k], k, m, w, lf, uf, mu, sg, inv, rok, arg));
+    return qt;
+}
+
+// ------------------------------------------------ fixed point and FP32 sums
+
+constexpr float kF0 = 12582912.0f;                 // 1.5 * 2^23
+constexpr double kM = 6755399441055744.0 + (double)0x4b400000;  // 1.5 * 2^52 + the bits of kF0
+constexpr unsigned kMHi = 0x43380000u;             // upper word of every in-range v
+
+// Scale and limits of one query at one cutoff, in units of 2^-K.
+struct Fix {
+    double scale;     // 2^K
+    double mid;       // units of the middle of the range
+    double eta;       // how far a sum (its root) may be off
+    float hi, lo;     // a total above hi exceeds the limit, one of at most lo does not
+    float a;          // ERP: the gap as F; MSM: the cost
+    float e1, e0;     // EDR, LCSS: a distance above e1 misses for certain, one below e0 matches
+    int most;         // EDR, LCSS: the misses the cutoff allows
+    bool exact;       // everything in FP64
+};
+
+template <int METRIC>
+__device__ __forceinline__ Fix make_fix(const QueryDev& q, double bsf, bool raw) {
+    Fix f;
+    const int m = q.m, lane = threadIdx.x & 31;
+    double xl = INFINITY, xh = -INFINITY;
+    for (int k = lane; k < m; k += 32) {
+        xl = fmin(xl, q.qn[k]);
+        xh = fmax(xh, q.qn[k]);
+    }
+    for (int o = 16; o; o >>= 1) {
+        xl = fmin(xl, __shfl_xor_sync(0xffffffffu, xl, o));
+        xh = fmax(xh, __shfl_xor_sync(0xffffffffu, xh, o));
+    }
+    const double ymax = raw ? 2.0 * (xh - xl) + 1.0 : fmax(fmax(xh, -xl), sqrt((double)m)) * 1.01 + 1.0;
+    f.exact = !(ymax < 1e200) || !(bsf < kGlbMax);
+    f.scale = scalbn(1.0, f.exact ? 0 : 21 - ilogb(ymax));  // ymax 2^K < 2^22
+    f.mid = raw && !f.exact ? rint(0.5 * (xl + xh) * f.scale) : 0.0;
+    f.exact |= !(fabs(f.mid) < 0x1p50);
+    const double U = bsf * f.scale, arg = q.arg * f.scale;
+    const double rho = (m + 16.0) * 0x1p-23;
+    f.hi = f.lo = f.a = f.e1 = f.e0 = 0.f;
+    f.eta = 0.0;
+    f.most = 0;
+    if (METRIC == DTW || METRIC == ERP || METRIC == MSM) {
+        double hi, lo;
+        if (METRIC == MSM) {
+            const double eta = 2.0 * (m + 4.0);
+            f.eta = eta;
+            hi = (U + eta) * (1.0 + rho);
+            lo = (U - eta) * (1.0 - rho);
+            f.a = (float)arg;
+            f.exact |= !(arg < 1e30);
+        } else {
+            double unit = 2.0;
+            if (METRIC == ERP) {
+                const double ga = rint(arg - f.mid);
+                if (!(fabs(ga) < 0x1p22)) unit += (fabs(ga) + 0x1p24) * 0x1p-22;
+                f.a = (float)(12582912.0 + ga);
+                f.exact |= !(fabs(ga) < 0x1p60);
+            }
+            const double eta = unit * sqrt(m + 2.0);
+            hi = (U + eta) * (U + eta) * (1.0 + rho);
+            lo = U > eta ? (U - eta) * (U - eta) * (1.0 - rho) : -1.0;
+            f.eta = eta;
+        }
+        f.hi = __double2float_ru(hi);
+        f.lo = __double2float_rd(lo);
+        f.exact |= !(hi < 1e37);
+    } else {
+        f.e1 = __double2float_ru(arg * (1.0 + 0x1p-22) + 2.0);
+        f.e0 = __double2float_rd(arg * (1.0 - 0x1p-22) - 2.0);
+        if (METRIC == EDR) {
+            f.most = f.exact ? 0 : (int)bsf;
+        } else {  // the fewest matches whose bound does not exceed the cutoff
+            int a = 0, b = m;
+            while (a < b) {
+                const int mid = (a + b) >> 1;
+                if (dmax0(dsub(1.0, ddiv((double)mid, (double)m))) > bsf) a = mid + 1;
+                else b = mid;
+            }
+            f.most = m - a;
+        }
+    }
+    return f;
+}
+
+// One candidate's map from raw points to F, with the upper bits collected.
+struct FixMap {
+    double A, B;
+    unsigned badh, badl;
+    __device__ __forceinline__ bool init(double mu, double sg, const Fix& f) {
+        A = __drcp_rn(sg) * f.scale;
+        const double p = mu * A;
+        B = fma(-mu, A, kM - f.mid);
+        badh = badl = 0u;
+        return fabs(p) < 0x1p51 && A < 0x1p900 && A > 0x1p-900;
+    }
+    __device__ __forceinline__ float at(double t) {  // with range check
+        const double v = fma(t, A, B);
+        const unsigned l = (unsigned)__double2loint(v);
+        badh |= (unsigned)__double2hiint(v) ^ kMHi;
+        badl |= l ^ 0x4b000000u;
+        return __uint_as_float(l);
+    }
+    __device__ __forceinline__ float at_checked(double t) const {  // a point already checked
+        return __uint_as_float((unsigned)__double2loint(fma(t, A, B)));
+    }
+    __device__ __forceinline__ bool bad() const { return (badh | (badl & 0xff800000u)) != 0u; }
+};
+
+// Sum (DTW, ERP, MSM) or certain / possible misses (EDR, LCSS).
+struct Acc {
+    float s = 0.f;
+    int c1 = 0, c2 = 0;
+};
+
+// the term of x against [lo, up]; gap: ERP's distance to the gap value
+template <int METRIC>
+__device__ __forceinline__ void acc_add(Acc& a, float x, float lo, float up, float gap, const Fix& f) {
+    if (METRIC == EDR || METRIC == LCSS) {
+        const float e = fmaxf(lo - x, x - up);  // signed: inside is certain for small tolerances too
+        a.c1 += e > f.e1 ? 1 : 0;
+        a.c2 += e >= f.e0 ? 1 : 0;
+        return;
+    }
+    float e = fmaxf(fmaxf(lo - x, x - up), 0.f);
+    if (METRIC == DTW) {
+        a.s = fmaf(e, e, a.s);
+    } else if (METRIC == ERP) {
+        e = fminf(e, fabsf(gap));
+        a.s = fmaf(e, e, a.s);
+    } else {
+        a.s += fminf(e, f.a);
+    }
+}
+
+// the boundary terms of points 0 and m-1 (and m-2), src/glb.cpp:200-230
+template <int METRIC>
+__device__ __forceinline__ Acc acc_boundary(FixMap& map, const double* __restrict__ tp, const float2* __restrict__ Qx,
+                                            int m, const Fix& f) {
+    Acc a;
+    if (METRIC == LCSS) return a;
+    const float TL = map.at(tp[m - 1]), ql = Qx[m - 1].x;
+    if (METRIC == EDR) {
+        const float e = fabsf(ql - TL);
+        a.c1 = e > f.e1 ? 1 : 0;
+        a.c2 = e >= f.e0 ? 1 : 0;
+    } else if (METRIC == ERP) {
+        const float d = fminf(fabsf(ql - TL), fminf(fabsf(ql - f.a), fabsf(TL - f.a)));
+        a.s = d * d;
+    } else {
+        const float d0 = map.at(tp[0]) - Qx[0].x, dl = fabsf(ql - TL);
+        if (METRIC == DTW) {
+            a.s = fmaf(d0, d0, dl * dl);
+        } else {
+            const float T2 = map.at(tp[m - 2]), ql2 = Qx[m - 2].x;
+            float b = fminf(dl, f.a);
+            if (!((T2 >= TL && TL >= ql) || (T2 <= TL && TL <= ql) || (ql2 <= ql && ql <= TL) ||
+                  (ql2 >= ql && ql >= TL)))
+                b = fminf(dl, fminf(f.a + fabsf(TL - T2), f.a + fabsf(ql - ql2)));
+            a.s = fabsf(d0) + b;
+        }
+    }
+    return a;
+}
+
+template <int METRIC>
+__device__ __forceinline__ bool acc_dead(const Acc& a, const Fix& f) {
+    return (METRIC == EDR || METRIC == LCSS) ? a.c1 > f.most : a.s > f.hi;
+}
+template <int METRIC>
+__device__ __forceinline__ bool acc_alive(const Acc& a, const Fix& f) {
+    return (METRIC == EDR || METRIC == LCSS) ? a.c2 <= f.most : a.s <= f.lo;
+}
+
+__device__ __forceinline__ float fix_units(double x, const Fix& f) {
+    return (float)(12582912.0 + rint(x * f.scale - f.mid));
+}
+
+}  // namespace
+
 template <int METRIC>
 __global__ void __launch_bounds__(256, 4) k_glb_tq(Geom g, GlbJob job) {
-    extern __shared__ double gq_smem[];
+    extern __shared__ __align__(16) float2 gtq_smem[];
     const QueryDev& q = job.q;
     const int m = q.m;
-    double* Q = gq_smem;
-    double* LQ = Q + m;
-    double* UQ = LQ + m;
-    for (int i = threadIdx.x; i < m; i += blockDim.x) { Q[i] = q.qn[i]; LQ[i] = q.LQ[i]; UQ[i] = q.UQ[i]; }
-    __syncthreads();
+    float2* LU = gtq_smem;  // [m] query envelope as F
+    float2* Qx = LU + m;    // [m] query points as F (x)
     const double bsf = job.cutoff_ptr ? *job.cutoff_ptr : q.cutoff;
-    const double sq = dmul(bsf, bsf);  // glb_exceeds_squared_bsf, src/glb.cpp:28-31
-    const double lim = (METRIC == DTW || METRIC == ERP) ? sq : bsf;
-    const double arg = q.arg;
+    const Fix f = make_fix<METRIC>(q, bsf, g.raw != 0);
+    for (int i = threadIdx.x; i < m; i += blockDim.x) {
+        LU[i] = make_float2(fix_units(q.LQ[i], f), fix_units(q.UQ[i], f));
+        Qx[i] = make_float2(fix_units(q.qn[i], f), 0.f);
+    }
+    __syncthreads();
+    constexpr int kb = METRIC == LCSS ? 0 : 1;
+    const int ke = METRIC == LCSS ? m : m - 1;
     const unsigned long long n_in = *job.n_in;
     const unsigned long long n_lim = n_in < (unsigned long long)job.in_cap ? n_in : job.in_cap;
     for (unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x; base < n_lim;
@@ -111,7 +429,7 @@ __global__ void __launch_bounds__(256, 4) k_glb_tq(Geom g, GlbJob job) {
         const unsigned long long idx = base + threadIdx.x;
         const bool active = idx < n_lim;
         long long gi = 0;
-        double mu = 0.0, sg = 1.0, inv = 1.0;
+        double mu = 0.0, sg = 1.0;
         if (active) {
             gi = job.in[idx];
             long long s;
@@ -119,80 +437,56 @@ __global__ void __launch_bounds__(256, 4) k_glb_tq(Geom g, GlbJob job) {
             g.locate(gi, &s, &j);
             mu = job.MU[s * g.kml + j];
             sg = job.SIG[s * g.kml + j];
-            inv = __drcp_rn(sg);
         }
-        const bool rok = rcp_div_in_range(sg);
-        const double* tp = job.target + gi;
-        bool alive = active;
-        double boundary = 0.0, tq = 0.0;
-        if (active) {
-#define TN(k) zdiv_i(dsub(tp[(k)], mu), sg, inv, rok)
-            const double T0 = TN(0), TL = TN(m - 1);
-            if (METRIC == DTW) {
-                boundary = dadd(dsq(T0, Q[0]), dsq(TL, Q[m - 1]));
-            } else if (METRIC == ERP) {
-                boundary = dmin3(dsq(Q[m - 1], TL), dsq(Q[m - 1], arg), dsq(TL, arg));
-            } else if (METRIC == EDR) {
-                boundary = dminv(edr_sub(Q[m - 1], TL, arg), 1.0);
-            } else if (METRIC == MSM) {
-                const double T2 = TN(m - 2);
-                const double q0 = Q[0], ql = Q[m - 1], ql2 = Q[m - 2];
-                if ((T2 >= TL && TL >= ql) || (T2 <= TL && TL <= ql) || (ql2 <= ql && ql <= TL) ||
-                    (ql2 >= ql && ql >= TL)) {
-                    boundary = dadd(fabs(dsub(q0, T0)), dminv(fabs(dsub(ql, TL)), arg));
+        const double* __restrict__ tp = job.target + gi;
+        FixMap map;
+        bool bad = !map.init(mu, sg, f) || f.exact;
+        bool dead = !active;
+        Acc a;
+        int inner = 0;  // certain misses without the boundary (the T->Q sum)
+        if (__any_sync(0xffffffffu, !dead && !bad)) {
+            a = acc_boundary<METRIC>(map, tp, Qx, m, f);
+            inner = a.c1;
+            for (int k = kb; k < ke; k += 8) {
+                if (k + 8 <= ke) {
+                    double t[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) t[u] = tp[k + u];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const float F = map.at(t[u]);
+                        const float2 e = LU[k + u];
+                        acc_add<METRIC>(a, F, e.x, e.y, F - f.a, f);
+                    }
                 } else {
-                    boundary = dadd(fabs(dsub(q0, T0)),
-                                    dmin3(fabs(dsub(ql, TL)), dadd(arg, fabs(dsub(TL, T2))),
-                                          dadd(arg, fabs(dsub(ql, ql2)))));
+                    for (int u = 0; k + u < ke; ++u) {
+                        const float F = map.at(tp[k + u]);
+                        const float2 e = LU[k + u];
+                        acc_add<METRIC>(a, F, e.x, e.y, F - f.a, f);
+                    }
                 }
+                bad = bad || map.bad();
+                dead = dead || (!bad && acc_dead<METRIC>(a, f));
+                if (!__any_sync(0xffffffffu, !dead && !bad)) break;
             }
-            if (METRIC == LCSS) {
-                // every point, no abandon (src/glb.cpp:238-252)
-                const double min_len = (double)m;
-                int k = 0;
-                for (; k + 4 <= m; k += 4) {
-                    double z4[4], t4[4];
-                    zdiv_group([&](int u) { return dsub(tp[k + u], mu); }, sg, inv, rok, z4);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) t4[u] = tq_term<LCSS>(z4[u], LQ[k + u], UQ[k + u], arg);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) tq = dadd(tq, t4[u]);
-                }
-                for (; k < m; ++k) tq = dadd(tq, tq_term<LCSS>(TN(k), LQ[k], UQ[k], arg));
-                if (dmax0(dsub(1.0, ddiv(tq, min_len))) > bsf) alive = false;
-            } else {
-                // points 1..m-2 four at a time: the four normalisations are
-                // independent, the sum takes them in the reference's order, and
-                // the abandon test runs once per group -- the sum never
-                // decreases, so a sum past the limit anywhere in the group is
-                // past it at the group's end (the same decision)
-                int k = 1;
-                for (; k + 4 <= m - 1; k += 4) {
-                    double z4[4], t4[4];
-                    zdiv_group([&](int u) { return dsub(tp[k + u], mu); }, sg, inv, rok, z4);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) t4[u] = tq_term<METRIC>(z4[u], LQ[k + u], UQ[k + u], arg);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) tq = dadd(tq, t4[u]);
-                    if (dadd(boundary, tq) > lim) { alive = false; break; }
-                }
-                if (alive) {
-                    for (; k < m - 1; ++k) tq = dadd(tq, tq_term<METRIC>(TN(k), LQ[k], UQ[k], arg));
-                    if (dadd(boundary, tq) > lim) alive = false;
-                }
-            }
-#undef TN
+            bad = bad || map.bad();  // no inner point: the boundary's own
+            dead = dead || (!bad && acc_dead<METRIC>(a, f));
+            inner = a.c1 - inner;
         }
-        if (active && !alive) {
+        bool alive = !dead && !bad && acc_alive<METRIC>(a, f);
+        double ob = dnan();  // certified: nothing to hand on but the T->Q count
+        double ot = METRIC == LCSS ? (double)(m - inner) : (double)inner;
+        if (!dead && !alive) {  // within the margin or out of range: the reference's operations
+            alive = exact_tq<METRIC>(q.qn, q.LQ, q.UQ, m, q.arg, tp, mu, sg, bsf, ob, ot);
             // abandoned: GLB returns MAX_VAL (src/glb.cpp:221 etc.); it survives only if
-            // MAX_VAL <= cutoff
-            if (kGlbMax <= bsf) alive = true, boundary = -1.0;  // marker: keep as MAX_VAL
+            // MAX_VAL <= cutoff (marker -1)
+            if (!alive && kGlbMax <= bsf) { alive = true; ob = -1.0; }
         }
         warp_append(alive, job.n_out, [&](unsigned long long o) {
             if (o < (unsigned long long)job.out_cap) {
                 job.out[o] = gi;
-                job.out_b[o] = boundary;
-                job.out_t[o] = tq;
+                job.out_b[o] = ob;
+                job.out_t[o] = ot;
             }
         });
     }
@@ -209,10 +503,15 @@ __global__ void __launch_bounds__(256, 4) k_glb_tq(Geom g, GlbJob job) {
 // replace the L reads per output of a direct scan, so the cost no longer
 // grows with the radius.  A CTA produces kFwdTile outputs per tile from the
 // tile plus its w-point halo, ping-ponging between two shared buffers.
+//
+// With clo/cup also the centred windows min/max(t[p-w .. p+w]) of the points
+// w .. n-1-w, each the min/max of the forward windows at p-w and p, from the
+// same tile with a halo of 2w points.
 __global__ void __launch_bounds__(kFwdThreads) k_fwd_env(const double* __restrict__ t, long long n, int w,
-                                                        double* __restrict__ lo, double* __restrict__ up) {
+                                                        double* __restrict__ lo, double* __restrict__ up,
+                                                        double* __restrict__ clo, double* __restrict__ cup) {
     extern __shared__ double fw_smem[];
-    const int ext = kFwdTile + w;  // tile plus halo
+    const int ext = kFwdTile + (clo ? 2 * w : w);  // tile plus halo
     double* An = fw_smem;
     double* Ax = An + ext;
     double* Bn = Ax + ext;
@@ -257,90 +556,162 @@ __global__ void __launch_bounds__(kFwdThreads) k_fwd_env(const double* __restric
             }
             lo[p] = mn;
             up[p] = mx;
+            if (clo && p + 2 * (long long)w <= n - 1) {
+                clo[p + w] = fmin(mn, fmin(An[i + w], An[i + w + off]));
+                cup[p + w] = fmax(mx, fmax(Ax[i + w], Ax[i + w + off]));
+            }
         }
         __syncthreads();
     }
 }
 
-size_t fwd_env_smem_bytes(int w) { return sizeof(double) * 4 * (size_t)(kFwdTile + w); }
+size_t fwd_env_smem_bytes(int w, bool centred) {
+    return sizeof(double) * 4 * (size_t)(kFwdTile + (centred ? 2 * w : w));
+}
 
-// one lane per T->Q survivor: Q->T terms added in the reference's order
 template <int METRIC>
-__global__ void __launch_bounds__(128) k_glb_qt(Geom g, GlbJob job) {
-    extern __shared__ double gqt_smem[];
+__global__ void __launch_bounds__(256, 3) k_glb_qt(Geom g, GlbJob job) {
+    extern __shared__ __align__(16) float2 gqt_smem[];
     const QueryDev& q = job.q;
     const int m = q.m, w = q.w;
-    double* Q = gqt_smem;
-    for (int i = threadIdx.x; i < m; i += blockDim.x) Q[i] = q.qn[i];
-    __syncthreads();
+    float2* Qx = gqt_smem;  // [m] query points as F, and (ERP) their distance to the gap
     const double bsf = job.cutoff_ptr ? *job.cutoff_ptr : q.cutoff;
-    const double sq = dmul(bsf, bsf);
-    const double arg = q.arg;
+    const Fix f = make_fix<METRIC>(q, bsf, g.raw != 0);
+    for (int i = threadIdx.x; i < m; i += blockDim.x) {
+        const float x = fix_units(q.qn[i], f);
+        Qx[i] = make_float2(x, x - f.a);
+    }
+    __syncthreads();
+    const double inv_scale = 1.0 / f.scale;
+    const double rho = (m + 16.0) * 0x1p-23;
+    constexpr int kb = METRIC == LCSS ? 0 : 1;
+    const int ke = METRIC == LCSS ? m : m - 1;
+    // interior points: the centred windows, where there are any
+    const bool ctr = job.clo != nullptr;
+    const int i0 = ctr ? min(max(kb, w), ke) : ke, i1 = ctr ? max(i0, min(ke, m - w)) : ke;
     const unsigned long long n_in = *job.n_in;
     const unsigned long long n_lim = n_in < (unsigned long long)job.in_cap ? n_in : job.in_cap;
-    for (unsigned long long c = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; c < n_lim;
-         c += (unsigned long long)gridDim.x * blockDim.x) {
-        const long long gi = job.in[c];
-        const double boundary = job.in_b[c];
-        const double tq = job.in_t[c];
-        long long s;
-        int j;
-        g.locate(gi, &s, &j);
-        double glb, qt = 0.0;
-        if (boundary == -1.0) {
-            glb = kGlbMax;  // abandoned in T->Q but MAX_VAL <= cutoff
-        } else {
-            const double mu = job.MU[s * g.kml + j], sg = job.SIG[s * g.kml + j];
-            const double inv = __drcp_rn(sg);
-            const bool rok = rcp_div_in_range(sg);
-            const double* lf = job.lraw + gi;
-            const double* uf = job.uraw + gi;
-            const int k0 = (METRIC == LCSS) ? 0 : 1, k1 = (METRIC == LCSS) ? m - 1 : m - 2;
-            // the terms are independent (unrolled so their loads and divisions
-            // overlap); only the sum is sequential, in the reference's order.
-            // Interior points (w <= k <= m-1-w) read the windows at k-w and k
-            // directly; the edges take the clamped indices.
-            const int i0 = max(k0, w), i1 = min(k1, m - 1 - w);
-            int k = k0;
-            for (; k <= k1 && k < i0; ++k) qt = dadd(qt, qt_term(METRIC, Q[k], k, m, w, lf, uf, mu, sg, inv, rok, arg));
-            for (; k + 1 <= i1; k += 2) {  // two points, four quotients, one range test
-                double z4[4];
-                zdiv_group(
-                    [&](int u) {
-                        const int kk = k + (u & 1);
-                        if (u < 2) { const double a0 = lf[kk - w], a1 = lf[kk]; return dsub((a1 < a0) ? a1 : a0, mu); }
-                        const double b0 = uf[kk - w], b1 = uf[kk];
-                        return dsub((b0 < b1) ? b1 : b0, mu);
-                    },
-                    sg, inv, rok, z4);
-                qt = dadd(qt, qt_term_norm(METRIC, Q[k], z4[0], z4[2], arg));
-                qt = dadd(qt, qt_term_norm(METRIC, Q[k + 1], z4[1], z4[3], arg));
+    for (unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x; base < n_lim;
+         base += (unsigned long long)gridDim.x * blockDim.x) {
+        const unsigned long long c = base + threadIdx.x;
+        const bool active = c < n_lim;
+        long long gi = 0, s = 0;
+        double mu = 0.0, sg = 1.0, boundary = 0.0, tq = 0.0;
+        if (active) {
+            gi = job.in[c];
+            boundary = job.in_b[c];
+            tq = job.in_t[c];
+            int j;
+            g.locate(gi, &s, &j);
+            mu = job.MU[s * g.kml + j];
+            sg = job.SIG[s * g.kml + j];
+        }
+        const double* __restrict__ lf = job.lraw + gi;
+        const double* __restrict__ uf = job.uraw + gi;
+        FixMap map;
+        bool keep = false;
+        const bool certified = map.init(mu, sg, f) && isnan(boundary);  // its points are in range
+        bool dead = !active || !certified;  // not certified: decided below
+        Acc a;
+        int edge = 0;
+        if (__any_sync(0xffffffffu, !dead)) {
+            a = acc_boundary<METRIC>(map, job.target + gi, Qx, m, f);
+            edge = a.c1;
+            auto term = [&](int k, float lo, float up) {
+                const float2 x = Qx[k];
+                acc_add<METRIC>(a, x.x, lo, up, x.y, f);
+            };
+            auto ends = [&](int k) {
+                const int p0 = qt_p0(k, w), p1 = qt_p1(k, m, w);
+                term(k, fminf(map.at_checked(lf[p0]), map.at_checked(lf[p1])),
+                     fmaxf(map.at_checked(uf[p0]), map.at_checked(uf[p1])));
+            };
+            auto done = [&] {
+                dead = dead || acc_dead<METRIC>(a, f);
+                return !__any_sync(0xffffffffu, !dead);
+            };
+            bool stop = false;
+            for (int k = kb; k < i0 && !stop; k += 4) {
+                if (k + 4 <= i0) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) ends(k + u);
+                } else {
+                    for (int u = 0; k + u < i0; ++u) ends(k + u);
+                }
+                stop = done();
             }
-            for (; k <= i1; ++k) {
-                const double a0 = lf[k - w], a1 = lf[k], b0 = uf[k - w], b1 = uf[k];
-                qt = dadd(qt, qt_term_env(METRIC, Q[k], (a1 < a0) ? a1 : a0, (b0 < b1) ? b1 : b0, mu, sg, inv, rok,
-                                          arg));
+            const double* __restrict__ cl = job.clo + gi;
+            const double* __restrict__ cu = job.cup + gi;
+            for (int k = i0; k < i1 && !stop; k += 8) {
+                if (k + 8 <= i1) {
+                    double lo[8], up[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) { lo[u] = cl[k + u]; up[u] = cu[k + u]; }
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) term(k + u, map.at_checked(lo[u]), map.at_checked(up[u]));
+                } else {
+                    for (int u = 0; k + u < i1; ++u) term(k + u, map.at_checked(cl[k + u]), map.at_checked(cu[k + u]));
+                }
+                stop = done();
             }
-            for (; k <= k1; ++k) qt = dadd(qt, qt_term(METRIC, Q[k], k, m, w, lf, uf, mu, sg, inv, rok, arg));
-            if (METRIC == LCSS) {
-                glb = dmax0(dsub(1.0, ddiv(dminv(tq, qt), (double)m)));
-            } else {
-                const double tot = dadd(boundary, qt);
-                if (METRIC == DTW || METRIC == ERP)
-                    glb = (tot > sq) ? kGlbMax : dsqrt(dmax0(dadd(boundary, dmaxv(tq, qt))));
-                else
-                    glb = (tot > bsf) ? kGlbMax : dadd(boundary, dmaxv(tq, qt));
+            for (int k = i1; k < ke && !stop; k += 4) {
+                if (k + 4 <= ke) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) ends(k + u);
+                } else {
+                    for (int u = 0; k + u < ke; ++u) ends(k + u);
+                }
+                stop = done();
+            }
+            dead = dead || acc_dead<METRIC>(a, f);
+        }
+        // what the abandon tests of the exact distances take: a lower bound of
+        // the Q->T sum (LCSS: an upper bound of the count), the T->Q count
+        double os, ot = tq;
+        if (METRIC == LCSS) os = (double)(m - (a.c1 - edge));
+        else if (METRIC == EDR) os = (double)(a.c1 - edge);
+        else {
+            // the boundary is part of a.s: taken off at its upper end
+            Acc b;
+            if (!dead) b = acc_boundary<METRIC>(map, job.target + gi, Qx, m, f);
+            const double v = fmax(0.0, ((double)a.s - (double)b.s * (1.0 + rho)) - (double)a.s * rho);
+            if (METRIC == MSM) os = fmax(0.0, v - f.eta) * inv_scale;
+            else {
+                const double r = fmax(0.0, sqrt(v) - f.eta) * inv_scale;
+                os = r * r * (1.0 - 0x1p-40);
             }
         }
-        if (glb <= bsf) {
-            const unsigned long long o = atomicAdd(job.n_out, 1ull);
+        keep = active && certified && !dead && acc_alive<METRIC>(a, f);
+        if (active && !keep && !(certified && dead)) {
+            double qt = 0.0, glb;
+            bool on = true;
+            if (certified) on = exact_tq<METRIC>(q.qn, q.LQ, q.UQ, m, q.arg, job.target + gi, mu, sg, bsf, boundary, tq);
+            if (boundary == -1.0 || !on) {
+                glb = kGlbMax;  // abandoned in T->Q but MAX_VAL <= cutoff
+            } else {
+                qt = exact_qt<METRIC>(q.qn, m, w, q.arg, lf, uf, mu, sg);
+                if (METRIC == LCSS) {
+                    glb = dmax0(dsub(1.0, ddiv(dminv(tq, qt), (double)m)));
+                } else {
+                    const double tot = dadd(boundary, qt);
+                    if (METRIC == DTW || METRIC == ERP)
+                        glb = (tot > dmul(bsf, bsf)) ? kGlbMax : dsqrt(dmax0(dadd(boundary, dmaxv(tq, qt))));
+                    else
+                        glb = (tot > bsf) ? kGlbMax : dadd(boundary, dmaxv(tq, qt));
+                }
+            }
+            keep = glb <= bsf;
+            os = boundary == -1.0 ? -1.0 : qt;
+            ot = boundary == -1.0 ? -1.0 : tq;
+        }
+        warp_append(keep, job.n_out, [&](unsigned long long o) {
             if (o < (unsigned long long)job.out_cap) {
                 job.out[o] = gi;
-                if (job.out_t) job.out_t[o] = (boundary == -1.0) ? -1.0 : qt;
-                if (job.out_b) job.out_b[o] = (boundary == -1.0) ? -1.0 : tq;
+                if (job.out_t) job.out_t[o] = os;
+                if (job.out_b) job.out_b[o] = ot;
             }
             if (job.segc && s < g.forsize) atomicAdd((unsigned long long*)&job.segc[3 * s + 2], 1ull);
-        }
+        });
     }
 }
 

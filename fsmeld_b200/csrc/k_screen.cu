@@ -32,7 +32,11 @@
 // dependent operations interleave.
 //
 // What bounds it: instruction issue (DTW about 6, MSM 13 instructions per
-// cell; the exact DP spends 30 to 110 on FP64 selects and compares).
+// cell; the exact DP spends 30 to 110 on FP64 selects and compares).  Measured
+// on the five-metric workload (2^24 points, m = 256, w = 13): MSM 82 ms by the
+// exact DP alone, 36 ms screen + 0.2 ms exact; ERP 2.6 -> 1.2 + 0.2 ms.  A warp
+// steps until its last candidate is dropped: 1.5 (MSM) to 1.9 (ERP, DTW) lane
+// rows per useful one.
 #include "common.cuh"
 #include "kernels.cuh"
 

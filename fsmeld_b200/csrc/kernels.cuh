@@ -33,10 +33,12 @@ struct GlbJob {
     const double* target;
     const double* lraw;         // forward windows min / max(t[p .. p+w]) of the raw target
     const double* uraw;
+    const double* clo;          // optional: centred windows min / max(t[p-w .. p+w])
+    const double* cup;
     const double* MU;
     const double* SIG;
     const long long* in;
-    const double* in_b;         // stage 2 input: boundary terms
+    const double* in_b;         // stage 2 input: boundary terms (NaN: T->Q decided without them, -1: abandoned)
     const double* in_t;         // stage 2 input: T->Q sums (LCSS: T->Q reward)
     const unsigned long long* n_in;
     long long in_cap;
@@ -142,8 +144,8 @@ __global__ void k_glb_qt(Geom g, GlbJob job);
 constexpr int kFwdThreads = 256;
 constexpr int kFwdTile = 2048;
 __global__ void k_fwd_env(const double* __restrict__ t, long long n, int w, double* __restrict__ lo,
-                          double* __restrict__ up);
-size_t fwd_env_smem_bytes(int w);
+                          double* __restrict__ up, double* __restrict__ clo, double* __restrict__ cup);
+size_t fwd_env_smem_bytes(int w, bool centred);
 template <int METRIC, bool GW>
 __global__ void k_dp(Geom g, DpJob job);
 // the DP kernel for a metric, with its band in shared memory or in job.gwork
