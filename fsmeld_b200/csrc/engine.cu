@@ -629,38 +629,24 @@ static int run_env(fsmeld_ctx* c, const Geom& g, int w, Stats* st, const std::st
 
 template <int T, int IPT>
 static int launch_thr(fsmeld_ctx* c, const Geom& g, const ThrJob* djobs, int njobs, int m) {
-    const size_t work = round256(threshold_work_bytes(T * IPT, threshold_sort_tmp_bytes<T, IPT>(), m));
-    unsigned char* gwork = nullptr;
-    size_t smem = work;
-    unsigned gx;
+    const ThrMem mem = threshold_mem<T, IPT>(m, (size_t)c->smem_optin);
+    const void* kf = mem.gw ? (const void*)k_threshold<T, IPT, true> : (const void*)k_threshold<T, IPT, false>;
     int r;
-    const bool gw_path = work + 16384 > (size_t)c->smem_optin;
-    if (!gw_path) {
-        if ((r = allow_smem(c, k_threshold<T, IPT, false>, smem))) return r;
-        int per_sm = 0;
-        FSM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_threshold<T, IPT, false>, T, smem));
-        gx = (unsigned)std::min<long long>(2 * g.S, (long long)std::max(1, per_sm) * c->sm_count * 4);
-    } else {
-        // global scratch for the runs, sorted values and sweep; the sort's temp
-        // storage in shared memory
-        smem = threshold_sort_tmp_bytes<T, IPT>();
-        if (smem + 8192 > (size_t)c->smem_optin)
-            return fail(FSMELD_E_UNSUPPORTED, "threshold sort does not fit in shared memory");
-        if ((r = allow_smem(c, k_threshold<T, IPT, true>, smem))) return r;
-        int per_sm = 0;
-        FSM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_threshold<T, IPT, true>, T, smem));
-        gx = (unsigned)std::min<long long>(2 * g.S, (long long)std::max(1, per_sm) * c->sm_count * 2);
-        const size_t gstride = round256(threshold_work_bytes(T * IPT, 0, m));
-        if ((r = bufT(c, "thrwork", gstride * gx * (size_t)njobs, &gwork))) return r;
-        dim3 grid(gx, njobs);
-        prof_begin(c, ST_THR);
-        k_threshold<T, IPT, true><<<grid, T, smem, c->stream>>>(g, djobs, gwork, (long long)gstride);
-        LAUNCH_CHECK(c);
-        return FSMELD_OK;
-    }
-    dim3 grid(gx, njobs);
+    if ((r = allow_smem(c, kf, mem.smem))) return r;
+    int per_sm = 0;
+    FSM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kf, T, mem.smem));
+    // shared memory: a few blocks per place even out the tail; global scratch:
+    // one scratch area per block
+    unsigned gx = (unsigned)std::min<long long>(2 * g.S, (long long)std::max(1, per_sm) * c->sm_count * (mem.gw ? 2 : 4));
+    unsigned char* gwork = nullptr;
+    long long gstride = (long long)round256(mem.gbytes);
+    if (mem.gw && (r = bufT(c, "thrwork", (size_t)gstride * gx * (size_t)njobs, &gwork))) return r;
+    Geom ga = g;
+    int z_shared = mem.z_shared;
+    void* args[] = {&ga, &djobs, &gwork, &gstride, &z_shared};
     prof_begin(c, ST_THR);
-    k_threshold<T, IPT, false><<<grid, T, smem, c->stream>>>(g, djobs, gwork, (long long)work);
+    const cudaError_t le = cudaLaunchKernel(kf, dim3(gx, njobs), dim3(T), args, mem.smem, c->stream);
+    if (le != cudaSuccess) return cuda_fail(le, "k_threshold launch", __FILE__, __LINE__);
     LAUNCH_CHECK(c);
     return FSMELD_OK;
 }

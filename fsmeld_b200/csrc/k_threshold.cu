@@ -9,9 +9,12 @@
 // and a penalty sum C, and scores LB[i] = h(t_i) * g_i; the argmax gives t.
 //
 // Here one CTA handles one (segment, side):
-//  1. dedup with a block scan, sort runs with a stable block merge sort on
-//     an order-preserving 64-bit key (total order: value, NaN last, ties by
-//     position through the sort's stability);
+//  1. dedup with a block scan, then the runs are sorted (total order: value,
+//     NaN last, ties by position): every run is counted into one of two
+//     buckets per run slot, equal in width over the values' range, and ranked
+//     by comparison with the few other runs of its bucket.  That took half of
+//     the kernel as a block merge sort of (64-bit key, run) pairs, which
+//     stays for values bunched in a few buckets (over kBucketMost in one);
 //  2. every pointer move of the sweep becomes an op with the sweep step at
 //     which it fires (a binary search over the sorted values); ops are
 //     ordered by (step, stream, rank) -- the order the reference's loops
@@ -23,6 +26,12 @@
 //  4. every candidate reads its state, scores LB in parallel, and a block
 //     reduction takes the first maximum (NaN at index 0 wins, as in
 //     findMaxIndex, src/find_t_lp.cpp:206-216).
+// Several blocks per SM hide each other's serial phases (the replay, 8 cycles
+// an add); the sort is a third of what is left.  Measured, five queries on 2^24
+// points (m = 256): 11.5 ms with the merge sort, predicated chains and a
+// quadratic op order for ERP, 5.9 ms now; 20 queries of mixed length on 2^22
+// points, most with 8192-point segments that used to lie in global scratch:
+// 17.6 -> 8.9 ms.
 // ERP's priority queues pop equal keys in an order the C++ library leaves
 // to its heap layout; here equal keys pop by query index.  The threshold is
 // the same unless two candidates' scores tie to the last bit.
@@ -39,6 +48,7 @@ namespace fsm {
 namespace {
 
 constexpr int kNever = INT_MAX;
+constexpr int kBucketMost = 24;  // runs of one bucket that are ranked by comparison
 
 // Order-preserving key of a double: ascending values map to ascending keys,
 // -0 and +0 to one key (they compare equal), NaN to the largest key (sorted
@@ -118,20 +128,64 @@ struct Plan {
 
 }  // namespace
 
-// Block working set: the runs (values and starts), region X (the sort's temp
-// storage, then the sorted values and counts) and region Z (the sweep: op
-// steps, op order, operand/state slots).  Z is used only after the runs are
-// dead, so it lives in the runs region whenever it fits there (segments of at
-// least 8m points, the usual case).
-__host__ __device__ inline size_t thr_runs_bytes(int cap) { return ((size_t)cap * 12 + 4 + 15) & ~size_t(15); }
-__host__ __device__ inline size_t thr_z_bytes(int m) { return (size_t)m * 24 + 16 + (size_t)(2 * m + 1) * 32; }
-__host__ __device__ inline bool thr_z_in_runs(int cap, int m) { return thr_z_bytes(m) <= thr_runs_bytes(cap); }
+// Block working set: region R, the runs (values and starts) and, in the same
+// place once the runs are in registers, the sorted values and counts; region Z,
+// the sort's temporaries and after it the sweep (op steps, op order,
+// operand/state slots).  Segments of up to 8192 core values keep both in shared
+// memory; longer ones keep R in global scratch with a second area for the
+// sorted values, and Z in shared memory when it fits.
+__host__ __device__ constexpr size_t thr_round16(size_t b) { return (b + 15) & ~size_t(15); }
+// counts and the bucket sort's counters are walked in runs of a few per thread:
+// one spare slot in 32 puts the walks on distinct banks
+__host__ __device__ constexpr int thr_pad(int i) { return i + (i >> 5); }
+__host__ __device__ constexpr size_t thr_r_bytes(int cap) {
+    return thr_round16((size_t)cap * 8 + ((size_t)thr_pad(cap) + 2) * 4);
+}
+__host__ __device__ inline size_t thr_z_bytes(int m) { return (size_t)m * 24 + 16 + (size_t)(2 * m + 9) * 32; }
+__host__ __device__ constexpr size_t thr_bucket_bytes(int cap, int nb) {
+    return thr_round16(((size_t)thr_pad(nb) + 1) * 4 + (size_t)cap * 2);
+}
+__host__ __device__ constexpr int thr_buckets(int cap, bool gw) { return gw ? cap : 2 * cap; }
+
+// The runs sorted by a block merge sort (thread t on runs t IPT ..) into the
+// sorted values and counts; in a function of its own for its registers.
+template <int T, int IPT>
+__device__ __noinline__ void merge_runs(typename cub::BlockMergeSort<unsigned long long, T, IPT, int>::TempStorage& tmp,
+                                        const double* rval, const int* rstart, double* tv, int* gp, int nr,
+                                        int upper) {
+    const int t = threadIdx.x;
+    unsigned long long keys[IPT];
+    int rid[IPT];
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+        const int r = t * IPT + k;
+        keys[k] = r < nr ? order_key(rval[r], upper ? 0 : 1) : ~0ull;  // padding after every run
+        rid[k] = r;
+    }
+    __syncthreads();
+    cub::BlockMergeSort<unsigned long long, T, IPT, int>(tmp).StableSort(keys, rid, KeyLess());
+    __syncthreads();
+    double rv[IPT];
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+        const int r = t * IPT + k < nr ? rid[k] : 0;
+        rv[k] = rval[r];
+        rid[k] = rstart[r + 1] - rstart[r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < IPT; ++k)
+        if (t * IPT + k < nr) {
+            tv[t * IPT + k] = rv[k];
+            gp[thr_pad(t * IPT + k)] = rid[k];
+        }
+}
 
 // 1024 / T blocks per SM: at most 64 registers a thread, so that several
 // blocks hide each other's serial phases
 template <int T, int IPT, bool GW>
 __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, const ThrJob* __restrict__ jobs,
-                                                 unsigned char* gwork, long long slot_stride) {
+                                                 unsigned char* gwork, long long slot_stride, int z_shared) {
     using Sort = cub::BlockMergeSort<unsigned long long, T, IPT, int>;
     using IScan = cub::BlockScan<int, T>;
     using AReduce = cub::BlockReduce<ArgMax, T>;
@@ -142,6 +196,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, const ThrJob*
     __shared__ typename AReduce::TempStorage red_tmp;
     __shared__ int s_nr, s_nfin, s_best, s_nops;
     __shared__ int s_cnt[2];
+    __shared__ double s_ext[64];
 
     const ThrJob& job = jobs[blockIdx.y];
     const QueryDev& q = job.q;
@@ -149,31 +204,26 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, const ThrJob*
     const int cnt = mk - 2 * m + 2;
     const int t = threadIdx.x;
 
-    // GW: working set in global scratch; otherwise provably shared memory
+    // GW: region R in global scratch; otherwise provably shared memory
+    constexpr size_t RB = thr_r_bytes(CAP);
     unsigned char* base = GW ? gwork + (long long)(blockIdx.y * gridDim.x + blockIdx.x) * slot_stride
                                 : thr_smem;
-    // runs (phases 1-3), then region X: sort temp (phase 2) / sorted values + g (phase 3)
-    double* rval = (double*)base;                                          // [CAP]
-    int* rstart = (int*)(base + (size_t)CAP * 8);                          // [CAP + 1]
-    unsigned char* xb = base + thr_runs_bytes(CAP);
-    // the sort's temp storage is always in shared memory (cub's block primitives
-    // work on shared memory): in the shared-memory form it shares region X with
-    // the sorted values, in the global-scratch form (GW) it is the block's whole
-    // dynamic shared memory and region X in global memory holds the values only
-    const size_t xbytes = GW ? (((size_t)CAP * 12 + 16 + 15) & ~size_t(15))
-                             : ((sizeof(typename Sort::TempStorage) > (size_t)CAP * 12 + 16
-                                     ? sizeof(typename Sort::TempStorage)
-                                     : (size_t)CAP * 12 + 16) + 15) & ~size_t(15);
-    typename Sort::TempStorage& sort_tmp =
-        *reinterpret_cast<typename Sort::TempStorage*>(GW ? thr_smem : xb);
-    double* tv = (double*)xb;                           // [CAP] sorted values
-    int* gp = (int*)(xb + (size_t)CAP * 8);             // [CAP] inclusive count sums
-    unsigned char* zb = thr_z_in_runs(CAP, m) ? base : xb + xbytes;
+    double* rval = (double*)base;                        // [CAP]
+    int* rstart = (int*)(base + (size_t)CAP * 8);        // [CAP + 1]
+    double* tv = (double*)(GW ? base + RB : base);       // [CAP] sorted values, over the runs
+    int* gp = (int*)((GW ? base + RB : base) + (size_t)CAP * 8);  // [thr_pad(CAP)] inclusive count sums
+    unsigned char* zb = GW ? (z_shared ? thr_smem : base + 2 * RB) : thr_smem + RB;
+    // the sorts' temporaries (shared memory in every form)
+    unsigned char* sortb = GW ? thr_smem : thr_smem + RB;
+    typename Sort::TempStorage& sort_tmp = *reinterpret_cast<typename Sort::TempStorage*>(sortb);
+    constexpr int NB = thr_buckets(CAP, GW);
+    int* bcnt = (int*)sortb;                                            // [thr_pad(NB) + 1]
+    unsigned short* bslot = (unsigned short*)(bcnt + thr_pad(NB) + 1);  // [CAP]
     int* sA = (int*)zb;                                 // [m]
     int* sB = sA + m;                                   // [m]
     int* opdesc = sB + m;                               // [2m]
     int* opstep = opdesc + 2 * m;                       // [2m]
-    double* st = (double*)(((uintptr_t)(opstep + 2 * m) + 15) & ~uintptr_t(15));  // [(2m+1)*4]
+    double* st = (double*)(((uintptr_t)(opstep + 2 * m) + 15) & ~uintptr_t(15));  // [(2m+9)*4]
 
     const int p = q.p;
     const int kind = (q.metric == DTW) ? 0 : (q.metric == ERP ? 2 : 1);
@@ -216,34 +266,107 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, const ThrJob*
         if (t == 0) { rstart[nr] = cnt; s_nr = nr; }
         __syncthreads();
 
-        // ---- 2. sort runs (src/find_t_lp.cpp:68-81)
-        unsigned long long keys[IPT];
-        int rid[IPT];
+        // ---- 2. sort runs (src/find_t_lp.cpp:68-81): ascending keys, ties by
+        // run; run t + k T is this thread's k-th
+        double rv[IPT];
+        int rank[IPT], rc[IPT], bk[IPT];
+        int nf = 0;  // this thread's runs that are not NaN
+        double vmn = INFINITY, vmx = -INFINITY;
 #pragma unroll
         for (int k = 0; k < IPT; ++k) {
-            const int r = t * IPT + k;
-            keys[k] = (r < nr) ? order_key(rval[r], upper ? 0 : 1) : ~0ull;  // padding after every run
-            rid[k] = r;
+            const int r = t + k * T;
+            rv[k] = r < nr ? rval[r] : dnan();
+            rc[k] = r < nr ? rstart[r + 1] - rstart[r] : 0;
+            nf += isnan(rv[k]) ? 0 : 1;
+            if (isfinite(rv[k])) { vmn = fmin(vmn, rv[k]); vmx = fmax(vmx, rv[k]); }
         }
-        Sort(sort_tmp).StableSort(keys, rid, KeyLess());
+        for (int o = 16; o; o >>= 1) {
+            vmn = fmin(vmn, __shfl_xor_sync(0xffffffffu, vmn, o));
+            vmx = fmax(vmx, __shfl_xor_sync(0xffffffffu, vmx, o));
+        }
+        if ((t & 31) == 0) { s_ext[t >> 5] = vmn; s_ext[32 + (t >> 5)] = vmx; }
+        for (int i = t; i <= thr_pad(NB); i += T) bcnt[i] = 0;
+        __syncthreads();
+        for (int i = 0; i < T / 32; ++i) { vmn = fmin(vmn, s_ext[i]); vmx = fmax(vmx, s_ext[32 + i]); }
+        // buckets of equal width over the finite values (the infinities in the
+        // outer ones, NaN in the last): the width is rounded, the order of the
+        // buckets is that of the values all the same
+        const double width = vmx > vmn ? (NB - 1) / (vmx - vmn) : 0.0;
+        const double scale = isfinite(width) ? width : 0.0;
+#pragma unroll
+        for (int k = 0; k < IPT; ++k) {
+            bk[k] = thr_pad(NB - 1);
+            rank[k] = 0;
+            if (t + k * T < nr) {
+                if (!isnan(rv[k])) {
+                    const int bu = isfinite(rv[k]) ? min(NB - 2, (int)dmul(dsub(rv[k], vmn), scale))
+                                                   : (rv[k] < 0.0 ? 0 : NB - 2);
+                    bk[k] = thr_pad(upper ? bu : NB - 2 - bu);
+                }
+                rank[k] = atomicAdd(&bcnt[bk[k]], 1);  // place inside the bucket, any order
+            }
+        }
+        __syncthreads();
+        constexpr int PER = NB / T;
+        int most = 0, bsum = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int x = bcnt[thr_pad(t * PER + i)];
+            most = max(most, x);
+            bsum += x;
+        }
+        int bbase;
+        IScan(iscan_tmp).ExclusiveSum(bsum, bbase);
+        if (!__syncthreads_or(most > kBucketMost)) {
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                const int x = bcnt[thr_pad(t * PER + i)];
+                bcnt[thr_pad(t * PER + i)] = bbase;
+                bbase += x;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < IPT; ++k)
+                if (t + k * T < nr) bslot[bcnt[bk[k]] + rank[k]] = (unsigned short)(t + k * T);
+            __syncthreads();
+            // rank inside the bucket by comparison with its other runs
+#pragma unroll
+            for (int k = 0; k < IPT; ++k) {
+                const int r = t + k * T;
+                if (r >= nr) continue;
+                const int lo = bcnt[bk[k]];
+                const int nb = bk[k] + (bk[k] % 33 == 31 ? 2 : 1);  // the next bucket's slot
+                const int hi = bk[k] < thr_pad(NB - 1) ? bcnt[nb] : nr;
+                int less = 0;
+                if (hi - lo > 1) {
+                    const unsigned long long key = order_key(rv[k], upper ? 0 : 1);
+                    for (int i = lo; i < hi; ++i) {
+                        const int o = bslot[i];
+                        const unsigned long long ko = order_key(rval[o], upper ? 0 : 1);
+                        less += (ko < key || (ko == key && o < r)) ? 1 : 0;
+                    }
+                }
+                rank[k] = lo + less;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < IPT; ++k) {
+                if (t + k * T < nr) {
+                    tv[rank[k]] = rv[k];
+                    gp[thr_pad(rank[k])] = rc[k];
+                }
+            }
+        } else {  // values bunched in a few buckets
+            merge_runs<T, IPT>(sort_tmp, rval, rstart, tv, gp, nr, upper);
+        }
         __syncthreads();
 
-        // ---- 3. sorted values, cumulative counts g_i, finite prefix length
-        int csum = 0, nf = 0;
-        double sv_[IPT];
-        int sc_[IPT];
+        // ---- 3. cumulative counts g_i, finite prefix length
+        int csum = 0;
 #pragma unroll
         for (int k = 0; k < IPT; ++k) {
             const int i = t * IPT + k;
-            sv_[k] = 0.0;
-            sc_[k] = 0;
-            if (i < nr) {
-                const int r = rid[k];
-                sv_[k] = rval[r];
-                sc_[k] = rstart[r + 1] - rstart[r];
-                csum += sc_[k];
-                nf += isnan(sv_[k]) ? 0 : 1;
-            }
+            if (i < nr) csum += gp[thr_pad(i)];
         }
         int cbase;
         IScan(iscan_tmp).ExclusiveSum(csum, cbase);
@@ -254,9 +377,8 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, const ThrJob*
         for (int k = 0; k < IPT; ++k) {
             const int i = t * IPT + k;
             if (i < nr) {
-                tv[i] = sv_[k];
-                cbase += sc_[k];
-                gp[i] = cbase;
+                cbase += gp[thr_pad(i)];
+                gp[thr_pad(i)] = cbase;
             }
         }
         if (t == 0) { s_nfin = nfin_total; s_cnt[0] = 0; s_cnt[1] = 0; }
@@ -369,7 +491,12 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, const ThrJob*
         // valid ops form a prefix of each stream (steps never go from finite to kNever and back)
         const int nAv = prefix_count(pl.nA, [&](int r) { return sA[r] != kNever; });
         const int nBv = prefix_count(pl.nB, [&](int r) { return sB[r] != kNever; });
-        const bool b_sorted = (kind != 2);
+        // ERP's steps of stream B ascend too (both the query points and their
+        // t_l / t_u ascend), unless rounding of t_l, t_u breaks it
+        int falls = 0;
+        if (kind == 2)
+            for (int r = t; r + 1 < nBv; r += T) falls |= sB[r] > sB[r + 1] ? 1 : 0;
+        const bool b_sorted = !__syncthreads_or(falls);
         for (int k = t; k < nAv + nBv; k += T) opdesc[k] = -1;
         __syncthreads();
         for (int r = t; r < nAv; r += T) {
@@ -428,54 +555,60 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, const ThrJob*
             o[0] = o0; o[1] = o1; o[2] = o2; o[3] = o3;
         }
         __syncthreads();
-        // initial sums: lane j of warp 0 owns accumulator j (the power sums
-        // m_0..m_2 for j < 3, the penalty sum C for j = 3) and adds its
-        // elements in the reference's order
+        // initial sums: lane j of one warp (a different one in each block, so that
+        // co-resident blocks' chains sit on different sub-partitions) owns
+        // accumulator j (the power sums m_0..m_2 for j < 3, the penalty sum C
+        // for j = 3) and adds its elements in the reference's order
+        const int jl = t - 32 * (int)(blockIdx.x % (T / 32));
         double acc = 0.0;
-        if (t < 4) {
-            const int jc = t;
-            // elements e0, e0+dir, ... (len of them); eight operands are loaded
-            // ahead of their adds
-            auto chain = [&](int e0, int dir, int len) {
-                for (int i0 = 0; i0 < len; i0 += 8) {
-                    double v[8];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const int i = i0 + u;
-                        v[u] = (i < len) ? st[4 * (e0 + dir * i) + jc] : 0.0;
-                    }
-#pragma unroll
-                    for (int u = 0; u < 8; ++u)
-                        if (i0 + u < len) acc = dadd(acc, v[u]);
-                }
-            };
-            if (jc < 3) {
+        if (jl >= 0 && jl < 4) {
+            // elements e0, e0+dir, ... (len of them)
+            int e0 = 0, dir = 1, len = 0;
+            if (kind == 2) {
+                len = m;
+            } else if (jl < 3) {
                 if (kind == 0) {
-                    if (!upper) chain(0, 1, pl.idx1 + 1);
-                    else chain(pl.idx1, 1, m - pl.idx1);
-                } else if (kind == 1) {
-                    if (!upper) chain(pl.idx1, -1, pl.idx1 - pl.idx2);
-                    else chain(pl.idx1, 1, pl.idx2 - pl.idx1);
+                    e0 = upper ? pl.idx1 : 0;
+                    len = upper ? m - pl.idx1 : pl.idx1 + 1;
                 } else {
-                    chain(0, 1, m);
+                    e0 = pl.idx1;
+                    dir = upper ? 1 : -1;
+                    len = upper ? pl.idx2 - pl.idx1 : pl.idx1 - pl.idx2;
                 }
-            } else {
-                if (kind == 1) {
-                    if (!upper) chain(0, 1, pl.idx2 + 1);
-                    else chain(pl.idx2, 1, m - pl.idx2);
-                } else if (kind == 2) {
-                    chain(0, 1, m);
-                }
+            } else if (kind == 1) {
+                e0 = upper ? pl.idx2 : 0;
+                len = upper ? m - pl.idx2 : pl.idx2 + 1;
             }
+            // eight operands are loaded ahead of their adds
+            const double* sp = st + 4 * e0 + jl;
+            const int step = 4 * dir, full = len & ~7;
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = full > 0 ? sp[u * step] : 0.0;
+            int i = 0;
+#pragma unroll 1
+            for (; i < full; i += 8) {
+                sp += 8 * step;
+                double nv[8];
+                const bool more = i + 8 < full;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) nv[u] = more ? sp[u * step] : 0.0;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) acc = dadd(acc, v[u]);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) v[u] = nv[u];
+            }
+#pragma unroll 1
+            for (; i < len; ++i, sp += step) acc = dadd(acc, sp[0]);
         }
         __syncthreads();
         // op payloads into the state slots the replay overwrites: op B
         // subtracts the element's powers, op A adds them and subtracts its
         // penalty
-        for (int k = t; k < nops; k += T) {
-            const int d = opdesc[k];
+        for (int k = t; k < ((nops + 7) & ~7); k += T) {
+            const int d = k < nops ? opdesc[k] : -1;
             double* o = st + 4 * (k + 1);
-            if (d < 0) {  // unreachable when the op order is a permutation; keeps reads in bounds
+            if (d < 0) {  // past the last op: no change
                 o[0] = o[1] = o[2] = o[3] = -0.0;
                 continue;
             }
@@ -497,30 +630,25 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, const ThrJob*
         // replay: lane j adds every op's operand to its accumulator j and
         // stores the state after each op, in chunks of eight (the next chunk's
         // operands are loaded before this chunk's states overwrite its slots)
-        if (t < 4) {
-            const int jc = t;
-            st[jc] = acc;
-            constexpr int RC = 8;
-            double a[RC];
+        if (jl >= 0 && jl < 4) {
+            double* sp = st + jl;
+            sp[0] = acc;
+            double a[8];
 #pragma unroll
-            for (int u = 0; u < RC; ++u) a[u] = (u < nops) ? st[4 * (u + 1) + jc] : 0.0;
-            for (int k0 = 0; k0 < nops; k0 += RC) {
-                double na[RC];
+            for (int u = 0; u < 8; ++u) a[u] = nops ? sp[4 * (u + 1)] : 0.0;
+            for (int k0 = 0; k0 < nops; k0 += 8) {
+                double na[8];
+                const bool more = k0 + 8 < nops;
 #pragma unroll
-                for (int u = 0; u < RC; ++u) {
-                    const int k = k0 + RC + u;
-                    na[u] = (k < nops) ? st[4 * (k + 1) + jc] : 0.0;
+                for (int u = 0; u < 8; ++u) na[u] = more ? sp[4 * (u + 9)] : 0.0;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    acc = dadd(acc, a[u]);
+                    sp[4 * (u + 1)] = acc;
                 }
 #pragma unroll
-                for (int u = 0; u < RC; ++u) {
-                    const int k = k0 + u;
-                    if (k < nops) {
-                        acc = dadd(acc, a[u]);
-                        st[4 * (k + 1) + jc] = acc;
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < RC; ++u) a[u] = na[u];
+                for (int u = 0; u < 8; ++u) a[u] = na[u];
+                sp += 32;
             }
         }
         __syncthreads();
@@ -528,24 +656,19 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, const ThrJob*
         // ---- 8. scores and first maximum
         ArgMax best{0.0, INT_MAX, 0};
         int nan0 = 0;
-        // each thread scores a contiguous range of steps, so the number of ops
-        // with step <= i is one binary search followed by a forward walk
-        const int per = (nr + T - 1) / T;
-        const int i_beg = t * per, i_end = min(i_beg + per, nr);
+        // thread t scores steps t, t + T, ...; the number of ops with step <= i
+        // is a binary search from the previous one on
         int lo = 0;
-        if (i_beg < i_end) {
+        for (int i = t; i < nr; i += T) {
             int hi = nops;
-            while (lo < hi) { const int mid = (lo + hi) >> 1; if (opstep[mid] <= i_beg) lo = mid + 1; else hi = mid; }
-        }
-        for (int i = i_beg; i < i_end; ++i) {
-            while (lo < nops && opstep[lo] <= i) ++lo;
+            while (lo < hi) { const int mid = (lo + hi) >> 1; if (opstep[mid] <= i) lo = mid + 1; else hi = mid; }
             const double* sv = st + 4 * lo;
             const double tt = tv[i];
             const double f = f_p(sv[0], sv[1], sv[2], p, tt);
             double h;
             if (kind == 0) h = upper ? f : fabs(f);
             else h = dadd(sv[3], upper ? f : fabs(f));
-            const double lb = dmul(h, (double)gp[i]);
+            const double lb = dmul(h, (double)gp[thr_pad(i)]);
             if (isnan(lb)) {
                 if (i == 0) nan0 = 1;  // findMaxIndex never leaves a NaN at index 0
             } else {
@@ -561,25 +684,32 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, const ThrJob*
     }
 }
 
-size_t threshold_work_bytes(int cap_items, size_t sort_tmp, int m) {
-    const size_t cap = (size_t)cap_items;
-    const size_t runs = thr_runs_bytes(cap_items);
-    const size_t x = ((sort_tmp > cap * 12 + 16 ? sort_tmp : cap * 12 + 16) + 15) & ~size_t(15);
-    const size_t z = thr_z_in_runs(cap_items, m) ? 0 : thr_z_bytes(m);
-    return runs + x + z + 64;
-}
-
 template <int T, int IPT>
-size_t threshold_sort_tmp_bytes() {
-    return sizeof(typename cub::BlockMergeSort<unsigned long long, T, IPT, int>::TempStorage);
+ThrMem threshold_mem(int m, size_t smem_optin) {
+    using Sort = cub::BlockMergeSort<unsigned long long, T, IPT, int>;
+    constexpr int CAP = T * IPT;
+    const size_t r = thr_r_bytes(CAP), z = thr_z_bytes(m), sort = sizeof(typename Sort::TempStorage);
+    auto most = [](size_t a, size_t b) { return a > b ? a : b; };
+    ThrMem mem;
+    mem.gw = false;
+    mem.z_shared = 1;
+    mem.smem = r + most(z, most(sort, thr_bucket_bytes(CAP, thr_buckets(CAP, false)))) + 16;
+    mem.gbytes = 0;
+    if (mem.smem + 8192 <= smem_optin) return mem;
+    const size_t sorts = most(sort, thr_bucket_bytes(CAP, thr_buckets(CAP, true)));
+    mem.gw = true;
+    mem.z_shared = most(z, sorts) + 16 + 8192 <= smem_optin;
+    mem.smem = (mem.z_shared ? most(z, sorts) : sorts) + 16;
+    mem.gbytes = 2 * r + (mem.z_shared ? 0 : z + 16);
+    return mem;
 }
 
 #define FSM_THR_INST(T, IPT)                                                                 \
     template __global__ void k_threshold<T, IPT, false>(Geom, const ThrJob*, unsigned char*,  \
-                                                        long long);                          \
+                                                        long long, int);                     \
     template __global__ void k_threshold<T, IPT, true>(Geom, const ThrJob*, unsigned char*,   \
-                                                       long long);                           \
-    template size_t threshold_sort_tmp_bytes<T, IPT>();
+                                                       long long, int);                      \
+    template ThrMem threshold_mem<T, IPT>(int, size_t);
 FSM_THR_INST(128, 4)
 FSM_THR_INST(256, 4)
 FSM_THR_INST(256, 8)

@@ -132,7 +132,7 @@ __global__ void k_envelope(const double* __restrict__ target, const double* __re
                            double* __restrict__ Ln, double* gwork, long long slot_stride);
 template <int T, int IPT, bool GW>
 __global__ void k_threshold(Geom g, const ThrJob* __restrict__ jobs, unsigned char* gwork,
-                            long long slot_stride);
+                            long long slot_stride, int z_shared);
 template <int T, bool GW>
 __global__ void k_lbip(Geom g, LbJob job, const double2* __restrict__ W, int P, int logP);
 template <int METRIC>
@@ -199,9 +199,15 @@ cudaError_t raise_smem_limit(const void* kernel, int device, size_t bytes);
 
 size_t mvmean_smem_bytes();
 size_t envelope_work_bytes(int m_k);
-size_t threshold_work_bytes(int cap_items, size_t sort_tmp, int m);
+// where a block of k_threshold keeps its working set
+struct ThrMem {
+    bool gw;         // runs and sorted values in global scratch
+    int z_shared;    // the sweep in shared memory
+    size_t smem;     // dynamic shared memory
+    size_t gbytes;   // global scratch per block
+};
 template <int T, int IPT>
-size_t threshold_sort_tmp_bytes();
+ThrMem threshold_mem(int m, size_t smem_optin);
 size_t lbip_smem_bytes(int P, int m_k, int m, int metric);
 int lbip_set_w16();
 // DP block size (2 warps: the per-warp band scratch sets the occupancy)

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from fsmeld_b200.synth import query_from, random_walk
-from tests.test_gpu_parity import _segments, api, bits_equal  # noqa: F401
+from tests.test_gpu_parity import _geom, _segments, api, bits_equal  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -91,3 +91,26 @@ def test_screened_distances(api, oracle, metric, arg, m, w, raw):  # noqa: F811
                 assert list(si) == list(yi) and sc["after_glb"] == yc["after_glb"], cut
     finally:
         oracle.set_normalization("zscore")
+
+
+# k_threshold: every block shape; values spread (bucket sort) and bunched by a
+# spike (merge sort), runs of equal values, NaN in the envelope core
+@pytest.mark.parametrize("m", [8, 32, 100, 200, 300, 800, 1500])
+@pytest.mark.parametrize("metric,arg", [("dtw", 0.0), ("erp", 0.4), ("msm", 0.5), ("lcss", 0.25)])
+def test_threshold_shapes(api, oracle, metric, arg, m):  # noqa: F811
+    w = m // 20
+    mk, kml, _, _ = _geom(m, 1 << 30)
+    t = random_walk(3 * kml + m + 7, [11, m])
+    t[kml + mk // 2] += 1e7                               # second segment: one far value
+    t[2 * kml + mk // 2: 2 * kml + mk // 2 + mk // 4] = 3.0  # third: a flat run
+    t[2 * kml + mk // 3] = np.nan
+    q, _ = query_from(t[:kml], m, np.random.default_rng([12, m]))
+    qn = oracle.normalize_query(q)
+    with api.Engine(t) as e:
+        thr = e.inspect(q, m, metric, w, arg, 4).reshape(-1, 2)
+        un = e.inspect(q, m, metric, w, arg, 2).reshape(-1, mk)
+        ln = e.inspect(q, m, metric, w, arg, 3).reshape(-1, mk)
+    for s in range(len(thr)):
+        tl = oracle.find_t(0, metric, ln[s], qn, m, arg)
+        tu = oracle.find_t(1, metric, un[s], qn, m, arg)
+        assert bits_equal(thr[s], [tl, tu]), (s, thr[s], tl, tu)
