@@ -568,29 +568,15 @@ static inline size_t round256(size_t b) { return (b + 255) & ~size_t(255); }
 
 template <int T, int OPT>
 static int launch_env(fsmeld_ctx* c, const Geom& g, int w, Stats* st) {
-    const size_t work = round256(envelope_work_bytes(g.m_k));
-    double* gwork = nullptr;
-    size_t smem = work;
-    unsigned grid;
+    const size_t smem = envelope_smem_bytes(T * OPT, g.m, w);
     int r;
-    const bool gw_path = work + 8192 > (size_t)c->smem_optin;
-    if (!gw_path) {
-        if ((r = allow_smem(c, k_envelope<T, OPT, false>, smem))) return r;
-        int per_sm = 0;
-        FSM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_envelope<T, OPT, false>, T, smem));
-        grid = (unsigned)std::min<long long>(g.S, (long long)std::max(1, per_sm) * c->sm_count);
-    } else {
-        smem = 0;
-        grid = (unsigned)std::min<long long>(g.S, (long long)c->sm_count * 2);
-        if ((r = bufT(c, "envwork", (work / 8) * grid, &gwork))) return r;
-    }
+    if ((r = allow_smem(c, k_envelope<T, OPT>, smem))) return r;
+    const int tiles = (g.m_k + T * OPT - 1) / (T * OPT);
+    const long long blocks = g.S * tiles;
+    if (blocks > 2147483647LL) return fail(FSMELD_E_UNSUPPORTED, "too many macro segments");
     prof_begin(c, ST_ENV);
-    if (gw_path)
-        k_envelope<T, OPT, true><<<grid, T, smem, c->stream>>>(c->d_target, st->MU, st->SIG, g, w, st->Un, st->Ln,
-                                                               gwork, (long long)(work / 8));
-    else
-        k_envelope<T, OPT, false><<<grid, T, smem, c->stream>>>(c->d_target, st->MU, st->SIG, g, w, st->Un, st->Ln,
-                                                                gwork, (long long)(work / 8));
+    k_envelope<T, OPT><<<(unsigned)blocks, T, smem, c->stream>>>(c->d_target, st->Lraw, st->Uraw, st->MU, st->SIG, g,
+                                                                 w, tiles, st->Un, st->Ln);
     LAUNCH_CHECK(c);
     return FSMELD_OK;
 }
@@ -619,12 +605,12 @@ static int run_env(fsmeld_ctx* c, const Geom& g, int w, Stats* st, const std::st
         LAUNCH_CHECK(c);
     }
     const int mk = g.m_k;
-    if (mk <= 1024) return launch_env<256, 4>(c, g, w, st);
-    if (mk <= 2048) return launch_env<512, 4>(c, g, w, st);
-    if (mk <= 4096) return launch_env<1024, 4>(c, g, w, st);
-    if (mk <= 8192) return launch_env<1024, 8>(c, g, w, st);
-    if (mk <= 16384) return launch_env<1024, 16>(c, g, w, st);
-    return fail(FSMELD_E_UNSUPPORTED, "macro segments longer than 16384 points are not supported");
+    if (mk > 16384) return fail(FSMELD_E_UNSUPPORTED, "macro segments longer than 16384 points are not supported");
+    // tiles of at least twice the window where that leaves enough blocks: the
+    // m - 1 points left of a tile are read again
+    if (mk <= 512 || (g.S * mk < 1024LL * c->sm_count && g.m <= 256)) return launch_env<128, 4>(c, g, w, st);
+    if (g.m <= 512) return launch_env<256, 4>(c, g, w, st);
+    return launch_env<512, 4>(c, g, w, st);
 }
 
 template <int T, int IPT>

@@ -12,16 +12,29 @@
 //  * with a NaN in the window: a NaN blocks every pop behind it, so the
 //    front is the extremum of the points before the first NaN, or NaN when
 //    the window starts with NaN.
-// NaN-free windows by doubling: after pass k, M[i] = min(x[i .. i+2^k-1]);
-// a window [a, b] of length L with 2^k <= L < 2^(k+1) is the union of the
-// runs of length 2^k at its two ends, min(M[a], M[b-2^k+1]), so each output
-// is taken right after the pass of its own level (full windows, and the
-// shorter windows at the segment's edges alike).  Every pass is one min and
-// one max per element with a block barrier, no scans.  Windows that contain
-// a NaN (detected with a NaN prefix count) are evaluated directly from their
-// start.
-#include <cub/block/block_scan.cuh>
-
+//
+// A block takes a tile of consecutive outputs of one segment.  Trailing
+// windows of m points (m >= 17): the tile and its m - 1 points to the left are
+// cut into runs of eight; a thread takes a run and leaves the extremum from
+// the run's start to each point and from each point to its end (van Herk, Gil
+// and Werman's blocks, but eight long whatever m is), and the runs' own
+// extrema are doubled to stretches of 2^L runs, 2^L the largest power that
+// fits between a window's two end runs.  A window is then four reads: its
+// first point's rest of run, its last point's start of run, and two stretches
+// that cover the runs between.  Shorter windows are read point by point.
+// Positions outside [0, n) hold NaN, which no comparison takes, so clipped
+// windows need no case of their own.  Centred windows of the raw points are the
+// min/max of two forward windows of the target (k_fwd_env) that lie inside the
+// segment.  Windows that do hold a NaN (a bit per position, only looked at
+// when the tile has any) end before the first one.
+//
+// What bounds it: shared-memory accesses, about 8 eight-byte ones per point,
+// series and extremum, and three reads of MU and SIG each (one from HBM).
+// Doubling over single points took log2(m) passes of the whole segment with a
+// block barrier each, one block per SM, and global scratch from 8192 points
+// on.  Measured: 2^24 points, m = 256: 1.89 -> 0.67 ms; 2^22 points, m = 64 ..
+// 1024 (19 lengths, most with 8192-point segments): 17.3 -> 3.9 ms; 2^21 points,
+// m = 1850: 0.86 -> 0.12 ms.
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -29,177 +42,202 @@ namespace fsm {
 
 namespace {
 
-// Padded index of the per-segment arrays: one spare slot after every 8
-// elements, so the blocked walks of the scans (thread t on elements
-// [8t, 8t+8)) fall on distinct banks.
-__device__ __forceinline__ int px(int i) { return i + (i >> 3); }
-// slots for indices 0..n (the NaN prefix count reads index n)
-__host__ __device__ inline int env_pad_len(int n) { return n + (n >> 3) + 2; }
+constexpr int kRun = 8;
 
-template <int T>
-struct EnvTemp {
-    typename cub::BlockScan<int, T>::TempStorage ic;
-};
+// one spare slot after every run, so threads on neighbouring runs meet
+// different banks
+__host__ __device__ __forceinline__ int px(int i) { return i + (i >> 3); }
+
+template <bool MAX>
+__device__ __forceinline__ double ext(double a, double b) {  // b unless NaN or worse
+    return MAX ? (b > a ? b : a) : (b < a ? b : a);
+}
+
+// first set bit at or after i and before n, or n
+__device__ __forceinline__ int next_bit(const unsigned* __restrict__ bits, int i, int n) {
+    while (i < n) {
+        const unsigned v = bits[i >> 5] >> (i & 31);
+        if (v) return min(n, i + __ffs(v) - 1);
+        i = (i | 31) + 1;
+    }
+    return n;
+}
 
 struct EnvWork {
-    double *raw, *Pmn, *Pmx, *Smn, *Smx;
-    int* ncnt;  // NaN prefix counts [n + 1]
+    double *P, *S;        // [px(len)] start of run .. point, point .. end of run
+    double *R0, *Ra, *Rb;  // [runs] run extrema; doubled stretches
+    unsigned* bits;        // [len / 32] NaN positions
 };
 
-// Sliding min/max of src[0..n) for nout windows; CENTRED selects
-// [o-w, o+w] (lemire) versus the trailing [o-m+1, o] (min_max_window), both
-// clipped to [0, n-1].  Work arrays: raw copy, two ping-pong pairs (Pmn/Pmx,
-// Smn/Smx) for the doubling passes, NaN prefix counts.
-template <int T, int OPT, bool CENTRED>
-__device__ void minmax_phase(const double* __restrict__ src, int n, int par, int nout,
-                             const EnvWork& wk, EnvTemp<T>& tmp, double (&omn)[OPT],
-                             double (&omx)[OPT]) {
-    const int t = threadIdx.x;
+// Extrema of src over [o - m + 1, o] for the tile's outputs o0 + t + k T,
+// clipped to [0, n).  Local position l is o0 - m + 1 + l.
+template <int T, int OPT, bool MAX>
+__device__ void trailing(const double* __restrict__ src, int n, int m, int o0, int nout, const EnvWork& wk,
+                         double (&out)[OPT]) {
+    constexpr double kNone = MAX ? -INFINITY : INFINITY;
+    const int t = threadIdx.x, b0 = o0 - (m - 1);
+    const int len = nout + m - 1, runs = (len + kRun - 1) / kRun, plen = (runs * kRun + 31) & ~31;
     int local_nan = 0;
-    for (int i = t; i < n; i += T) {
-        const double v = src[i];
-        wk.raw[px(i)] = v;
-        wk.Pmn[px(i)] = v;
-        wk.Pmx[px(i)] = v;
-        local_nan |= isnan(v) ? 1 : 0;
+    for (int l = t; l < plen; l += T) {
+        const int p = b0 + l;
+        const bool in = l < len && p >= 0 && p < n;
+        const double v = in ? src[p] : dnan();
+        if (l < runs * kRun) wk.P[px(l)] = v;
+        const unsigned bad = __ballot_sync(0xffffffffu, in && isnan(v));
+        if ((l & 31) == 0) wk.bits[l >> 5] = bad;
+        local_nan |= bad != 0u;
     }
     const int any_nan = __syncthreads_or(local_nan);
-    if (any_nan) {
-        const int c = (n + T - 1) / T;
-        const int lo = t * c, hi = min(n, lo + c);
-        int cnt = 0;
-        for (int i = lo; i < hi; ++i) cnt += isnan(wk.raw[px(i)]) ? 1 : 0;
-        int off;
-        cub::BlockScan<int, T>(tmp.ic).ExclusiveSum(cnt, off);
-        for (int i = lo; i < hi; ++i) {
-            wk.ncnt[px(i)] = off;
-            off += isnan(wk.raw[px(i)]) ? 1 : 0;
-        }
-        if (hi == n && lo < hi) wk.ncnt[px(n)] = off;  // the chunk holding n-1 closes the count
-        __syncthreads();
-    }
-    // each output's window [ws, we] (recomputed where needed, to keep the
-    // per-thread state to the outputs themselves)
-    auto window = [&](int o, int& ws, int& we) {
-        if (CENTRED) { ws = max(0, o - par); we = min(n - 1, o + par); }
-        else { ws = max(0, o - par + 1); we = min(o, n - 1); }
-    };
-    auto has_nan = [&](int ws, int we) {
-        return any_nan && (wk.ncnt[px(we + 1)] - wk.ncnt[px(ws)] > 0);
-    };
+    const bool by_runs = m > 2 * kRun;
+    int L = 0;
+    const double* Rt = wk.R0;
+    if (by_runs) {
+        for (int r = t; r < runs; r += T) {
+            double v[kRun];
 #pragma unroll
-    for (int k = 0; k < OPT; ++k) { omn[k] = 0.0; omx[k] = 0.0; }
-    // the deepest level any window needs: the full window length, clipped to n
-    const int maxlen = CENTRED ? min(n, 2 * par + 1) : min(n, par);
-    const int levels = 31 - __clz(max(1, maxlen));
-    double* An = wk.Pmn;
-    double* Ax = wk.Pmx;
-    double* Bn = wk.Smn;
-    double* Bx = wk.Smx;
-    for (int lv = 0; lv <= levels; ++lv) {
-        if (lv > 0) {
-            const int s = 1 << (lv - 1);
-            for (int i = t; i < n; i += T) {
-                const bool in = i + s < n;
-                const double a0 = An[px(i)], x0 = Ax[px(i)];
-                const double a1 = in ? An[px(i + s)] : a0, x1 = in ? Ax[px(i + s)] : x0;
-                Bn[px(i)] = (a1 < a0) ? a1 : a0;
-                Bx[px(i)] = (x1 > x0) ? x1 : x0;
+            for (int u = 0; u < kRun; ++u) v[u] = wk.P[px(r * kRun) + u];
+            double e = kNone;
+#pragma unroll
+            for (int u = kRun - 1; u >= 0; --u) {
+                e = ext<MAX>(e, v[u]);
+                wk.S[px(r * kRun) + u] = e;
             }
-            __syncthreads();
-            double* tn = An; An = Bn; Bn = tn;
-            double* tx = Ax; Ax = Bx; Bx = tx;
-        }
-        // outputs whose window length has this level: the two end runs
+            wk.R0[r] = e;
+            e = kNone;
 #pragma unroll
-        for (int k = 0; k < OPT; ++k) {
-            const int o = t + k * T;
-            if (o >= nout) continue;
-            int ws, we;
-            window(o, ws, we);
-            if (31 - __clz(we - ws + 1) != lv || has_nan(ws, we)) continue;
-            const int b2 = we - (1 << lv) + 1;
-            const double a0 = An[px(ws)], a1 = An[px(b2)];
-            const double x0 = Ax[px(ws)], x1 = Ax[px(b2)];
-            omn[k] = (a1 < a0) ? a1 : a0;
-            omx[k] = (x1 > x0) ? x1 : x0;
+            for (int u = 0; u < kRun; ++u) {
+                e = ext<MAX>(e, v[u]);
+                wk.P[px(r * kRun) + u] = e;
+            }
+        }
+        __syncthreads();
+        // whole runs between a window's end runs: (m-1)/8 - 1 or one more
+        L = 31 - __clz((m - 1) / kRun - 1);
+        double* w0 = wk.Ra;
+        double* w1 = wk.Rb;
+        for (int lv = 1; lv <= L; ++lv) {
+            const int s = 1 << (lv - 1);
+            for (int r = t; r < runs; r += T) w0[r] = r + s < runs ? ext<MAX>(Rt[r], Rt[r + s]) : Rt[r];
+            __syncthreads();
+            Rt = w0;
+            double* x = w0; w0 = w1; w1 = x;
         }
     }
-    // windows holding a NaN: the deque's front from the window's start
 #pragma unroll
     for (int k = 0; k < OPT; ++k) {
-        const int o = t + k * T;
-        if (!any_nan || o >= nout) continue;
-        int ws, we;
-        window(o, ws, we);
-        if (!has_nan(ws, we)) continue;
-        double a = wk.raw[px(ws)];
-        double vmn = a, vmx = a;
-        if (!isnan(a)) {
-            for (int i = ws + 1; i <= we; ++i) {
-                const double v = wk.raw[px(i)];
-                if (isnan(v)) break;
-                vmn = (v <= vmn) ? v : vmn;
-                vmx = (v >= vmx) ? v : vmx;
+        const int a = t + k * T;
+        out[k] = kNone;
+        if (a >= nout) continue;
+        int b = a + m - 1;
+        if (any_nan) {
+            const int first = max(a, -b0), last = min(b, n - 1 - b0);  // inside [0, n)
+            const int f = next_bit(wk.bits, first, last + 1);
+            if (f <= last) {  // only the points before the first NaN
+                double e = kNone;
+                if (f == first) {
+                    e = dnan();
+                } else if (!by_runs || (f - 1) / kRun == first / kRun) {
+                    for (int l = first; l < f; ++l) e = ext<MAX>(e, src[b0 + l]);
+                } else {
+                    e = ext<MAX>(wk.S[px(first)], wk.P[px(f - 1)]);
+                    for (int r = first / kRun + 1; r < (f - 1) / kRun; ++r) e = ext<MAX>(e, wk.R0[r]);
+                }
+                out[k] = e;
+                continue;
             }
         }
-        omn[k] = vmn;
-        omx[k] = vmx;
+        double e;
+        if (by_runs) {
+            const int ra = a / kRun + 1, rb = b / kRun - (1 << L);
+            e = ext<MAX>(ext<MAX>(wk.S[px(a)], wk.P[px(b)]), ext<MAX>(Rt[ra], Rt[rb]));
+        } else {
+            e = kNone;
+            for (; b >= a; --b) e = ext<MAX>(e, wk.P[px(b)]);
+        }
+        out[k] = e;
     }
     __syncthreads();
 }
 
 }  // namespace
 
-template <int T, int OPT, bool GW>
-__global__ void __launch_bounds__(T) k_envelope(const double* __restrict__ target,
-                                                const double* __restrict__ MU,
-                                                const double* __restrict__ SIG, Geom g, int w,
-                                                double* __restrict__ Un, double* __restrict__ Ln,
-                                                double* gwork, long long slot_stride) {
+template <int T, int OPT>
+__global__ void __launch_bounds__(T) k_envelope(const double* __restrict__ target, const double* __restrict__ Lraw,
+                                                const double* __restrict__ Uraw, const double* __restrict__ MU,
+                                                const double* __restrict__ SIG, Geom g, int w, int tiles,
+                                                double* __restrict__ Un, double* __restrict__ Ln) {
     extern __shared__ __align__(16) unsigned char env_smem[];
-    __shared__ EnvTemp<T> tmp;
-    const int mk = g.m_k, kml = g.kml, m = g.m;
-    double* base = GW ? gwork + (long long)blockIdx.x * slot_stride : (double*)env_smem;
+    constexpr int O = T * OPT;
+    const int mk = g.m_k, kml = g.kml, m = g.m, t = threadIdx.x;
+    const int runs = (O + m - 1 + kRun - 1) / kRun;
     EnvWork wk;
-    const int pk = env_pad_len(mk);  // padded length of each array
-    wk.raw = base;
-    wk.Pmn = base + pk;
-    wk.Pmx = base + 2 * pk;
-    wk.Smn = base + 3 * pk;
-    wk.Smx = base + 4 * pk;
-    wk.ncnt = (int*)(base + 5 * pk);
-    for (long long s = blockIdx.x; s < g.S; s += gridDim.x) {
-        double simn[OPT], simx[OPT], mumn[OPT], mumx[OPT], lmn[OPT], lmx[OPT];
-        minmax_phase<T, OPT, false>(SIG + s * kml, kml, m, mk, wk, tmp, simn, simx);
-        minmax_phase<T, OPT, false>(MU + s * kml, kml, m, mk, wk, tmp, mumn, mumx);
-        minmax_phase<T, OPT, true>(target + g.off(s), mk, w, mk, wk, tmp, lmn, lmx);
+    wk.P = (double*)env_smem;
+    wk.S = wk.P + px(runs * kRun);
+    wk.R0 = wk.S + px(runs * kRun);
+    wk.Ra = wk.R0 + runs;
+    wk.Rb = wk.Ra + runs;
+    wk.bits = (unsigned*)(wk.Rb + runs);
+    const long long s = blockIdx.x / tiles;
+    const int o0 = (int)(blockIdx.x % tiles) * O, nout = min(O, mk - o0);
+    double simn[OPT], simx[OPT], mumn[OPT], mumx[OPT];
+    trailing<T, OPT, false>(SIG + s * kml, kml, m, o0, nout, wk, simn);
+    trailing<T, OPT, true>(SIG + s * kml, kml, m, o0, nout, wk, simx);
+    trailing<T, OPT, false>(MU + s * kml, kml, m, o0, nout, wk, mumn);
+    trailing<T, OPT, true>(MU + s * kml, kml, m, o0, nout, wk, mumx);
+    // centred windows of the raw segment: NaN positions o0 - w + l
+    const long long off = g.off(s);
+    const double* __restrict__ seg = target + off;
+    const int c0 = o0 - w, clen = (nout + 2 * w + 31) & ~31;
+    int local_nan = 0;
+    for (int l = t; l < clen; l += T) {
+        const int p = c0 + l;
+        const unsigned bad = __ballot_sync(0xffffffffu, p >= 0 && p < mk && isnan(seg[min(max(p, 0), mk - 1)]));
+        if ((l & 31) == 0) wk.bits[l >> 5] = bad;
+        local_nan |= bad != 0u;
+    }
+    const int any_nan = __syncthreads_or(local_nan);
+    const double* __restrict__ lf = Lraw + off;
+    const double* __restrict__ uf = Uraw + off;
 #pragma unroll
-        for (int k = 0; k < OPT; ++k) {
-            const int o = threadIdx.x + k * T;
-            if (o < mk) {
-                const double nu = dsub(lmx[k], mumn[k]);
-                const double un = (nu >= 0) ? ddiv(nu, simn[k]) : ddiv(nu, simx[k]);
-                const double nl = dsub(lmn[k], mumx[k]);
-                const double ln = (nl <= 0) ? ddiv(nl, simn[k]) : ddiv(nl, simx[k]);
-                Un[s * mk + o] = un;
-                Ln[s * mk + o] = ln;
+    for (int k = 0; k < OPT; ++k) {
+        const int x = t + k * T, o = o0 + x;
+        if (x >= nout) continue;
+        const int ws = max(0, o - w), we = min(mk - 1, o + w);
+        const int p1 = we - w;  // the forward windows at ws and we - w cover [ws, we]
+        double lmn = lf[ws], lmx = uf[ws];
+        lmn = ext<false>(lmn, lf[p1]);
+        lmx = ext<true>(lmx, uf[p1]);
+        if (any_nan) {
+            const int f = next_bit(wk.bits, ws - c0, we - c0 + 1) + c0;
+            if (f <= we) {
+                lmn = f == ws ? dnan() : INFINITY;
+                lmx = f == ws ? dnan() : -INFINITY;
+                for (int p = ws; p < f; ++p) {
+                    lmn = ext<false>(lmn, seg[p]);
+                    lmx = ext<true>(lmx, seg[p]);
+                }
             }
         }
+        const double nu = dsub(lmx, mumn[k]);
+        const double un = (nu >= 0) ? ddiv(nu, simn[k]) : ddiv(nu, simx[k]);
+        const double nl = dsub(lmn, mumx[k]);
+        const double ln = (nl <= 0) ? ddiv(nl, simn[k]) : ddiv(nl, simx[k]);
+        Un[s * mk + o] = un;
+        Ln[s * mk + o] = ln;
     }
 }
 
-size_t envelope_work_bytes(int m_k) { return (size_t)env_pad_len(m_k) * (5 * sizeof(double) + sizeof(int)) + 16; }
+size_t envelope_smem_bytes(int tile, int m, int w) {
+    const int runs = (tile + m - 1 + kRun - 1) / kRun;
+    const size_t bits = (size_t)(runs * kRun > tile + 2 * w ? runs * kRun : tile + 2 * w) / 32 + 2;
+    return (2 * (size_t)px(runs * kRun) + 3 * (size_t)runs) * 8 + bits * 4;
+}
 
-#define FSM_ENV_INST(T, OPT)                                                                          \
-    template __global__ void k_envelope<T, OPT, false>(const double*, const double*, const double*,  \
-                                                       Geom, int, double*, double*, double*, long long); \
-    template __global__ void k_envelope<T, OPT, true>(const double*, const double*, const double*,   \
-                                                      Geom, int, double*, double*, double*, long long);
+#define FSM_ENV_INST(T, OPT)                                                                                    \
+    template __global__ void k_envelope<T, OPT>(const double*, const double*, const double*, const double*,    \
+                                                const double*, Geom, int, int, double*, double*);
+FSM_ENV_INST(128, 4)
 FSM_ENV_INST(256, 4)
 FSM_ENV_INST(512, 4)
-FSM_ENV_INST(1024, 4)
-FSM_ENV_INST(1024, 8)
-FSM_ENV_INST(1024, 16)
 
 }  // namespace fsm

@@ -126,10 +126,12 @@ constexpr int kMvmeanThreads = 288;
 __global__ void k_mvmean(const double* __restrict__ target, Geom g, double* __restrict__ mu,
                          double* __restrict__ sig, int seg);
 int mvmean_segments(long long S, int sm_count);
-template <int T, int OPT, bool GW>
-__global__ void k_envelope(const double* __restrict__ target, const double* __restrict__ MU,
-                           const double* __restrict__ SIG, Geom g, int w, double* __restrict__ Un,
-                           double* __restrict__ Ln, double* gwork, long long slot_stride);
+// one block per tile of T * OPT outputs of a segment
+template <int T, int OPT>
+__global__ void k_envelope(const double* __restrict__ target, const double* __restrict__ Lraw,
+                           const double* __restrict__ Uraw, const double* __restrict__ MU,
+                           const double* __restrict__ SIG, Geom g, int w, int tiles, double* __restrict__ Un,
+                           double* __restrict__ Ln);
 template <int T, int IPT, bool GW>
 __global__ void k_threshold(Geom g, const ThrJob* __restrict__ jobs, unsigned char* gwork,
                             long long slot_stride, int z_shared);
@@ -198,7 +200,7 @@ __global__ void k_seed(Geom g, const double* __restrict__ z, const double* __res
 cudaError_t raise_smem_limit(const void* kernel, int device, size_t bytes);
 
 size_t mvmean_smem_bytes();
-size_t envelope_work_bytes(int m_k);
+size_t envelope_smem_bytes(int tile, int m, int w);
 // where a block of k_threshold keeps its working set
 struct ThrMem {
     bool gw;         // runs and sorted values in global scratch

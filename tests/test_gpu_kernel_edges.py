@@ -114,3 +114,27 @@ def test_threshold_shapes(api, oracle, metric, arg, m):  # noqa: F811
         tl = oracle.find_t(0, metric, ln[s], qn, m, arg)
         tu = oracle.find_t(1, metric, un[s], qn, m, arg)
         assert bits_equal(thr[s], [tl, tu]), (s, thr[s], tl, tu)
+
+
+# k_envelope: windows read point by point (m <= 16) and by runs of eight, tiles
+# of 512, 1024 and 2048 outputs with a remainder, clipped segments, NaN at the
+# start, inside and at the end of windows and runs
+@pytest.mark.parametrize("n,m,w", [(4000, 2, 0), (4000, 9, 8), (5000, 16, 3), (5001, 17, 1), (5002, 24, 5),
+                                   (5003, 25, 24), (20_000, 100, 9), (9000, 257, 40), (90_000, 600, 30),
+                                   (4300, 1500, 200), (16_001, 8000, 50)])
+def test_envelope_tiles(api, oracle, n, m, w):  # noqa: F811
+    for bad in ([], [7, 8, 1023, 1024 + m, n // 2, n // 2 + 1, n - 1]):
+        t = _target(n, [13, m], bad)
+        q = random_walk(m, 14)
+        segs, mk, kml = _segments(t, m)
+        with api.Engine(t) as e:
+            un = e.inspect(q, m, "dtw", w, 0.0, 2).reshape(-1, mk)
+            ln = e.inspect(q, m, "dtw", w, 0.0, 3).reshape(-1, mk)
+        for s, ts in enumerate(segs):
+            omu, osg = oracle.mvmean(ts, m)
+            mn, mx = oracle.min_max_window(omu, mk, m)
+            smn, smx = oracle.min_max_window(osg, mk, m)
+            L, U = oracle.lemire(ts, w)
+            oun, oln = oracle.normalized(U, L, mx, mn, smx, smn)
+            assert bits_equal(un[s], oun), (s, len(bad))
+            assert bits_equal(ln[s], oln), (s, len(bad))
