@@ -858,7 +858,8 @@ static int run_dp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
     const bool gw_path = smem > (size_t)c->smem_optin - 4096;
     // wide bands (and FSMELD_DP_FORM=wave): one warp per candidate, band in registers
     int form = c->dp_form;
-    if (screened) form = 2;  // few candidates: a warp each
+    // few candidates (what the screen leaves, the top-k seeds): a warp each
+    if (c->dp_form == 0 && (screened || (job.list && expected <= 32LL * c->sm_count))) form = 2;
     else if (form == 0) form = tuned(c, job.list ? 0 : 3, job.q.metric, g.m_k, w);
     const void* wk = form == 1 ? nullptr : dpw_kernel(job.q.metric, w);
     const size_t wsm = dpw_smem_bytes(job.q.m, kDpwThreads / 32);

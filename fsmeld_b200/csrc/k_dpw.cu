@@ -19,6 +19,12 @@
 //            the next chunk);  diag = own O (old value)
 //
 // so one shuffle per chunk and step carries the only cross-lane operand.
+//
+// What bounds it: the latency of a step (shuffle, two minima, an add) and the
+// instructions of its K chunks, one warp against a full-length candidate of
+// 2m steps; the lists it gets are short.  Away from the matrix's corners a pair
+// of steps runs without index arithmetic or tests; blocks of one warp spread
+// a short list over the SMs.
 // Cells outside the band or outside the matrix hold the reference's
 // out-of-band value (MAX_VAL = 1e18, 0 for LCSS), which is exactly what the
 // reference reads for such neighbours; row 0 and column 0 of ERP, EDR and
@@ -110,6 +116,37 @@ __device__ __forceinline__ double wave_cell(int i, int j, double up, double left
         const double c1 = dadd(diag, fabs(dsub(X[i], Y[j])));
         const double c2 = dadd(up, wmsm_c(X[i], X[i - 1], Y[j], arg));
         const double c3 = dadd(left, wmsm_c(Y[j], X[i], Y[j - 1], arg));
+        return wmin(wmin(c1, c2), c3);
+    }
+}
+
+// One cell away from the matrix's first row and column: x, y the cell's points,
+// xp, yp the ones before them (MSM).  Everything is computed, then selected.
+template <int METRIC>
+__device__ __forceinline__ double inner_cell(double up, double left, double diag, double x, double xp, double y,
+                                             double yp, double arg) {
+    if (METRIC == DTW) {
+        return dadd(wmin(wmin(up, diag), left), dsq(x, y));
+    } else if (METRIC == LCSS) {
+        const double hit1 = dadd(diag, 1.0);
+        const double best = (fabs(dsub(x, y)) <= arg) ? hit1 : diag;
+        return wmax(wmax(best, up), left);
+    } else if (METRIC == ERP) {
+        const double match = dadd(diag, dsq(x, y));
+        const double ins = dadd(left, dsq(y, arg));
+        const double del = dadd(up, dsq(x, arg));
+        return wmin(wmin(match, del), ins);
+    } else if (METRIC == EDR) {
+        const double sub = (fabs(dsub(x, y)) <= arg) ? 0.0 : 1.0;
+        return wmin(wmin(dadd(up, 1.0), dadd(diag, sub)), dadd(left, 1.0));
+    } else {  // MSM
+        const double axy = fabs(dsub(x, y));
+        const double c1 = dadd(diag, axy);
+        const bool xle = x <= y, yle = y <= x;
+        const bool b2 = (xp <= x && xle) || (yle && x <= xp);
+        const double c2 = dadd(up, b2 ? arg : dadd(arg, wmin(fabs(dsub(x, xp)), axy)));
+        const bool b3 = (xle && y <= yp) || (yp <= y && yle);
+        const double c3 = dadd(left, b3 ? arg : dadd(arg, wmin(axy, fabs(dsub(y, yp)))));
         return wmin(wmin(c1, c2), c3);
     }
 }
@@ -216,58 +253,137 @@ __global__ void __launch_bounds__(kDpwThreads) k_dpw(Geom g, DpJob job) {
         }
         bool stop = false;
         int a = 0;
-        for (; a <= 2 * R; ++a) {
-            if (((a + w) & 1) == 0) {
-                double rot[K];
+        // one anti-diagonal with every test (near the matrix's corners)
+        auto even_step = [&](int a) {
+            double rot[K];
+#pragma unroll
+            for (int c = 0; c < K; ++c) rot[c] = __shfl_sync(0xffffffffu, O[c], (lane + 31) & 31);
+#pragma unroll
+            for (int c = 0; c < K; ++c) {
+                const int d = 64 * c + 2 * lane;
+                const double left = (lane == 0) ? (c == 0 ? SENT : rot[c > 0 ? c - 1 : 0]) : rot[c];
+                const int i = (a - d + w) >> 1, j = i + d - w;
+                const bool ok = d < W2 && i >= 0 && j >= 0 && i <= R && j <= R;
+                const int ic = ok ? i : 0, jc = ok ? j : 0;
+                const double v = wave_cell<METRIC>(ic, jc, O[c], left, E[c], X, Y, arg);
+                E[c] = ok ? v : SENT;
+            }
+        };
+        auto odd_step = [&](int a) {
+            double rot[K];
+#pragma unroll
+            for (int c = 0; c < K; ++c) rot[c] = __shfl_sync(0xffffffffu, E[c], (lane + 1) & 31);
+#pragma unroll
+            for (int c = 0; c < K; ++c) {
+                const int d = 64 * c + 2 * lane + 1;
+                const double up = (lane == 31) ? (c == K - 1 ? SENT : rot[c < K - 1 ? c + 1 : c]) : rot[c];
+                const int i = (a - d + w) >> 1, j = i + d - w;
+                const bool ok = d < W2 && i >= 0 && j >= 0 && i <= R && j <= R;
+                const int ic = ok ? i : 0, jc = ok ? j : 0;
+                const double v = wave_cell<METRIC>(ic, jc, up, E[c], O[c], X, Y, arg);
+                O[c] = ok ? v : SENT;
+            }
+        };
+        auto abandon = [&](int a) {
+            // bound over anti-diagonals a-1 and a
+            double ext = SENT;
+            if (METRIC == LCSS) {
+#pragma unroll
+                for (int c = 0; c < K; ++c) ext = wmax(ext, wmax(E[c], O[c]));
+                for (int o = 16; o; o >>= 1) ext = wmax(ext, __shfl_xor_sync(0xffffffffu, ext, o));
+                const int imin = max(0, (a - 1 - w) >> 1);  // no row of the pair lies above imin
+                double rest = (double)(R - imin);
+                if (cascade) rest = fmin(rest, S4[(imin + 1) >> 2]);
+                if (dadd(ext, rest) < lcss_lim) stop = true;
+            } else {
+#pragma unroll
+                for (int c = 0; c < K; ++c) ext = wmin(ext, wmin(E[c], O[c]));
+                for (int o = 16; o; o >>= 1) ext = wmin(ext, __shfl_xor_sync(0xffffffffu, ext, o));
+                const int imax = min(R, (a + w) >> 1);  // no row of the pair lies below imax
+                const double rest = cascade ? S4[min(nblk, (imax + 4) >> 2)] : 0.0;
+                const double bnd = dadd(ext, rest);
+                if (METRIC == DTW || METRIC == ERP) stop = neg_lim || bnd > cut_sq;
+                else stop = bnd > cut_s;
+            }
+        };
+        auto edge_steps = [&](int to) {  // anti-diagonals a .. to - 1
+            for (; a < to && !stop; ++a) {
+                if (((a + w) & 1) == 0) even_step(a);
+                else odd_step(a);
+                if ((a & 7) == 7 && a < 2 * R) abandon(a);
+            }
+            if (stop) --a;
+        };
+        // Interior: with h = (a + w) / 2 rounded down, the even step at h and
+        // the odd step at h read query point i = h - lane - 32 c and candidate
+        // points j = h + lane + 32 c - w and j + 1, and the next h one point
+        // further each, so a pair of steps loads one new point per side and
+        // chunk.  All cells of the band lie inside the matrix, off its first
+        // row and column, for w < h < R.
+        constexpr int SH = ONE_BASED ? 1 : 0;  // grid (i, j) reads points i - 1, j - 1
+        const int hlo = w + 1, hhi = R;        // interior: hlo <= h < hhi
+        edge_steps(hhi > hlo ? 2 * hlo - w : 2 * R + 1);
+        if (!stop && hhi > hlo) {
+            // lanes past the band in the last chunk read the band's last points
+            const int dlast = 64 * (K - 1) + 2 * lane;
+            const bool oke = dlast < W2, oko = dlast + 1 < W2;
+            const int ll = oke ? lane : w - 32 * (K - 1);
+            double xq[K], yq[K], xp[K], yp[K];
+            const double* px = X + (hlo - SH);
+            const double* py = Y + (hlo - w - SH);
+#pragma unroll
+            for (int c = 0; c < K; ++c) {
+                const int o = (c == K - 1 ? ll : lane) + 32 * c;
+                yq[c] = py[o];
+                xp[c] = METRIC == MSM ? px[-o - 1] : 0.0;
+                yp[c] = METRIC == MSM ? py[o - 1] : 0.0;
+            }
+            for (int h = hlo; h < hhi; ++h) {
+                a = 2 * h - w;
+                double rot[K], yn[K];
+#pragma unroll
+                for (int c = 0; c < K; ++c) {
+                    const int o = (c == K - 1 ? ll : lane) + 32 * c;
+                    xq[c] = px[-o];
+                    yn[c] = py[o + 1];
+                }
 #pragma unroll
                 for (int c = 0; c < K; ++c) rot[c] = __shfl_sync(0xffffffffu, O[c], (lane + 31) & 31);
 #pragma unroll
                 for (int c = 0; c < K; ++c) {
-                    const int d = 64 * c + 2 * lane;
                     const double left = (lane == 0) ? (c == 0 ? SENT : rot[c > 0 ? c - 1 : 0]) : rot[c];
-                    const int i = (a - d + w) >> 1, j = i + d - w;
-                    const bool ok = d < W2 && i >= 0 && j >= 0 && i <= R && j <= R;
-                    const int ic = ok ? i : 0, jc = ok ? j : 0;
-                    const double v = wave_cell<METRIC>(ic, jc, O[c], left, E[c], X, Y, arg);
-                    E[c] = ok ? v : SENT;
+                    const double v = inner_cell<METRIC>(O[c], left, E[c], xq[c], xp[c], yq[c], yp[c], arg);
+                    E[c] = (c < K - 1 || oke) ? v : SENT;
                 }
-            } else {
-                double rot[K];
+                if (((a & 7) == 7)) {
+                    abandon(a);
+                    if (stop) break;
+                }
+                ++a;
 #pragma unroll
                 for (int c = 0; c < K; ++c) rot[c] = __shfl_sync(0xffffffffu, E[c], (lane + 1) & 31);
 #pragma unroll
                 for (int c = 0; c < K; ++c) {
-                    const int d = 64 * c + 2 * lane + 1;
                     const double up = (lane == 31) ? (c == K - 1 ? SENT : rot[c < K - 1 ? c + 1 : c]) : rot[c];
-                    const int i = (a - d + w) >> 1, j = i + d - w;
-                    const bool ok = d < W2 && i >= 0 && j >= 0 && i <= R && j <= R;
-                    const int ic = ok ? i : 0, jc = ok ? j : 0;
-                    const double v = wave_cell<METRIC>(ic, jc, up, E[c], O[c], X, Y, arg);
-                    O[c] = ok ? v : SENT;
+                    const double v = inner_cell<METRIC>(up, E[c], O[c], xq[c], xp[c], yn[c], yq[c], arg);
+                    O[c] = (c < K - 1 || oko) ? v : SENT;
                 }
+                if (((a & 7) == 7)) {
+                    abandon(a);
+                    if (stop) break;
+                }
+#pragma unroll
+                for (int c = 0; c < K; ++c) {
+                    yp[c] = yq[c];
+                    yq[c] = yn[c];
+                    xp[c] = xq[c];
+                }
+                ++px;
+                ++py;
             }
-            if ((a & 7) == 7 && a < 2 * R) {
-                // bound over anti-diagonals a-1 and a
-                double ext = SENT;
-                if (METRIC == LCSS) {
-#pragma unroll
-                    for (int c = 0; c < K; ++c) ext = wmax(ext, wmax(E[c], O[c]));
-                    for (int o = 16; o; o >>= 1) ext = wmax(ext, __shfl_xor_sync(0xffffffffu, ext, o));
-                    const int imin = max(0, (a - 1 - w) >> 1);  // no row of the pair lies above imin
-                    double rest = (double)(R - imin);
-                    if (cascade) rest = fmin(rest, S4[(imin + 1) >> 2]);
-                    if (dadd(ext, rest) < lcss_lim) stop = true;
-                } else {
-#pragma unroll
-                    for (int c = 0; c < K; ++c) ext = wmin(ext, wmin(E[c], O[c]));
-                    for (int o = 16; o; o >>= 1) ext = wmin(ext, __shfl_xor_sync(0xffffffffu, ext, o));
-                    const int imax = min(R, (a + w) >> 1);  // no row of the pair lies below imax
-                    const double rest = cascade ? S4[min(nblk, (imax + 4) >> 2)] : 0.0;
-                    const double bnd = dadd(ext, rest);
-                    if (METRIC == DTW || METRIC == ERP) stop = neg_lim || bnd > cut_sq;
-                    else stop = bnd > cut_s;
-                }
-                if (stop) break;
+            if (!stop) {
+                a = 2 * hhi - w;
+                edge_steps(2 * R + 1);
             }
         }
         if (stop) {

@@ -156,7 +156,7 @@ const void* dp_kernel(int metric, bool gw);
 // in registers (K chunks of 64 band offsets per warp, 2w+1 <= 64 K)
 template <int METRIC, int K>
 __global__ void k_dpw(Geom g, DpJob job);
-constexpr int kDpwThreads = 128;
+constexpr int kDpwThreads = 32;  // one warp: a short list spreads over the SMs
 constexpr int kDpwMaxChunks = 8;  // w <= 255
 // the wavefront kernel for (metric, w), or null when the band is too wide
 const void* dpw_kernel(int metric, int w);
