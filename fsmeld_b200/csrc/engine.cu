@@ -659,13 +659,58 @@ static int run_thr(fsmeld_ctx* c, const Geom& g, const std::vector<ThrJob>& jobs
     return FSMELD_OK;
 }
 
+// The largest inner product zz whose bound passes the prune test at the
+// cutoff (trans and fsmeld_lbip_exceeds_cutoff, the operations of common.cuh
+// and k_lbip): both are monotone, so it is bisected over the doubles.
+static double lbip_keep_max(const QueryDev& q) {
+    auto keeps = [&](double zz) {
+        double z = zz;
+        if (q.metric == DTW || q.metric == ERP) z = std::sqrt(zz > 0.0 ? zz : 0.0);
+        else if (q.metric == LCSS) z = zz / (double)q.m;
+        if (!std::isfinite(z) || !(z > q.cutoff + kLbTol)) return true;
+        if (q.metric == DTW || q.metric == ERP) {
+            const double limit = q.cutoff + kLbTol;
+            return !(z > std::sqrt(limit * limit + kLbTol));
+        }
+        return false;
+    };
+    long long lo = order_int(0.0), hi = order_int(DBL_MAX);
+    if (keeps(DBL_MAX)) return DBL_MAX;
+    while (hi - lo > 1) {  // keeps(lo), not keeps(hi)
+        const long long mid = lo + (hi - lo) / 2;
+        if (keeps(from_order_int(mid))) lo = mid;
+        else hi = mid;
+    }
+    return from_order_int(lo);
+}
+
+// EDR and LCSS by popcounts; the others by the changes of their masks unless
+// the band is so narrow (100 (w+1) < m) that there may be too many of them
+template <bool POPC>
+static int run_lbip_runs(fsmeld_ctx* c, const Geom& g, const LbJob& job) {
+    const size_t smem = lbip_runs_smem_bytes(g.m_k, g.kml, g.m, POPC);
+    int r;
+    if ((r = allow_smem(c, k_lbip_runs<256, POPC>, smem))) return r;
+    int per_sm = 0;
+    FSM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lbip_runs<256, POPC>, 256, smem));
+    const unsigned grid = (unsigned)std::min<long long>(g.S, (long long)std::max(1, per_sm) * c->sm_count);
+    prof_begin(c, ST_LBIP);
+    k_lbip_runs<256, POPC><<<grid, 256, smem, c->stream>>>(g, job, job.surv ? lbip_keep_max(job.q) : 0.0);
+    LAUNCH_CHECK(c);
+    return FSMELD_OK;
+}
+
 static int run_lbip(fsmeld_ctx* c, const Geom& g, LbJob job) {
+    if (job.q.metric == EDR || job.q.metric == LCSS) return run_lbip_runs<true>(c, g, job);
+    if (100LL * (job.q.w + 1) >= g.m && g.m_k <= 65536 &&
+        lbip_runs_smem_bytes(g.m_k, g.kml, g.m, false) + 8192 <= (size_t)c->smem_optin)
+        return run_lbip_runs<false>(c, g, job);
     int P = 1, logP = 0;
     while (P < g.m_k) { P <<= 1; ++logP; }
     const double2* W;
     int r;
     if ((r = twiddle_table(c, P, &W))) return r;
-    size_t smem = lbip_smem_bytes(P, g.m_k, g.m, job.q.metric);
+    size_t smem = lbip_smem_bytes(P);
     unsigned grid;
     if (smem + 8192 <= (size_t)c->smem_optin) {
         job.gwork = nullptr;

@@ -8,8 +8,22 @@
 // test fsmeld_lbip_exceeds_cutoff (include/fsmeld_internal.h:9-19).
 //
 // z_l[m-1+j] + z_u[m-1+j] = sum_k h_l[k] g_l[j+k] + h_u[k] g_u[j+k] for the
-// kml windows j.  Two paths:
-//  * DTW, ERP, MSM: one complex FFT packs (g_l + i g_u), one packs the
+// kml windows j.  Three ways:
+//  * k_lbip_runs, DTW, ERP, MSM with 100 (w+1) >= m: the masks g come from
+//    envelopes of radius w and change value rarely, so with H[k] = h[0] + .. +
+//    h[k-1] an inner product is a signed sum of H over the changes inside the
+//    window (summation by parts): a few adds per window instead of a
+//    transform.  A run in which the radius-w maximum exceeds a level is at least
+//    2w+1 long, so a window has about m / (w+1) changes a side at most; at the
+//    limit of the rule, 200 for both, that costs what the transform does.
+//    Measured on 2^24 points (m = 256, w = 13): DTW 1.16 -> 0.65 ms; 20 mixed queries on
+//    2^22 points (m to 1024) 7.5 -> 2.7 ms with the popcounts below (0.75 -> 0.28 ms
+//    for LCSS on the 2^24 points).  H is a tree sum of
+//    non-negative terms; the result is off by the order of 1e-16 of H[m] per
+//    change, below the transform's error and far below the prune test's 1e-9.
+//  * k_lbip_runs, EDR and LCSS: h and g are 0/1, so the products are popcounts
+//    of bit masks: exact integers.
+//  * k_lbip, narrower bands: one complex FFT packs (g_l + i g_u), one packs the
 //    reversed penalties, the two real spectra of each are separated, the
 //    products are summed, and one inverse FFT gives z_l + z_u directly
 //    (3 complex FFTs of length P >= m_k instead of the reference's 6 real
@@ -17,8 +31,6 @@
 //    passes with a padded layout (one pad every 16 points) so strided
 //    stores are bank-conflict free.  Rounding differs from FFTW's at the
 //    1e-13 level; the prune test's 1e-9 guard makes the decision the same.
-//  * EDR, LCSS: h and g are 0/1, so the products are popcounts of bit
-//    masks: exact integers, no FFT.
 #include <cub/block/block_reduce.cuh>
 #include <cub/block/block_scan.cuh>
 
@@ -161,20 +173,11 @@ __global__ void __launch_bounds__(T) k_lbip(Geom g, LbJob job, const double2* __
     const QueryDev& q = job.q;
     const int m = q.m, mk = g.m_k, kml = g.kml, metric = q.metric;
     const int tid = threadIdx.x;
-    const bool popc_path = (metric == EDR || metric == LCSS);
     const int Pp = P + (P >> 4) + 1;
     unsigned char* lbase = GW ? job.gwork + (long long)blockIdx.x * job.slot_stride : lb_smem;
     double2* bufA = (double2*)lbase;
     double2* bufB = bufA + Pp;
     double2* bufC = bufB + Pp;
-    // popcount path: words of g_l, g_u, h_l, h_u
-    const int gw = (mk + 63) / 64 + 2, hw = (m + 63) / 64;
-    unsigned long long* GL = (unsigned long long*)lbase;
-    unsigned long long* GU = GL + gw;
-    unsigned long long* HL = GU + gw;
-    unsigned long long* HU = HL + hw;
-    double* zpop = (double*)(HU + hw);
-
     for (long long s = blockIdx.x; s < g.S; s += gridDim.x) {
         if (tid == 0) { s_tl = job.thr[2 * s]; s_tu = job.thr[2 * s + 1]; }
         __syncthreads();
@@ -182,79 +185,42 @@ __global__ void __launch_bounds__(T) k_lbip(Geom g, LbJob job, const double2* __
         const double* Ln = job.Ln + s * mk;
         const double* Un = job.Un + s * mk;
         const double* zsrc;
-        if (!popc_path) {
-            // X = g_l + i g_u, Y = reversed h_l + i reversed h_u (src/sip.cpp:16-29)
-            for (int i = tid; i < P; i += T) {
-                double2 x = make_double2(0.0, 0.0), y = make_double2(0.0, 0.0);
-                if (i < mk) x = make_double2(Ln[i] >= tl ? 1.0 : 0.0, Un[i] <= tu ? 1.0 : 0.0);
-                if (i < m) {
-                    const double qv = q.qn[m - 1 - i];
-                    y = make_double2(q_to_h(metric, false, qv, tl, q.arg), q_to_h(metric, true, qv, tu, q.arg));
-                }
-                bufA[padi(i)] = x;
-                bufC[padi(i)] = y;
+        // X = g_l + i g_u, Y = reversed h_l + i reversed h_u (src/sip.cpp:16-29)
+        for (int i = tid; i < P; i += T) {
+            double2 x = make_double2(0.0, 0.0), y = make_double2(0.0, 0.0);
+            if (i < mk) x = make_double2(Ln[i] >= tl ? 1.0 : 0.0, Un[i] <= tu ? 1.0 : 0.0);
+            if (i < m) {
+                const double qv = q.qn[m - 1 - i];
+                y = make_double2(q_to_h(metric, false, qv, tl, q.arg), q_to_h(metric, true, qv, tu, q.arg));
             }
-            __syncthreads();
-            double2* X = fft_run<T>(bufA, bufB, P, logP, W, false);
-            double2* freeb = (X == bufA) ? bufB : bufA;
-            double2* Y = fft_run<T>(bufC, freeb, P, logP, W, false);
-            double2* Zb = (Y == bufC) ? freeb : bufC;  // the buffer holding neither X nor Y
-            const double half = 0.5;
-            for (int k = tid; k < P; k += T) {
-                const int kn = (P - k) & (P - 1);
-                const double2 xk = X[padi(k)], xn = X[padi(kn)];
-                const double2 yk = Y[padi(k)], yn = Y[padi(kn)];
-                // split two real spectra packed in one complex FFT
-                const double2 gl = make_double2(half * (xk.x + xn.x), half * (xk.y - xn.y));
-                const double2 gu = make_double2(half * (xk.y + xn.y), -half * (xk.x - xn.x));
-                const double2 hl = make_double2(half * (yk.x + yn.x), half * (yk.y - yn.y));
-                const double2 hu = make_double2(half * (yk.y + yn.y), -half * (yk.x - yn.x));
-                Zb[padi(k)] = cadd(cmul(gl, hl), cmul(gu, hu));
-            }
-            __syncthreads();
-            double2* Z = fft_run<T>(Zb, X, P, logP, W, true);
-            const double invP = 1.0 / (double)P;
-            // z_l + z_u for window j sits at m-1+j; stash it in the free buffer as doubles
-            double* zs = (double*)((Z == Zb) ? X : Zb);
-            for (int j = tid; j < kml; j += T) zs[j] = Z[padi(m - 1 + j)].x * invP;
-            __syncthreads();
-            zsrc = zs;
-        } else {
-            // bit masks (src/lb.cpp:18-34, src/q_to_h.cpp EDR/LCSS branches)
-            const int lane = tid & 31, warp = tid >> 5;
-            for (int base = warp * 32; base < gw * 64; base += T) {
-                const int i = base + lane;
-                const unsigned bl = __ballot_sync(0xffffffffu, i < mk && Ln[min(i, mk - 1)] >= tl);
-                const unsigned bu = __ballot_sync(0xffffffffu, i < mk && Un[min(i, mk - 1)] <= tu);
-                if (lane == 0) {
-                    unsigned* gl32 = (unsigned*)GL;
-                    unsigned* gu32 = (unsigned*)GU;
-                    gl32[base >> 5] = bl;
-                    gu32[base >> 5] = bu;
-                }
-            }
-            for (int base = warp * 32; base < hw * 64; base += T) {
-                const int k = base + lane;
-                const double qv = (k < m) ? q.qn[k] : 0.0;
-                const unsigned bl = __ballot_sync(0xffffffffu, k < m && q_to_h(metric, false, qv, tl, q.arg) != 0.0);
-                const unsigned bu = __ballot_sync(0xffffffffu, k < m && q_to_h(metric, true, qv, tu, q.arg) != 0.0);
-                if (lane == 0) {
-                    ((unsigned*)HL)[base >> 5] = bl;
-                    ((unsigned*)HU)[base >> 5] = bu;
-                }
-            }
-            __syncthreads();
-            for (int j = tid; j < kml; j += T) {
-                int cnt = 0;
-                for (int wd = 0; wd < hw; ++wd) {
-                    cnt += __popcll(HL[wd] & bits64(GL, j + 64 * wd));
-                    cnt += __popcll(HU[wd] & bits64(GU, j + 64 * wd));
-                }
-                zpop[j] = (double)cnt;
-            }
-            __syncthreads();
-            zsrc = zpop;
+            bufA[padi(i)] = x;
+            bufC[padi(i)] = y;
         }
+        __syncthreads();
+        double2* X = fft_run<T>(bufA, bufB, P, logP, W, false);
+        double2* freeb = (X == bufA) ? bufB : bufA;
+        double2* Y = fft_run<T>(bufC, freeb, P, logP, W, false);
+        double2* Zb = (Y == bufC) ? freeb : bufC;  // the buffer holding neither X nor Y
+        const double half = 0.5;
+        for (int k = tid; k < P; k += T) {
+            const int kn = (P - k) & (P - 1);
+            const double2 xk = X[padi(k)], xn = X[padi(kn)];
+            const double2 yk = Y[padi(k)], yn = Y[padi(kn)];
+            // split two real spectra packed in one complex FFT
+            const double2 gl = make_double2(half * (xk.x + xn.x), half * (xk.y - xn.y));
+            const double2 gu = make_double2(half * (xk.y + xn.y), -half * (xk.x - xn.x));
+            const double2 hl = make_double2(half * (yk.x + yn.x), half * (yk.y - yn.y));
+            const double2 hu = make_double2(half * (yk.y + yn.y), -half * (yk.x - yn.x));
+            Zb[padi(k)] = cadd(cmul(gl, hl), cmul(gu, hu));
+        }
+        __syncthreads();
+        double2* Z = fft_run<T>(Zb, X, P, logP, W, true);
+        const double invP = 1.0 / (double)P;
+        // z_l + z_u for window j sits at m-1+j; stash it in the free buffer as doubles
+        double* zs = (double*)((Z == Zb) ? X : Zb);
+        for (int j = tid; j < kml; j += T) zs[j] = Z[padi(m - 1 + j)].x * invP;
+        __syncthreads();
+        zsrc = zs;
 
         // trans + validity + prune, in window order
         const int lo = g.lo(s);
@@ -273,7 +239,6 @@ __global__ void __launch_bounds__(T) k_lbip(Geom g, LbJob job, const double2* __
             const double zz = zsrc[j];
             double z;
             if (metric == DTW || metric == ERP) z = dsqrt(dmax0(zz));
-            else if (metric == LCSS) z = dmax0(ddiv(zz, (double)m));
             else z = zz;
             if (job.zout) job.zout[s * kml + j] = z;
             if (job.surv && !lbip_exceeds(z, q.cutoff, metric)) ++nsurv;
@@ -295,7 +260,6 @@ __global__ void __launch_bounds__(T) k_lbip(Geom g, LbJob job, const double2* __
                     const double zz = zsrc[j];
                     double z;
                     if (metric == DTW || metric == ERP) z = dsqrt(dmax0(zz));
-                    else if (metric == LCSS) z = dmax0(ddiv(zz, (double)m));
                     else z = zz;
                     if (!lbip_exceeds(z, q.cutoff, metric)) {
                         if (o < (unsigned long long)job.surv_cap) job.surv[o] = gi;
@@ -315,13 +279,209 @@ __global__ void __launch_bounds__(T) k_lbip(Geom g, LbJob job, const double2* __
     }
 }
 
-size_t lbip_smem_bytes(int P, int m_k, int m, int metric) {
-    if (metric == EDR || metric == LCSS) {
-        const int gw = (m_k + 63) / 64 + 2, hw = (m + 63) / 64;
-        return (size_t)(2 * gw + 2 * hw) * 8 + (size_t)(m_k + 1) * 8 + 64;
+// One block per segment.  POPC: EDR, LCSS.
+template <int T, bool POPC>
+__global__ void __launch_bounds__(T) k_lbip_runs(Geom g, LbJob job, double keep_max) {
+    using DScan = cub::BlockScan<double, T>;
+    using IScan = cub::BlockScan<int, T>;
+    extern __shared__ __align__(16) unsigned char lr_smem[];
+    __shared__ typename DScan::TempStorage dscan_tmp;
+    __shared__ typename IScan::TempStorage iscan_tmp;
+    __shared__ unsigned long long s_base;
+    __shared__ double s_tot[2];
+    __shared__ int s_cnt[2], s_off[T / 32 + 1];
+    constexpr unsigned kAll = 0xffffffffu;
+    const QueryDev& q = job.q;
+    const int m = q.m, mk = g.m_k, kml = g.kml, metric = q.metric;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int gw = (mk + 63) / 64 + 2, hw = (m + 63) / 64;
+    // mask words of the two sides, survivor bits of the windows, then either
+    // the penalty words (POPC) or H of the two sides, the changes and, per mask
+    // word, the number of changes before it
+    unsigned long long* G[2] = {(unsigned long long*)lr_smem, (unsigned long long*)lr_smem + gw};
+    unsigned* keepw = (unsigned*)(G[1] + gw);
+    unsigned char* rest = (unsigned char*)keepw + (((size_t)(kml + 31) / 32 * 4 + 15) & ~size_t(15));
+    unsigned long long* Hb[2] = {(unsigned long long*)rest, (unsigned long long*)rest + hw};
+    double* H[2] = {(double*)rest, (double*)rest + (m + 1)};
+    int* pre[2] = {(int*)(H[1] + m + 1), (int*)(H[1] + m + 1) + gw};
+    unsigned short* edge[2] = {(unsigned short*)(pre[1] + gw), (unsigned short*)(pre[1] + gw) + mk};
+
+    for (long long s = blockIdx.x; s < g.S; s += gridDim.x) {
+        const double tl = job.thr[2 * s], tu = job.thr[2 * s + 1];
+        const double* __restrict__ Ln = job.Ln + s * mk;
+        const double* __restrict__ Un = job.Un + s * mk;
+        for (int base = warp * 32; base < gw * 64; base += T) {
+            const int i = base + lane;
+            const unsigned bl = __ballot_sync(kAll, i < mk && Ln[min(i, mk - 1)] >= tl);
+            const unsigned bu = __ballot_sync(kAll, i < mk && Un[min(i, mk - 1)] <= tu);
+            if (lane == 0) {
+                ((unsigned*)G[0])[base >> 5] = bl;
+                ((unsigned*)G[1])[base >> 5] = bu;
+            }
+        }
+        bool plain = true;  // every penalty finite
+        if (POPC) {
+            for (int base = warp * 32; base < hw * 64; base += T) {
+                const int k = base + lane;
+                const double qv = (k < m) ? q.qn[k] : 0.0;
+                const unsigned bl = __ballot_sync(kAll, k < m && q_to_h(metric, false, qv, tl, q.arg) != 0.0);
+                const unsigned bu = __ballot_sync(kAll, k < m && q_to_h(metric, true, qv, tu, q.arg) != 0.0);
+                if (lane == 0) {
+                    ((unsigned*)Hb[0])[base >> 5] = bl;
+                    ((unsigned*)Hb[1])[base >> 5] = bu;
+                }
+            }
+            __syncthreads();
+        } else {
+            // H by a tree: each thread's own stretch, then a block scan
+            const int per = (m + T - 1) / T, k0 = min(m, tid * per), k1 = min(m, k0 + per);
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                double sum = 0.0;
+                for (int k = k0; k < k1; ++k) sum += q_to_h(metric, side == 1, q.qn[k], side ? tu : tl, q.arg);
+                double off;
+                DScan(dscan_tmp).ExclusiveSum(sum, off);
+                for (int k = k0; k < k1; ++k) {
+                    H[side][k] = off;
+                    off += q_to_h(metric, side == 1, q.qn[k], side ? tu : tl, q.arg);
+                }
+                if (k1 == m && k0 < m) { H[side][m] = off; s_tot[side] = off; }
+                __syncthreads();
+            }
+            plain = isfinite(s_tot[0]) && isfinite(s_tot[1]);
+            // changes: positions p with g[p] != g[p-1]; even ones start a run
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                int before = 0;  // gw <= 258 words: one or two rounds
+                for (int w0 = 0; w0 < gw; w0 += T) {
+                    const int wi = w0 + tid;
+                    unsigned long long x = 0;
+                    if (wi < gw) x = G[side][wi] ^ ((G[side][wi] << 1) | (wi ? G[side][wi - 1] >> 63 : 0ull));
+                    int off, tot;
+                    IScan(iscan_tmp).ExclusiveSum(__popcll(x), off, tot);
+                    __syncthreads();
+                    if (wi < gw) {
+                        off += before;
+                        pre[side][wi] = off;
+                        while (x) {
+                            const int b = __ffsll((long long)x) - 1;
+                            x &= x - 1;
+                            if (wi * 64 + b < mk) edge[side][off++] = (unsigned short)(wi * 64 + b);
+                        }
+                    }
+                    before += tot;
+                }
+            }
+            __syncthreads();
+        }
+
+        // windows in order: warp by warp stretches of whole 32-window words
+        const int lo = g.lo(s), words = (kml + 31) / 32, wper = (words + T / 32 - 1) / (T / 32);
+        const int wd0 = min(words, warp * wper), wd1 = min(words, wd0 + wper);
+        int nvalid = 0, nsurv = 0;
+        for (int wd = wd0; wd < wd1; ++wd) {
+            const int j = wd * 32 + lane;
+            const bool in = j < kml && j >= lo;
+            const long long gi = in ? g.gidx(s, j) : 0;
+            const bool ok = in && !window_invalid(job.SIG[s * kml + j], g, gi);
+            bool keep = false;
+            double zz = 0.0;
+            if (ok) {
+                if (POPC) {
+                    int cnt = 0;
+                    for (int i = 0; i < hw; ++i) {
+                        cnt += __popcll(Hb[0][i] & bits64(G[0], j + 64 * i));
+                        cnt += __popcll(Hb[1][i] & bits64(G[1], j + 64 * i));
+                    }
+                    zz = (double)cnt;
+                } else if (plain) {
+#pragma unroll
+                    for (int side = 0; side < 2; ++side) {
+                        // changes at most x, x = j and j+m-1: those of the words before and of the word itself
+                        const unsigned long long* Gs = G[side];
+                        auto upto = [&](int x) {
+                            const int wi = x >> 6;
+                            const unsigned long long c =
+                                Gs[wi] ^ ((Gs[wi] << 1) | (wi ? Gs[wi - 1] >> 63 : 0ull));
+                            return pre[side][wi] + __popcll(c & (~0ull >> (63 - (x & 63))));
+                        };
+                        int e = upto(j);
+                        const int e1 = upto(j + m - 1);
+                        const unsigned short* __restrict__ E = edge[side];
+                        const double* __restrict__ Hs = H[side] - j;
+                        // an odd change ends a run (+H), an even one starts it (-H); H[0] = 0
+                        double z0 = 0.0, z1 = 0.0;
+                        if ((e & 1) && e < e1) { z0 = Hs[E[e]]; ++e; }
+                        for (; e + 1 < e1; e += 2) {
+                            z1 += Hs[E[e]];
+                            z0 += Hs[E[e + 1]];
+                        }
+                        if (e < e1) z1 += Hs[E[e]];
+                        if (e1 & 1) z0 += Hs[j + m];
+                        zz += z0 - z1;
+                    }
+                } else {
+                    zz = dnan();  // as the transform of infinite penalties
+                }
+                ++nvalid;
+                keep = !(zz > keep_max && zz <= 1.7976931348623157e308);
+            }
+            if (job.zout && in) {
+                double z;
+                if (metric == DTW || metric == ERP) z = dsqrt(dmax0(zz));
+                else if (metric == LCSS) z = dmax0(ddiv(zz, (double)m));
+                else z = zz;
+                job.zout[s * kml + j] = ok ? z : dnan();
+            }
+            const unsigned mask = __ballot_sync(kAll, keep);
+            if (lane == 0) keepw[wd] = mask;
+            nsurv += __popc(mask);  // the same in every lane
+        }
+        for (int o = 16; o; o >>= 1) nvalid += __shfl_xor_sync(kAll, nvalid, o);
+        if (lane == 0) s_off[warp] = nsurv;
+        if (tid == 0) s_cnt[0] = 0;
+        __syncthreads();
+        if (lane == 0 && nvalid) atomicAdd(&s_cnt[0], nvalid);
+        int off = 0, total = 0;
+        for (int i = 0; i < T / 32; ++i) {
+            if (i < warp) off += s_off[i];
+            total += s_off[i];
+        }
+        __syncthreads();
+        if (tid == 0) {
+            if (s_cnt[0]) atomicAdd(job.nvalid, (unsigned long long)s_cnt[0]);
+            if (job.surv) s_base = total ? atomicAdd(job.nsurv, (unsigned long long)total) : 0ull;
+            if (job.surv && job.segc) {
+                job.segc[3 * s] = s_cnt[0];
+                job.segc[3 * s + 1] = total;
+                job.segc[3 * s + 2] = 0;
+            }
+        }
+        __syncthreads();
+        if (job.surv) {
+            unsigned long long o = s_base + off;
+            for (int wd = wd0; wd < wd1; ++wd) {
+                const unsigned mask = keepw[wd];
+                if (mask >> lane & 1u) {
+                    const unsigned long long at = o + __popc(mask & ((1u << lane) - 1));
+                    if (at < (unsigned long long)job.surv_cap) job.surv[at] = g.gidx(s, wd * 32 + lane);
+                }
+                o += __popc(mask);
+            }
+        }
+        __syncthreads();
     }
+}
+
+size_t lbip_smem_bytes(int P) {
     const size_t Pp = (size_t)P + (P >> 4) + 1;
     return 3 * Pp * sizeof(double2) + 64;
+}
+
+size_t lbip_runs_smem_bytes(int m_k, int kml, int m, bool popc) {
+    const size_t gw = (m_k + 63) / 64 + 2, hw = (m + 63) / 64;
+    const size_t keep = (((size_t)(kml + 31) / 32 * 4) + 15) & ~size_t(15);
+    return 2 * gw * 8 + keep + (popc ? 2 * hw * 8 : 2 * ((size_t)m + 1) * 8 + 2 * gw * 4 + 2 * (size_t)m_k * 2) + 64;
 }
 
 int lbip_set_w16() {
@@ -336,7 +496,7 @@ int lbip_set_w16() {
 
 template __global__ void k_lbip<256, false>(Geom, LbJob, const double2*, int, int);
 template __global__ void k_lbip<256, true>(Geom, LbJob, const double2*, int, int);
-template __global__ void k_lbip<512, false>(Geom, LbJob, const double2*, int, int);
-template __global__ void k_lbip<512, true>(Geom, LbJob, const double2*, int, int);
+template __global__ void k_lbip_runs<256, false>(Geom, LbJob, double);
+template __global__ void k_lbip_runs<256, true>(Geom, LbJob, double);
 
 }  // namespace fsm

@@ -137,6 +137,11 @@ __global__ void k_threshold(Geom g, const ThrJob* __restrict__ jobs, unsigned ch
                             long long slot_stride, int z_shared);
 template <int T, bool GW>
 __global__ void k_lbip(Geom g, LbJob job, const double2* __restrict__ W, int P, int logP);
+// LB_IP by the changes of the masks (DTW, ERP, MSM) or by popcounts (EDR,
+// LCSS); keep_max: the largest inner product the prune test keeps
+template <int T, bool POPC>
+__global__ void k_lbip_runs(Geom g, LbJob job, double keep_max);
+size_t lbip_runs_smem_bytes(int m_k, int kml, int m, bool popc);
 template <int METRIC>
 __global__ void k_glb_tq(Geom g, GlbJob job);
 template <int METRIC>
@@ -210,7 +215,7 @@ struct ThrMem {
 };
 template <int T, int IPT>
 ThrMem threshold_mem(int m, size_t smem_optin);
-size_t lbip_smem_bytes(int P, int m_k, int m, int metric);
+size_t lbip_smem_bytes(int P);
 int lbip_set_w16();
 // DP block size (2 warps: the per-warp band scratch sets the occupancy)
 constexpr int kDpThreads = 64;

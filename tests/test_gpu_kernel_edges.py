@@ -138,3 +138,33 @@ def test_envelope_tiles(api, oracle, n, m, w):  # noqa: F811
             oun, oln = oracle.normalized(U, L, mx, mn, smx, smn)
             assert bits_equal(un[s], oun), (s, len(bad))
             assert bits_equal(ln[s], oln), (s, len(bad))
+
+
+# k_lbip_runs: sums over mask changes and popcounts, word borders of the masks,
+# walks (few changes) and noise (many), the tail segment; the same tolerance as
+# the transform's (1e-9 absolute, 1e-12 relative, squared domain for DTW, ERP).
+# Narrow bands (100 (w+1) < m) keep the transform.
+@pytest.mark.parametrize("m,w", [(2, 0), (31, 1), (64, 2), (65, 10), (200, 1), (300, 2), (600, 30)])
+@pytest.mark.parametrize("metric,arg", [("dtw", 0.0), ("erp", 0.4), ("edr", 0.25), ("lcss", 0.25), ("msm", 0.5)])
+def test_lbip_runs(api, oracle, metric, arg, m, w):  # noqa: F811
+    mk, kml, _, _ = _geom(m, 1 << 30)
+    t = random_walk(2 * kml + m + 5, [15, m])
+    t[kml:kml + mk // 2] += np.random.default_rng([16, m]).normal(0.0, 5.0, mk // 2)
+    q, _ = query_from(t, m, np.random.default_rng([17, m]))
+    qn = oracle.normalize_query(q)
+    with api.Engine(t) as e:
+        z = e.inspect(q, m, metric, w, arg, 5).reshape(-1, kml)
+        thr = e.inspect(q, m, metric, w, arg, 4).reshape(-1, 2)
+        un = e.inspect(q, m, metric, w, arg, 2).reshape(-1, mk)
+        ln = e.inspect(q, m, metric, w, arg, 3).reshape(-1, mk)
+    _, _, forsize, tail = _geom(m, len(t))
+    for s in range(len(z)):
+        ref = np.correlate(oracle.s_to_g(0, ln[s], thr[s, 0]), oracle.q_to_h(0, metric, qn, thr[s, 0], arg), "valid")
+        ref = ref + np.correlate(oracle.s_to_g(1, un[s], thr[s, 1]), oracle.q_to_h(1, metric, qn, thr[s, 1], arg),
+                                 "valid")
+        got = z[s] ** 2 if metric in ("dtw", "erp") else z[s] * m if metric == "lcss" else z[s]
+        ok = ~np.isnan(got)
+        if s == forsize:  # the tail segment's windows before the tail belong to other segments
+            ok[:kml - tail] = False
+        assert ok.sum() > 0
+        assert np.all(np.abs(got - ref)[ok] <= 1e-9 + 1e-12 * np.abs(ref[ok])), s
