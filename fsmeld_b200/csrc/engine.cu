@@ -218,25 +218,37 @@ int prepare_query(const double* q, int m, int metric, int w, double arg, HostQue
     const std::vector<double>& qn = hq->qn;
     // query envelope (src/fsmeld.cpp:721): window extremes, most recent on ties
     hq->LQ.resize(m); hq->UQ.resize(m);
-    for (int o = 0; o < m; ++o) {
-        const int a = std::max(0, o - w), b = std::min(m - 1, o + w);
-        double lo = qn[a], hi = qn[a];
-        for (int i = a + 1; i <= b; ++i) {
-            lo = (qn[i] <= lo) ? qn[i] : lo;
-            hi = (qn[i] >= hi) ? qn[i] : hi;
+    {
+        // monotone queues of the candidates for the minimum and the maximum
+        std::vector<int> lo(m), hi(m);
+        int l0 = 0, l1 = 0, h0 = 0, h1 = 0;
+        for (int o = 0, i = 0; o < m; ++o) {
+            for (; i <= std::min(m - 1, o + w); ++i) {
+                while (l1 > l0 && qn[i] <= qn[lo[l1 - 1]]) --l1;
+                lo[l1++] = i;
+                while (h1 > h0 && qn[i] >= qn[hi[h1 - 1]]) --h1;
+                hi[h1++] = i;
+            }
+            while (lo[l0] < o - w) ++l0;
+            while (hi[h0] < o - w) ++h0;
+            hq->LQ[o] = qn[lo[l0]];
+            hq->UQ[o] = qn[hi[h0]];
         }
-        hq->LQ[o] = lo; hq->UQ[o] = hi;
     }
     hq->qs = qn;
     std::sort(hq->qs.begin(), hq->qs.end());
     hq->pw.resize(3 * m); hq->opw.resize(3 * m);
     hq->Dq.resize(m); hq->tlq.resize(m); hq->tuq.resize(m);
     hq->oD.resize(m); hq->otl.resize(m); hq->otu.resize(m);
+    const volatile double two = 2.0;
     for (int j = 0; j < m; ++j) {
-        for (int a = 0; a < 3; ++a) {
-            hq->pw[a * m + j] = std::pow(hq->qs[j], a);
-            hq->opw[a * m + j] = std::pow(qn[j], a);
-        }
+        // pow(x, 0) = 1 and pow(x, 1) = x exactly; the square is the C library's
+        // pow, not a product the compiler would put in its place
+        hq->pw[j] = hq->opw[j] = 1.0;
+        hq->pw[m + j] = hq->qs[j];
+        hq->opw[m + j] = qn[j];
+        hq->pw[2 * m + j] = std::pow(hq->qs[j], two);
+        hq->opw[2 * m + j] = std::pow(qn[j], two);
         hq->Dq[j] = fn_D(hq->qs[j], arg, metric);
         hq->tlq[j] = fn_tl(hq->qs[j], arg, metric);
         hq->tuq[j] = fn_tu(hq->qs[j], arg, metric);
@@ -313,6 +325,15 @@ struct fsmeld_ctx {
     std::map<std::string, Buf> bufs;
     std::map<int, double2*> twiddles;
     // opt-in per-stage device timing (CUDA events around each launch)
+    // pinned host memory: query uploads (grow-only, the size of the largest
+    // query's tables) and what k_finish writes
+    unsigned char* pin_up = nullptr;
+    size_t pin_up_bytes = 0;
+    cudaEvent_t ev_up = nullptr;  // the last upload has been read
+    FinishOut* pin_out = nullptr;
+    // work counters of this query's DP launches, zeroed with the query's counters
+    unsigned long long* next = nullptr;
+    int next_used = 0;
     bool prof = false;
     struct ProfRec { int stage; cudaEvent_t a, b; };
     std::vector<ProfRec> pending;
@@ -470,6 +491,23 @@ static int twiddle_table(fsmeld_ctx* c, int P, const double2** out) {
     return FSMELD_OK;
 }
 
+// the context's pinned host memory, at least `bytes` for an upload; the last
+// upload's copy is waited for before its place is written again
+static int pinned(fsmeld_ctx* c, size_t bytes) {
+    if (!c->pin_out) FSM_CUDA_TRY(cudaHostAlloc(&c->pin_out, sizeof(FinishOut), cudaHostAllocDefault));
+    if (!c->ev_up) FSM_CUDA_TRY(cudaEventCreateWithFlags(&c->ev_up, cudaEventDisableTiming));
+    FSM_CUDA_TRY(cudaEventSynchronize(c->ev_up));
+    if (c->pin_up_bytes < bytes) {
+        if (c->pin_up) cudaFreeHost(c->pin_up);
+        c->pin_up = nullptr;
+        c->pin_up_bytes = 0;
+        const size_t want = bytes + bytes / 2;
+        FSM_CUDA_TRY(cudaHostAlloc(&c->pin_up, want, cudaHostAllocDefault));
+        c->pin_up_bytes = want;
+    }
+    return FSMELD_OK;
+}
+
 // upload a prepared query into a named device slot
 static int upload_query(fsmeld_ctx* c, const HostQuery& hq, const std::string& slot, QueryDev* qd) {
     const int m = hq.m;
@@ -478,8 +516,11 @@ static int upload_query(fsmeld_ctx* c, const HostQuery& hq, const std::string& s
     const bool bits = !hq.bitE.empty();
     const size_t bytes0 = nd * 8 + ni * 4;
     const size_t nbit = bits ? hq.bitE.size() * 8 + 2 * (size_t)m * 4 + hq.bitGrid.size() * 2 : 0;
-    std::vector<unsigned char> host(bytes0 + nbit);
-    double* d = (double*)host.data();
+    const size_t bytes = bytes0 + nbit;
+    int r;
+    if ((r = pinned(c, bytes))) return r;
+    unsigned char* host = c->pin_up;
+    double* d = (double*)host;
     size_t o = 0;
     auto put = [&](const std::vector<double>& v) { memcpy(d + o, v.data(), v.size() * 8); size_t at = o; o += v.size(); return at; };
     const size_t o_qn = put(hq.qn), o_LQ = put(hq.LQ), o_UQ = put(hq.UQ), o_qs = put(hq.qs);
@@ -491,7 +532,7 @@ static int upload_query(fsmeld_ctx* c, const HostQuery& hq, const std::string& s
     memcpy(ip + 2 * m, hq.ordA_u.data(), m * 4);
     memcpy(ip + 3 * m, hq.ordB_u.data(), m * 4);
     if (bits) {
-        unsigned char* b = host.data() + bytes0;
+        unsigned char* b = host + bytes0;
         memcpy(b, hq.bitE.data(), hq.bitE.size() * 8);
         b += hq.bitE.size() * 8;
         memcpy(b, hq.bitA.data(), (size_t)m * 4);
@@ -499,9 +540,9 @@ static int upload_query(fsmeld_ctx* c, const HostQuery& hq, const std::string& s
         memcpy(b + 2 * (size_t)m * 4, hq.bitGrid.data(), hq.bitGrid.size() * 2);
     }
     void* dev;
-    int r = buf(c, slot, host.size(), &dev);
-    if (r) return r;
-    FSM_CUDA_TRY(cudaMemcpyAsync(dev, host.data(), host.size(), cudaMemcpyHostToDevice, c->stream));
+    if ((r = buf(c, slot, bytes, &dev))) return r;
+    FSM_CUDA_TRY(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, c->stream));
+    FSM_CUDA_TRY(cudaEventRecord(c->ev_up, c->stream));
     qd->bit = BitTab{};
     if (bits) {
         BitTab& bt = qd->bit;
@@ -523,7 +564,6 @@ static int upload_query(fsmeld_ctx* c, const HostQuery& hq, const std::string& s
         k_bit_table<<<grid, 256, 0, c->stream>>>(pa, pa + m, m, bt.pad, bt.rs, tab);
         LAUNCH_CHECK(c);
     }
-    FSM_CUDA_TRY(cudaStreamSynchronize(c->stream));  // host staging buffer is released on return
     const double* D = (const double*)dev;
     const int* I = (const int*)(D + nd);
     qd->m = m; qd->w = hq.w; qd->metric = hq.metric; qd->p = hq.p; qd->arg = hq.arg;
@@ -614,7 +654,7 @@ static int run_env(fsmeld_ctx* c, const Geom& g, int w, Stats* st, const std::st
 }
 
 template <int T, int IPT>
-static int launch_thr(fsmeld_ctx* c, const Geom& g, const ThrJob* djobs, int njobs, int m) {
+static int launch_thr(fsmeld_ctx* c, const Geom& g, ThrJob job, int m) {
     const ThrMem mem = threshold_mem<T, IPT>(m, (size_t)c->smem_optin);
     const void* kf = mem.gw ? (const void*)k_threshold<T, IPT, true> : (const void*)k_threshold<T, IPT, false>;
     int r;
@@ -626,37 +666,27 @@ static int launch_thr(fsmeld_ctx* c, const Geom& g, const ThrJob* djobs, int njo
     unsigned gx = (unsigned)std::min<long long>(2 * g.S, (long long)std::max(1, per_sm) * c->sm_count * (mem.gw ? 2 : 4));
     unsigned char* gwork = nullptr;
     long long gstride = (long long)round256(mem.gbytes);
-    if (mem.gw && (r = bufT(c, "thrwork", (size_t)gstride * gx * (size_t)njobs, &gwork))) return r;
+    if (mem.gw && (r = bufT(c, "thrwork", (size_t)gstride * gx, &gwork))) return r;
     Geom ga = g;
     int z_shared = mem.z_shared;
-    void* args[] = {&ga, &djobs, &gwork, &gstride, &z_shared};
+    void* args[] = {&ga, &job, &gwork, &gstride, &z_shared};
     prof_begin(c, ST_THR);
-    const cudaError_t le = cudaLaunchKernel(kf, dim3(gx, njobs), dim3(T), args, mem.smem, c->stream);
+    const cudaError_t le = cudaLaunchKernel(kf, dim3(gx), dim3(T), args, mem.smem, c->stream);
     if (le != cudaSuccess) return cuda_fail(le, "k_threshold launch", __FILE__, __LINE__);
     LAUNCH_CHECK(c);
     return FSMELD_OK;
 }
 
-static int run_thr(fsmeld_ctx* c, const Geom& g, const std::vector<ThrJob>& jobs) {
-    if (jobs.empty()) return FSMELD_OK;
-    ThrJob* dj;
-    int r;
-    if ((r = bufT(c, "thrjobs", jobs.size(), &dj))) return r;
-    FSM_CUDA_TRY(cudaMemcpyAsync(dj, jobs.data(), sizeof(ThrJob) * jobs.size(), cudaMemcpyHostToDevice, c->stream));
+static int run_thr(fsmeld_ctx* c, const Geom& g, const ThrJob& job) {
     const int m = g.m;
     const int cnt = g.m_k - 2 * m + 2;
-    const int nj = (int)jobs.size();
-    if (cnt <= 512) r = launch_thr<128, 4>(c, g, dj, nj, m);
-    else if (cnt <= 1024) r = launch_thr<256, 4>(c, g, dj, nj, m);
-    else if (cnt <= 2048) r = launch_thr<256, 8>(c, g, dj, nj, m);
-    else if (cnt <= 4096) r = launch_thr<512, 8>(c, g, dj, nj, m);
-    else if (cnt <= 8192) r = launch_thr<1024, 8>(c, g, dj, nj, m);
-    else if (cnt <= 16384) r = launch_thr<1024, 16>(c, g, dj, nj, m);
-    else r = fail(FSMELD_E_UNSUPPORTED, "envelope core longer than 16384 points is not supported");
-    if (r) return r;
-    // the job array is read by the kernel: keep it alive until it finishes
-    FSM_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    return FSMELD_OK;
+    if (cnt <= 512) return launch_thr<128, 4>(c, g, job, m);
+    if (cnt <= 1024) return launch_thr<256, 4>(c, g, job, m);
+    if (cnt <= 2048) return launch_thr<256, 8>(c, g, job, m);
+    if (cnt <= 4096) return launch_thr<512, 8>(c, g, job, m);
+    if (cnt <= 8192) return launch_thr<1024, 8>(c, g, job, m);
+    if (cnt <= 16384) return launch_thr<1024, 16>(c, g, job, m);
+    return fail(FSMELD_E_UNSUPPORTED, "envelope core longer than 16384 points is not supported");
 }
 
 // The largest inner product zz whose bound passes the prune test at the
@@ -877,9 +907,22 @@ static int run_screen(fsmeld_ctx* c, const Geom& g, DpJob* job) {
     job->n_list = job->n_screened;
     job->list_s = nullptr;
     job->n_valid = nullptr;
-    FSM_CUDA_TRY(cudaMemsetAsync(job->next, 0, sizeof(unsigned long long), c->stream));
+    job->next = job->next + 1;  // its own counter (run_dp takes it off the list)
     return FSMELD_OK;
 }
+
+// the query's counters, all zero, and behind them the work counters of its DP
+// launches (the seeds' and the survivors', a screen and an exact DP each)
+constexpr int kNexts = 4;
+static int zero_counters(fsmeld_ctx* c, unsigned long long** cnt) {
+    int r;
+    if ((r = bufT(c, "counters", C_N + kNexts, cnt))) return r;
+    FSM_CUDA_TRY(cudaMemsetAsync(*cnt, 0, sizeof(unsigned long long) * (C_N + kNexts), c->stream));
+    c->next = *cnt + C_N;
+    c->next_used = 0;
+    return FSMELD_OK;
+}
+static unsigned long long* next_counter(fsmeld_ctx* c) { return c->next + c->next_used++; }
 
 static int run_dp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
     const int w = job.q.w;
@@ -887,10 +930,7 @@ static int run_dp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
     const size_t per_warp = dp_warp_doubles(w);
     size_t smem = sizeof(double) * per_warp * warps;
     int r;
-    unsigned long long* next;
-    if ((r = bufT(c, "dpnext", 1, &next))) return r;
-    FSM_CUDA_TRY(cudaMemsetAsync(next, 0, sizeof(unsigned long long), c->stream));
-    job.next = next;
+    job.next = next_counter(c);
     job.gwork = nullptr;
     job.force_exact = c->dp_exact ? 1 : 0;
     unsigned grid;
@@ -898,6 +938,7 @@ static int run_dp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
     const bool screened = use_screen(c, job);
     if (screened) {
         if ((r = run_screen(c, g, &job))) return r;
+        next_counter(c);
         expected = (long long)c->sm_count * 16 * 128;
     }
     const bool gw_path = smem > (size_t)c->smem_optin - 4096;
@@ -987,6 +1028,37 @@ static int sort_lex(fsmeld_ctx* c, long long* idx, double* dist, long long n) {
     return FSMELD_OK;
 }
 
+// Ends a query's device work: results ordered (by index, or by distance and
+// index), counters in h, and the first `want` results (at most what there are)
+// in the caller's buffers.  One wait for up to kFinishOut results; more than
+// kFinishSort are sorted by radix.
+static int finish(fsmeld_ctx* c, const unsigned long long* cnt, long long cap, bool lex, long long* oi, double* od,
+                  long long want, int64_t* out_idx, double* out_dist, unsigned long long* h) {
+    const size_t smem = 16 * (size_t)kFinishSort;
+    int r;
+    if ((r = allow_smem(c, k_finish, smem))) return r;
+    prof_begin(c, ST_SELECT);
+    k_finish<<<1, kFinishThreads, smem, c->stream>>>(cnt, C_N, C_OUT, cap, lex ? 1 : 0, oi, od, c->pin_out);
+    LAUNCH_CHECK(c);
+    FSM_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    memcpy(h, c->pin_out->cnt, sizeof(unsigned long long) * C_N);
+    const long long nout = std::min<long long>((long long)h[C_OUT], cap);
+    const long long n = std::min(nout, want);
+    if (n <= 0) return FSMELD_OK;
+    if (nout <= kFinishSort && n <= kFinishOut) {
+        if (out_idx) memcpy(out_idx, c->pin_out->idx, sizeof(long long) * n);
+        if (out_dist) memcpy(out_dist, c->pin_out->dist, sizeof(double) * n);
+        return FSMELD_OK;
+    }
+    if (nout > kFinishSort && (r = lex ? sort_lex(c, oi, od, nout) : sort_pairs_i64(c, oi, od, nout))) return r;
+    if (out_idx)
+        FSM_CUDA_TRY(cudaMemcpyAsync(out_idx, oi, sizeof(long long) * n, cudaMemcpyDeviceToHost, c->stream));
+    if (out_dist && od)
+        FSM_CUDA_TRY(cudaMemcpyAsync(out_dist, od, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
+    FSM_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    return FSMELD_OK;
+}
+
 struct QueryRun {
     const HostQuery* hq;
     int mode;  // 0 search, 1 cutoff, 2 exact
@@ -1025,17 +1097,11 @@ static int search_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     dj.screened = surv; dj.n_screened = cnt + C_SCREEN;  // the LB_IP survivors are done with
     dj.out_idx = oi; dj.out_dist = od; dj.n_out = cnt + C_OUT; dj.n_cells = cnt + C_CELLS; dj.out_cap = cap; dj.n_valid = nullptr;
     if ((r = run_dp(c, g, dj, (long long)c->sm_count * 16 * 128))) return r;
-    FSM_CUDA_TRY(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-    FSM_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    const long long nout = (long long)h[C_OUT];
-    if ((r = sort_pairs_i64(c, oi, nullptr, nout))) return r;
-    const long long ncopy = std::min<long long>(nout, qr.cap);
-    if (ncopy > 0)
-        FSM_CUDA_TRY(cudaMemcpyAsync(qr.out_idx, oi, sizeof(long long) * ncopy, cudaMemcpyDeviceToHost, c->stream));
     if (qr.seg_counts && segc && g.forsize > 0)
         FSM_CUDA_TRY(cudaMemcpyAsync(qr.seg_counts, segc, sizeof(long long) * 3 * g.forsize,
                                      cudaMemcpyDeviceToHost, c->stream));
-    FSM_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if ((r = finish(c, cnt, cap, false, oi, nullptr, qr.cap, qr.out_idx, nullptr, h))) return r;
+    const long long nout = (long long)h[C_OUT];
     out.valid = (long long)h[C_VALID];
     out.invalid = g.tsn - out.valid;
     out.after_lb = (long long)h[C_SURV];
@@ -1075,8 +1141,9 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     double* sd;
     if ((r = bufT(c, "seedi", (size_t)nslot, &si))) return r;
     if ((r = bufT(c, "seedd", (size_t)nslot, &sd))) return r;
-    // unused seed slots hold all-ones bit patterns, which sort after every distance
-    FSM_CUDA_TRY(cudaMemsetAsync(sd, 0xff, sizeof(double) * (size_t)nslot, c->stream));
+    const bool tau_block = nslot <= kFinishSort;
+    // (radix sort) unused seed slots hold all-ones bit patterns, which sort after every distance
+    if (!tau_block) FSM_CUDA_TRY(cudaMemsetAsync(sd, 0xff, sizeof(double) * (size_t)nslot, c->stream));
     DpJob sj{};
     sj.q = qd; sj.target = c->d_target; sj.MU = st.MU; sj.SIG = st.SIG;
     sj.list = seeds; sj.n_list = cnt + C_SEED; sj.list_cap = nslot; sj.mode = 1; sj.cutoff = DBL_MAX;
@@ -1084,11 +1151,16 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     if ((r = run_dp(c, g, sj, nslot))) return r;
     // tau = k-th smallest seed distance, selected on the device: the rest of
     // the query reads it from device memory, so the host waits only once
-    unsigned long long* sdk;
     double* tau_dev;
-    if ((r = bufT(c, "seedsort", (size_t)nslot, &sdk))) return r;
     if ((r = bufT(c, "tau", 1, &tau_dev))) return r;
-    {
+    if (tau_block) {
+        const size_t smem = 16 * (size_t)kFinishSort;
+        if ((r = allow_smem(c, k_tau_block, smem))) return r;
+        k_tau_block<<<1, kFinishThreads, smem, c->stream>>>(sd, cnt + C_SEEDOUT, nslot, qr.k, tau_dev);
+        LAUNCH_CHECK(c);
+    } else {
+        unsigned long long* sdk;
+        if ((r = bufT(c, "seedsort", (size_t)nslot, &sdk))) return r;
         size_t tmp = 0;
         FSM_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, tmp, (const unsigned long long*)sd, sdk, (int)nslot, 0,
                                                     64, c->stream));
@@ -1123,18 +1195,15 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     if (nslot >= qr.k) { dj.screened = f1; dj.n_screened = cnt + C_SCREEN; }  // fewer seeds than k: tau is no bound
     dj.out_idx = oi; dj.out_dist = od; dj.n_out = cnt + C_OUT; dj.n_cells = cnt + C_CELLS; dj.out_cap = cap;
     if ((r = run_dp(c, g, dj, (long long)c->sm_count * 16 * 128))) return r;
-    FSM_CUDA_TRY(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-    FSM_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    std::vector<int64_t> ki(qr.k);
+    std::vector<double> kd(qr.k);
+    if ((r = finish(c, cnt, cap, true, oi, od, qr.k, ki.data(), kd.data(), h))) return r;
     const long long nvalid = (long long)h[C_VALID];
     const long long nseed = (long long)h[C_SEEDOUT];
     if (nvalid < qr.k) return fail(FSMELD_E_FEWER_K, "Fewer valid, non-excluded candidates than requested k.");
     const long long nout = (long long)h[C_OUT];
     if (nout < qr.k) return fail(FSMELD_E_FEWER_K, "Fewer valid, non-excluded candidates than requested k.");
-    if ((r = sort_lex(c, oi, od, nout))) return r;
-    FSM_CUDA_TRY(cudaMemcpyAsync(qr.out_idx, oi, sizeof(long long) * qr.k, cudaMemcpyDeviceToHost, c->stream));
-    std::vector<double> kd(qr.k);
-    FSM_CUDA_TRY(cudaMemcpyAsync(kd.data(), od, sizeof(double) * qr.k, cudaMemcpyDeviceToHost, c->stream));
-    FSM_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    memcpy(qr.out_idx, ki.data(), sizeof(int64_t) * qr.k);
     if (qr.out_dist) memcpy(qr.out_dist, kd.data(), sizeof(double) * qr.k);
     out.valid = nvalid;
     out.invalid = g.tsn - nvalid;
@@ -1158,8 +1227,7 @@ static int run_query(fsmeld_ctx* c, const QueryRun& qr, const Geom& g0, Stats& s
     QueryDev qd;
     if ((r = upload_query(c, hq, "query", &qd))) return r;
     unsigned long long* cnt;
-    if ((r = bufT(c, "counters", C_N, &cnt))) return r;
-    FSM_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * C_N, c->stream));
+    if ((r = zero_counters(c, &cnt))) return r;
     const long long cap = g.tsn;
     unsigned long long h[C_N] = {0};
     fsmeld_counters out{};
@@ -1180,16 +1248,8 @@ static int run_query(fsmeld_ctx* c, const QueryRun& qr, const Geom& g0, Stats& s
         dj.n_screened = cnt + C_SCREEN;
         dj.out_idx = oi; dj.out_dist = od; dj.n_out = cnt + C_OUT; dj.n_cells = cnt + C_CELLS; dj.out_cap = cap; dj.n_valid = cnt + C_VALID;
         if ((r = run_dp(c, g, dj, g.tsn))) return r;
-        FSM_CUDA_TRY(cudaMemcpyAsync(h, cnt, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-        FSM_CUDA_TRY(cudaStreamSynchronize(c->stream));
+        if ((r = finish(c, cnt, cap, false, oi, od, qr.cap, qr.out_idx, qr.out_dist, h))) return r;
         const long long nout = (long long)h[C_OUT];
-        if ((r = sort_pairs_i64(c, oi, od, nout))) return r;
-        const long long ncopy = std::min<long long>(nout, qr.cap);
-        if (ncopy > 0) {
-            FSM_CUDA_TRY(cudaMemcpyAsync(qr.out_idx, oi, sizeof(long long) * ncopy, cudaMemcpyDeviceToHost, c->stream));
-            if (qr.out_dist) FSM_CUDA_TRY(cudaMemcpyAsync(qr.out_dist, od, sizeof(double) * ncopy, cudaMemcpyDeviceToHost, c->stream));
-        }
-        FSM_CUDA_TRY(cudaStreamSynchronize(c->stream));
         out.valid = (long long)h[C_VALID];
         out.invalid = g.tsn - out.valid;
         out.after_lb = out.after_glb = out.exact_evals = out.valid;
@@ -1204,9 +1264,9 @@ static int run_query(fsmeld_ctx* c, const QueryRun& qr, const Geom& g0, Stats& s
     // thresholds
     double* thr;
     if ((r = bufT(c, "thr", (size_t)2 * g.S, &thr))) return r;
-    std::vector<ThrJob> jobs(1);
-    jobs[0].q = qd; jobs[0].Un = st.Un; jobs[0].Ln = st.Ln; jobs[0].thr = thr;
-    if ((r = run_thr(c, g, jobs))) return r;
+    ThrJob tj{};
+    tj.q = qd; tj.Un = st.Un; tj.Ln = st.Ln; tj.thr = thr;
+    if ((r = run_thr(c, g, tj))) return r;
     (void)have_env;
 
     long long* segc = nullptr;
@@ -1285,9 +1345,9 @@ static int gemm_thresholds(fsmeld_ctx* c, const Geom& g, const Stats& st, const 
     if ((r = upload_query(c, rep, "query", &qd))) return r;
     double* thr;
     if ((r = bufT(c, "thr", (size_t)2 * g.S, &thr))) return r;
-    std::vector<ThrJob> jobs(1);
-    jobs[0].q = qd; jobs[0].Un = st.Un; jobs[0].Ln = st.Ln; jobs[0].thr = thr;
-    if ((r = run_thr(c, g, jobs))) return r;
+    ThrJob tj{};
+    tj.q = qd; tj.Un = st.Un; tj.Ln = st.Ln; tj.thr = thr;
+    if ((r = run_thr(c, g, tj))) return r;
     std::vector<double> h(2 * (size_t)g.S);
     FSM_CUDA_TRY(cudaMemcpyAsync(h.data(), thr, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, c->stream));
     FSM_CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -1473,8 +1533,7 @@ static int run_search_gemm(fsmeld_ctx* c, const Geom& g0, Stats& st, const std::
             if ((rr = upload_query(x, *qr.hq, "query", &qd))) return rr;
             qd.cutoff = qr.cutoff;
             unsigned long long* cnt;
-            if ((rr = bufT(x, "counters", C_N, &cnt))) return rr;
-            FSM_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * C_N, x->stream));
+            if ((rr = zero_counters(x, &cnt))) return rr;
             FSM_CUDA_TRY(cudaMemcpyAsync(cnt + C_VALID, dcnt + nq + i, 8, cudaMemcpyDeviceToDevice, x->stream));
             if (topk) {
                 if ((long long)hc[nq + i] < qr.k)
@@ -1973,6 +2032,9 @@ int fsmeld_close(fsmeld_ctx* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (auto& kv : c->bufs) if (kv.second.p) cudaFree(kv.second.p);
     for (auto& kv : c->twiddles) cudaFree(kv.second);
+    if (c->pin_up) cudaFreeHost(c->pin_up);
+    if (c->pin_out) cudaFreeHost(c->pin_out);
+    if (c->ev_up) cudaEventDestroy(c->ev_up);
     for (auto& r : c->pending) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
     for (auto e : c->pool) cudaEventDestroy(e);
     if (c->own_target && c->d_target) cudaFree(c->d_target);
@@ -2227,9 +2289,9 @@ int64_t fsmeld_inspect(fsmeld_ctx* c, const double* query, int m, int metric, in
             if ((r = upload_query(c, hq, "query", &qd))) return r;
             double* thr;
             if ((r = bufT(c, "thr", (size_t)2 * g.S, &thr))) return r;
-            std::vector<ThrJob> jobs(1);
-            jobs[0].q = qd; jobs[0].Un = st.Un; jobs[0].Ln = st.Ln; jobs[0].thr = thr;
-            if ((r = run_thr(c, g, jobs))) return r;
+            ThrJob tj{};
+            tj.q = qd; tj.Un = st.Un; tj.Ln = st.Ln; tj.thr = thr;
+            if ((r = run_thr(c, g, tj))) return r;
             if (what == 4) {
                 src = thr;
                 count = 2 * g.S;
@@ -2253,8 +2315,7 @@ int64_t fsmeld_inspect(fsmeld_ctx* c, const double* query, int m, int metric, in
                 }
             } else {
                 unsigned long long* cnt;
-                if ((r = bufT(c, "counters", C_N, &cnt))) return r;
-                FSM_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long) * C_N, c->stream));
+                if ((r = zero_counters(c, &cnt))) return r;
                 double* z;
                 if ((r = bufT(c, "zbuf", (size_t)g.S * g.kml, &z))) return r;
                 LbJob lj{};

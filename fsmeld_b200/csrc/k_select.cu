@@ -103,6 +103,93 @@ __global__ void __launch_bounds__(256) k_seed(Geom g, const double* __restrict__
     }
 }
 
+namespace {
+
+// (key, index) pairs of shared memory in ascending order, n2 a power of two
+template <typename Less>
+__device__ void bitonic(int n2, Less less, double* __restrict__ d, long long* __restrict__ x) {
+    for (int k = 2; k <= n2; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int i = threadIdx.x; i < n2; i += blockDim.x) {
+                const int o = i ^ j;
+                if (o > i) {
+                    const double da = d[i], db = d[o];
+                    const long long xa = x[i], xb = x[o];
+                    if (less(db, xb, da, xa) == ((i & k) == 0)) {
+                        d[i] = db; d[o] = da;
+                        x[i] = xb; x[o] = xa;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+}
+
+}  // namespace
+
+// The end of a query in one block: up to kFinishSort results in their order (by
+// index, or by distance and index), in place, the first kFinishOut of them and
+// the counters also in host memory the device can write, so that the host waits
+// once and copies nothing.  More results are left as they are (the host sorts
+// them by radix).
+__global__ void __launch_bounds__(kFinishThreads) k_finish(const unsigned long long* __restrict__ cnt, int ncnt,
+                                                           int out_slot, long long cap, int lex,
+                                                           long long* __restrict__ idx, double* __restrict__ dist,
+                                                           FinishOut* __restrict__ host) {
+    extern __shared__ __align__(16) unsigned char fin_smem[];
+    double* d = (double*)fin_smem;
+    long long* x = (long long*)(d + kFinishSort);
+    for (int i = threadIdx.x; i < ncnt; i += blockDim.x) host->cnt[i] = cnt[i];
+    const unsigned long long n_all = cnt[out_slot];
+    const int n = n_all < (unsigned long long)cap ? (int)min(n_all, (unsigned long long)kFinishSort + 1)
+                                                  : (int)min(cap, (long long)kFinishSort + 1);
+    if (n > kFinishSort) return;
+    int n2 = 1;
+    while (n2 < n) n2 <<= 1;
+    for (int i = threadIdx.x; i < n2; i += blockDim.x) {
+        d[i] = i < n ? (dist ? dist[i] : 0.0) : INFINITY;
+        x[i] = i < n ? idx[i] : 0x7fffffffffffffffLL;
+    }
+    __syncthreads();
+    if (lex)
+        bitonic(n2, [](double da, long long xa, double db, long long xb) { return da < db || (da == db && xa < xb); },
+                d, x);
+    else
+        bitonic(n2, [](double, long long xa, double, long long xb) { return xa < xb; }, d, x);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        idx[i] = x[i];
+        if (dist) dist[i] = d[i];
+        if (i < kFinishOut) {
+            host->idx[i] = x[i];
+            host->dist[i] = d[i];
+        }
+    }
+}
+
+// The same bound tau as k_tau from at most kFinishSort unsorted seed distances.
+__global__ void __launch_bounds__(kFinishThreads) k_tau_block(const double* __restrict__ dist,
+                                                              const unsigned long long* __restrict__ n_seed,
+                                                              long long cap, long long k, double* tau) {
+    extern __shared__ __align__(16) unsigned char tau_smem[];
+    double* d = (double*)tau_smem;
+    long long* x = (long long*)(d + kFinishSort);
+    const long long n_all = (long long)*n_seed;
+    const int n = (int)(n_all < cap ? n_all : cap);
+    if (k > n) {
+        if (threadIdx.x == 0) *tau = DBL_MAX;
+        return;
+    }
+    int n2 = 1;
+    while (n2 < n) n2 <<= 1;
+    for (int i = threadIdx.x; i < n2; i += blockDim.x) {
+        d[i] = i < n ? dist[i] : INFINITY;
+        x[i] = 0;
+    }
+    __syncthreads();
+    bitonic(n2, [](double da, long long, double db, long long) { return da < db; }, d, x);
+    if (threadIdx.x == 0) *tau = d[k - 1];
+}
+
 // The k-th smallest seed distance, as the search bound tau: the seed
 // distances (non-negative, so their bit patterns order like the values) were
 // sorted as 64-bit keys over all n slots, the unused slots pre-filled with

@@ -184,8 +184,8 @@ __device__ __noinline__ void merge_runs(typename cub::BlockMergeSort<unsigned lo
 // 1024 / T blocks per SM: at most 64 registers a thread, so that several
 // blocks hide each other's serial phases
 template <int T, int IPT, bool GW>
-__global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, const ThrJob* __restrict__ jobs,
-                                                 unsigned char* gwork, long long slot_stride, int z_shared) {
+__global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, ThrJob job, unsigned char* gwork,
+                                                                   long long slot_stride, int z_shared) {
     using Sort = cub::BlockMergeSort<unsigned long long, T, IPT, int>;
     using IScan = cub::BlockScan<int, T>;
     using AReduce = cub::BlockReduce<ArgMax, T>;
@@ -198,7 +198,6 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, const ThrJob*
     __shared__ int s_cnt[2];
     __shared__ double s_ext[64];
 
-    const ThrJob& job = jobs[blockIdx.y];
     const QueryDev& q = job.q;
     const int m = q.m, mk = g.m_k;
     const int cnt = mk - 2 * m + 2;
@@ -206,7 +205,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, const ThrJob*
 
     // GW: region R in global scratch; otherwise provably shared memory
     constexpr size_t RB = thr_r_bytes(CAP);
-    unsigned char* base = GW ? gwork + (long long)(blockIdx.y * gridDim.x + blockIdx.x) * slot_stride
+    unsigned char* base = GW ? gwork + (long long)blockIdx.x * slot_stride
                                 : thr_smem;
     double* rval = (double*)base;                        // [CAP]
     int* rstart = (int*)(base + (size_t)CAP * 8);        // [CAP + 1]
@@ -705,10 +704,10 @@ ThrMem threshold_mem(int m, size_t smem_optin) {
 }
 
 #define FSM_THR_INST(T, IPT)                                                                 \
-    template __global__ void k_threshold<T, IPT, false>(Geom, const ThrJob*, unsigned char*,  \
-                                                        long long, int);                     \
-    template __global__ void k_threshold<T, IPT, true>(Geom, const ThrJob*, unsigned char*,   \
-                                                       long long, int);                      \
+    template __global__ void k_threshold<T, IPT, false>(Geom, ThrJob, unsigned char*,  \
+                                                        long long, int);              \
+    template __global__ void k_threshold<T, IPT, true>(Geom, ThrJob, unsigned char*,   \
+                                                       long long, int);               \
     template ThrMem threshold_mem<T, IPT>(int, size_t);
 FSM_THR_INST(128, 4)
 FSM_THR_INST(256, 4)

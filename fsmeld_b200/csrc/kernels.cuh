@@ -133,8 +133,7 @@ __global__ void k_envelope(const double* __restrict__ target, const double* __re
                            const double* __restrict__ SIG, Geom g, int w, int tiles, double* __restrict__ Un,
                            double* __restrict__ Ln);
 template <int T, int IPT, bool GW>
-__global__ void k_threshold(Geom g, const ThrJob* __restrict__ jobs, unsigned char* gwork,
-                            long long slot_stride, int z_shared);
+__global__ void k_threshold(Geom g, ThrJob job, unsigned char* gwork, long long slot_stride, int z_shared);
 template <int T, bool GW>
 __global__ void k_lbip(Geom g, LbJob job, const double2* __restrict__ W, int P, int logP);
 // LB_IP by the changes of the masks (DTW, ERP, MSM) or by popcounts (EDR,
@@ -196,6 +195,19 @@ size_t screen_warp_bytes(int w);
 __global__ void k_lb_filter(Geom g, const double* __restrict__ z, const double* __restrict__ SIG,
                             const double* __restrict__ cutoff, int metric, long long* out,
                             unsigned long long* n_out, long long cap);
+// results of a query that k_finish leaves in host memory
+constexpr int kFinishThreads = 512;
+constexpr int kFinishSort = 4096;  // results sorted in one block
+constexpr int kFinishOut = 1024;   // results copied
+struct FinishOut {
+    unsigned long long cnt[16];
+    long long idx[kFinishOut];
+    double dist[kFinishOut];
+};
+__global__ void k_finish(const unsigned long long* __restrict__ cnt, int ncnt, int out_slot, long long cap, int lex,
+                         long long* __restrict__ idx, double* __restrict__ dist, FinishOut* __restrict__ host);
+__global__ void k_tau_block(const double* __restrict__ dist, const unsigned long long* __restrict__ n_seed,
+                            long long cap, long long k, double* tau);
 __global__ void k_tau(const unsigned long long* __restrict__ sorted, long long k, long long n, double* tau);
 __global__ void k_seed(Geom g, const double* __restrict__ z, const double* __restrict__ SIG, int per_seg,
                        long long* out, unsigned long long* n_out, long long cap);
