@@ -767,7 +767,7 @@ static int run_lbip(fsmeld_ctx* c, const Geom& g, LbJob job) {
 }
 
 // counters slot layout
-enum { C_SURV, C_G1, C_G2, C_OUT, C_VALID, C_SEED, C_SEEDOUT, C_DPNEXT, C_CELLS, C_SCREEN, C_N };
+enum { C_SURV, C_G1, C_G2, C_OUT, C_VALID, C_SEED, C_SEEDOUT, C_DPNEXT, C_CELLS, C_SCREEN, C_REF, C_REFOUT, C_N };
 
 static bool use_bitdp(const fsmeld_ctx* c, const QueryDev& q) { return q.bit.E && c->dp_form == 0 && !c->dp_exact; }
 
@@ -1128,8 +1128,11 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     out.segments = g.forsize;
     out.tail = g.tsn % g.kml;
     // seeds
-    // seeds per segment: enough for k of them (2k over all segments), at most 32
-    const int per_seg = (int)std::min<long long>(32, std::max<long long>(1, (2 * qr.k + g.S - 1) / g.S));
+    // seeds per segment: enough for k of them (2k over all segments), eight on
+    // short targets (the seeds' DP is one wave up to some thousands), at most 32
+    const long long few_seg = std::min<long long>(8, (1024 + g.S - 1) / g.S);
+    const int per_seg =
+        (int)std::min<long long>(32, std::max<long long>(std::max<long long>(1, few_seg), (2 * qr.k + g.S - 1) / g.S));
     const long long nslot = g.S * per_seg;
     long long* seeds;
     if ((r = bufT(c, "seeds", (size_t)nslot, &seeds))) return r;
@@ -1153,23 +1156,56 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     // the query reads it from device memory, so the host waits only once
     double* tau_dev;
     if ((r = bufT(c, "tau", 1, &tau_dev))) return r;
-    if (tau_block) {
-        const size_t smem = 16 * (size_t)kFinishSort;
-        if ((r = allow_smem(c, k_tau_block, smem))) return r;
-        k_tau_block<<<1, kFinishThreads, smem, c->stream>>>(sd, cnt + C_SEEDOUT, nslot, qr.k, tau_dev);
-        LAUNCH_CHECK(c);
-    } else {
+    // refining windows: about 1024 of them or 2k; large k and seeds that give no
+    // bound go without
+    const long long span = 2 * kRefineReach + 1;
+    const int picks = qr.k <= 2048 && nslot >= qr.k
+                          ? (int)std::min<long long>(kRefinePicks, (std::max<long long>(1024, 2 * qr.k) + span - 1) / span)
+                          : 0;
+    const double* sdist = sd;
+    const long long* sidx = si;
+    if (!tau_block) {
         unsigned long long* sdk;
+        long long* sik;
         if ((r = bufT(c, "seedsort", (size_t)nslot, &sdk))) return r;
+        if ((r = bufT(c, "seedsorti", (size_t)nslot, &sik))) return r;
         size_t tmp = 0;
-        FSM_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, tmp, (const unsigned long long*)sd, sdk, (int)nslot, 0,
-                                                    64, c->stream));
+        FSM_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp, (const unsigned long long*)sd, sdk, (const long long*)si,
+                                                     sik, (int)nslot, 0, 64, c->stream));
         void* tp;
         if ((r = buf(c, "seedsorttmp", tmp, &tp))) return r;
-        FSM_CUDA_TRY(cub::DeviceRadixSort::SortKeys(tp, tmp, (const unsigned long long*)sd, sdk, (int)nslot, 0, 64,
-                                                    c->stream));
-        k_tau<<<1, 32, 0, c->stream>>>(sdk, qr.k, nslot, tau_dev);
+        FSM_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tp, tmp, (const unsigned long long*)sd, sdk, (const long long*)si,
+                                                     sik, (int)nslot, 0, 64, c->stream));
+        sdist = (const double*)sdk;
+        sidx = sik;
+    }
+    {
+        const size_t smem = 16 * (size_t)kFinishSort;
+        long long *rl = nullptr, *ri = nullptr;
+        double* rd = nullptr;
+        if (picks) {
+            if ((r = bufT(c, "refl", (size_t)kFinishSort, &rl))) return r;
+            if ((r = bufT(c, "refi", (size_t)kFinishSort, &ri))) return r;
+            if ((r = bufT(c, "refd", (size_t)kFinishSort, &rd))) return r;
+        }
+        if ((r = allow_smem(c, k_tau_block, smem))) return r;
+        prof_begin(c, ST_SELECT);
+        k_tau_block<<<1, kFinishThreads, smem, c->stream>>>(sdist, sidx, tau_block ? 0 : 1, cnt + C_SEEDOUT, nslot, qr.k,
+                                                            g.tsn, picks, tau_dev, rl, cnt + C_REF);
         LAUNCH_CHECK(c);
+        if (picks) {
+            DpJob rj{};
+            rj.q = qd; rj.target = c->d_target; rj.MU = st.MU; rj.SIG = st.SIG;
+            rj.list = rl; rj.n_list = cnt + C_REF; rj.list_cap = kFinishSort; rj.mode = 1; rj.cutoff = DBL_MAX;
+            rj.cutoff_ptr = tau_dev;
+            rj.out_idx = ri; rj.out_dist = rd; rj.n_out = cnt + C_REFOUT; rj.n_cells = cnt + C_CELLS;
+            rj.out_cap = kFinishSort;
+            if ((r = run_dp(c, g, rj, picks * span))) return r;
+            if ((r = allow_smem(c, k_tau_refine, smem))) return r;
+            prof_begin(c, ST_SELECT);
+            k_tau_refine<<<1, kFinishThreads, smem, c->stream>>>(rd, cnt + C_REFOUT, qr.k, tau_dev);
+            LAUNCH_CHECK(c);
+        }
     }
     // filter, GLB and DP at tau
     long long* f1;
@@ -1209,7 +1245,7 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     out.invalid = g.tsn - nvalid;
     out.after_lb = (long long)h[C_SURV];
     out.after_glb = (long long)h[C_G2];
-    out.exact_evals = (long long)h[C_G2] + nseed;
+    out.exact_evals = (long long)h[C_G2] + nseed + (long long)h[C_REF];
     out.matches = qr.k;
     out.dp_cells = (long long)h[C_CELLS];
     out.threshold = kd[qr.k - 1];

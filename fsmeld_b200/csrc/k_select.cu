@@ -7,19 +7,22 @@
 // (distance, index) pairs among valid candidates.  The device form reaches
 // the same set without the serial scan:
 //  1. LB_IP per window (k_lbip with z output);
-//  2. seeds: the windows with the smallest LB of each segment (k_seed,
-//     ceil(2k/S) per segment, at most 32, so that there are at least k seeds
-//     unless k > 32 S); the k-th smallest exact distance among the seeds is
-//     an upper bound tau on the k-th smallest distance overall (with fewer
-//     than k seeds there is no bound and every candidate is evaluated);
+//  2. seeds: the windows with the smallest LB of each stretch of each segment
+//     (k_seed, ceil(2k/S) stretches per segment, eight on short targets, at
+//     most 32, so that there are at least k seeds unless k > 32 S); the k-th
+//     smallest exact distance among the seeds is an upper bound tau on the
+//     k-th smallest distance overall (with fewer than k seeds there is no
+//     bound and every candidate is evaluated); the windows around the best
+//     seeds lower it (k_tau_block, k_tau_refine), to the k-th distance itself
+//     when the best matches are neighbours of theirs.  Without that step the
+//     filters and the DP ran at a bound that left tens of times the
+//     candidates;
 //  3. every valid window whose LB does not exceed tau (k_lb_filter) goes
 //     through GLB at tau and then the exact DP; any window whose distance is
 //     at most the true k-th distance survives both admissible bounds;
 //  4. a lexicographic sort of the surviving (distance, index) pairs gives the
 //     ranking and the threshold.
 #include <cfloat>
-
-#include <cub/block/block_reduce.cuh>
 
 #include "common.cuh"
 #include "kernels.cuh"
@@ -66,39 +69,33 @@ struct MinZOp {
     }
 };
 
-// one block per segment: its per_seg valid windows with the smallest LB
-// (ties: lowest index), by repeated block-wide argmin strictly after the
-// previous pick in (LB, index) order
+// One block per segment, cut into per_seg stretches of windows: the valid
+// window with the smallest LB of each stretch (ties: lowest index), one pass
+// over the bounds.
 __global__ void __launch_bounds__(256) k_seed(Geom g, const double* __restrict__ z,
                                               const double* __restrict__ SIG, int per_seg,
                                               long long* out, unsigned long long* n_out, long long cap) {
-    using Red = cub::BlockReduce<MinZ, 256>;
-    __shared__ typename Red::TempStorage tmp;
-    __shared__ MinZ s_last;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (long long s = blockIdx.x; s < g.S; s += gridDim.x) {
-        MinZ last{-INFINITY, -1};
-        for (int p = 0; p < per_seg; ++p) {
+        const int lo = g.lo(s), len = (g.kml - lo + per_seg - 1) / per_seg;
+        for (int p = warp; p < per_seg; p += 8) {
+            const int j0 = lo + p * len, j1 = min(g.kml, j0 + len);
             MinZ best{INFINITY, -1};
-            for (int j = g.lo(s) + threadIdx.x; j < g.kml; j += blockDim.x) {
+            for (int j = j0 + lane; j < j1; j += 32) {
                 const long long gi = g.gidx(s, j);
                 if (window_invalid(SIG[s * g.kml + j], g, gi)) continue;
-                double zz = z[s * g.kml + j];
-                if (isnan(zz)) zz = INFINITY;
-                if (zz < last.z || (zz == last.z && gi <= last.gi)) continue;  // picked already
-                best = MinZOp()(best, MinZ{zz, gi});
+                const double zz = z[s * g.kml + j];
+                const MinZ c{isnan(zz) ? INFINITY : zz, gi};
+                best = best.gi < 0 ? c : MinZOp()(best, c);
             }
-            const MinZ r = Red(tmp).Reduce(best, MinZOp());
-            if (threadIdx.x == 0) {
-                s_last = r;
-                if (r.gi >= 0) {
-                    const unsigned long long o = atomicAdd(n_out, 1ull);
-                    if (o < (unsigned long long)cap) out[o] = r.gi;
-                }
+            for (int o = 16; o; o >>= 1) {
+                const MinZ c{__shfl_xor_sync(0xffffffffu, best.z, o), __shfl_xor_sync(0xffffffffu, best.gi, o)};
+                if (c.gi >= 0) best = best.gi < 0 ? c : MinZOp()(best, c);
             }
-            __syncthreads();
-            last = s_last;
-            __syncthreads();
-            if (last.gi < 0) break;
+            if (lane == 0 && best.gi >= 0) {
+                const unsigned long long o = atomicAdd(n_out, 1ull);
+                if (o < (unsigned long long)cap) out[o] = best.gi;
+            }
         }
     }
 }
@@ -166,19 +163,74 @@ __global__ void __launch_bounds__(kFinishThreads) k_finish(const unsigned long l
     }
 }
 
-// The same bound tau as k_tau from at most kFinishSort unsorted seed distances.
+// The bound tau (the k-th smallest seed distance, DBL_MAX with fewer than k
+// seeds) and the windows to refine it with.  Seeds lie at the smallest bound of
+// their stretch; the windows next to a good match are good matches too, and
+// most of the ranking usually, so the kRefineReach windows on either side of
+// the best seeds are evaluated next.  The seeds taken lie more than twice the
+// reach apart, so no window is listed twice and the k-th smallest of their
+// distances is a bound again (k_tau_refine).  sorted: the seeds are in
+// ascending order, else there are at most kFinishSort of them.
 __global__ void __launch_bounds__(kFinishThreads) k_tau_block(const double* __restrict__ dist,
+                                                              const long long* __restrict__ idx, int sorted,
                                                               const unsigned long long* __restrict__ n_seed,
-                                                              long long cap, long long k, double* tau) {
+                                                              long long cap, long long k, long long tsn, int picks,
+                                                              double* tau, long long* __restrict__ list,
+                                                              unsigned long long* __restrict__ n_list) {
     extern __shared__ __align__(16) unsigned char tau_smem[];
+    __shared__ long long s_pick[kRefinePicks];
+    __shared__ int s_np, s_n;
     double* d = (double*)tau_smem;
     long long* x = (long long*)(d + kFinishSort);
-    const long long n_all = (long long)*n_seed;
-    const int n = (int)(n_all < cap ? n_all : cap);
-    if (k > n) {
-        if (threadIdx.x == 0) *tau = DBL_MAX;
-        return;
+    const long long n_all = min((long long)*n_seed, cap);
+    const int n = (int)min(n_all, (long long)kFinishSort);
+    int n2 = 1;
+    while (n2 < n) n2 <<= 1;
+    for (int i = threadIdx.x; i < n2; i += blockDim.x) {
+        d[i] = i < n ? dist[i] : INFINITY;
+        x[i] = i < n ? idx[i] : 0x7fffffffffffffffLL;
     }
+    if (threadIdx.x == 0) s_np = s_n = 0;
+    __syncthreads();
+    if (!sorted)
+        bitonic(n2, [](double da, long long xa, double db, long long xb) { return da < db || (da == db && xa < xb); },
+                d, x);
+    if (threadIdx.x == 0) *tau = k <= n_all ? (k <= n ? d[k - 1] : dist[k - 1]) : DBL_MAX;
+    if (!picks) return;
+    if (threadIdx.x < 32) {
+        int np = 0;
+        for (int i = 0; i < min(n, 8 * kRefinePicks) && np < picks; ++i) {
+            bool clash = false;
+            for (int q = threadIdx.x; q < np; q += 32) {
+                const long long gap = x[i] - s_pick[q];
+                clash = clash || (gap <= 2 * kRefineReach && gap >= -2 * kRefineReach);
+            }
+            if (__any_sync(0xffffffffu, clash)) continue;
+            if (threadIdx.x == 0) s_pick[np] = x[i];
+            ++np;
+            __syncwarp();
+        }
+        if (threadIdx.x == 0) s_np = np;
+    }
+    __syncthreads();
+    constexpr int kSpan = 2 * kRefineReach + 1;
+    for (int e = threadIdx.x; e < s_np * kSpan; e += blockDim.x) {
+        const long long w = s_pick[e / kSpan] + e % kSpan - kRefineReach;
+        if (w >= 0 && w < tsn) list[atomicAdd(&s_n, 1)] = w;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) *n_list = (unsigned long long)s_n;
+}
+
+// tau lowered to the k-th smallest of the refining distances
+__global__ void __launch_bounds__(kFinishThreads) k_tau_refine(const double* __restrict__ dist,
+                                                               const unsigned long long* __restrict__ n_dist,
+                                                               long long k, double* tau) {
+    extern __shared__ __align__(16) unsigned char ref_smem[];
+    double* d = (double*)ref_smem;
+    long long* x = (long long*)(d + kFinishSort);
+    const int n = (int)min(*n_dist, (unsigned long long)kFinishSort);
+    if (k > n) return;
     int n2 = 1;
     while (n2 < n) n2 <<= 1;
     for (int i = threadIdx.x; i < n2; i += blockDim.x) {
@@ -187,22 +239,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_tau_block(const double* __re
     }
     __syncthreads();
     bitonic(n2, [](double da, long long, double db, long long) { return da < db; }, d, x);
-    if (threadIdx.x == 0) *tau = d[k - 1];
-}
-
-// The k-th smallest seed distance, as the search bound tau: the seed
-// distances (non-negative, so their bit patterns order like the values) were
-// sorted as 64-bit keys over all n slots, the unused slots pre-filled with
-// all-ones (a NaN pattern, sorted last).  Fewer than k seeds: no bound.
-__global__ void k_tau(const unsigned long long* __restrict__ sorted, long long k, long long n, double* tau) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double v = DBL_MAX;
-        if (k >= 1 && k <= n) {
-            const double s = __longlong_as_double((long long)sorted[k - 1]);
-            if (!isnan(s)) v = s;
-        }
-        *tau = v;
-    }
+    if (threadIdx.x == 0 && d[k - 1] < *tau) *tau = d[k - 1];
 }
 
 }  // namespace fsm

@@ -206,9 +206,15 @@ struct FinishOut {
 };
 __global__ void k_finish(const unsigned long long* __restrict__ cnt, int ncnt, int out_slot, long long cap, int lex,
                          long long* __restrict__ idx, double* __restrict__ dist, FinishOut* __restrict__ host);
-__global__ void k_tau_block(const double* __restrict__ dist, const unsigned long long* __restrict__ n_seed,
-                            long long cap, long long k, double* tau);
-__global__ void k_tau(const unsigned long long* __restrict__ sorted, long long k, long long n, double* tau);
+// top-k: tau from the seeds, and the windows around the best of them
+constexpr int kRefineReach = 15;
+constexpr int kRefinePicks = 132;  // 132 x 31 windows fit kFinishSort
+__global__ void k_tau_block(const double* __restrict__ dist, const long long* __restrict__ idx, int sorted,
+                            const unsigned long long* __restrict__ n_seed, long long cap, long long k, long long tsn,
+                            int picks, double* tau, long long* __restrict__ list,
+                            unsigned long long* __restrict__ n_list);
+__global__ void k_tau_refine(const double* __restrict__ dist, const unsigned long long* __restrict__ n_dist,
+                             long long k, double* tau);
 __global__ void k_seed(Geom g, const double* __restrict__ z, const double* __restrict__ SIG, int per_seg,
                        long long* out, unsigned long long* n_out, long long cap);
 
