@@ -1034,7 +1034,7 @@ static int sort_lex(fsmeld_ctx* c, long long* idx, double* dist, long long n) {
 // kFinishSort are sorted by radix.
 static int finish(fsmeld_ctx* c, const unsigned long long* cnt, long long cap, bool lex, long long* oi, double* od,
                   long long want, int64_t* out_idx, double* out_dist, unsigned long long* h) {
-    const size_t smem = 16 * (size_t)kFinishSort;
+    const size_t smem = finish_smem_bytes();
     int r;
     if ((r = allow_smem(c, k_finish, smem))) return r;
     prof_begin(c, ST_SELECT);
@@ -1180,7 +1180,7 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
         sidx = sik;
     }
     {
-        const size_t smem = 16 * (size_t)kFinishSort;
+        const size_t smem = finish_smem_bytes();
         long long *rl = nullptr, *ri = nullptr;
         double* rd = nullptr;
         if (picks) {
@@ -1211,7 +1211,7 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     long long* f1;
     if ((r = bufT(c, "surv", (size_t)cap, &f1))) return r;
     prof_begin(c, ST_SELECT);
-    k_lb_filter<<<(unsigned)std::min<long long>((g.tsn + 255) / 256, (long long)c->sm_count * 16), 256, 0, c->stream>>>(
+    k_lb_filter<<<(unsigned)std::min<long long>((g.tsn + 2047) / 2048, (long long)c->sm_count * 8), 256, 0, c->stream>>>(
         g, z, st.SIG, tau_dev, qd.metric, f1, cnt + C_SURV, cap);
     LAUNCH_CHECK(c);
     QueryDev qt = qd;

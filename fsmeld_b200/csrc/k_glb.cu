@@ -116,6 +116,36 @@ __device__ __forceinline__ double tq_term(double t, double lo, double hi, double
     }
 }
 
+// boundary term in the reference's operations (src/glb.cpp:200-230)
+template <int METRIC>
+__device__ __forceinline__ double boundary_exact(const double* __restrict__ Q, int m, double arg,
+                                                 const double* __restrict__ tp, double mu, double sg, double inv,
+                                                 bool rok) {
+    if (METRIC == LCSS) return 0.0;
+#define TN(k) zdiv_i(dsub(tp[(k)], mu), sg, inv, rok)
+    const double T0 = TN(0), TL = TN(m - 1);
+    if (METRIC == DTW) {
+        return dadd(dsq(T0, Q[0]), dsq(TL, Q[m - 1]));
+    } else if (METRIC == ERP) {
+        return dmin3(dsq(Q[m - 1], TL), dsq(Q[m - 1], arg), dsq(TL, arg));
+    } else if (METRIC == EDR) {
+        return dminv(edr_sub(Q[m - 1], TL, arg), 1.0);
+    } else if (METRIC == MSM) {
+        const double T2 = TN(m - 2);
+        const double q0 = Q[0], ql = Q[m - 1], ql2 = Q[m - 2];
+        if ((T2 >= TL && TL >= ql) || (T2 <= TL && TL <= ql) || (ql2 <= ql && ql <= TL) ||
+            (ql2 >= ql && ql >= TL)) {
+            return dadd(fabs(dsub(q0, T0)), dminv(fabs(dsub(ql, TL)), arg));
+        } else {
+            return dadd(fabs(dsub(q0, T0)),
+                            dmin3(fabs(dsub(ql, TL)), dadd(arg, fabs(dsub(TL, T2))),
+                                  dadd(arg, fabs(dsub(ql, ql2)))));
+        }
+    }
+#undef TN
+    return 0.0;
+}
+
 // boundary term and T->Q sum in the reference's operations; false: abandoned
 template <int METRIC>
 __device__ __noinline__ bool exact_tq(const double* __restrict__ Q, const double* __restrict__ LQ,
@@ -129,25 +159,7 @@ __device__ __noinline__ bool exact_tq(const double* __restrict__ Q, const double
     bool alive = true;
     boundary = tq = 0.0;
 #define TN(k) zdiv_i(dsub(tp[(k)], mu), sg, inv, rok)
-    const double T0 = TN(0), TL = TN(m - 1);
-    if (METRIC == DTW) {
-        boundary = dadd(dsq(T0, Q[0]), dsq(TL, Q[m - 1]));
-    } else if (METRIC == ERP) {
-        boundary = dmin3(dsq(Q[m - 1], TL), dsq(Q[m - 1], arg), dsq(TL, arg));
-    } else if (METRIC == EDR) {
-        boundary = dminv(edr_sub(Q[m - 1], TL, arg), 1.0);
-    } else if (METRIC == MSM) {
-        const double T2 = TN(m - 2);
-        const double q0 = Q[0], ql = Q[m - 1], ql2 = Q[m - 2];
-        if ((T2 >= TL && TL >= ql) || (T2 <= TL && TL <= ql) || (ql2 <= ql && ql <= TL) ||
-            (ql2 >= ql && ql >= TL)) {
-            boundary = dadd(fabs(dsub(q0, T0)), dminv(fabs(dsub(ql, TL)), arg));
-        } else {
-            boundary = dadd(fabs(dsub(q0, T0)),
-                            dmin3(fabs(dsub(ql, TL)), dadd(arg, fabs(dsub(TL, T2))),
-                                  dadd(arg, fabs(dsub(ql, ql2)))));
-        }
-    }
+    boundary = boundary_exact<METRIC>(Q, m, arg, tp, mu, sg, inv, rok);
     if (METRIC == LCSS) {
         // every point, no abandon (src/glb.cpp:238-252)
         const double min_len = (double)m;
@@ -226,6 +238,56 @@ __device__ __noinline__ double exact_qt(const double* __restrict__ Q, int m, int
     for (; k <= k1; ++k) qt = dadd(qt, qt_term(METRIC, Q[k], k, m, w, lf, uf, mu, sg, inv, rok, arg));
     return qt;
 }
+
+// The same two sums with a warp per candidate, every lane with the same
+// arguments and the same results: the terms of 32 points at a time, added in
+// the reference's order.  One lane alone waits for each of its loads; most
+// warps that come here have one candidate to decide.
+template <int METRIC>
+__device__ __noinline__ bool warp_tq(const double* __restrict__ Q, const double* __restrict__ LQ,
+                                     const double* __restrict__ UQ, int m, double arg,
+                                     const double* __restrict__ tp, double mu, double sg, double bsf,
+                                     double& boundary_out, double& tq_out) {
+    const int lane = threadIdx.x & 31;
+    const double inv = __drcp_rn(sg);
+    const bool rok = rcp_div_in_range(sg);
+    const double lim = (METRIC == DTW || METRIC == ERP) ? dmul(bsf, bsf) : bsf;
+    double boundary = boundary_exact<METRIC>(Q, m, arg, tp, mu, sg, inv, rok), tq = 0.0;
+    bool alive = true;
+    const int kb = METRIC == LCSS ? 0 : 1, ke = METRIC == LCSS ? m : m - 1;
+    for (int k0 = kb; k0 < ke && alive; k0 += 32) {
+        const int k = min(k0 + lane, ke - 1);
+        const double term = tq_term<METRIC>(zdiv_i(dsub(tp[k], mu), sg, inv, rok), LQ[k], UQ[k], arg);
+        for (int j = 0; j < min(32, ke - k0); ++j) tq = dadd(tq, __shfl_sync(0xffffffffu, term, j));
+        if (METRIC != LCSS && dadd(boundary, tq) > lim) alive = false;
+    }
+    if (METRIC == LCSS) {
+        if (dmax0(dsub(1.0, ddiv(tq, (double)m))) > bsf) alive = false;
+    } else if (dadd(boundary, tq) > lim) {
+        alive = false;
+    }
+    boundary_out = boundary;
+    tq_out = tq;
+    return alive;
+}
+
+template <int METRIC>
+__device__ __noinline__ double warp_qt(const double* __restrict__ Q, int m, int w, double arg,
+                                       const double* __restrict__ lf, const double* __restrict__ uf, double mu,
+                                       double sg) {
+    const int lane = threadIdx.x & 31;
+    const double inv = __drcp_rn(sg);
+    const bool rok = rcp_div_in_range(sg);
+    const int kb = METRIC == LCSS ? 0 : 1, ke = METRIC == LCSS ? m : m - 1;
+    double qt = 0.0;
+    for (int k0 = kb; k0 < ke; k0 += 32) {
+        const int k = min(k0 + lane, ke - 1);
+        const double term = qt_term(METRIC, Q[k], k, m, w, lf, uf, mu, sg, inv, rok, arg);
+        for (int j = 0; j < min(32, ke - k0); ++j) qt = dadd(qt, __shfl_sync(0xffffffffu, term, j));
+    }
+    return qt;
+}
+constexpr int kWarpExact = 6;  // candidates of a warp decided one after another by the whole warp
 
 // ------------------------------------------------ fixed point and FP32 sums
 
@@ -476,7 +538,23 @@ __global__ void __launch_bounds__(256, 4) k_glb_tq(Geom g, GlbJob job) {
         bool alive = !dead && !bad && acc_alive<METRIC>(a, f);
         double ob = dnan();  // certified: nothing to hand on but the T->Q count
         double ot = METRIC == LCSS ? (double)(m - inner) : (double)inner;
-        if (!dead && !alive) {  // within the margin or out of range: the reference's operations
+        // within the margin or out of range: the reference's operations
+        const unsigned open = __ballot_sync(0xffffffffu, !dead && !alive);
+        if (__popc(open) <= kWarpExact) {
+            for (unsigned left = open; left; left &= left - 1) {
+                const int L = __ffs(left) - 1;
+                const long long gL = __shfl_sync(0xffffffffu, gi, L);
+                const double muL = __shfl_sync(0xffffffffu, mu, L), sgL = __shfl_sync(0xffffffffu, sg, L);
+                double b, t;
+                const bool on = warp_tq<METRIC>(q.qn, q.LQ, q.UQ, m, q.arg, job.target + gL, muL, sgL, bsf, b, t);
+                if ((threadIdx.x & 31) == L) {
+                    alive = on;
+                    ob = b;
+                    ot = t;
+                }
+            }
+            if ((open >> (threadIdx.x & 31) & 1u) && !alive && kGlbMax <= bsf) { alive = true; ob = -1.0; }
+        } else if (!dead && !alive) {
             alive = exact_tq<METRIC>(q.qn, q.LQ, q.UQ, m, q.arg, tp, mu, sg, bsf, ob, ot);
             // abandoned: GLB returns MAX_VAL (src/glb.cpp:221 etc.); it survives only if
             // MAX_VAL <= cutoff (marker -1)
@@ -682,15 +760,40 @@ __global__ void __launch_bounds__(256, 3) k_glb_qt(Geom g, GlbJob job) {
             }
         }
         keep = active && certified && !dead && acc_alive<METRIC>(a, f);
-        if (active && !keep && !(certified && dead)) {
-            double qt = 0.0, glb;
+        const bool want = active && !keep && !(certified && dead);
+        const unsigned open = __ballot_sync(0xffffffffu, want);
+        if (open) {
+            double qt = 0.0;
             bool on = true;
-            if (certified) on = exact_tq<METRIC>(q.qn, q.LQ, q.UQ, m, q.arg, job.target + gi, mu, sg, bsf, boundary, tq);
-            if (boundary == -1.0 || !on) {
-                glb = kGlbMax;  // abandoned in T->Q but MAX_VAL <= cutoff
-            } else {
-                qt = exact_qt<METRIC>(q.qn, m, w, q.arg, lf, uf, mu, sg);
-                if (METRIC == LCSS) {
+            if (__popc(open) <= kWarpExact) {
+                for (unsigned left = open; left; left &= left - 1) {
+                    const int L = __ffs(left) - 1;
+                    const long long gL = __shfl_sync(0xffffffffu, gi, L);
+                    const double muL = __shfl_sync(0xffffffffu, mu, L), sgL = __shfl_sync(0xffffffffu, sg, L);
+                    double bL = __shfl_sync(0xffffffffu, boundary, L), tL = __shfl_sync(0xffffffffu, tq, L);
+                    bool onL = true;
+                    if (__shfl_sync(0xffffffffu, (int)certified, L))
+                        onL = warp_tq<METRIC>(q.qn, q.LQ, q.UQ, m, q.arg, job.target + gL, muL, sgL, bsf, bL, tL);
+                    double v = 0.0;
+                    if (bL != -1.0 && onL)
+                        v = warp_qt<METRIC>(q.qn, m, w, q.arg, job.lraw + gL, job.uraw + gL, muL, sgL);
+                    if ((threadIdx.x & 31) == L) {
+                        boundary = bL;
+                        tq = tL;
+                        on = onL;
+                        qt = v;
+                    }
+                }
+            } else if (want) {
+                if (certified)
+                    on = exact_tq<METRIC>(q.qn, q.LQ, q.UQ, m, q.arg, job.target + gi, mu, sg, bsf, boundary, tq);
+                if (boundary != -1.0 && on) qt = exact_qt<METRIC>(q.qn, m, w, q.arg, lf, uf, mu, sg);
+            }
+            if (want) {
+                double glb;
+                if (boundary == -1.0 || !on) {
+                    glb = kGlbMax;  // abandoned in T->Q but MAX_VAL <= cutoff
+                } else if (METRIC == LCSS) {
                     glb = dmax0(dsub(1.0, ddiv(dminv(tq, qt), (double)m)));
                 } else {
                     const double tot = dadd(boundary, qt);
@@ -699,10 +802,10 @@ __global__ void __launch_bounds__(256, 3) k_glb_qt(Geom g, GlbJob job) {
                     else
                         glb = (tot > bsf) ? kGlbMax : dadd(boundary, dmaxv(tq, qt));
                 }
+                keep = glb <= bsf;
+                os = boundary == -1.0 ? -1.0 : qt;
+                ot = boundary == -1.0 ? -1.0 : tq;
             }
-            keep = glb <= bsf;
-            os = boundary == -1.0 ? -1.0 : qt;
-            ot = boundary == -1.0 ? -1.0 : tq;
         }
         warp_append(keep, job.n_out, [&](unsigned long long o) {
             if (o < (unsigned long long)job.out_cap) {

@@ -24,36 +24,63 @@
 //     ranking and the threshold.
 #include <cfloat>
 
+#include <cub/block/block_merge_sort.cuh>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
 namespace fsm {
 
+// A block takes 2048 windows and appends its survivors, in order, with one
+// atomic: one per warp (2^23 windows: 262,144 on one address) took 0.15 ms where
+// reading the bounds takes 0.02.
 __global__ void __launch_bounds__(256) k_lb_filter(Geom g, const double* __restrict__ z,
                                                    const double* __restrict__ SIG,
                                                    const double* __restrict__ cutoff_dev, int metric,
                                                    long long* out, unsigned long long* n_out, long long cap) {
+    constexpr int kPer = 8;
+    __shared__ unsigned s_mask[kPer * 8];
+    __shared__ unsigned long long s_base;
     const double cutoff = *cutoff_dev;
-    const int lane = threadIdx.x & 31;
-    for (long long base = (long long)blockIdx.x * blockDim.x; base < g.tsn;
-         base += (long long)gridDim.x * blockDim.x) {
-        const long long gi = base + threadIdx.x;
-        bool keep = false;
-        if (gi < g.tsn) {
-            long long s;
-            int j;
-            g.locate(gi, &s, &j);
-            const double sg = SIG[s * g.kml + j];
-            keep = !window_invalid(sg, g, gi) && !lbip_exceeds(z[s * g.kml + j], cutoff, metric);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (long long base = (long long)blockIdx.x * 256 * kPer; base < g.tsn; base += (long long)gridDim.x * 256 * kPer) {
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            const long long gi = base + u * 256 + threadIdx.x;
+            bool keep = false;
+            if (gi < g.tsn) {
+                long long s;
+                int j;
+                g.locate(gi, &s, &j);
+                const double sg = SIG[s * g.kml + j];
+                keep = !window_invalid(sg, g, gi) && !lbip_exceeds(z[s * g.kml + j], cutoff, metric);
+            }
+            const unsigned mask = __ballot_sync(0xffffffffu, keep);
+            if (lane == 0) s_mask[u * 8 + warp] = mask;
         }
-        const unsigned mask = __ballot_sync(0xffffffffu, keep);
-        if (mask) {
-            unsigned long long o = 0;
-            const int leader = __ffs(mask) - 1;
-            if (lane == leader) o = atomicAdd(n_out, (unsigned long long)__popc(mask));
-            o = __shfl_sync(0xffffffffu, o, leader) + __popc(mask & ((1u << lane) - 1));
-            if (keep && o < (unsigned long long)cap) out[o] = gi;
+        __syncthreads();
+        // survivors before each of the 64 words
+        const int c0 = __popc(s_mask[2 * lane]), c1 = __popc(s_mask[2 * lane + 1]);
+        int inc = c0 + c1;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += v;
         }
+        const int total = __shfl_sync(0xffffffffu, inc, 31);
+        if (threadIdx.x == 0) s_base = total ? atomicAdd(n_out, (unsigned long long)total) : 0ull;
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kPer; ++u) {
+            const int wd = u * 8 + warp;
+            const int before = __shfl_sync(0xffffffffu, inc - c0 - c1, wd >> 1) +
+                               ((wd & 1) ? __shfl_sync(0xffffffffu, c0, wd >> 1) : 0);
+            const unsigned mask = s_mask[wd];
+            if (mask >> lane & 1u) {
+                const unsigned long long o = s_base + before + __popc(mask & ((1u << lane) - 1));
+                if (o < (unsigned long long)cap) out[o] = base + u * 256 + threadIdx.x;
+            }
+        }
+        __syncthreads();
     }
 }
 
@@ -75,13 +102,17 @@ struct MinZOp {
 __global__ void __launch_bounds__(256) k_seed(Geom g, const double* __restrict__ z,
                                               const double* __restrict__ SIG, int per_seg,
                                               long long* out, unsigned long long* n_out, long long cap) {
+    __shared__ MinZ s_best[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // few stretches: the whole block on each, else a warp each
+    const bool whole = per_seg < 8;
+    const int t0 = whole ? (int)threadIdx.x : lane, step = whole ? 256 : 32;
     for (long long s = blockIdx.x; s < g.S; s += gridDim.x) {
         const int lo = g.lo(s), len = (g.kml - lo + per_seg - 1) / per_seg;
-        for (int p = warp; p < per_seg; p += 8) {
+        for (int p = whole ? 0 : warp; p < per_seg; p += whole ? 1 : 8) {
             const int j0 = lo + p * len, j1 = min(g.kml, j0 + len);
             MinZ best{INFINITY, -1};
-            for (int j = j0 + lane; j < j1; j += 32) {
+            for (int j = j0 + t0; j < j1; j += step) {
                 const long long gi = g.gidx(s, j);
                 if (window_invalid(SIG[s * g.kml + j], g, gi)) continue;
                 const double zz = z[s * g.kml + j];
@@ -92,7 +123,16 @@ __global__ void __launch_bounds__(256) k_seed(Geom g, const double* __restrict__
                 const MinZ c{__shfl_xor_sync(0xffffffffu, best.z, o), __shfl_xor_sync(0xffffffffu, best.gi, o)};
                 if (c.gi >= 0) best = best.gi < 0 ? c : MinZOp()(best, c);
             }
-            if (lane == 0 && best.gi >= 0) {
+            if (whole) {
+                if (lane == 0) s_best[warp] = best;
+                __syncthreads();
+                for (int i = 0; i < 8; ++i) {
+                    const MinZ c = s_best[i];
+                    if (c.gi >= 0) best = best.gi < 0 ? c : MinZOp()(best, c);
+                }
+                __syncthreads();
+            }
+            if (lane == 0 && (!whole || warp == 0) && best.gi >= 0) {
                 const unsigned long long o = atomicAdd(n_out, 1ull);
                 if (o < (unsigned long long)cap) out[o] = best.gi;
             }
@@ -102,24 +142,48 @@ __global__ void __launch_bounds__(256) k_seed(Geom g, const double* __restrict__
 
 namespace {
 
-// (key, index) pairs of shared memory in ascending order, n2 a power of two
-template <typename Less>
-__device__ void bitonic(int n2, Less less, double* __restrict__ d, long long* __restrict__ x) {
-    for (int k = 2; k <= n2; k <<= 1)
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-                const int o = i ^ j;
-                if (o > i) {
-                    const double da = d[i], db = d[o];
-                    const long long xa = x[i], xb = x[o];
-                    if (less(db, xb, da, xa) == ((i & k) == 0)) {
-                        d[i] = db; d[o] = da;
-                        x[i] = xb; x[o] = xa;
-                    }
-                }
-            }
-            __syncthreads();
+struct Pair {
+    double d;
+    long long x;
+};
+struct PairLess {
+    __device__ bool operator()(const Pair& a, const Pair& b) const { return a.d < b.d || (a.d == b.d && a.x < b.x); }
+};
+using PairSort = cub::BlockMergeSort<Pair, kFinishThreads, kFinishSort / kFinishThreads>;
+
+// n pairs of shared memory in ascending (distance, index) order: up to 1024 by
+// counting the smaller ones of each (no barriers; 6 us at 1024), a merge sort of
+// all kFinishSort slots beyond (45 us).  Pairs are distinct.
+__device__ void sort_pairs(Pair* __restrict__ v, int n, PairSort::TempStorage& tmp) {
+    constexpr int kPer = kFinishSort / kFinishThreads;
+    if (n > 2 * kFinishThreads) {
+        Pair own[kPer];
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            const int i = threadIdx.x * kPer + k;
+            own[k] = i < n ? v[i] : Pair{INFINITY, 0x7fffffffffffffffLL};
         }
+        __syncthreads();
+        PairSort(tmp).Sort(own, PairLess());
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) v[threadIdx.x * kPer + k] = own[k];
+        __syncthreads();
+        return;
+    }
+    const int i0 = threadIdx.x, i1 = i0 + kFinishThreads;
+    const Pair a = i0 < n ? v[i0] : Pair{INFINITY, 0}, b = i1 < n ? v[i1] : Pair{INFINITY, 0};
+    int ra = 0, rb = 0;
+    if ((i0 & ~31) < n)
+        for (int j = 0; j < n; ++j) {
+            const Pair c = v[j];
+            ra += PairLess()(c, a) ? 1 : 0;
+            rb += PairLess()(c, b) ? 1 : 0;
+        }
+    __syncthreads();
+    if (i0 < n) v[ra] = a;
+    if (i1 < n) v[rb] = b;
+    __syncthreads();
 }
 
 }  // namespace
@@ -134,31 +198,37 @@ __global__ void __launch_bounds__(kFinishThreads) k_finish(const unsigned long l
                                                            long long* __restrict__ idx, double* __restrict__ dist,
                                                            FinishOut* __restrict__ host) {
     extern __shared__ __align__(16) unsigned char fin_smem[];
-    double* d = (double*)fin_smem;
-    long long* x = (long long*)(d + kFinishSort);
+    Pair* v = (Pair*)fin_smem;
+    PairSort::TempStorage& tmp = *reinterpret_cast<PairSort::TempStorage*>(v + kFinishSort);
     for (int i = threadIdx.x; i < ncnt; i += blockDim.x) host->cnt[i] = cnt[i];
     const unsigned long long n_all = cnt[out_slot];
     const int n = n_all < (unsigned long long)cap ? (int)min(n_all, (unsigned long long)kFinishSort + 1)
                                                   : (int)min(cap, (long long)kFinishSort + 1);
     if (n > kFinishSort) return;
-    int n2 = 1;
-    while (n2 < n) n2 <<= 1;
-    for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-        d[i] = i < n ? (dist ? dist[i] : 0.0) : INFINITY;
-        x[i] = i < n ? idx[i] : 0x7fffffffffffffffLL;
-    }
+    // by index: the distances ride along in idx order (a second read)
+    for (int i = threadIdx.x; i < n; i += blockDim.x) v[i] = Pair{lex ? dist[i] : 0.0, lex ? idx[i] : idx[i] << 13 | i};
     __syncthreads();
-    if (lex)
-        bitonic(n2, [](double da, long long xa, double db, long long xb) { return da < db || (da == db && xa < xb); },
-                d, x);
-    else
-        bitonic(n2, [](double, long long xa, double, long long xb) { return xa < xb; }, d, x);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        idx[i] = x[i];
-        if (dist) dist[i] = d[i];
+    sort_pairs(v, n, tmp);
+    double keep[kFinishSort / kFinishThreads];
+    if (!lex) {
+#pragma unroll
+        for (int u = 0; u < kFinishSort / kFinishThreads; ++u) {
+            const int i = threadIdx.x + u * kFinishThreads;
+            keep[u] = i < n && dist ? dist[v[i].x & 8191] : 0.0;
+        }
+        __syncthreads();  // every distance is read before its place is written
+    }
+#pragma unroll
+    for (int u = 0; u < kFinishSort / kFinishThreads; ++u) {
+        const int i = threadIdx.x + u * kFinishThreads;
+        if (i >= n) continue;
+        const long long x = lex ? v[i].x : v[i].x >> 13;
+        const double d = lex ? v[i].d : keep[u];
+        idx[i] = x;
+        if (dist) dist[i] = d;
         if (i < kFinishOut) {
-            host->idx[i] = x[i];
-            host->dist[i] = d[i];
+            host->idx[i] = x;
+            host->dist[i] = d;
         }
     }
 }
@@ -180,34 +250,35 @@ __global__ void __launch_bounds__(kFinishThreads) k_tau_block(const double* __re
     extern __shared__ __align__(16) unsigned char tau_smem[];
     __shared__ long long s_pick[kRefinePicks];
     __shared__ int s_np, s_n;
-    double* d = (double*)tau_smem;
-    long long* x = (long long*)(d + kFinishSort);
+    Pair* v = (Pair*)tau_smem;
+    PairSort::TempStorage& tmp = *reinterpret_cast<PairSort::TempStorage*>(v + kFinishSort);
     const long long n_all = min((long long)*n_seed, cap);
     const int n = (int)min(n_all, (long long)kFinishSort);
-    int n2 = 1;
-    while (n2 < n) n2 <<= 1;
-    for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-        d[i] = i < n ? dist[i] : INFINITY;
-        x[i] = i < n ? idx[i] : 0x7fffffffffffffffLL;
-    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) v[i] = Pair{dist[i], idx[i]};
     if (threadIdx.x == 0) s_np = s_n = 0;
     __syncthreads();
-    if (!sorted)
-        bitonic(n2, [](double da, long long xa, double db, long long xb) { return da < db || (da == db && xa < xb); },
-                d, x);
-    if (threadIdx.x == 0) *tau = k <= n_all ? (k <= n ? d[k - 1] : dist[k - 1]) : DBL_MAX;
+    if (!sorted) sort_pairs(v, n, tmp);
+    if (threadIdx.x == 0) *tau = k <= n_all ? (k <= n ? v[k - 1].d : dist[k - 1]) : DBL_MAX;
     if (!picks) return;
     if (threadIdx.x < 32) {
+        // best first, 32 seeds at a time: those that clash with no pick so far,
+        // then the first of them again and again
         int np = 0;
-        for (int i = 0; i < min(n, 8 * kRefinePicks) && np < picks; ++i) {
-            bool clash = false;
-            for (int q = threadIdx.x; q < np; q += 32) {
-                const long long gap = x[i] - s_pick[q];
-                clash = clash || (gap <= 2 * kRefineReach && gap >= -2 * kRefineReach);
+        const int lane = threadIdx.x;
+        for (int i0 = 0; i0 < min(n, 8 * kRefinePicks) && np < picks; i0 += 32) {
+            const bool in = i0 + lane < n;
+            const long long x = in ? v[i0 + lane].x : 0;
+            auto near = [&](long long c) { return x - c <= 2 * kRefineReach && c - x <= 2 * kRefineReach; };
+            bool free = in;
+            for (int q = 0; q < np; ++q) free = free && !near(s_pick[q]);
+            unsigned left = __ballot_sync(0xffffffffu, free);
+            while (left && np < picks) {
+                const long long c = __shfl_sync(0xffffffffu, x, __ffs(left) - 1);
+                if (lane == 0) s_pick[np] = c;
+                ++np;
+                free = free && !near(c);
+                left = __ballot_sync(0xffffffffu, free);
             }
-            if (__any_sync(0xffffffffu, clash)) continue;
-            if (threadIdx.x == 0) s_pick[np] = x[i];
-            ++np;
             __syncwarp();
         }
         if (threadIdx.x == 0) s_np = np;
@@ -227,19 +298,16 @@ __global__ void __launch_bounds__(kFinishThreads) k_tau_refine(const double* __r
                                                                const unsigned long long* __restrict__ n_dist,
                                                                long long k, double* tau) {
     extern __shared__ __align__(16) unsigned char ref_smem[];
-    double* d = (double*)ref_smem;
-    long long* x = (long long*)(d + kFinishSort);
+    Pair* v = (Pair*)ref_smem;
+    PairSort::TempStorage& tmp = *reinterpret_cast<PairSort::TempStorage*>(v + kFinishSort);
     const int n = (int)min(*n_dist, (unsigned long long)kFinishSort);
     if (k > n) return;
-    int n2 = 1;
-    while (n2 < n) n2 <<= 1;
-    for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-        d[i] = i < n ? dist[i] : INFINITY;
-        x[i] = 0;
-    }
+    for (int i = threadIdx.x; i < n; i += blockDim.x) v[i] = Pair{dist[i], i};
     __syncthreads();
-    bitonic(n2, [](double da, long long, double db, long long) { return da < db; }, d, x);
-    if (threadIdx.x == 0 && d[k - 1] < *tau) *tau = d[k - 1];
+    sort_pairs(v, n, tmp);
+    if (threadIdx.x == 0 && v[k - 1].d < *tau) *tau = v[k - 1].d;
 }
+
+size_t finish_smem_bytes() { return sizeof(Pair) * kFinishSort + sizeof(PairSort::TempStorage) + 16; }
 
 }  // namespace fsm

@@ -199,6 +199,7 @@ __global__ void k_lb_filter(Geom g, const double* __restrict__ z, const double* 
 constexpr int kFinishThreads = 512;
 constexpr int kFinishSort = 4096;  // results sorted in one block
 constexpr int kFinishOut = 1024;   // results copied
+size_t finish_smem_bytes();
 struct FinishOut {
     unsigned long long cnt[16];
     long long idx[kFinishOut];
