@@ -325,8 +325,8 @@ struct fsmeld_ctx {
     std::map<std::string, Buf> bufs;
     std::map<int, double2*> twiddles;
     // opt-in per-stage device timing (CUDA events around each launch)
-    // pinned host memory: query uploads (grow-only, the size of the largest
-    // query's tables) and what k_finish writes
+    // pinned host memory, one block: what k_finish writes, then query uploads
+    // (grow-only, the size of the largest query's tables)
     unsigned char* pin_up = nullptr;
     size_t pin_up_bytes = 0;
     cudaEvent_t ev_up = nullptr;  // the last upload has been read
@@ -494,15 +494,15 @@ static int twiddle_table(fsmeld_ctx* c, int P, const double2** out) {
 // the context's pinned host memory, at least `bytes` for an upload; the last
 // upload's copy is waited for before its place is written again
 static int pinned(fsmeld_ctx* c, size_t bytes) {
-    if (!c->pin_out) FSM_CUDA_TRY(cudaHostAlloc(&c->pin_out, sizeof(FinishOut), cudaHostAllocDefault));
     if (!c->ev_up) FSM_CUDA_TRY(cudaEventCreateWithFlags(&c->ev_up, cudaEventDisableTiming));
     FSM_CUDA_TRY(cudaEventSynchronize(c->ev_up));
     if (c->pin_up_bytes < bytes) {
-        if (c->pin_up) cudaFreeHost(c->pin_up);
-        c->pin_up = nullptr;
+        if (c->pin_out) cudaFreeHost(c->pin_out);
+        c->pin_out = nullptr;
         c->pin_up_bytes = 0;
-        const size_t want = bytes + bytes / 2;
-        FSM_CUDA_TRY(cudaHostAlloc(&c->pin_up, want, cudaHostAllocDefault));
+        const size_t want = std::max<size_t>(bytes + bytes / 2, 64 << 10);
+        FSM_CUDA_TRY(cudaHostAlloc(&c->pin_out, sizeof(FinishOut) + want, cudaHostAllocDefault));
+        c->pin_up = (unsigned char*)(c->pin_out + 1);
         c->pin_up_bytes = want;
     }
     return FSMELD_OK;
@@ -590,8 +590,8 @@ struct Stats {
 
 static int run_stats(fsmeld_ctx* c, const Geom& g, Stats* st, const std::string& tag) {
     int r;
-    if ((r = bufT(c, "mu" + tag, (size_t)g.S * g.kml, &st->MU))) return r;
-    if ((r = bufT(c, "sig" + tag, (size_t)g.S * g.kml, &st->SIG))) return r;
+    if ((r = bufT(c, "stats" + tag, 2 * (size_t)g.S * g.kml, &st->MU))) return r;
+    st->SIG = st->MU + (size_t)g.S * g.kml;
     const size_t smem = mvmean_smem_bytes();
     if ((r = allow_smem(c, k_mvmean, smem))) return r;
     const int seg = mvmean_segments(g.S, c->sm_count);
@@ -623,16 +623,12 @@ static int launch_env(fsmeld_ctx* c, const Geom& g, int w, Stats* st) {
 
 static int run_env(fsmeld_ctx* c, const Geom& g, int w, Stats* st, const std::string& tag) {
     int r;
-    if ((r = bufT(c, "un" + tag, (size_t)g.S * g.m_k, &st->Un))) return r;
-    if ((r = bufT(c, "ln" + tag, (size_t)g.S * g.m_k, &st->Ln))) return r;
-    if ((r = bufT(c, "lraw" + tag, (size_t)g.n, &st->Lraw))) return r;
-    if ((r = bufT(c, "uraw" + tag, (size_t)g.n, &st->Uraw))) return r;
+    if ((r = bufT(c, "env" + tag, 2 * (size_t)g.S * g.m_k + 2 * (size_t)g.n, &st->Un))) return r;
+    st->Ln = st->Un + (size_t)g.S * g.m_k;
+    st->Lraw = st->Ln + (size_t)g.S * g.m_k;
+    st->Uraw = st->Lraw + (size_t)g.n;
     st->Clo = st->Cup = nullptr;
-    if (!c->lean) {
-        if (buf_optional(c, "clo" + tag, sizeof(double) * (size_t)g.n, &st->Clo) &&
-            !buf_optional(c, "cup" + tag, sizeof(double) * (size_t)g.n, &st->Cup))
-            st->Clo = nullptr;
-    }
+    if (!c->lean && buf_optional(c, "ctr" + tag, sizeof(double) * 2 * (size_t)g.n, &st->Clo)) st->Cup = st->Clo + g.n;
     {
         const size_t fsm = fwd_env_smem_bytes(w, st->Clo != nullptr);
         if ((r = allow_smem(c, k_fwd_env, fsm))) return r;
@@ -766,6 +762,21 @@ static int run_lbip(fsmeld_ctx* c, const Geom& g, LbJob job) {
     return FSMELD_OK;
 }
 
+// A query's lists of up to `cap` windows, in one buffer (an allocation takes the
+// driver as long as a small query): the LB_IP survivors, later what the screen
+// leaves; the results; and, where GLB runs, its two stages.
+enum { L_SURV, L_OUTI, L_OUTD, L_EXACT, L_G1 = L_EXACT, L_G1B, L_G1T, L_G2, L_G2T, L_ALL };
+struct Lists {
+    double* p = nullptr;
+    size_t cap = 0;
+    double* d(int slot) const { return p + (size_t)slot * cap; }
+    long long* i(int slot) const { return (long long*)d(slot); }
+};
+static int lists(fsmeld_ctx* c, long long cap, int slots, Lists* l) {
+    l->cap = (size_t)cap;
+    return bufT(c, "lists", (size_t)slots * (size_t)cap, &l->p);
+}
+
 // counters slot layout
 enum { C_SURV, C_G1, C_G2, C_OUT, C_VALID, C_SEED, C_SEEDOUT, C_DPNEXT, C_CELLS, C_SCREEN, C_REF, C_REFOUT, C_N };
 
@@ -774,13 +785,11 @@ static bool use_bitdp(const fsmeld_ctx* c, const QueryDev& q) { return q.bit.E &
 static int run_glb(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const Stats& st, const long long* in,
                    unsigned long long* cnt, long long cap, long long* segc, long long** out_list,
                    double** out_qt, double** out_tq, const double* cutoff_ptr = nullptr) {
-    long long *g1, *g2;
-    double *g1b, *g1t;
     int r;
-    if ((r = bufT(c, "g1", (size_t)cap, &g1))) return r;
-    if ((r = bufT(c, "g1b", (size_t)cap, &g1b))) return r;
-    if ((r = bufT(c, "g1t", (size_t)cap, &g1t))) return r;
-    if ((r = bufT(c, "g2", (size_t)cap, &g2))) return r;
+    Lists l;
+    if ((r = lists(c, cap, L_ALL, &l))) return r;
+    long long *g1 = l.i(L_G1), *g2 = l.i(L_G2);
+    double *g1b = l.d(L_G1B), *g1t = l.d(L_G1T), *g2t = l.d(L_G2T);
     GlbJob j1{};
     j1.q = qd; j1.target = c->d_target; j1.MU = st.MU; j1.SIG = st.SIG;
     j1.lraw = st.Lraw; j1.uraw = st.Uraw; j1.clo = st.Clo; j1.cup = st.Cup;
@@ -804,8 +813,6 @@ static int run_glb(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const Stats
     }
     LAUNCH_CHECK(c);
     GlbJob j2 = j1;
-    double* g2t;
-    if ((r = bufT(c, "g2t", (size_t)cap, &g2t))) return r;
     j2.in = g1; j2.in_b = g1b; j2.in_t = g1t; j2.n_in = cnt + C_G1;
     j2.out = g2; j2.out_b = nullptr; j2.out_t = g2t; j2.n_out = cnt + C_G2;
     // the bit-vector DP bounds what is to come by the T->Q sums, the others by
@@ -1086,10 +1093,10 @@ static int search_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     long long* g2;
     double *g2t, *g2q;
     if ((r = run_glb(c, g, qd, st, surv, cnt, cap, segc, &g2, &g2t, &g2q))) return r;
-    long long* oi;
-    double* od;
-    if ((r = bufT(c, "outi", (size_t)cap, &oi))) return r;
-    if ((r = bufT(c, "outd", (size_t)cap, &od))) return r;
+    Lists l;
+    if ((r = lists(c, cap, L_ALL, &l))) return r;
+    long long* oi = l.i(L_OUTI);
+    double* od = l.d(L_OUTD);
     DpJob dj{};
     dj.q = qd; dj.target = c->d_target; dj.MU = st.MU; dj.SIG = st.SIG;
     dj.lraw = st.Lraw; dj.uraw = st.Uraw;
@@ -1134,16 +1141,15 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     const int per_seg =
         (int)std::min<long long>(32, std::max<long long>(std::max<long long>(1, few_seg), (2 * qr.k + g.S - 1) / g.S));
     const long long nslot = g.S * per_seg;
+    // seeds: windows, evaluated windows and distances; refining windows likewise; tau
     long long* seeds;
-    if ((r = bufT(c, "seeds", (size_t)nslot, &seeds))) return r;
+    if ((r = bufT(c, "seeds", 3 * (size_t)nslot + 3 * (size_t)kFinishSort + 1, &seeds))) return r;
     prof_begin(c, ST_SELECT);
     k_seed<<<(unsigned)std::min<long long>(g.S, (long long)c->sm_count * 8), 256, 0, c->stream>>>(
         g, z, st.SIG, per_seg, seeds, cnt + C_SEED, nslot);
     LAUNCH_CHECK(c);
-    long long* si;
-    double* sd;
-    if ((r = bufT(c, "seedi", (size_t)nslot, &si))) return r;
-    if ((r = bufT(c, "seedd", (size_t)nslot, &sd))) return r;
+    long long* si = seeds + nslot;
+    double* sd = (double*)(si + nslot);
     const bool tau_block = nslot <= kFinishSort;
     // (radix sort) unused seed slots hold all-ones bit patterns, which sort after every distance
     if (!tau_block) FSM_CUDA_TRY(cudaMemsetAsync(sd, 0xff, sizeof(double) * (size_t)nslot, c->stream));
@@ -1154,8 +1160,8 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     if ((r = run_dp(c, g, sj, nslot))) return r;
     // tau = k-th smallest seed distance, selected on the device: the rest of
     // the query reads it from device memory, so the host waits only once
-    double* tau_dev;
-    if ((r = bufT(c, "tau", 1, &tau_dev))) return r;
+    long long *rl = (long long*)(sd + nslot), *ri = rl + kFinishSort;
+    double *rd = (double*)(ri + kFinishSort), *tau_dev = rd + kFinishSort;
     // refining windows: about 1024 of them or 2k; large k and seeds that give no
     // bound go without
     const long long span = 2 * kRefineReach + 1;
@@ -1181,13 +1187,6 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     }
     {
         const size_t smem = finish_smem_bytes();
-        long long *rl = nullptr, *ri = nullptr;
-        double* rd = nullptr;
-        if (picks) {
-            if ((r = bufT(c, "refl", (size_t)kFinishSort, &rl))) return r;
-            if ((r = bufT(c, "refi", (size_t)kFinishSort, &ri))) return r;
-            if ((r = bufT(c, "refd", (size_t)kFinishSort, &rd))) return r;
-        }
         if ((r = allow_smem(c, k_tau_block, smem))) return r;
         prof_begin(c, ST_SELECT);
         k_tau_block<<<1, kFinishThreads, smem, c->stream>>>(sdist, sidx, tau_block ? 0 : 1, cnt + C_SEEDOUT, nslot, qr.k,
@@ -1208,8 +1207,9 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
         }
     }
     // filter, GLB and DP at tau
-    long long* f1;
-    if ((r = bufT(c, "surv", (size_t)cap, &f1))) return r;
+    Lists l;
+    if ((r = lists(c, cap, L_ALL, &l))) return r;
+    long long* f1 = l.i(L_SURV);
     prof_begin(c, ST_SELECT);
     k_lb_filter<<<(unsigned)std::min<long long>((g.tsn + 2047) / 2048, (long long)c->sm_count * 8), 256, 0, c->stream>>>(
         g, z, st.SIG, tau_dev, qd.metric, f1, cnt + C_SURV, cap);
@@ -1219,10 +1219,8 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     long long* g2;
     double *g2t, *g2q;
     if ((r = run_glb(c, g, qt, st, f1, cnt, cap, nullptr, &g2, &g2t, &g2q, tau_dev))) return r;
-    long long* oi;
-    double* od;
-    if ((r = bufT(c, "outi", (size_t)cap, &oi))) return r;
-    if ((r = bufT(c, "outd", (size_t)cap, &od))) return r;
+    long long* oi = l.i(L_OUTI);
+    double* od = l.d(L_OUTD);
     DpJob dj{};
     dj.q = qt; dj.target = c->d_target; dj.MU = st.MU; dj.SIG = st.SIG;
     dj.lraw = st.Lraw; dj.uraw = st.Uraw;
@@ -1272,15 +1270,15 @@ static int run_query(fsmeld_ctx* c, const QueryRun& qr, const Geom& g0, Stats& s
     out.tail = g.tsn % g.kml;
 
     if (qr.mode == 2) {  // exact: every valid window through the DP
-        long long *oi;
-        double* od;
-        if ((r = bufT(c, "outi", (size_t)cap, &oi))) return r;
-        if ((r = bufT(c, "outd", (size_t)cap, &od))) return r;
+        Lists l;
+        if ((r = lists(c, cap, L_EXACT, &l))) return r;
+        long long* oi = l.i(L_OUTI);
+        double* od = l.d(L_OUTD);
         qd.cutoff = qr.cutoff;
         DpJob dj{};
         dj.q = qd; dj.target = c->d_target; dj.MU = st.MU; dj.SIG = st.SIG;
         dj.list = nullptr; dj.n_windows = g.tsn; dj.list_cap = cap; dj.mode = 0; dj.cutoff = qr.cutoff;
-        if ((r = bufT(c, "surv", (size_t)cap, &dj.screened))) return r;
+        dj.screened = l.i(L_SURV);
         dj.n_screened = cnt + C_SCREEN;
         dj.out_idx = oi; dj.out_dist = od; dj.n_out = cnt + C_OUT; dj.n_cells = cnt + C_CELLS; dj.out_cap = cap; dj.n_valid = cnt + C_VALID;
         if ((r = run_dp(c, g, dj, g.tsn))) return r;
@@ -1309,8 +1307,9 @@ static int run_query(fsmeld_ctx* c, const QueryRun& qr, const Geom& g0, Stats& s
     if ((r = bufT(c, "segc", (size_t)3 * g.S, &segc))) return r;
 
     if (qr.mode == 0) {  // search
-        long long* surv;
-        if ((r = bufT(c, "surv", (size_t)cap, &surv))) return r;
+        Lists l;
+        if ((r = lists(c, cap, L_ALL, &l))) return r;
+        long long* surv = l.i(L_SURV);
         qd.cutoff = qr.cutoff;
         LbJob lj{};
         lj.q = qd; lj.Un = st.Un; lj.Ln = st.Ln; lj.thr = thr; lj.SIG = st.SIG;
@@ -1576,8 +1575,9 @@ static int run_search_gemm(fsmeld_ctx* c, const Geom& g0, Stats& st, const std::
                     return fail(FSMELD_E_FEWER_K, "Fewer valid, non-excluded candidates than requested k.");
                 return cutoff_tail(x, g, qd, st, zq + (size_t)i * g0.S * g0.kml, cnt, qr);
             }
-            long long* surv;
-            if ((rr = bufT(x, "surv", (size_t)cap, &surv))) return rr;
+            Lists l;
+            if ((rr = lists(x, cap, L_ALL, &l))) return rr;
+            long long* surv = l.i(L_SURV);
             prof_begin(x, ST_LBIP);
             k_bits_to_list<<<(unsigned)std::min<long long>((words + 255) / 256, (long long)x->sm_count * 8), 256, 0,
                              x->stream>>>(dbits + (size_t)i * words, words, surv, cap, cnt + C_SURV);
@@ -1811,8 +1811,7 @@ static int run_tasks_parallel(fsmeld_ctx* c, std::vector<QueryRun>& runs, const 
 static void drop_centred(fsmeld_ctx* c, Stats& st) {
     if (!st.Clo) return;
     st.Clo = st.Cup = nullptr;
-    release_buf(c, "clo");
-    release_buf(c, "cup");
+    release_buf(c, "ctr");
 }
 
 // One call over many queries: statistics per distinct m, envelopes per distinct
@@ -1981,11 +1980,11 @@ static int open_common(int device, fsmeld_ctx** out) {
     c->device = device;
     cudaError_t e = cudaSetDevice(device);
     if (e != cudaSuccess) { delete c; return cuda_fail(e, "cudaSetDevice", __FILE__, __LINE__); }
-    cudaDeviceProp prop;
-    e = cudaGetDeviceProperties(&prop, device);
-    if (e != cudaSuccess) { delete c; return cuda_fail(e, "cudaGetDeviceProperties", __FILE__, __LINE__); }
-    c->sm_count = prop.multiProcessorCount;
-    c->smem_optin = (int)prop.sharedMemPerBlockOptin;
+    if ((e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&c->smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device)) != cudaSuccess) {
+        delete c;
+        return cuda_fail(e, "cudaDeviceGetAttribute", __FILE__, __LINE__);
+    }
     if (const char* ex = getenv("FSMELD_DP_EXACT")) c->dp_exact = ex[0] == '1';
     if (const char* f = getenv("FSMELD_DP_FORM")) c->dp_form = !strcmp(f, "lane") ? 1 : !strcmp(f, "wave") ? 2 : 0;
     if (const char* f = getenv("FSMELD_LB_FORM")) c->lb_form = !strcmp(f, "fft") ? 1 : !strcmp(f, "gemm") ? 2 : 0;
@@ -2068,7 +2067,6 @@ int fsmeld_close(fsmeld_ctx* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     for (auto& kv : c->bufs) if (kv.second.p) cudaFree(kv.second.p);
     for (auto& kv : c->twiddles) cudaFree(kv.second);
-    if (c->pin_up) cudaFreeHost(c->pin_up);
     if (c->pin_out) cudaFreeHost(c->pin_out);
     if (c->ev_up) cudaEventDestroy(c->ev_up);
     for (auto& r : c->pending) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
