@@ -1461,7 +1461,11 @@ static int run_search_gemm(fsmeld_ctx* c, const Geom& g0, Stats& st, const std::
                 // split's residual and a relative 2^-40 for these host sums
                 marg[2 * i + side] = (R + 4.0 * nadd * std::ldexp(S, -23)) * (1.0 + std::ldexp(1.0, -40)) + 1e-300;
             }
-            cut[i] = topk ? DBL_MAX : qr.cutoff;
+            {
+                QueryDev kq{};
+                kq.metric = hq.metric; kq.m = m; kq.cutoff = topk ? DBL_MAX : qr.cutoff;
+                cut[i] = topk ? DBL_MAX : lbip_keep_max(kq);
+            }
             met[i] = hq.metric;
             const bool ex = qr.eb >= 0 && qr.ee > qr.eb;
             eb[i] = ex ? qr.eb : -1;
@@ -1496,7 +1500,7 @@ static int run_search_gemm(fsmeld_ctx* c, const Geom& g0, Stats& st, const std::
         GemmJob gj{};
         gj.Un = st.Un; gj.Ln = st.Ln; gj.SIG = st.SIG; gj.t_l = th.t_l; gj.t_u = th.t_u;
         gj.B = (const uint4*)dB; gj.m = m; gj.nq = nq; gj.kchunks = kchunks;
-        gj.margin_l = dM; gj.margin_u = dM + nq; gj.metric = dMet; gj.cutoff = dC;
+        gj.margin_l = dM; gj.margin_u = dM + nq; gj.metric = dMet; gj.keep_max = dC;
         gj.excl_b = dE; gj.excl_e = dE + nq;
         double* zq = zout_dev;
         if (topk && !zq && (r = bufT(c, "gemmZ", (size_t)nq * g0.S * g0.kml, &zq))) return r;

@@ -37,8 +37,9 @@
 // them to an mbarrier; the next chunk's operands are written once that
 // mbarrier says the MMAs have read the current ones.  The epilogue: thread r
 // reads TMEM lane r (window j0 + r) with tcgen05.ld, forms each query's
-// bound (src/fsmeld.cpp:84-106) and prune test (include/fsmeld_internal.h:
-// 9-19) in FP64, and sets the survivors' bits in the query's window bit mask
+// inner product and compares it with the largest one the prune test keeps
+// (src/fsmeld.cpp:84-106, include/fsmeld_internal.h:9-19; the host's bisection),
+// and sets the survivors' bits in the query's window bit mask
 // (one atomic OR per warp, query and word); k_bits_to_list turns a mask into
 // the survivor list the GLB stage reads.
 //
@@ -257,20 +258,23 @@ __global__ void __launch_bounds__(kGemmThreads) k_lbgemm(Geom g, GemmJob job) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const int q = q0 + i;
-                double z = dnan();
+                const bool ok = q < job.nq && sig_ok && !(job.excl_b[q] >= 0 && gi >= job.excl_b[q] && gi < job.excl_e[q]);
                 bool keep = false;
-                if (q < job.nq && sig_ok && !(job.excl_b[q] >= 0 && gi >= job.excl_b[q] && gi < job.excl_e[q])) {
+                double zz = 0.0;
+                if (ok) {
                     const double zl = dmax0(dsub((double)__uint_as_float(rl[i]), job.margin_l[q]));
                     const double zu = dmax0(dsub((double)__uint_as_float(ru[i]), job.margin_u[q]));
-                    const double zz = dadd(zl, zu);
+                    zz = dadd(zl, zu);
+                    keep = !(zz > job.keep_max[q]);  // the prune test, without its square roots
+                }
+                if (job.zout && j < kml && q < job.nq) {
                     const int metric = job.metric[q];
+                    double z = zz;
                     if (metric == DTW || metric == ERP) z = dsqrt(zz);
                     else if (metric == LCSS) z = ddiv(zz, (double)m);
-                    else z = zz;
-                    keep = !lbip_exceeds(z, job.cutoff[q], metric);
+                    job.zout[(size_t)q * job.zstride + s * kml + j] = ok ? z : dnan();
                 }
-                if (job.zout && j < kml && q < job.nq) job.zout[(size_t)q * job.zstride + s * kml + j] = z;
-                const unsigned bv = __ballot_sync(0xffffffffu, !isnan(z));
+                const unsigned bv = __ballot_sync(0xffffffffu, ok);
                 const unsigned bk = __ballot_sync(0xffffffffu, keep);
                 if (lane == 0 && q < job.nq) {
                     if (bv) atomicAdd(&s_valid[i], __popc(bv));
@@ -334,34 +338,42 @@ __global__ void __launch_bounds__(256) k_gemm_masks(Geom g, const double* __rest
 }
 
 // survivor bit mask -> list of window indices (ascending within a block of
-// 8192 windows; blocks append in any order)
+// 8192 windows; blocks append in any order).  A warp takes 32 words: their
+// counts by a shuffle scan, then a word at a time, a lane per bit, so the
+// stores are coalesced.
 __global__ void __launch_bounds__(256) k_bits_to_list(const unsigned* __restrict__ bits, long long words,
                                                       long long* __restrict__ out, long long cap,
                                                       unsigned long long* __restrict__ n) {
-    __shared__ int s_pre[256];
+    __shared__ int s_cnt[8];
     __shared__ unsigned long long s_off;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (long long b0 = (long long)blockIdx.x * 256; b0 < words; b0 += (long long)gridDim.x * 256) {
         const long long wi = b0 + tid;
         const unsigned v = wi < words ? bits[wi] : 0u;
         const int c = __popc(v);
-        s_pre[tid] = c;
-        __syncthreads();
-        for (int d = 1; d < 256; d <<= 1) {
-            const int x = tid >= d ? s_pre[tid - d] : 0;
-            __syncthreads();
-            s_pre[tid] += x;
-            __syncthreads();
+        int inc = c;
+        for (int d = 1; d < 32; d <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += x;
         }
-        if (tid == 255) s_off = s_pre[255] ? atomicAdd(n, (unsigned long long)s_pre[255]) : 0ull;
+        if (lane == 31) s_cnt[warp] = inc;
         __syncthreads();
-        unsigned long long o = s_off + s_pre[tid] - c;
-        unsigned r = v;
-        while (r) {
-            const int bit = __ffs(r) - 1;
-            r &= r - 1;
-            if (o < (unsigned long long)cap) out[o] = wi * 32 + bit;
-            ++o;
+        int before = 0, total = 0;
+        for (int i = 0; i < 8; ++i) {
+            before += i < warp ? s_cnt[i] : 0;
+            total += s_cnt[i];
+        }
+        if (tid == 0) s_off = total ? atomicAdd(n, (unsigned long long)total) : 0ull;
+        __syncthreads();
+        const unsigned long long o = s_off + before;
+        const unsigned below = (1u << lane) - 1;
+        for (int i = 0; i < 32; ++i) {
+            const unsigned x = __shfl_sync(0xffffffffu, v, i);
+            const int at = __shfl_sync(0xffffffffu, inc - c, i);
+            if (x >> lane & 1u) {
+                const unsigned long long p = o + at + __popc(x & below);
+                if (p < (unsigned long long)cap) out[p] = (b0 + warp * 32 + i) * 32 + lane;
+            }
         }
         __syncthreads();
     }

@@ -92,7 +92,7 @@ struct GemmJob {
     const double* margin_l;     // rounding-error margins of the lower / upper inner products
     const double* margin_u;
     const int* metric;
-    const double* cutoff;
+    const double* keep_max;     // the largest inner product the prune test keeps
     const long long* excl_b;    // exclusion interval per query (-1: none)
     const long long* excl_e;
     double* zout;               // optional: bound per window, [q][zstride]
