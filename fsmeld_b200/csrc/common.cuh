@@ -216,6 +216,7 @@ struct QueryDev {
     int m, w, metric, p;
     double arg;
     double cutoff;
+    double qlo, qhi;       // smallest and largest point of qn
     const double* qn;      // normalised query, original order [m]
     const double* LQ;      // query envelope (radius w) [m]
     const double* UQ;

@@ -155,7 +155,7 @@ static double match_end(double x, double eps) {
 // candidate values y with A_i <= y < B_i.  The bucket of an end comes from the
 // operations of the device's lookup (bit_rank), so equal values fall in equal
 // buckets and the buckets ascend with the values.
-static void match_table(HostQuery* hq) {
+void match_table(HostQuery* hq) {
     const int m = hq->m, ne = 2 * m;
     std::vector<std::pair<double, int>> ev(ne);
     for (int i = 0; i < m; ++i) {
@@ -568,6 +568,8 @@ static int upload_query(fsmeld_ctx* c, const HostQuery& hq, const std::string& s
     const int* I = (const int*)(D + nd);
     qd->m = m; qd->w = hq.w; qd->metric = hq.metric; qd->p = hq.p; qd->arg = hq.arg;
     qd->cutoff = 0.0;
+    qd->qlo = hq.qs.front();
+    qd->qhi = hq.qs.back();
     qd->qn = D + o_qn; qd->LQ = D + o_LQ; qd->UQ = D + o_UQ; qd->qs = D + o_qs;
     qd->pw = D + o_pw; qd->Dq = D + o_Dq; qd->tlq = D + o_tlq; qd->tuq = D + o_tuq;
     qd->opw = D + o_opw; qd->oD = D + o_oD; qd->otl = D + o_otl; qd->otu = D + o_otu;
@@ -803,13 +805,16 @@ static int run_glb(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const Stats
                     : qd.metric == EDR ? (const void*)k_glb_tq<EDR>
                     : qd.metric == LCSS ? (const void*)k_glb_tq<LCSS> : (const void*)k_glb_tq<MSM>;
     if ((r = allow_smem(c, tqf, sm1))) return r;
+    int tq_sm = 0;
+    FSM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&tq_sm, tqf, 256, sm1));
+    const unsigned g1grid = (unsigned)(std::max(1, tq_sm) * c->sm_count);
     prof_begin(c, ST_GLB1);
     switch (qd.metric) {
-        case DTW: k_glb_tq<DTW><<<c->sm_count * 8, 256, sm1, c->stream>>>(g, j1); break;
-        case ERP: k_glb_tq<ERP><<<c->sm_count * 8, 256, sm1, c->stream>>>(g, j1); break;
-        case EDR: k_glb_tq<EDR><<<c->sm_count * 8, 256, sm1, c->stream>>>(g, j1); break;
-        case LCSS: k_glb_tq<LCSS><<<c->sm_count * 8, 256, sm1, c->stream>>>(g, j1); break;
-        default: k_glb_tq<MSM><<<c->sm_count * 8, 256, sm1, c->stream>>>(g, j1); break;
+        case DTW: k_glb_tq<DTW><<<g1grid, 256, sm1, c->stream>>>(g, j1); break;
+        case ERP: k_glb_tq<ERP><<<g1grid, 256, sm1, c->stream>>>(g, j1); break;
+        case EDR: k_glb_tq<EDR><<<g1grid, 256, sm1, c->stream>>>(g, j1); break;
+        case LCSS: k_glb_tq<LCSS><<<g1grid, 256, sm1, c->stream>>>(g, j1); break;
+        default: k_glb_tq<MSM><<<g1grid, 256, sm1, c->stream>>>(g, j1); break;
     }
     LAUNCH_CHECK(c);
     GlbJob j2 = j1;

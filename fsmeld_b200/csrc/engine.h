@@ -23,6 +23,8 @@ struct HostQuery {
 
 // raw: the query is used as given (no z-normalisation; raw mode)
 int prepare_query(const double* q, int m, int metric, int w, double arg, HostQuery* hq, bool raw = false);
+// the matching intervals of an EDR or LCSS query (qn, arg set)
+void match_table(HostQuery* hq);
 int macro_length(int m, long long available);
 extern thread_local std::string g_last_error;
 

@@ -211,9 +211,7 @@ __global__ void __launch_bounds__(kDpThreads) k_dp(Geom g, DpJob job) {
     } else if (METRIC == LCSS) {
         ylim = (fabs(arg) < 1e299) ? INFINITY : -1.0;  // padding must never match
     } else {
-        double xm = 0.0;
-        for (int k = lane; k < m; k += 32) xm = fmax(xm, fabs(X[k]));
-        for (int o = 16; o; o >>= 1) xm = fmax(xm, __shfl_xor_sync(0xffffffffu, xm, o));
+        const double xm = fmax(-q.qlo, q.qhi);
         ylim = sqrt(1e17 / (2.0 * m + 2.0)) - xm - fabs(arg) - 2.0;
     }
     const bool query_exact = job.force_exact || !(ylim > 0.0);

@@ -310,16 +310,8 @@ struct Fix {
 template <int METRIC>
 __device__ __forceinline__ Fix make_fix(const QueryDev& q, double bsf, bool raw) {
     Fix f;
-    const int m = q.m, lane = threadIdx.x & 31;
-    double xl = INFINITY, xh = -INFINITY;
-    for (int k = lane; k < m; k += 32) {
-        xl = fmin(xl, q.qn[k]);
-        xh = fmax(xh, q.qn[k]);
-    }
-    for (int o = 16; o; o >>= 1) {
-        xl = fmin(xl, __shfl_xor_sync(0xffffffffu, xl, o));
-        xh = fmax(xh, __shfl_xor_sync(0xffffffffu, xh, o));
-    }
+    const int m = q.m;
+    const double xl = q.qlo, xh = q.qhi;
     const double ymax = raw ? 2.0 * (xh - xl) + 1.0 : fmax(fmax(xh, -xl), sqrt((double)m)) * 1.01 + 1.0;
     f.exact = !(ymax < 1e200) || !(bsf < kGlbMax);
     f.scale = scalbn(1.0, f.exact ? 0 : 21 - ilogb(ymax));  // ymax 2^K < 2^22
@@ -476,7 +468,10 @@ __global__ void __launch_bounds__(256, 4) k_glb_tq(Geom g, GlbJob job) {
     float2* LU = gtq_smem;  // [m] query envelope as F
     float2* Qx = LU + m;    // [m] query points as F (x)
     const double bsf = job.cutoff_ptr ? *job.cutoff_ptr : q.cutoff;
-    const Fix f = make_fix<METRIC>(q, bsf, g.raw != 0);
+    __shared__ Fix s_fix;  // one thread's divisions and roots serve the block
+    if (threadIdx.x == 0) s_fix = make_fix<METRIC>(q, bsf, g.raw != 0);
+    __syncthreads();
+    const Fix f = s_fix;
     for (int i = threadIdx.x; i < m; i += blockDim.x) {
         LU[i] = make_float2(fix_units(q.LQ[i], f), fix_units(q.UQ[i], f));
         Qx[i] = make_float2(fix_units(q.qn[i], f), 0.f);
@@ -654,7 +649,10 @@ __global__ void __launch_bounds__(256, 3) k_glb_qt(Geom g, GlbJob job) {
     const int m = q.m, w = q.w;
     float2* Qx = gqt_smem;  // [m] query points as F, and (ERP) their distance to the gap
     const double bsf = job.cutoff_ptr ? *job.cutoff_ptr : q.cutoff;
-    const Fix f = make_fix<METRIC>(q, bsf, g.raw != 0);
+    __shared__ Fix s_fix;
+    if (threadIdx.x == 0) s_fix = make_fix<METRIC>(q, bsf, g.raw != 0);
+    __syncthreads();
+    const Fix f = s_fix;
     for (int i = threadIdx.x; i < m; i += blockDim.x) {
         const float x = fix_units(q.qn[i], f);
         Qx[i] = make_float2(x, x - f.a);

@@ -109,9 +109,7 @@ __global__ void __launch_bounds__(kScreenThreads) k_screen(Geom g, DpJob job, lo
     const double cut = job.cutoff_ptr ? *job.cutoff_ptr : job.cutoff;
     const float arg = (float)q.arg;
 
-    double xm = 0.0;
-    for (int k = lane; k < m; k += 32) xm = fmax(xm, fabs(X[k]));
-    for (int o = 16; o; o >>= 1) xm = fmax(xm, __shfl_xor_sync(kAll, xm, o));
+    const double xm = fmax(-q.qlo, q.qhi);
     const double ymax = 2.0 * xm + 8.0;
     const double cut_s = cut + 1e-9 * (1.0 + fabs(cut));
     const double delta = 0x1p-22 * (xm + ymax + fabs(q.arg)) * 1.01;

@@ -233,6 +233,30 @@ __global__ void __launch_bounds__(kFinishThreads) k_finish(const unsigned long l
     }
 }
 
+// Up to kFinishSort matches in window order into the caller's buffers; *total
+// is their number, or kFinishSort + 1 or more when they are left as they are.
+__global__ void __launch_bounds__(kFinishThreads) k_order(const unsigned long long* __restrict__ n_in,
+                                                          const long long* __restrict__ idx,
+                                                          const double* __restrict__ dist,
+                                                          long long* __restrict__ out_idx,
+                                                          double* __restrict__ out_dist, long long cap,
+                                                          unsigned long long* __restrict__ total) {
+    extern __shared__ __align__(16) unsigned char ord_smem[];
+    Pair* v = (Pair*)ord_smem;
+    PairSort::TempStorage& tmp = *reinterpret_cast<PairSort::TempStorage*>(v + kFinishSort);
+    const unsigned long long n_all = *n_in;
+    if (threadIdx.x == 0) *total = n_all;
+    if (n_all > (unsigned long long)kFinishSort) return;
+    const int n = (int)n_all;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) v[i] = Pair{0.0, idx[i] << 13 | i};
+    __syncthreads();
+    sort_pairs(v, n, tmp);
+    for (int i = threadIdx.x; i < n && i < cap; i += blockDim.x) {
+        out_idx[i] = v[i].x >> 13;
+        out_dist[i] = dist[v[i].x & 8191];
+    }
+}
+
 // The bound tau (the k-th smallest seed distance, DBL_MAX with fewer than k
 // seeds) and the windows to refine it with.  Seeds lie at the smallest bound of
 // their stretch; the windows next to a good match are good matches too, and

@@ -207,6 +207,9 @@ struct FinishOut {
 };
 __global__ void k_finish(const unsigned long long* __restrict__ cnt, int ncnt, int out_slot, long long cap, int lex,
                          long long* __restrict__ idx, double* __restrict__ dist, FinishOut* __restrict__ host);
+__global__ void k_order(const unsigned long long* __restrict__ n_in, const long long* __restrict__ idx,
+                        const double* __restrict__ dist, long long* __restrict__ out_idx,
+                        double* __restrict__ out_dist, long long cap, unsigned long long* __restrict__ total);
 // top-k: tau from the seeds, and the windows around the best of them
 constexpr int kRefineReach = 15;
 constexpr int kRefinePicks = 132;  // 132 x 31 windows fit kFinishSort

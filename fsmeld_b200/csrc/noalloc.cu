@@ -7,9 +7,17 @@
 // (every valid window through the banded elastic DP, matches at or below the
 // cutoff) with caller-owned device inputs and outputs and a caller stream.
 // Its scratch -- window statistics, the DP's work and match counters and
-// match list, and an ordering buffer -- lives in one file-scope
+// match list, an ordering buffer (first the list of what the FP32 screen
+// leaves) and the matching table of EDR and LCSS -- lives in one file-scope
 // `static __device__` array of kScratchBytes (12 MiB), which every GPU that
 // loads the library holds until the process exits.
+//
+// The DPs are those of the allocating path: DTW, ERP and MSM go through the
+// FP32 screen and the wavefront DP, EDR and LCSS through the bit vectors, a
+// cutoff that no bound can reach and bands below 2 through the lane DP.  Up to
+// kFinishSort matches are put in window order by one block; more are marked at
+// their windows and compacted.  120,000 points, DTW, m = 200, w = 10: 0.47 ms
+// with the lane DP on every window and a serial compaction, 0.24 ms now.
 //
 // Limits: at most FSMELD_NOALLOC_MAX_WINDOWS windows (n - m + 1) and
 // m <= FSMELD_NOALLOC_MAX_M per call; the DP band and candidate ring of the
@@ -53,7 +61,8 @@ constexpr size_t kOffSig = kOffMu + sizeof(double) * kStatN;           // window
 constexpr size_t kOffLi = kOffSig + sizeof(double) * kStatN;           // DP match indices
 constexpr size_t kOffLd = kOffLi + sizeof(long long) * kMaxWin;        // DP match distances
 constexpr size_t kOffWin = kOffLd + sizeof(double) * kMaxWin;          // distance per window
-constexpr size_t kNeed = kOffWin + sizeof(double) * kMaxWin;
+constexpr size_t kOffBit = kOffWin + sizeof(double) * kMaxWin;         // EDR, LCSS: matching table and its inputs
+constexpr size_t kNeed = kOffBit;
 constexpr size_t kScratchBytes = 12u << 20;
 static_assert(kNeed <= kScratchBytes, "scratch layout exceeds the static array");
 
@@ -196,9 +205,6 @@ static int exact_noalloc(int device, const double* device_target, int64_t n, con
     if ((e = cudaMemcpyAsync(qn, t_qn, sizeof(double) * m, cudaMemcpyHostToDevice, st)) != cudaSuccess)
         return cuda_fail(e, "cudaMemcpyAsync(query)", __FILE__, __LINE__);
     if ((e = cudaMemsetAsync(cnt, 0, 256, st)) != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync", __FILE__, __LINE__);
-    if ((e = cudaMemsetAsync(win, 0xff, sizeof(double) * g.tsn, st)) != cudaSuccess)
-        return cuda_fail(e, "cudaMemsetAsync", __FILE__, __LINE__);
-
     const size_t sm_stats = mvmean_smem_bytes();
     if ((e = raise_smem_limit((const void*)k_mvmean, device, sm_stats)) != cudaSuccess)
         return cuda_fail(e, "cudaFuncSetAttribute", __FILE__, __LINE__);
@@ -208,32 +214,107 @@ static int exact_noalloc(int device, const double* device_target, int64_t n, con
 
     QueryDev qd{};
     qd.m = m; qd.w = w; qd.metric = metric; qd.arg = arg; qd.cutoff = cutoff; qd.qn = qn;
+    qd.qlo = *std::min_element(t_qn, t_qn + m);
+    qd.qhi = *std::max_element(t_qn, t_qn + m);
     DpJob dj{};
     dj.q = qd; dj.target = device_target; dj.MU = MU; dj.SIG = SIG;
     dj.list = nullptr; dj.n_windows = g.tsn; dj.mode = 0; dj.cutoff = cutoff;
     dj.out_idx = li; dj.out_dist = ld; dj.n_out = cnt + 0; dj.out_cap = kMaxWin;
     dj.n_valid = cnt + 1; dj.next = cnt + 2; dj.gwork = nullptr;
-    const void* kf = dp_kernel(metric, false);
-    if ((e = raise_smem_limit(kf, device, smem)) != cudaSuccess)
-        return cuda_fail(e, "cudaFuncSetAttribute", __FILE__, __LINE__);
-    int per_sm = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kf, warps * 32, smem)) != cudaSuccess)
-        return cuda_fail(e, "occupancy", __FILE__, __LINE__);
-    const unsigned grid = (unsigned)std::max(1, per_sm) * (unsigned)sms;
-    {
-        void* args[] = {&g, &dj};
-        if ((e = cudaLaunchKernel(kf, dim3(grid), dim3(warps * 32), args, smem, st)) != cudaSuccess)
-            return cuda_fail(e, "k_dp", __FILE__, __LINE__);
+    auto launch = [&](const void* kf, void** args, int threads, size_t bytes, const char* what) -> int {
+        cudaError_t le;
+        if ((le = raise_smem_limit(kf, device, bytes)) != cudaSuccess)
+            return cuda_fail(le, "cudaFuncSetAttribute", __FILE__, __LINE__);
+        int per_sm = 0;
+        if ((le = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kf, threads, bytes)) != cudaSuccess)
+            return cuda_fail(le, "occupancy", __FILE__, __LINE__);
+        const unsigned grid = (unsigned)std::max(1, per_sm) * (unsigned)sms;
+        if ((le = cudaLaunchKernel(kf, dim3(grid), dim3(threads), args, bytes, st)) != cudaSuccess)
+            return cuda_fail(le, what, __FILE__, __LINE__);
+        if ((le = cudaGetLastError()) != cudaSuccess) return cuda_fail(le, what, __FILE__, __LINE__);
+        return FSMELD_OK;
+    };
+    int r = FSMELD_OK;
+    HostQuery hq;  // the matching table's inputs; host memory until the call's last wait
+    bool done = false;
+    if (metric == EDR || metric == LCSS) {
+        BitTab bt;
+        bt.pad = (w + 31) / 32;
+        bt.rs = (bt.pad + (m + 31) / 32 + bit_words(w) + 1) | 1;
+        const size_t ends = sizeof(double) * (2 * (size_t)m + 1), ranks = sizeof(int) * 2 * (size_t)m;
+        const size_t grid_b = (sizeof(unsigned short) * (kBitBuckets + 1) + 15) & ~size_t(15);
+        const size_t tab = sizeof(unsigned) * (size_t)(2 * m + 1) * bt.rs;
+        if (bit_words(w) > 0 && kOffBit + ends + ranks + grid_b + tab <= kScratchBytes) {
+            hq.m = m; hq.w = w; hq.metric = metric; hq.arg = arg;
+            hq.qn.assign(t_qn, t_qn + m);
+            match_table(&hq);
+            unsigned char* b = base + kOffBit;
+            double* dE = (double*)b;
+            int* pa = (int*)(b + ends);
+            unsigned short* dg = (unsigned short*)(b + ends + ranks);
+            unsigned* dt = (unsigned*)(b + ends + ranks + grid_b);
+            if ((e = cudaMemcpyAsync(dE, hq.bitE.data(), ends, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+                (e = cudaMemcpyAsync(pa, hq.bitA.data(), ranks / 2, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+                (e = cudaMemcpyAsync(pa + m, hq.bitB.data(), ranks / 2, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+                (e = cudaMemcpyAsync(dg, hq.bitGrid.data(), sizeof(unsigned short) * (kBitBuckets + 1),
+                                     cudaMemcpyHostToDevice, st)) != cudaSuccess)
+                return cuda_fail(e, "cudaMemcpyAsync(matching table)", __FILE__, __LINE__);
+            k_bit_table<<<(unsigned)sms, 256, 0, st>>>(pa, pa + m, m, bt.pad, bt.rs, dt);
+            if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_bit_table", __FILE__, __LINE__);
+            bt.E = dE; bt.grid = dg; bt.table = dt;
+            bt.e0 = hq.bit_e0; bt.elast = hq.bit_elast; bt.scale = hq.bit_scale;
+            size_t bytes = bit_table_offset(m);
+            bt.in_smem = bytes + tab <= 54 * 1024;
+            if (bt.in_smem) bytes += tab;
+            void* args[] = {&g, &dj, &bt};
+            if ((r = launch(bitdp_kernel(metric, w), args, kBitThreads, bytes, "k_bitdp"))) return r;
+            done = true;
+        }
+    } else if (w >= 2 && cutoff < 1e12 && dpw_kernel(metric, w) &&
+               dpw_smem_bytes(m, kDpwThreads / 32) + 1024 <= (size_t)dev_optin) {
+        const size_t per_warp = screen_warp_bytes(w);
+        const int nw = per_warp * 4 <= 64 * 1024 ? 4 : per_warp * 2 <= 96 * 1024 ? 2 : 1;
+        long long few = 32LL * sms;
+        long long* list = (long long*)win;
+        unsigned long long* n_list = cnt + 4;
+        void* args[] = {&g, &dj, &list, &n_list, &few};
+        if ((r = launch(screen_kernel(metric), args, nw * 32, per_warp * nw, "k_screen"))) return r;
+        dj.list = list; dj.n_list = n_list; dj.list_cap = kMaxWin; dj.n_valid = nullptr; dj.next = cnt + 5;
+        void* args2[] = {&g, &dj};
+        if ((r = launch(dpw_kernel(metric, w), args2, kDpwThreads, dpw_smem_bytes(m, kDpwThreads / 32), "k_dpw")))
+            return r;
+        done = true;
     }
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_dp", __FILE__, __LINE__);
-    k_noalloc_scatter<<<(unsigned)sms * 4, 256, 0, st>>>(li, ld, cnt + 0, win);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_noalloc_scatter", __FILE__, __LINE__);
-    k_noalloc_compact<<<1, 1024, 0, st>>>(win, g.tsn, (long long*)device_out_idx, device_out_dist, capacity, cnt + 3);
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_noalloc_compact", __FILE__, __LINE__);
+    if (!done) {
+        void* args[] = {&g, &dj};
+        if ((r = launch(dp_kernel(metric, false), args, warps * 32, smem, "k_dp"))) return r;
+    }
     unsigned long long total = 0;
-    if ((e = cudaMemcpyAsync(&total, cnt + 3, sizeof(total), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
-        return cuda_fail(e, "cudaMemcpyAsync(count)", __FILE__, __LINE__);
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize", __FILE__, __LINE__);
+    auto wait = [&]() -> int {
+        if ((e = cudaMemcpyAsync(&total, cnt + 3, sizeof(total), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
+            return cuda_fail(e, "cudaMemcpyAsync(count)", __FILE__, __LINE__);
+        if ((e = cudaStreamSynchronize(st)) != cudaSuccess)
+            return cuda_fail(e, "cudaStreamSynchronize", __FILE__, __LINE__);
+        return FSMELD_OK;
+    };
+    {
+        const size_t bytes = finish_smem_bytes();
+        if ((e = raise_smem_limit((const void*)k_order, device, bytes)) != cudaSuccess)
+            return cuda_fail(e, "cudaFuncSetAttribute", __FILE__, __LINE__);
+        k_order<<<1, kFinishThreads, bytes, st>>>(cnt + 0, li, ld, (long long*)device_out_idx, device_out_dist, capacity,
+                                                  cnt + 3);
+        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_order", __FILE__, __LINE__);
+        if ((r = wait())) return r;
+    }
+    if (total > (unsigned long long)kFinishSort) {
+        if ((e = cudaMemsetAsync(win, 0xff, sizeof(double) * g.tsn, st)) != cudaSuccess)
+            return cuda_fail(e, "cudaMemsetAsync", __FILE__, __LINE__);
+        k_noalloc_scatter<<<(unsigned)sms * 4, 256, 0, st>>>(li, ld, cnt + 0, win);
+        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_noalloc_scatter", __FILE__, __LINE__);
+        k_noalloc_compact<<<1, 1024, 0, st>>>(win, g.tsn, (long long*)device_out_idx, device_out_dist, capacity, cnt + 3);
+        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_noalloc_compact", __FILE__, __LINE__);
+        if ((r = wait())) return r;
+    }
     *host_out_count = (int64_t)total;
     return FSMELD_OK;
 }

@@ -168,3 +168,29 @@ def test_lbip_runs(api, oracle, metric, arg, m, w):  # noqa: F811
             ok[:kml - tail] = False
         assert ok.sum() > 0
         assert np.all(np.abs(got - ref)[ok] <= 1e-9 + 1e-12 * np.abs(ref[ok])), s
+
+
+# fsmeld_exact_noalloc: each DP it may take (screen + wavefront, bit vectors,
+# lane DP for w < 2 and unreachable cutoffs), few and many matches (one block's
+# order, marking and compaction), a buffer that is too small
+@pytest.mark.parametrize("metric,arg", [("dtw", 0.0), ("erp", 0.4), ("msm", 0.5), ("edr", 0.25), ("lcss", 0.25)])
+@pytest.mark.parametrize("m,w", [(24, 0), (24, 3), (65, 40), (2048, 20)])
+def test_noalloc_paths(api, oracle, metric, arg, m, w):  # noqa: F811
+    import torch
+
+    n = 7000 + m if m < 100 else 2 * m + 300
+    t = random_walk(n, [18, m])
+    t[100] = np.nan
+    q, _ = query_from(t, m, np.random.default_rng([19, m]))
+    oi, od, _ = oracle.exact(t, q, m, 1e300, metric, w, arg)
+    ranked = np.sort(od)
+    d_t = torch.from_numpy(t).cuda()
+    idx = torch.full((n,), -7, dtype=torch.int64, device="cuda")
+    dist = torch.full((n,), -7.0, dtype=torch.float64, device="cuda")
+    for cut, cap in ((ranked[10], n), (ranked[-1], n), (1e300, n), (ranked[10], 4), (ranked[-1], 5000)):
+        keep = od <= cut
+        c = api.exact_noalloc(d_t.data_ptr(), n, q, m, float(cut), metric, w, arg, idx.data_ptr(), dist.data_ptr(), cap)
+        assert c == keep.sum()
+        k = min(c, cap)
+        assert np.array_equal(idx[:k].cpu().numpy(), oi[keep][:k])
+        assert bits_equal(dist[:k].cpu().numpy(), od[keep][:k])
