@@ -26,12 +26,14 @@
 //  4. every candidate reads its state, scores LB in parallel, and a block
 //     reduction takes the first maximum (NaN at index 0 wins, as in
 //     findMaxIndex, src/find_t_lp.cpp:206-216).
-// Several blocks per SM hide each other's serial phases (the replay, 8 cycles
-// an add); the sort is a third of what is left.  Measured, five queries on 2^24
-// points (m = 256): 11.5 ms with the merge sort, predicated chains and a
-// quadratic op order for ERP, 5.9 ms now; 20 queries of mixed length on 2^22
-// points, most with 8192-point segments that used to lie in global scratch:
-// 17.6 -> 8.9 ms.
+// Several blocks per SM hide each other's serial phases (the sums before the
+// sweep and the replay, 11 cycles an add); the sort is a quarter of what is left.
+// Measured, five queries on 2^24 points (m = 256): 11.5 ms with the merge sort,
+// predicated chains and a quadratic op order for ERP; 5.9 ms with buckets; 4.5 ms
+// with the runs found by ballots, a bucket's values side by side and the counts
+// of ops kept for every 32nd step.  20 queries of mixed length on 2^22 points,
+// most with 8192-point segments that used to lie in global scratch: 17.6, 8.9,
+// 7.3 ms.
 // ERP's priority queues pop equal keys in an order the C++ library leaves
 // to its heap layout; here equal keys pop by query index.  The threshold is
 // the same unless two candidates' scores tie to the last bit.
@@ -141,11 +143,42 @@ __host__ __device__ constexpr int thr_pad(int i) { return i + (i >> 5); }
 __host__ __device__ constexpr size_t thr_r_bytes(int cap) {
     return thr_round16((size_t)cap * 8 + ((size_t)thr_pad(cap) + 2) * 4);
 }
-__host__ __device__ inline size_t thr_z_bytes(int m) { return (size_t)m * 24 + 16 + (size_t)(2 * m + 9) * 32; }
+constexpr int kChainPad = 32;  // slots past the last op: a whole chunk and the loads ahead
+__host__ __device__ inline size_t thr_z_bytes(int m) { return (size_t)m * 24 + 16 + (size_t)(2 * m + kChainPad) * 32; }
 __host__ __device__ constexpr size_t thr_bucket_bytes(int cap, int nb) {
     return thr_round16(((size_t)thr_pad(nb) + 1) * 4 + (size_t)cap * 2);
 }
 __host__ __device__ constexpr int thr_buckets(int cap, bool gw) { return gw ? cap : 2 * cap; }
+
+// acc plus n operands in order, 4 doubles apart, the sum left in each operand's
+// place if STORE; operands up to the next multiple of 16 leave the sum as it
+// is.  A serial chain of additions: 8 operands are loaded under the 8 additions
+// before theirs, at fixed distances and without a test, up to 8 past the end.
+// (Strides and ends known only at run time cost 22 cycles an addition, these 11.)
+template <bool STORE>
+__device__ __forceinline__ double chain(double acc, double* p, int n) {
+    double a[8], b[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) a[u] = p[4 * u];
+#pragma unroll 1
+    for (int i = 0; i < n; i += 16, p += 64) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) b[u] = p[4 * (u + 8)];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            acc = dadd(acc, a[u]);
+            if (STORE) p[4 * u] = acc;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) a[u] = p[4 * (u + 16)];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            acc = dadd(acc, b[u]);
+            if (STORE) p[4 * (u + 8)] = acc;
+        }
+    }
+    return acc;
+}
 
 // The runs sorted by a block merge sort (thread t on runs t IPT ..) into the
 // sorted values and counts; in a function of its own for its registers.
@@ -189,19 +222,21 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, ThrJob job, u
     using Sort = cub::BlockMergeSort<unsigned long long, T, IPT, int>;
     using IScan = cub::BlockScan<int, T>;
     using AReduce = cub::BlockReduce<ArgMax, T>;
-    constexpr int CAP = T * IPT;
+    constexpr int CAP = T * IPT, NW = T / 32;
 
     extern __shared__ __align__(16) unsigned char thr_smem[];
     __shared__ typename IScan::TempStorage iscan_tmp;
     __shared__ typename AReduce::TempStorage red_tmp;
-    __shared__ int s_nr, s_nfin, s_best, s_nops;
+    __shared__ int s_nfin, s_best, s_nops;
     __shared__ int s_cnt[2];
-    __shared__ double s_ext[64];
+    __shared__ unsigned s_ext[64];
+    __shared__ int s_wc[NW * IPT];
+    __shared__ int s_lo[CAP / 32 + 2];
 
     const QueryDev& q = job.q;
     const int m = q.m, mk = g.m_k;
     const int cnt = mk - 2 * m + 2;
-    const int t = threadIdx.x;
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
 
     // GW: region R in global scratch; otherwise provably shared memory
     constexpr size_t RB = thr_r_bytes(CAP);
@@ -222,7 +257,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, ThrJob job, u
     int* sB = sA + m;                                   // [m]
     int* opdesc = sB + m;                               // [2m]
     int* opstep = opdesc + 2 * m;                       // [2m]
-    double* st = (double*)(((uintptr_t)(opstep + 2 * m) + 15) & ~uintptr_t(15));  // [(2m+9)*4]
+    double* st = (double*)(((uintptr_t)(opstep + 2 * m) + 15) & ~uintptr_t(15));  // [(2m + kChainPad) * 4]
 
     const int p = q.p;
     const int kind = (q.metric == DTW) ? 0 : (q.metric == ERP ? 2 : 1);
@@ -232,64 +267,68 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, ThrJob job, u
         const int upper = (int)(bid & 1);
         const double* env = (upper ? job.Un : job.Ln) + s * mk + (m - 1);
 
-        // ---- 1. run-length dedup (src/find_t_lp.cpp:53-67)
+        // ---- 1. run-length dedup (src/find_t_lp.cpp:53-67), value t + k T per
+        // thread; the extremes of the finite values as the upper words of their
+        // order keys
         double v[IPT];
-        int nflag = 0;
+        unsigned fl = 0, kmn = ~0u, kmx = 0;
+#pragma unroll
+        for (int k = 0; k < IPT; ++k) v[k] = t + k * T < cnt ? env[t + k * T] : 0.0;
 #pragma unroll
         for (int k = 0; k < IPT; ++k) {
-            const int i = t * IPT + k;
-            v[k] = (i < cnt) ? env[i] : 0.0;
-        }
-        bool flag[IPT];
-#pragma unroll
-        for (int k = 0; k < IPT; ++k) {
-            const int i = t * IPT + k;
-            bool f = false;
-            if (i < cnt) {
-                const double prev = (k > 0) ? v[k - 1] : (i > 0 ? env[i - 1] : 0.0);
-                f = (i == 0) || (v[k] != prev);
+            const int i = t + k * T;
+            double prev = __shfl_up_sync(0xffffffffu, v[k], 1);
+            if (lane == 0 && i > 0 && i < cnt) prev = env[i - 1];
+            const bool f = i < cnt && (i == 0 || v[k] != prev);
+            const unsigned hw = (unsigned)__double2hiint(v[k]);
+            if (i < cnt && (hw & 0x7ff00000u) != 0x7ff00000u) {
+                const unsigned key = (hw >> 31) ? ~hw : hw | 0x80000000u;
+                kmn = min(kmn, key);
+                kmx = max(kmx, key);
             }
-            flag[k] = f;
-            nflag += f ? 1 : 0;
+            fl |= f ? 1u << k : 0u;
+            const int c = __popc(__ballot_sync(0xffffffffu, f));
+            if (lane == 0) s_wc[k * NW + wid] = c;
         }
-        int roff, nr;
-        IScan(iscan_tmp).ExclusiveSum(nflag, roff, nr);
+        kmn = __reduce_min_sync(0xffffffffu, kmn);
+        kmx = __reduce_max_sync(0xffffffffu, kmx);
+        if (lane == 0) { s_ext[wid] = kmn; s_ext[32 + wid] = kmx; }
+        for (int i = t; i <= thr_pad(NB); i += T) bcnt[i] = 0;
+        __syncthreads();
+        kmn = __reduce_min_sync(0xffffffffu, s_ext[min(lane, NW - 1)]);
+        kmx = __reduce_max_sync(0xffffffffu, s_ext[32 + min(lane, NW - 1)]);
+        int wbase, nr;
+        IScan(iscan_tmp).ExclusiveSum(t < NW * IPT ? s_wc[t] : 0, wbase, nr);
+        if (t < NW * IPT) s_wc[t] = wbase;
+        __syncthreads();
 #pragma unroll
         for (int k = 0; k < IPT; ++k) {
-            if (flag[k]) {
-                rstart[roff] = t * IPT + k;
-                rval[roff] = v[k];
-                ++roff;
+            const bool f = (fl >> k) & 1;
+            const unsigned bal = __ballot_sync(0xffffffffu, f);
+            if (f) {
+                const int o = s_wc[k * NW + wid] + __popc(bal & ((1u << lane) - 1));
+                rstart[o] = t + k * T;
+                rval[o] = v[k];
             }
         }
-        if (t == 0) { rstart[nr] = cnt; s_nr = nr; }
+        if (t == 0) rstart[nr] = cnt;
         __syncthreads();
 
         // ---- 2. sort runs (src/find_t_lp.cpp:68-81): ascending keys, ties by
         // run; run t + k T is this thread's k-th
         double rv[IPT];
         int rank[IPT], rc[IPT], bk[IPT];
-        int nf = 0;  // this thread's runs that are not NaN
-        double vmn = INFINITY, vmx = -INFINITY;
 #pragma unroll
         for (int k = 0; k < IPT; ++k) {
             const int r = t + k * T;
             rv[k] = r < nr ? rval[r] : dnan();
             rc[k] = r < nr ? rstart[r + 1] - rstart[r] : 0;
-            nf += isnan(rv[k]) ? 0 : 1;
-            if (isfinite(rv[k])) { vmn = fmin(vmn, rv[k]); vmx = fmax(vmx, rv[k]); }
         }
-        for (int o = 16; o; o >>= 1) {
-            vmn = fmin(vmn, __shfl_xor_sync(0xffffffffu, vmn, o));
-            vmx = fmax(vmx, __shfl_xor_sync(0xffffffffu, vmx, o));
-        }
-        if ((t & 31) == 0) { s_ext[t >> 5] = vmn; s_ext[32 + (t >> 5)] = vmx; }
-        for (int i = t; i <= thr_pad(NB); i += T) bcnt[i] = 0;
-        __syncthreads();
-        for (int i = 0; i < T / 32; ++i) { vmn = fmin(vmn, s_ext[i]); vmx = fmax(vmx, s_ext[32 + i]); }
         // buckets of equal width over the finite values (the infinities in the
-        // outer ones, NaN in the last): the width is rounded, the order of the
-        // buckets is that of the values all the same
+        // outer ones, NaN in the last): the range and the width are rounded, the
+        // order of the buckets is that of the values all the same
+        const double vmn = __hiloint2double((int)((kmn >> 31) ? kmn ^ 0x80000000u : ~kmn), (kmn >> 31) ? 0 : -1);
+        const double vmx = __hiloint2double((int)((kmx >> 31) ? kmx ^ 0x80000000u : ~kmx), (kmx >> 31) ? -1 : 0);
         const double width = vmx > vmn ? (NB - 1) / (vmx - vmn) : 0.0;
         const double scale = isfinite(width) ? width : 0.0;
 #pragma unroll
@@ -314,6 +353,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, ThrJob job, u
             most = max(most, x);
             bsum += x;
         }
+        if (t == T - 1) s_nfin = nr - bcnt[thr_pad(NB - 1)];  // the last bucket holds the NaN
         int bbase;
         IScan(iscan_tmp).ExclusiveSum(bsum, bbase);
         if (!__syncthreads_or(most > kBucketMost)) {
@@ -324,28 +364,57 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, ThrJob job, u
                 bbase += x;
             }
             __syncthreads();
+            // the runs by buckets, values over the unsorted ones
 #pragma unroll
             for (int k = 0; k < IPT; ++k)
-                if (t + k * T < nr) bslot[bcnt[bk[k]] + rank[k]] = (unsigned short)(t + k * T);
-            __syncthreads();
-            // rank inside the bucket by comparison with its other runs
-#pragma unroll
-            for (int k = 0; k < IPT; ++k) {
-                const int r = t + k * T;
-                if (r >= nr) continue;
-                const int lo = bcnt[bk[k]];
-                const int nb = bk[k] + (bk[k] % 33 == 31 ? 2 : 1);  // the next bucket's slot
-                const int hi = bk[k] < thr_pad(NB - 1) ? bcnt[nb] : nr;
-                int less = 0;
-                if (hi - lo > 1) {
-                    const unsigned long long key = order_key(rv[k], upper ? 0 : 1);
-                    for (int i = lo; i < hi; ++i) {
-                        const int o = bslot[i];
-                        const unsigned long long ko = order_key(rval[o], upper ? 0 : 1);
-                        less += (ko < key || (ko == key && o < r)) ? 1 : 0;
-                    }
+                if (t + k * T < nr) {
+                    const int pos = bcnt[bk[k]] + rank[k];
+                    tv[pos] = rv[k];
+                    bslot[pos] = (unsigned short)(t + k * T);
                 }
-                rank[k] = lo + less;
+            __syncthreads();
+            // rank inside the bucket by comparison with its runs, four runs'
+            // buckets side by side
+            constexpr int G = IPT < 4 ? IPT : 4;
+#pragma unroll
+            for (int k0 = 0; k0 < IPT; k0 += G) {
+                int lo[G], num[G], less[G], eq[G], most_here = 0;
+#pragma unroll
+                for (int u = 0; u < G; ++u) {
+                    const int k = k0 + u;
+                    less[u] = eq[u] = lo[u] = num[u] = 0;
+                    if (t + k * T < nr) {
+                        lo[u] = bcnt[bk[k]];
+                        const int nb = bk[k] + (bk[k] % 33 == 31 ? 2 : 1);  // the next bucket's slot
+                        num[u] = (bk[k] < thr_pad(NB - 1) ? bcnt[nb] : nr) - lo[u];
+                    }
+                    most_here = max(most_here, num[u]);
+                }
+                most_here = __reduce_max_sync(0xffffffffu, most_here);
+                if (most_here > 1)
+#pragma unroll 1
+                    for (int i = 0; i < most_here; ++i) {
+#pragma unroll
+                        for (int u = 0; u < G; ++u) {
+                            if (i >= num[u]) continue;
+                            const double vo = tv[lo[u] + i];
+                            less[u] += (upper ? vo < rv[k0 + u] : vo > rv[k0 + u]) ? 1 : 0;
+                            eq[u] += vo == rv[k0 + u] ? 1 : 0;
+                        }
+                    }
+#pragma unroll
+                for (int u = 0; u < G; ++u) {
+                    if (num[u] > 1 && eq[u] != 1) {  // equal values or NaN: by run
+                        const double x = rv[k0 + u];
+                        less[u] = 0;
+                        for (int i = 0; i < num[u]; ++i) {
+                            const double vo = tv[lo[u] + i];
+                            const bool before = upper ? vo < x : vo > x, after = upper ? vo > x : vo < x;
+                            less[u] += before || (!after && (int)bslot[lo[u] + i] < t + (k0 + u) * T) ? 1 : 0;
+                        }
+                    }
+                    rank[k0 + u] = lo[u] + less[u];
+                }
             }
             __syncthreads();
 #pragma unroll
@@ -369,9 +438,6 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, ThrJob job, u
         }
         int cbase;
         IScan(iscan_tmp).ExclusiveSum(csum, cbase);
-        __syncthreads();
-        int nfin_total;
-        IScan(iscan_tmp).ExclusiveSum(nf, nf, nfin_total);
 #pragma unroll
         for (int k = 0; k < IPT; ++k) {
             const int i = t * IPT + k;
@@ -380,7 +446,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, ThrJob job, u
                 gp[thr_pad(i)] = cbase;
             }
         }
-        if (t == 0) { s_nfin = nfin_total; s_cnt[0] = 0; s_cnt[1] = 0; }
+        if (t == 0) { s_cnt[0] = 0; s_cnt[1] = 0; }
         __syncthreads();
         const int nfin = s_nfin;
         double* out = job.thr + s * 2 + upper;
@@ -540,18 +606,37 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, ThrJob job, u
         // for every x, signed zeros included).
         const double* pw0 = (kind == 2) ? q.opw : q.pw;
         const double* Dt = (kind == 2) ? q.oD : q.Dq;
-        for (int j = t; j < m; j += T) {
-            double o0 = pw0[j], o1 = pw0[m + j], o2 = pw0[2 * m + j], o3 = Dt[j];
-            if (kind == 2) {  // which initial sum the element enters, if any
-                const double qv = q.qn[j];
+        // (the power sums' elements and the penalty sum's, in the order they are
+        // added; past the last one no change, to a whole number of chunks)
+        int em = 0, dm = 1, lm = m, ec = 0, lc = m;
+        if (kind == 0) {
+            em = upper ? pl.idx1 : 0;
+            lm = upper ? m - pl.idx1 : pl.idx1 + 1;
+            lc = 0;
+        } else if (kind == 1) {
+            em = pl.idx1;
+            dm = upper ? 1 : -1;
+            lm = upper ? pl.idx2 - pl.idx1 : pl.idx1 - pl.idx2;
+            ec = upper ? pl.idx2 : 0;
+            lc = upper ? m - pl.idx2 : pl.idx2 + 1;
+        }
+        const int ninit = (max(lm, lc) + 15) & ~15;
+        for (int i = t; i < ninit; i += T) {
+            bool in_m = i < lm, in_c = i < lc;
+            if (kind == 2 && i < m) {  // which initial sum the element enters, if any
+                const double qv = q.qn[i];
                 int cd;
-                if (!upper) cd = (qv >= t0) ? 0 : (q.otl[j] >= t0 ? 1 : 2);
-                else cd = (qv <= t0) ? 0 : (q.otu[j] <= t0 ? 1 : 2);
-                if (cd != 1) o0 = o1 = o2 = -0.0;
-                if (cd != 2) o3 = -0.0;
+                if (!upper) cd = (qv >= t0) ? 0 : (q.otl[i] >= t0 ? 1 : 2);
+                else cd = (qv <= t0) ? 0 : (q.otu[i] <= t0 ? 1 : 2);
+                in_m = cd == 1;
+                in_c = cd == 2;
             }
-            double* o = st + 4 * j;
-            o[0] = o0; o[1] = o1; o[2] = o2; o[3] = o3;
+            const int jm = em + dm * i;
+            double* o = st + 4 * i;
+            o[0] = in_m ? pw0[jm] : -0.0;
+            o[1] = in_m ? pw0[m + jm] : -0.0;
+            o[2] = in_m ? pw0[2 * m + jm] : -0.0;
+            o[3] = in_c ? Dt[ec + i] : -0.0;
         }
         __syncthreads();
         // initial sums: lane j of one warp (a different one in each block, so that
@@ -560,51 +645,14 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, ThrJob job, u
         // for j = 3) and adds its elements in the reference's order
         const int jl = t - 32 * (int)(blockIdx.x % (T / 32));
         double acc = 0.0;
-        if (jl >= 0 && jl < 4) {
-            // elements e0, e0+dir, ... (len of them)
-            int e0 = 0, dir = 1, len = 0;
-            if (kind == 2) {
-                len = m;
-            } else if (jl < 3) {
-                if (kind == 0) {
-                    e0 = upper ? pl.idx1 : 0;
-                    len = upper ? m - pl.idx1 : pl.idx1 + 1;
-                } else {
-                    e0 = pl.idx1;
-                    dir = upper ? 1 : -1;
-                    len = upper ? pl.idx2 - pl.idx1 : pl.idx1 - pl.idx2;
-                }
-            } else if (kind == 1) {
-                e0 = upper ? pl.idx2 : 0;
-                len = upper ? m - pl.idx2 : pl.idx2 + 1;
-            }
-            // eight operands are loaded ahead of their adds
-            const double* sp = st + 4 * e0 + jl;
-            const int step = 4 * dir, full = len & ~7;
-            double v[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = full > 0 ? sp[u * step] : 0.0;
-            int i = 0;
-#pragma unroll 1
-            for (; i < full; i += 8) {
-                sp += 8 * step;
-                double nv[8];
-                const bool more = i + 8 < full;
-#pragma unroll
-                for (int u = 0; u < 8; ++u) nv[u] = more ? sp[u * step] : 0.0;
-#pragma unroll
-                for (int u = 0; u < 8; ++u) acc = dadd(acc, v[u]);
-#pragma unroll
-                for (int u = 0; u < 8; ++u) v[u] = nv[u];
-            }
-#pragma unroll 1
-            for (; i < len; ++i, sp += step) acc = dadd(acc, sp[0]);
-        }
+        if (jl >= 0 && jl < 4) acc = chain<false>(acc, st + jl, ninit);
         __syncthreads();
+        // ops before every 32nd step
+        for (int b = t; b <= (nr + 31) / 32; b += T) s_lo[b] = prefix_count(nops, [&](int k) { return opstep[k] < 32 * b; });
         // op payloads into the state slots the replay overwrites: op B
         // subtracts the element's powers, op A adds them and subtracts its
         // penalty
-        for (int k = t; k < ((nops + 7) & ~7); k += T) {
+        for (int k = t; k < ((nops + 15) & ~15); k += T) {
             const int d = k < nops ? opdesc[k] : -1;
             double* o = st + 4 * (k + 1);
             if (d < 0) {  // past the last op: no change
@@ -627,39 +675,20 @@ __global__ void __launch_bounds__(T, 1024 / T) k_threshold(Geom g, ThrJob job, u
         }
         __syncthreads();
         // replay: lane j adds every op's operand to its accumulator j and
-        // stores the state after each op, in chunks of eight (the next chunk's
-        // operands are loaded before this chunk's states overwrite its slots)
+        // stores the state after each op in the operand's place
         if (jl >= 0 && jl < 4) {
-            double* sp = st + jl;
-            sp[0] = acc;
-            double a[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) a[u] = nops ? sp[4 * (u + 1)] : 0.0;
-            for (int k0 = 0; k0 < nops; k0 += 8) {
-                double na[8];
-                const bool more = k0 + 8 < nops;
-#pragma unroll
-                for (int u = 0; u < 8; ++u) na[u] = more ? sp[4 * (u + 9)] : 0.0;
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    acc = dadd(acc, a[u]);
-                    sp[4 * (u + 1)] = acc;
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u) a[u] = na[u];
-                sp += 32;
-            }
+            st[jl] = acc;
+            chain<true>(acc, st + 4 + jl, nops);
         }
         __syncthreads();
 
         // ---- 8. scores and first maximum
         ArgMax best{0.0, INT_MAX, 0};
         int nan0 = 0;
-        // thread t scores steps t, t + T, ...; the number of ops with step <= i
-        // is a binary search from the previous one on
-        int lo = 0;
+        // the number of ops with step <= i lies between the counts at the ends of
+        // the step's 32
         for (int i = t; i < nr; i += T) {
-            int hi = nops;
+            int lo = s_lo[i >> 5], hi = s_lo[(i >> 5) + 1];
             while (lo < hi) { const int mid = (lo + hi) >> 1; if (opstep[mid] <= i) lo = mid + 1; else hi = mid; }
             const double* sv = st + 4 * lo;
             const double tt = tv[i];
