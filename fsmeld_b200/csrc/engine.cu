@@ -1514,7 +1514,7 @@ static int run_search_gemm(fsmeld_ctx* c, const Geom& g0, Stats& st, const std::
         gj.nsurv = dcnt; gj.nvalid = dcnt + nq; gj.err = (unsigned*)(dcnt + 2 * nq);
         // the group's window masks, once for all tiles
         {
-            const int mw = gemm_mask_words(g0.m_k, g0.kml, m);
+            const int mw = (g0.m_k + 31) / 32;
             unsigned* dmask;
             if ((r = bufT(c, "gemmMask", 2 * (size_t)g0.S * mw, &dmask))) return r;
             gj.mask_l = dmask;
@@ -1529,11 +1529,11 @@ static int run_search_gemm(fsmeld_ctx* c, const Geom& g0, Stats& st, const std::
             LAUNCH_CHECK(c);
         }
         const void* kf = lbgemm_kernel(NQ);
-        const size_t smem = lbgemm_smem_bytes(NQ, m);
+        const size_t smem = lbgemm_smem_bytes(NQ, m, &gj.resident);
         if ((r = allow_smem(c, kf, smem))) return r;
         // resident CTAs per SM from the kernel's own resources: shared memory
         // (dynamic + static + the 1 KB the SM reserves per block), registers,
-        // threads, and TMEM (512 columns per SM, 2 NQ (>= 32) per CTA)
+        // threads, and TMEM
         int per_sm = 0;
         {
             cudaFuncAttributes fa;
@@ -1546,9 +1546,9 @@ static int run_search_gemm(fsmeld_ctx* c, const Geom& g0, Stats& st, const std::
             per_sm = (int)std::min<size_t>((size_t)smem_sm / per_block, (size_t)thr_sm / kLbGemmThreads);
             if (fa.numRegs > 0) per_sm = std::min(per_sm, regs_sm / (fa.numRegs * kLbGemmThreads));
         }
-        const int cols = std::max(32, 2 * NQ);
-        per_sm = std::max(1, std::min(per_sm, 512 / cols));  // TMEM: 512 columns per SM
-        const long long items = g0.S * ((g0.kml + 127) / 128);
+        per_sm = std::max(1, std::min(per_sm, 512 / lbgemm_cols(NQ)));  // TMEM: 512 columns per SM
+        const int span = 128 * lbgemm_tiles(NQ);
+        const long long items = g0.S * ((g0.kml + span - 1) / span);
         const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(items, (long long)per_sm * c->sm_count));
         Geom ga = g0;
         void* args[] = {&ga, &gj};

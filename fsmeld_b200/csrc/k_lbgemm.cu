@@ -23,25 +23,33 @@
 // threshold gives a valid bound (the reference picks one per segment and
 // query to make it tight; here one pair serves the whole group).
 //
-// Tiles: a CTA of 128 threads takes one (segment, 128-window tile) at a
+// Tiles: a CTA of 256 threads takes kTiles 128-window tiles of one segment at a
 // time.  The group's window masks g (one bit per segment position and side)
 // are computed once before the product (k_gemm_masks, one ballot per 32
-// positions).  Per 64-wide K chunk, the threads write the A tiles of both
-// sides from the mask words of the tile's span (positions j0 .. j0+127+m) and
-// copy the chunk of B (pre-arranged on the host in the operand layout), in
-// the canonical no-swizzle K-major layout (8-row x 16-byte core matrices:
-// rows 16 B apart, row groups SBO = 128 B apart, 8-element K groups LBO
-// apart); one thread issues 4 K-steps x 2 sides x 3 splits of
-// tcgen05.mma.cta_group::1.kind::f16 (M = 128, N = NQ, K = 16) into two
-// TMEM accumulators (columns [0, NQ) lower, [NQ, 2 NQ) upper) and commits
-// them to an mbarrier; the next chunk's operands are written once that
-// mbarrier says the MMAs have read the current ones.  The epilogue: thread r
-// reads TMEM lane r (window j0 + r) with tcgen05.ld, forms each query's
-// inner product and compares it with the largest one the prune test keeps
-// (src/fsmeld.cpp:84-106, include/fsmeld_internal.h:9-19; the host's bisection),
-// and sets the survivors' bits in the query's window bit mask
-// (one atomic OR per warp, query and word); k_bits_to_list turns a mask into
-// the survivor list the GLB stage reads.
+// positions).  Row r of A is g[j0 + r ...], so the eight elements of row r and
+// K group kg depend on r + 8 kg alone: in the canonical no-swizzle K-major
+// layout (8-row x 16-byte core matrices) with 128 bytes from row group to row
+// group and also from K group to K group, all tiles' rows and K groups lie in
+// one array, 16 bytes per position (the operand that is read repeats, the one
+// that is stored does not).  B is arranged on the host in the operand layout
+// and stays in shared memory where it and A leave room for two CTAs per SM
+// (NQ m up to about 7000); otherwise a chunk of 64 K elements at a time is staged.  One
+// thread issues kTiles x 4 K-steps x 2 sides x 3 splits of
+// tcgen05.mma.cta_group::1.kind::f16 (M = 128, N = NQ, K = 16) per chunk into
+// the TMEM accumulators (per tile columns [0, NQ) lower, [NQ, 2 NQ) upper) and
+// commits them to an mbarrier.  The epilogue: a warp reads its TMEM lanes (32
+// windows) with tcgen05.ld, 16 queries at a time, forms each query's inner
+// product and compares it with the largest one the prune test keeps
+// (src/fsmeld.cpp:84-106, include/fsmeld_internal.h:9-19; the host's bisection);
+// lane i collects query i's ballot and sets the survivors' bits in the query's
+// window bit mask; k_bits_to_list turns a mask into the survivor list the GLB
+// stage reads.
+//
+// What bounds it: instruction issue of the epilogue (about 25 instructions per
+// query and 32 windows) beside the MMAs' operand reads (4 KB of A per MMA).
+// Writing A out per chunk (16 KB and 16 expanded bytes a thread and side) and
+// counting by shared-memory atomics took 1.64 ms for 32 queries of m = 128 on 2^22
+// points, this takes 0.60.
 //
 // Waits are bounded (about a second of clock cycles): on a timeout the
 // kernel records an error flag, waits once more for its MMAs, frees its
@@ -55,10 +63,9 @@ namespace fsm {
 
 namespace {
 
-constexpr int kGemmThreads = 128;
+constexpr int kGemmThreads = 256;
 constexpr int kKChunk = 64;                         // K elements per chunk
-constexpr int kAChunkBytes = 128 * kKChunk * 2;     // one side's A chunk (16 KB)
-constexpr int kALbo = 16 * 128;                     // A: bytes between K groups (16 row groups x 128 B)
+constexpr size_t kResident = 104 * 1024;            // operands of two CTAs per SM
 constexpr long long kWaitCycles = 2000000000LL;     // ~1 s at 2 GHz
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -123,47 +130,54 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
         : "r"(taddr));
 }
 
-// eight 0/1 mask bits -> eight BF16 values (1.0 = 0x3F80) packed in 16 bytes
+// eight 0/1 mask bits -> eight BF16 values (1.0 = 0x3F80) packed in 16 bytes:
+// bits 2i and 2i+1 are brought 16 apart and multiplied by 0x3F80 >> 2i
 __device__ __forceinline__ uint4 bits_to_bf16x8(uint32_t b) {
-    uint4 v;
-    v.x = ((b & 1u) ? 0x3F80u : 0u) | ((b & 2u) ? 0x3F800000u : 0u);
-    v.y = ((b & 4u) ? 0x3F80u : 0u) | ((b & 8u) ? 0x3F800000u : 0u);
-    v.z = ((b & 16u) ? 0x3F80u : 0u) | ((b & 32u) ? 0x3F800000u : 0u);
-    v.w = ((b & 64u) ? 0x3F80u : 0u) | ((b & 128u) ? 0x3F800000u : 0u);
-    return v;
+    const uint32_t t = b * 0x8001u;
+    return make_uint4((t & 0x00010001u) * 0x3F80u, (t & 0x00040004u) * 0x0FE0u, (t & 0x00100010u) * 0x03F8u,
+                      (t & 0x00400040u) * 0x00FEu);
 }
 
-__device__ __forceinline__ unsigned long long bits_at(const unsigned long long* w, int p) {
-    const int q = p >> 6, r = p & 63;
-    return r ? ((w[q] >> r) | (w[q + 1] << (64 - r))) : w[q];
-}
+// one query's limits in the epilogue
+struct __align__(16) Limits {
+    double ml, mu;    // margins of the two inner products
+    double keep_max;
+    double unused;
+};
 
 }  // namespace
 
-size_t lbgemm_smem_bytes(int nq_pad, int m) {
-    const int kpad = (m + kKChunk - 1) / kKChunk * kKChunk;
-    const int words = (128 + kpad + 63) / 64 + 2;
-    return 2 * (size_t)kAChunkBytes + 6 * (size_t)nq_pad * kKChunk * 2 + 2 * (size_t)words * 8 + 64;
+size_t lbgemm_smem_bytes(int nq_pad, int m, int* resident) {
+    const size_t kpad = (size_t)(m + kKChunk - 1) / kKChunk * kKChunk;
+    const size_t rows = 128 * (size_t)lbgemm_tiles(nq_pad), fixed = nq_pad * (sizeof(Limits) + 8);
+    const size_t all = 2 * (rows + kpad) * 16 + 12 * (size_t)nq_pad * kpad + fixed;
+    *resident = all <= kResident;
+    return *resident ? all : 2 * (rows + kKChunk) * 16 + 12 * (size_t)nq_pad * kKChunk + fixed;
 }
 
 template <int NQ>
-__global__ void __launch_bounds__(kGemmThreads) k_lbgemm(Geom g, GemmJob job) {
+__global__ void __launch_bounds__(kGemmThreads, NQ <= 64 ? 3 : 2) k_lbgemm(Geom g, GemmJob job) {
+    constexpr int kTiles = lbgemm_tiles(NQ);
+    constexpr int kBlocks = NQ / 16;                        // 16-query blocks of the epilogue
+    constexpr int kOwn = kBlocks > 1 ? kBlocks / 2 : 1;     // those of one warpgroup
+    constexpr int kBChunk = 12 * NQ * kKChunk;              // bytes of a B chunk
     extern __shared__ __align__(1024) unsigned char gm_smem[];
-    unsigned char* As = gm_smem;                             // [2 sides] A chunk (canonical layout)
-    unsigned char* Bs = As + 2 * kAChunkBytes;              // [2 sides][3 splits] B chunk
-    const int kpad = job.kchunks * kKChunk;
-    const int words = (128 + kpad + 63) / 64 + 2;
-    unsigned long long* GLb = (unsigned long long*)(Bs + 6 * NQ * kKChunk * 2);
-    unsigned long long* GUb = GLb + words;
+    const int kc = job.resident ? job.kchunks : 1;          // K chunks staged at a time
+    const int rows = 128 * kTiles + kc * kKChunk;           // A positions staged at a time
+    unsigned char* As = gm_smem;                            // [2 sides][rows] eight elements per position
+    unsigned char* Bs = As + 2 * rows * 16;                 // [kc] B chunks
+    Limits* lim = (Limits*)(Bs + kc * kBChunk);             // [NQ]
+    int* s_cnt = (int*)(lim + NQ);                          // [NQ] survivors, [NQ] valid windows
+    int* s_valid = s_cnt + NQ;
     __shared__ __align__(8) unsigned long long s_bar;
     __shared__ uint32_t s_tmem;
-    __shared__ int s_cnt[16], s_valid[16];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int m = job.m, mk = g.m_k, kml = g.kml;
-    const int tiles = (kml + 127) / 128;
-    const long long items = g.S * tiles;
-    constexpr uint32_t kCols = (2 * NQ < 32) ? 32 : 2 * NQ;
+    const int half = warp >> 2;                             // warpgroup
+    const int m = job.m, kml = g.kml;
+    const int per_seg = (kml + 128 * kTiles - 1) / (128 * kTiles);
+    const long long items = g.S * per_seg;
+    constexpr uint32_t kCols = lbgemm_cols(NQ);
     const uint32_t idesc = gemm_idesc<NQ>();
     const uint32_t bar = smem_u32(&s_bar);
 
@@ -176,54 +190,61 @@ __global__ void __launch_bounds__(kGemmThreads) k_lbgemm(Geom g, GemmJob job) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
+    bool ex = false;
+    for (int q = tid; q < NQ; q += kGemmThreads) {
+        const bool in = q < job.nq;
+        lim[q] = Limits{in ? job.margin_l[q] : 0.0, in ? job.margin_u[q] : 0.0, in ? job.keep_max[q] : 0.0, 0.0};
+        s_cnt[q] = s_valid[q] = 0;
+        ex = ex || (in && job.excl_b[q] >= 0);
+    }
+    if (job.resident)
+        for (int i = tid; i < kc * (kBChunk / 16); i += kGemmThreads) ((uint4*)Bs)[i] = job.B[i];
     asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
+    const bool any_excl = __syncthreads_or(ex) != 0;
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = s_tmem;
     uint32_t phase = 0;
     bool failed = false;
+    int cnt[kOwn], val[kOwn];  // lane i: query i of each own block
+#pragma unroll
+    for (int b = 0; b < kOwn; ++b) cnt[b] = val[b] = 0;
 
     for (long long it = blockIdx.x; it < items && !failed; it += gridDim.x) {
-        const long long s = it / tiles;
-        const int j0 = (int)(it - s * tiles) * 128;
-        // masks of the tile's span: positions j0 .. j0 + 128 + kpad (0 past the
-        // segment), copied from the group's precomputed mask words
-        {
-            const unsigned* ml = job.mask_l + s * (long long)job.mask_words + (j0 >> 5);
-            const unsigned* mu = job.mask_u + s * (long long)job.mask_words + (j0 >> 5);
-            for (int i = tid; i < 2 * words; i += kGemmThreads) {
-                ((unsigned*)GLb)[i] = ml[i];
-                ((unsigned*)GUb)[i] = mu[i];
+        const long long s = it / per_seg;
+        const int j0 = (int)(it - s * per_seg) * 128 * kTiles;
+        const unsigned* ml = job.mask_l + s * (long long)job.mask_words;
+        const unsigned* mu = job.mask_u + s * (long long)job.mask_words;
+        for (int c = 0; c < job.kchunks; c += kc) {
+            // A: positions j0 + 64 c + i, eight mask bits each (0 past the segment)
+            for (int i = tid; i < rows; i += kGemmThreads) {
+                const int p = j0 + c * kKChunk + i, w = p >> 5;
+                const unsigned l0 = w < job.mask_words ? ml[w] : 0u, l1 = w + 1 < job.mask_words ? ml[w + 1] : 0u;
+                const unsigned u0 = w < job.mask_words ? mu[w] : 0u, u1 = w + 1 < job.mask_words ? mu[w + 1] : 0u;
+                ((uint4*)As)[i] = bits_to_bf16x8(__funnelshift_r(l0, l1, p & 31) & 0xFFu);
+                ((uint4*)As)[rows + i] = bits_to_bf16x8(__funnelshift_r(u0, u1, p & 31) & 0xFFu);
             }
-        }
-        __syncthreads();
-        for (int c = 0; c < job.kchunks; ++c) {
-            // A chunk: row r = tid, K groups kg = 0..7 (elements j0 + r + 64c + 8kg .. +7)
-            const unsigned long long wl = bits_at(GLb, tid + c * kKChunk);
-            const unsigned long long wu = bits_at(GUb, tid + c * kKChunk);
-            const int rowoff = (tid >> 3) * 128 + (tid & 7) * 16;
-#pragma unroll
-            for (int kg = 0; kg < 8; ++kg) {
-                *(uint4*)(As + kg * kALbo + rowoff) = bits_to_bf16x8((uint32_t)(wl >> (8 * kg)) & 0xFFu);
-                *(uint4*)(As + kAChunkBytes + kg * kALbo + rowoff) = bits_to_bf16x8((uint32_t)(wu >> (8 * kg)) & 0xFFu);
+            if (!job.resident) {
+                const uint4* src = job.B + (size_t)c * (kBChunk / 16);
+                for (int i = tid; i < kBChunk / 16; i += kGemmThreads) ((uint4*)Bs)[i] = src[i];
             }
-            // B chunk: pre-arranged, 6 NQ x 64 BF16
-            const uint4* src = job.B + (size_t)c * (6 * NQ * kKChunk * 2 / 16);
-            for (int i = tid; i < 6 * NQ * kKChunk * 2 / 16; i += kGemmThreads) ((uint4*)Bs)[i] = src[i];
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncthreads();
             if (tid == 0) {
                 asm volatile("tcgen05.fence::after_thread_sync;");
-#pragma unroll
-                for (int ks = 0; ks < kKChunk / 16; ++ks) {
+                for (int ks = 0; ks < kc * (kKChunk / 16); ++ks) {
+                    const unsigned char* bk = Bs + (ks / (kKChunk / 16)) * kBChunk + 2 * (ks % (kKChunk / 16)) * (NQ * 16);
 #pragma unroll
                     for (int side = 0; side < 2; ++side) {
-                        const uint64_t ad = umma_desc(smem_u32(As + side * kAChunkBytes + 2 * ks * kALbo), kALbo, 128);
 #pragma unroll
-                        for (int sp = 0; sp < 3; ++sp) {
-                            const unsigned char* bsub = Bs + (side * 3 + sp) * NQ * kKChunk * 2;
-                            const uint64_t bd = umma_desc(smem_u32(bsub + 2 * ks * (NQ * 16)), NQ * 16, 128);
-                            mma_bf16(tmem + side * NQ, ad, bd, idesc, (c > 0 || ks > 0 || sp > 0) ? 1u : 0u);
+                        for (int t = 0; t < kTiles; ++t) {
+                            const uint64_t ad =
+                                umma_desc(smem_u32(As + (side * rows + t * 128 + ks * 16) * 16), 128, 128);
+#pragma unroll
+                            for (int sp = 0; sp < 3; ++sp) {
+                                const uint64_t bd =
+                                    umma_desc(smem_u32(bk + (side * 3 + sp) * NQ * kKChunk * 2), NQ * 16, 128);
+                                mma_bf16(tmem + (2 * t + side) * NQ, ad, bd, idesc, (c > 0 || ks > 0 || sp > 0) ? 1u : 0u);
+                            }
                         }
                     }
                 }
@@ -239,80 +260,90 @@ __global__ void __launch_bounds__(kGemmThreads) k_lbgemm(Geom g, GemmJob job) {
         }
         if (failed) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
-        // epilogue: thread tid <-> TMEM lane tid <-> window j0 + tid, 16 queries at a time
-        const int j = j0 + tid;
-        const bool inwin = j < kml && j >= g.lo(s);
-        const long long gi = inwin ? g.gidx(s, j) : 0;
-        const double sg = inwin ? job.SIG[s * kml + j] : 0.0;
-        const bool sig_ok = inwin && isfinite(sg) && sg > kSigmaFloor;
-        const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-        for (int q0 = 0; q0 < NQ && q0 < job.nq; q0 += 16) {
-            uint32_t rl[16], ru[16];
-            tmem_ld16(trow + q0, rl);
-            tmem_ld16(trow + NQ + q0, ru);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (tid < 16) { s_cnt[tid] = 0; s_valid[tid] = 0; }
-            __syncthreads();
+        // epilogue: warp w <-> TMEM lanes 32 (w mod 4) ...; a warpgroup takes every
+        // second block of 16 queries (every second tile where there is one block)
+#pragma unroll 1
+        for (int t = kBlocks > 1 ? 0 : half; t < kTiles; t += kBlocks > 1 ? 1 : 2) {
+            const int jw = j0 + 128 * t + 32 * (warp & 3), j = jw + lane;
+            if (jw >= kml) break;
+            const bool inwin = j < kml && j >= g.lo(s);
+            const long long gi = inwin ? g.gidx(s, j) : 0;
+            const double sg = inwin ? job.SIG[s * kml + j] : 0.0;
+            const bool sig_ok = inwin && isfinite(sg) && sg > kSigmaFloor;
+            const unsigned valid = __ballot_sync(0xffffffffu, sig_ok);
             // survivor bits of this warp's 32 consecutive windows: positions p0 .. p0+31
-            const long long p0 = s * (long long)kml + (j0 + 32 * warp) - g.lo(s);
+            const long long p0 = s * (long long)kml + jw - g.lo(s);
+            const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 2 * t * NQ;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int q = q0 + i;
-                const bool ok = q < job.nq && sig_ok && !(job.excl_b[q] >= 0 && gi >= job.excl_b[q] && gi < job.excl_e[q]);
-                bool keep = false;
-                double zz = 0.0;
-                if (ok) {
-                    const double zl = dmax0(dsub((double)__uint_as_float(rl[i]), job.margin_l[q]));
-                    const double zu = dmax0(dsub((double)__uint_as_float(ru[i]), job.margin_u[q]));
-                    zz = dadd(zl, zu);
-                    keep = !(zz > job.keep_max[q]);  // the prune test, without its square roots
+            for (int b = 0; b < kOwn; ++b) {
+                const int q0 = 16 * (kBlocks > 1 ? 2 * b + half : 0);
+                if (q0 >= job.nq) continue;
+                uint32_t rl[16], ru[16];
+                tmem_ld16(trow + q0, rl);
+                tmem_ld16(trow + NQ + q0, ru);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                auto bound = [&](int i) {  // the inner product, lowered by its margins
+                    const Limits& L = lim[q0 + i];
+                    return dadd(dmax0(dsub((double)__uint_as_float(rl[i]), L.ml)),
+                                dmax0(dsub((double)__uint_as_float(ru[i]), L.mu)));
+                };
+                unsigned mine = 0, mine_v = valid;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {  // the prune test, without its square roots
+                    const unsigned bk = __ballot_sync(0xffffffffu, !(bound(i) > lim[q0 + i].keep_max));
+                    if (lane == i) mine = bk;
                 }
-                if (job.zout && j < kml && q < job.nq) {
-                    const int metric = job.metric[q];
-                    double z = zz;
-                    if (metric == DTW || metric == ERP) z = dsqrt(zz);
-                    else if (metric == LCSS) z = ddiv(zz, (double)m);
-                    job.zout[(size_t)q * job.zstride + s * kml + j] = ok ? z : dnan();
+                if (any_excl) {
+                    for (int i = 0; i < 16 && q0 + i < job.nq; ++i) {
+                        const long long eb = job.excl_b[q0 + i], ee = job.excl_e[q0 + i];
+                        const unsigned out = __ballot_sync(0xffffffffu, eb >= 0 && gi >= eb && gi < ee);
+                        if (lane == i) mine_v &= ~out;
+                    }
                 }
-                const unsigned bv = __ballot_sync(0xffffffffu, ok);
-                const unsigned bk = __ballot_sync(0xffffffffu, keep);
-                if (lane == 0 && q < job.nq) {
-                    if (bv) atomicAdd(&s_valid[i], __popc(bv));
-                    if (bk && job.bits) {
-                        atomicAdd(&s_cnt[i], __popc(bk));
-                        unsigned* bq = job.bits + (size_t)q * job.bit_words;
+                mine &= mine_v;
+                if (job.zout) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const bool ok = __shfl_sync(0xffffffffu, mine_v, i) >> lane & 1u;
+                        if (q0 + i >= job.nq || j >= kml) continue;
+                        const int metric = job.metric[q0 + i];
+                        double z = bound(i);
+                        if (metric == DTW || metric == ERP) z = dsqrt(z);
+                        else if (metric == LCSS) z = ddiv(z, (double)m);
+                        job.zout[(size_t)(q0 + i) * job.zstride + s * kml + j] = ok ? z : dnan();
+                    }
+                }
+                if (lane < 16 && q0 + lane < job.nq) {
+                    val[b] += __popc(mine_v);
+                    if (mine && job.bits) {
+                        cnt[b] += __popc(mine);
+                        unsigned* bq = job.bits + (size_t)(q0 + lane) * job.bit_words;
                         const long long w0 = p0 >> 5;  // floor for negative p0 (short targets' tail)
                         const int sh = (int)(p0 & 31);
-                        const unsigned lo_bits = bk << sh;
+                        const unsigned lo_bits = mine << sh;
                         if (w0 >= 0 && lo_bits) atomicOr(bq + w0, lo_bits);
-                        if (sh && (bk >> (32 - sh))) atomicOr(bq + w0 + 1, bk >> (32 - sh));
+                        if (sh && (mine >> (32 - sh))) atomicOr(bq + w0 + 1, mine >> (32 - sh));
                     }
                 }
             }
-            __syncthreads();
-            if (tid < 16 && q0 + tid < job.nq) {
-                const int q = q0 + tid;
-                if (s_cnt[tid]) atomicAdd(job.nsurv + q, (unsigned long long)s_cnt[tid]);
-                if (s_valid[tid]) atomicAdd(job.nvalid + q, (unsigned long long)s_valid[tid]);
-            }
-            __syncthreads();
         }
         // the accumulators are read: the next tile may overwrite them
         asm volatile("tcgen05.fence::before_thread_sync;");
         __syncthreads();
     }
     if (failed) mbar_wait(bar, phase ^ 1);  // let issued MMAs drain (bounded) before freeing TMEM
+#pragma unroll
+    for (int b = 0; b < kOwn; ++b) {
+        const int q = 16 * (kBlocks > 1 ? 2 * b + half : 0) + lane;
+        if (lane < 16 && val[b]) atomicAdd(&s_valid[q], val[b]);
+        if (lane < 16 && cnt[b]) atomicAdd(&s_cnt[q], cnt[b]);
+    }
     __syncthreads();
+    for (int q = tid; q < job.nq; q += kGemmThreads) {
+        if (s_cnt[q]) atomicAdd(job.nsurv + q, (unsigned long long)s_cnt[q]);
+        if (s_valid[q]) atomicAdd(job.nvalid + q, (unsigned long long)s_valid[q]);
+    }
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
-}
-
-int gemm_mask_words(int m_k, int kml, int m) {
-    const int kpad = (m + kKChunk - 1) / kKChunk * kKChunk;
-    const int words = (128 + kpad + 63) / 64 + 2;  // 64-bit words a tile reads (k_lbgemm)
-    const int tiles = (kml + 127) / 128;
-    const int need = (tiles - 1) * 4 + 2 * words;   // 32-bit words up to the last tile's span
-    const int cover = (m_k + 31) / 32;
-    return (need > cover ? need : cover) + 1;
 }
 
 // One warp per 32 positions: the ballot of the threshold tests is the word.

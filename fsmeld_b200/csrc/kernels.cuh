@@ -88,7 +88,7 @@ struct GemmJob {
     const double* SIG;          // [S][kml]
     double t_l, t_u;            // the group's thresholds
     const uint4* B;             // BF16 penalty operand, per K chunk [side][split][NQ x 64] (operand layout)
-    int m, nq, kchunks;
+    int m, nq, kchunks, resident;
     const double* margin_l;     // rounding-error margins of the lower / upper inner products
     const double* margin_u;
     const int* metric;
@@ -111,13 +111,15 @@ __global__ void k_lbgemm(Geom g, GemmJob job);
 // bit p of segment s: Ln[s][p] >= t_l (mask_l), Un[s][p] <= t_u (mask_u); 0 for p >= m_k
 __global__ void k_gemm_masks(Geom g, const double* __restrict__ Ln, const double* __restrict__ Un, double t_l,
                              double t_u, unsigned* __restrict__ mask_l, unsigned* __restrict__ mask_u, int words);
-// 32-bit mask words per segment: the positions every tile of the segment reads
-int gemm_mask_words(int m_k, int kml, int m);
 const void* lbgemm_kernel(int nq_pad);  // NQ in {16, 32, 64, 128}
 __global__ void k_bits_to_list(const unsigned* __restrict__ bits, long long words, long long* __restrict__ out,
                                long long cap, unsigned long long* __restrict__ n);
-size_t lbgemm_smem_bytes(int nq_pad, int m);
-constexpr int kLbGemmThreads = 128;
+// shared memory a CTA, and whether all of B stays in it
+size_t lbgemm_smem_bytes(int nq_pad, int m, int* resident);
+// 128-window tiles of a CTA at a time, and their TMEM columns
+__host__ __device__ constexpr int lbgemm_tiles(int nq_pad) { return nq_pad >= 64 ? 1 : 64 / nq_pad; }
+__host__ __device__ constexpr int lbgemm_cols(int nq_pad) { return lbgemm_tiles(nq_pad) * 2 * nq_pad; }
+constexpr int kLbGemmThreads = 256;
 constexpr int kLbGemmKChunk = 64;
 
 // window statistics: one block per seg (mvmean_segments) segments, one warp runs the running sums

@@ -194,3 +194,33 @@ def test_noalloc_paths(api, oracle, metric, arg, m, w):  # noqa: F811
         k = min(c, cap)
         assert np.array_equal(idx[:k].cpu().numpy(), oi[keep][:k])
         assert bits_equal(dist[:k].cpu().numpy(), od[keep][:k])
+
+
+# k_lbgemm: 16 .. 128 operand columns (4 to 1 tiles at a time), the penalty
+# operand resident or by chunks, lengths off the 64-element chunks, exclusions.
+# A query's accumulators see the same terms in the same order in every group
+# that starts with the same query (which picks the thresholds), so its survivor
+# and valid counts do not depend on the group; matches are the per-query path's.
+@pytest.mark.parametrize("m,w", [(33, 2), (64, 3), (129, 6), (300, 15), (700, 30)])
+def test_lbgemm_groups(api, m, w):  # noqa: F811
+    _, kml, _, _ = _geom(m, 1 << 30)
+    t = random_walk(3 * kml + m + 77, [20, m])
+    t[kml + 50] = np.nan
+    rng = np.random.default_rng([21, m])
+    batch = []
+    for i in range(70):
+        q, _ = query_from(t, m, rng)
+        batch.append(dict(query=q, m=m, metric="dtw", w=w, arg=0.0, cutoff=0.2 * m ** 0.5))
+    batch[2]["exclude"] = (kml - 40, kml + 300)
+    with api.Engine(t) as e:
+        e.set_lb_form("fft")
+        ref = e.batch("search", batch)
+        e.set_lb_form("gemm")
+        groups = [e.batch("search", batch[:k]) for k in (3, 17, 40, 70)]
+    for got in groups:
+        for g, full, r in zip(got, groups[-1], ref):
+            assert g["status"] == 0
+            assert np.array_equal(g["idx"], r["idx"])
+            assert g["counters"]["valid"] == r["counters"]["valid"]
+            assert g["counters"]["matches"] == r["counters"]["matches"]
+            assert g["counters"]["after_lb"] == full["counters"]["after_lb"] >= r["counters"]["matches"]
