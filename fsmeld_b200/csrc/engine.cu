@@ -586,8 +586,8 @@ struct Stats {
     double* Ln = nullptr;
     double* Lraw = nullptr;  // forward windows min / max(t[p .. p+w]) of the raw target
     double* Uraw = nullptr;
-    double* Clo = nullptr;   // centred windows (GLB's Q->T terms); null when the workspace has no room for them
-    double* Cup = nullptr;
+    float* rel = nullptr;    // FP32 points and windows by segment (k_rel); null on short targets and
+    double2* rseg = nullptr;  // when the workspace has no room for them
 };
 
 static int run_stats(fsmeld_ctx* c, const Geom& g, Stats* st, const std::string& tag) {
@@ -623,25 +623,42 @@ static int launch_env(fsmeld_ctx* c, const Geom& g, int w, Stats* st) {
     return FSMELD_OK;
 }
 
+// GLB's FP32 rows: from 2^18 points on; below, the launch costs what they save
+static int run_rel(fsmeld_ctx* c, const Geom& g, int w, Stats* st, const std::string& tag) {
+    st->rel = nullptr;
+    st->rseg = nullptr;
+    const size_t N = (size_t)g.S * g.m_k;
+    double* p;
+    if (c->lean || g.n < (1 << 18) || !buf_optional(c, "rel" + tag, sizeof(double2) * g.S + sizeof(float) * 3 * N, &p))
+        return FSMELD_OK;
+    st->rseg = (double2*)p;
+    st->rel = (float*)(st->rseg + g.S);
+    const int threads = g.m_k <= 2048 ? 256 : g.m_k <= 4096 ? 512 : 1024;
+    prof_begin(c, ST_FWD);
+    k_rel<<<(unsigned)std::min<long long>(g.S, 2147483647LL), threads, 0, c->stream>>>(c->d_target, st->Lraw, st->Uraw,
+                                                                                      g, w, st->rel, st->rseg);
+    LAUNCH_CHECK(c);
+    return FSMELD_OK;
+}
+
 static int run_env(fsmeld_ctx* c, const Geom& g, int w, Stats* st, const std::string& tag) {
     int r;
     if ((r = bufT(c, "env" + tag, 2 * (size_t)g.S * g.m_k + 2 * (size_t)g.n, &st->Un))) return r;
     st->Ln = st->Un + (size_t)g.S * g.m_k;
     st->Lraw = st->Ln + (size_t)g.S * g.m_k;
     st->Uraw = st->Lraw + (size_t)g.n;
-    st->Clo = st->Cup = nullptr;
-    if (!c->lean && buf_optional(c, "ctr" + tag, sizeof(double) * 2 * (size_t)g.n, &st->Clo)) st->Cup = st->Clo + g.n;
     {
-        const size_t fsm = fwd_env_smem_bytes(w, st->Clo != nullptr);
+        const size_t fsm = fwd_env_smem_bytes(w);
         if ((r = allow_smem(c, k_fwd_env, fsm))) return r;
         int per_sm = 0;
         FSM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fwd_env, kFwdThreads, fsm));
         const unsigned fgrid = (unsigned)std::max<long long>(
             1, std::min<long long>((g.n + kFwdTile - 1) / kFwdTile, (long long)std::max(1, per_sm) * c->sm_count));
         prof_begin(c, ST_FWD);
-        k_fwd_env<<<fgrid, kFwdThreads, fsm, c->stream>>>(c->d_target, g.n, w, st->Lraw, st->Uraw, st->Clo, st->Cup);
+        k_fwd_env<<<fgrid, kFwdThreads, fsm, c->stream>>>(c->d_target, g.n, w, st->Lraw, st->Uraw);
         LAUNCH_CHECK(c);
     }
+    if ((r = run_rel(c, g, w, st, tag))) return r;
     const int mk = g.m_k;
     if (mk > 16384) return fail(FSMELD_E_UNSUPPORTED, "macro segments longer than 16384 points are not supported");
     // tiles of at least twice the window where that leaves enough blocks: the
@@ -794,12 +811,12 @@ static int run_glb(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const Stats
     double *g1b = l.d(L_G1B), *g1t = l.d(L_G1T), *g2t = l.d(L_G2T);
     GlbJob j1{};
     j1.q = qd; j1.target = c->d_target; j1.MU = st.MU; j1.SIG = st.SIG;
-    j1.lraw = st.Lraw; j1.uraw = st.Uraw; j1.clo = st.Clo; j1.cup = st.Cup;
+    j1.lraw = st.Lraw; j1.uraw = st.Uraw; j1.rel = st.rel; j1.rseg = st.rseg;
     j1.in = in; j1.n_in = cnt + C_SURV; j1.in_cap = cap;
     j1.out = g1; j1.out_b = g1b; j1.out_t = g1t; j1.n_out = cnt + C_G1; j1.out_cap = cap;
     j1.segc = segc;
     j1.cutoff_ptr = cutoff_ptr;
-    const size_t sm1 = sizeof(float2) * 2 * qd.m;
+    const size_t sm1 = sizeof(float2) * (2 * qd.m + 1);
     const void* tqf = qd.metric == DTW ? (const void*)k_glb_tq<DTW>
                     : qd.metric == ERP ? (const void*)k_glb_tq<ERP>
                     : qd.metric == EDR ? (const void*)k_glb_tq<EDR>
@@ -1816,11 +1833,12 @@ static int run_tasks_parallel(fsmeld_ctx* c, std::vector<QueryRun>& runs, const 
     return first_err;
 }
 
-// gives the centred windows back (GLB then reads two forward windows per point)
-static void drop_centred(fsmeld_ctx* c, Stats& st) {
-    if (!st.Clo) return;
-    st.Clo = st.Cup = nullptr;
-    release_buf(c, "ctr");
+// gives GLB's FP32 rows back (it then reads FP64 points and two forward windows per point)
+static void drop_rel(fsmeld_ctx* c, Stats& st) {
+    if (!st.rel) return;
+    st.rel = nullptr;
+    st.rseg = nullptr;
+    release_buf(c, "rel");
 }
 
 // One call over many queries: statistics per distinct m, envelopes per distinct
@@ -1885,12 +1903,12 @@ int run_batch(fsmeld_ctx* c, std::vector<QueryRun>& runs, std::vector<int>* stat
         std::vector<char> done(oj, 0);
         if ((r = group_gemm(c, g, st, runs, order, oi, oj, status, &done, true)) == FSMELD_E_CUDA) return r;
         // a grouped query refused for workspace runs again by itself, without
-        // the centred windows
+        // the FP32 rows
         for (size_t k = oi; k < oj; ++k)
-            if (done[k] && (*status)[order[k]] == FSMELD_E_NOMEM && st.Clo) done[k] = 2;
+            if (done[k] && (*status)[order[k]] == FSMELD_E_NOMEM && st.rel) done[k] = 2;
         if (std::count(done.begin(), done.end(), 2)) {
             for (fsmeld_ctx* w : c->workers) release_bufs(w);
-            drop_centred(c, st);
+            drop_rel(c, st);
             for (char& d : done) if (d == 2) d = 0;
         }
         std::vector<size_t> rest;
@@ -1909,8 +1927,8 @@ int run_batch(fsmeld_ctx* c, std::vector<QueryRun>& runs, std::vector<int>* stat
                     for (fsmeld_ctx* w : c->workers) release_bufs(w);
                     q = run_query(c, runs[k], g, st, have_env);
                 }
-                if (q == FSMELD_E_NOMEM && st.Clo) {
-                    drop_centred(c, st);
+                if (q == FSMELD_E_NOMEM && st.rel) {
+                    drop_rel(c, st);
                     q = run_query(c, runs[k], g, st, have_env);
                 }
                 (*status)[k] = q;
@@ -1954,7 +1972,7 @@ int run_batch(fsmeld_ctx* c, std::vector<QueryRun>& runs, std::vector<int>* stat
             }
             if (nomem && !dead) {
                 for (fsmeld_ctx* w : c->workers) release_bufs(w);
-                drop_centred(c, st);
+                drop_rel(c, st);
                 for (size_t k : rest) {
                     if ((*status)[k] != FSMELD_E_NOMEM) continue;
                     const int q = run_query(c, runs[k], g, st, have_env);

@@ -9,7 +9,8 @@
 //    the minimum of the normalised points equals the normalised minimum of the
 //    raw points, bit for bit; every envelope point is the min/max of two
 //    forward windows of the target, an interior one (w <= k <= m-1-w) a value
-//    of the centred windows (k_fwd_env).
+//    of the centred windows (k_rel).  On short lists 8 lanes share a candidate:
+//    one lane's chain of loads is what such a launch waits for.
 // What GLB decides is whether boundary + T->Q and boundary + Q->T stay within
 // the cutoff (LCSS: whether both counts reach it): running sums never decrease
 // and rounding is monotone, so glb <= cutoff exactly when both hold, and when
@@ -37,12 +38,18 @@
 //     is continuous in its arguments); the FP32 sums by a relative (m+16) 2^-23.
 //   * EDR, LCSS: terms are 0 or 1; those within 2 units of the tolerance count
 //     as 0 in one total and as 1 in the other.
-// What bounds it: instruction issue, about 14 instructions a point (T->Q) and
-// 18 (Q->T, with two unaligned 8-byte loads that keep the L1 path 84% busy)
-// where the FP64 sums took 45 and 90 issue slots.  Measured on the five-metric
-// workload (2^24 points, m = 256, w = 13), T->Q and Q->T of all five queries:
-// 19.3 and 14.6 ms with FP64 sums, 9.3 and 7.4 ms here; 8 top-k queries (m =
-// 512, 2^23 points) 18.6 and 7.6 ms -> 9.6 and 5.0 ms.
+//   * From 2^18 points on the points come in FP32, relative to the middle of
+//     their segment's range (k_rel): one FP32 multiply-add gives F, from half the
+//     bytes and without a range test (RelMap).  A warp with a window whose sigma
+//     is small against that range takes the FP64 points.
+// What bounds it: instruction issue, about 8 instructions a point (T->Q; 14 with
+// FP64 points) and 11 (Q->T; 18, with the L1 path 84% busy) where the FP64 sums
+// took 45 and 90 issue slots.  Measured on the five-metric workload (2^24 points,
+// m = 256, w = 13), T->Q and Q->T of all five queries: 19.3 and 14.6 ms with FP64
+// sums, 10.1 and 6.5 ms with fixed point, 8.0 and 5.2 ms with FP32 points (and
+// 0.1 ms for k_rel); 8 top-k queries (m = 512, 2^23 points) 18.6 and 7.6, 4.5 and
+// 1.4, 3.5 and 1.3 ms.  Q->T of 20 queries of mixed length with some thousand
+// candidates each: 1.5 ms a lane per candidate, 1.05 ms 8 lanes.
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -308,13 +315,19 @@ struct Fix {
 };
 
 template <int METRIC>
-__device__ __forceinline__ Fix make_fix(const QueryDev& q, double bsf, bool raw) {
+__device__ __forceinline__ Fix make_fix(const QueryDev& q, double bsf, bool raw, bool rel) {
     Fix f;
     const int m = q.m;
     const double xl = q.qlo, xh = q.qhi;
     const double ymax = raw ? 2.0 * (xh - xl) + 1.0 : fmax(fmax(xh, -xl), sqrt((double)m)) * 1.01 + 1.0;
     f.exact = !(ymax < 1e200) || !(bsf < kGlbMax);
-    f.scale = scalbn(1.0, f.exact ? 0 : 21 - ilogb(ymax));  // ymax 2^K < 2^22
+    int K = f.exact ? 0 : 21 - ilogb(ymax);  // ymax 2^K < 2^22
+    // FP32 points need H 2^K / sigma <= 2^21 (H: half the segment's range): K no
+    // larger than leaves room for H up to 64 (32) sigma, which one warp of 32
+    // neighbouring windows in 1000 exceeds on random walks; a unit stays far
+    // below what separates candidates (the linear sums and counts take more)
+    if (rel && !f.exact) K = raw ? K - 5 : min(K, METRIC == DTW || METRIC == ERP ? 15 : 16);
+    f.scale = scalbn(1.0, K);
     f.mid = raw && !f.exact ? rint(0.5 * (xl + xh) * f.scale) : 0.0;
     f.exact |= !(fabs(f.mid) < 0x1p50);
     const double U = bsf * f.scale, arg = q.arg * f.scale;
@@ -389,6 +402,23 @@ struct FixMap {
     __device__ __forceinline__ bool bad() const { return (badh | (badl & 0xff800000u)) != 0u; }
 };
 
+// One candidate's map from FP32 points relative to its segment to F: off by
+// less than 1.4 units where the segment allows it (ok), 0.125 from the point,
+// 0.25 from A, 0.5 from B, 0.5 from the sum, and always in range.
+struct RelMap {
+    float A, B;
+    bool ok;
+    __device__ __forceinline__ RelMap() : A(0.f), B(0.f), ok(false) {}
+    __device__ __forceinline__ RelMap(double a, double mu, double2 seg, double mid) {
+        constexpr double kMost = 0x1p21 * (1.0 - 0x1p-10);
+        A = (float)a;
+        const double p = fma(mu - seg.x, (double)A, mid);
+        B = (float)(12582912.0 - p);
+        ok = A > 1e-30f && A < 1e30f && seg.y < 1e30 && seg.y * (double)A <= kMost && fabs(p) <= kMost;
+    }
+    __device__ __forceinline__ float at(float t) const { return fmaf(t, A, B); }
+};
+
 // Sum (DTW, ERP, MSM) or certain / possible misses (EDR, LCSS).
 struct Acc {
     float s = 0.f;
@@ -445,6 +475,20 @@ __device__ __forceinline__ Acc acc_boundary(FixMap& map, const double* __restric
     return a;
 }
 
+// the sums of the 8 lanes that share a candidate
+__device__ __forceinline__ Acc group_sum(Acc a) {
+    for (int o = 4; o; o >>= 1) {
+        a.s += __shfl_xor_sync(0xffffffffu, a.s, o);
+        a.c1 += __shfl_xor_sync(0xffffffffu, a.c1, o);
+        a.c2 += __shfl_xor_sync(0xffffffffu, a.c2, o);
+    }
+    return a;
+}
+// candidates per resident group of 8 lanes up to which they share (57,000 on 148
+// SMs; T->Q lists are rarely that short, and its kernel has no registers to spare:
+// the same there made long lists 5% slower)
+constexpr unsigned long long kGrouped = 4;
+
 template <int METRIC>
 __device__ __forceinline__ bool acc_dead(const Acc& a, const Fix& f) {
     return (METRIC == EDR || METRIC == LCSS) ? a.c1 > f.most : a.s > f.hi;
@@ -465,11 +509,12 @@ __global__ void __launch_bounds__(256, 4) k_glb_tq(Geom g, GlbJob job) {
     extern __shared__ __align__(16) float2 gtq_smem[];
     const QueryDev& q = job.q;
     const int m = q.m;
-    float2* LU = gtq_smem;  // [m] query envelope as F
-    float2* Qx = LU + m;    // [m] query points as F (x)
+    constexpr int kb = METRIC == LCSS ? 0 : 1;
+    float2* LU = gtq_smem + kb;       // [m] query envelope as F, points kb, kb + 1 16-byte aligned
+    float2* Qx = gtq_smem + m + 1;    // [m] query points as F (x)
     const double bsf = job.cutoff_ptr ? *job.cutoff_ptr : q.cutoff;
     __shared__ Fix s_fix;  // one thread's divisions and roots serve the block
-    if (threadIdx.x == 0) s_fix = make_fix<METRIC>(q, bsf, g.raw != 0);
+    if (threadIdx.x == 0) s_fix = make_fix<METRIC>(q, bsf, g.raw != 0, job.rel != nullptr);
     __syncthreads();
     const Fix f = s_fix;
     for (int i = threadIdx.x; i < m; i += blockDim.x) {
@@ -477,7 +522,6 @@ __global__ void __launch_bounds__(256, 4) k_glb_tq(Geom g, GlbJob job) {
         Qx[i] = make_float2(fix_units(q.qn[i], f), 0.f);
     }
     __syncthreads();
-    constexpr int kb = METRIC == LCSS ? 0 : 1;
     const int ke = METRIC == LCSS ? m : m - 1;
     const unsigned long long n_in = *job.n_in;
     const unsigned long long n_lim = n_in < (unsigned long long)job.in_cap ? n_in : job.in_cap;
@@ -485,12 +529,11 @@ __global__ void __launch_bounds__(256, 4) k_glb_tq(Geom g, GlbJob job) {
          base += (unsigned long long)gridDim.x * blockDim.x) {
         const unsigned long long idx = base + threadIdx.x;
         const bool active = idx < n_lim;
-        long long gi = 0;
+        long long gi = 0, s = 0;
         double mu = 0.0, sg = 1.0;
+        int j = 0;
         if (active) {
             gi = job.in[idx];
-            long long s;
-            int j;
             g.locate(gi, &s, &j);
             mu = job.MU[s * g.kml + j];
             sg = job.SIG[s * g.kml + j];
@@ -502,29 +545,50 @@ __global__ void __launch_bounds__(256, 4) k_glb_tq(Geom g, GlbJob job) {
         Acc a;
         int inner = 0;  // certain misses without the boundary (the T->Q sum)
         if (__any_sync(0xffffffffu, !dead && !bad)) {
+            RelMap rm;
+            if (job.rel && active) rm = RelMap(map.A, mu, job.rseg[s], f.mid);
+            const bool fast = __all_sync(0xffffffffu, !active || (rm.ok && !bad));
             a = acc_boundary<METRIC>(map, tp, Qx, m, f);
             inner = a.c1;
-            for (int k = kb; k < ke; k += 8) {
-                if (k + 8 <= ke) {
-                    double t[8];
+            auto add = [&](int k, float F) {
+                const float2 e = LU[k];
+                acc_add<METRIC>(a, F, e.x, e.y, F - f.a, f);
+            };
+            if (fast) {
+                const float* __restrict__ rp = job.rel + (s * g.m_k + j);
+                for (int k = kb; k < ke; k += 8) {
+                    if (k + 8 <= ke) {
+                        float t[8];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) t[u] = tp[k + u];
+                        for (int u = 0; u < 8; ++u) t[u] = rp[k + u];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const float F = map.at(t[u]);
-                        const float2 e = LU[k + u];
-                        acc_add<METRIC>(a, F, e.x, e.y, F - f.a, f);
+                        for (int u = 0; u < 8; u += 2) {
+                            const float4 e = *(const float4*)(LU + k + u);
+                            const float F0 = rm.at(t[u]), F1 = rm.at(t[u + 1]);
+                            acc_add<METRIC>(a, F0, e.x, e.y, F0 - f.a, f);
+                            acc_add<METRIC>(a, F1, e.z, e.w, F1 - f.a, f);
+                        }
+                    } else {
+                        for (int u = 0; k + u < ke; ++u) add(k + u, rm.at(rp[k + u]));
                     }
-                } else {
-                    for (int u = 0; k + u < ke; ++u) {
-                        const float F = map.at(tp[k + u]);
-                        const float2 e = LU[k + u];
-                        acc_add<METRIC>(a, F, e.x, e.y, F - f.a, f);
-                    }
+                    dead = dead || acc_dead<METRIC>(a, f);
+                    if (!__any_sync(0xffffffffu, !dead)) break;
                 }
-                bad = bad || map.bad();
-                dead = dead || (!bad && acc_dead<METRIC>(a, f));
-                if (!__any_sync(0xffffffffu, !dead && !bad)) break;
+            } else {
+                for (int k = kb; k < ke; k += 8) {
+                    if (k + 8 <= ke) {
+                        double t[8];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) t[u] = tp[k + u];
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) add(k + u, map.at(t[u]));
+                    } else {
+                        for (int u = 0; k + u < ke; ++u) add(k + u, map.at(tp[k + u]));
+                    }
+                    bad = bad || map.bad();
+                    dead = dead || (!bad && acc_dead<METRIC>(a, f));
+                    if (!__any_sync(0xffffffffu, !dead && !bad)) break;
+                }
             }
             bad = bad || map.bad();  // no inner point: the boundary's own
             dead = dead || (!bad && acc_dead<METRIC>(a, f));
@@ -577,14 +641,10 @@ __global__ void __launch_bounds__(256, 4) k_glb_tq(Geom g, GlbJob job) {
 // grows with the radius.  A CTA produces kFwdTile outputs per tile from the
 // tile plus its w-point halo, ping-ponging between two shared buffers.
 //
-// With clo/cup also the centred windows min/max(t[p-w .. p+w]) of the points
-// w .. n-1-w, each the min/max of the forward windows at p-w and p, from the
-// same tile with a halo of 2w points.
 __global__ void __launch_bounds__(kFwdThreads) k_fwd_env(const double* __restrict__ t, long long n, int w,
-                                                        double* __restrict__ lo, double* __restrict__ up,
-                                                        double* __restrict__ clo, double* __restrict__ cup) {
+                                                        double* __restrict__ lo, double* __restrict__ up) {
     extern __shared__ double fw_smem[];
-    const int ext = kFwdTile + (clo ? 2 * w : w);  // tile plus halo
+    const int ext = kFwdTile + w;  // tile plus halo
     double* An = fw_smem;
     double* Ax = An + ext;
     double* Bn = Ax + ext;
@@ -629,17 +689,53 @@ __global__ void __launch_bounds__(kFwdThreads) k_fwd_env(const double* __restric
             }
             lo[p] = mn;
             up[p] = mx;
-            if (clo && p + 2 * (long long)w <= n - 1) {
-                clo[p + w] = fmin(mn, fmin(An[i + w], An[i + w + off]));
-                cup[p + w] = fmax(mx, fmax(Ax[i + w], Ax[i + w + off]));
-            }
         }
         __syncthreads();
     }
 }
 
-size_t fwd_env_smem_bytes(int w, bool centred) {
-    return sizeof(double) * 4 * (size_t)(kFwdTile + (centred ? 2 * w : w));
+size_t fwd_env_smem_bytes(int w) { return sizeof(double) * 4 * (size_t)(kFwdTile + w); }
+
+// The points and the centred windows min/max(t[p-w .. p+w]) of every macro
+// segment in FP32, relative to the middle of the segment's range, for GLB: half
+// the bytes, and one FP32 multiply-add makes F of them.  A block per segment:
+// its extremes (finite points), then the three rows (the windows where they lie
+// inside the segment).  Bound by memory: 24 bytes read (two of the three reads
+// twice, from L2) and 12 written per point.
+__global__ void k_rel(const double* __restrict__ t, const double* __restrict__ lraw, const double* __restrict__ uraw,
+                      Geom g, int w, float* __restrict__ rel, double2* __restrict__ seg) {
+    __shared__ double s_mn[32], s_mx[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5, mk = g.m_k;
+    const long long N = g.S * mk;
+    for (long long s = blockIdx.x; s < g.S; s += gridDim.x) {
+        const long long off = g.off(s);
+        double mn = INFINITY, mx = -INFINITY;
+        for (int p = tid; p < mk; p += blockDim.x) {
+            const double v = t[off + p];
+            if (isfinite(v)) {
+                mn = fmin(mn, v);
+                mx = fmax(mx, v);
+            }
+        }
+        for (int o = 16; o; o >>= 1) {
+            mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+            mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        }
+        if (lane == 0) { s_mn[warp] = mn; s_mx[warp] = mx; }
+        __syncthreads();
+        for (int i = 0; i < nw; ++i) { mn = fmin(mn, s_mn[i]); mx = fmax(mx, s_mx[i]); }
+        const double c = mn <= mx ? 0.5 * mn + 0.5 * mx : 0.0;
+        if (tid == 0) seg[s] = make_double2(c, mn <= mx ? fmax(mx - c, c - mn) * (1.0 + 0x1p-40) : INFINITY);
+        for (int p = tid; p < mk; p += blockDim.x) {
+            const long long o = s * mk + p;
+            rel[o] = (float)(t[off + p] - c);
+            if (p >= w && p < mk - w) {
+                rel[N + o] = (float)(fmin(lraw[off + p - w], lraw[off + p]) - c);
+                rel[2 * N + o] = (float)(fmax(uraw[off + p - w], uraw[off + p]) - c);
+            }
+        }
+        __syncthreads();
+    }
 }
 
 template <int METRIC>
@@ -650,7 +746,7 @@ __global__ void __launch_bounds__(256, 3) k_glb_qt(Geom g, GlbJob job) {
     float2* Qx = gqt_smem;  // [m] query points as F, and (ERP) their distance to the gap
     const double bsf = job.cutoff_ptr ? *job.cutoff_ptr : q.cutoff;
     __shared__ Fix s_fix;
-    if (threadIdx.x == 0) s_fix = make_fix<METRIC>(q, bsf, g.raw != 0);
+    if (threadIdx.x == 0) s_fix = make_fix<METRIC>(q, bsf, g.raw != 0, job.rel != nullptr);
     __syncthreads();
     const Fix f = s_fix;
     for (int i = threadIdx.x; i < m; i += blockDim.x) {
@@ -662,22 +758,25 @@ __global__ void __launch_bounds__(256, 3) k_glb_qt(Geom g, GlbJob job) {
     const double rho = (m + 16.0) * 0x1p-23;
     constexpr int kb = METRIC == LCSS ? 0 : 1;
     const int ke = METRIC == LCSS ? m : m - 1;
-    // interior points: the centred windows, where there are any
-    const bool ctr = job.clo != nullptr;
-    const int i0 = ctr ? min(max(kb, w), ke) : ke, i1 = ctr ? max(i0, min(ke, m - w)) : ke;
+    // interior points: the centred windows
+    const int in0 = min(max(kb, w), ke), in1 = max(in0, min(ke, m - w));
     const unsigned long long n_in = *job.n_in;
     const unsigned long long n_lim = n_in < (unsigned long long)job.in_cap ? n_in : job.in_cap;
-    for (unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x; base < n_lim;
-         base += (unsigned long long)gridDim.x * blockDim.x) {
-        const unsigned long long c = base + threadIdx.x;
-        const bool active = c < n_lim;
+    // short lists: 8 lanes per candidate, each every eighth point
+    const bool grouped = n_lim <= kGrouped * (unsigned long long)gridDim.x * blockDim.x / 8;
+    const int share = grouped ? 3 : 0, sub = grouped ? threadIdx.x & 7 : 0;
+    const unsigned per_block = blockDim.x >> share;
+    for (unsigned long long base = (unsigned long long)blockIdx.x * per_block; base < n_lim;
+         base += (unsigned long long)gridDim.x * per_block) {
+        const unsigned long long c = base + (threadIdx.x >> share);
+        bool active = c < n_lim;
         long long gi = 0, s = 0;
         double mu = 0.0, sg = 1.0, boundary = 0.0, tq = 0.0;
+        int j = 0;
         if (active) {
             gi = job.in[c];
             boundary = job.in_b[c];
             tq = job.in_t[c];
-            int j;
             g.locate(gi, &s, &j);
             mu = job.MU[s * g.kml + j];
             sg = job.SIG[s * g.kml + j];
@@ -691,7 +790,11 @@ __global__ void __launch_bounds__(256, 3) k_glb_qt(Geom g, GlbJob job) {
         Acc a;
         int edge = 0;
         if (__any_sync(0xffffffffu, !dead)) {
-            a = acc_boundary<METRIC>(map, job.target + gi, Qx, m, f);
+            RelMap rm;
+            if (job.rel && active) rm = RelMap(map.A, mu, job.rseg[s], f.mid);
+            const bool fast = __all_sync(0xffffffffu, dead || rm.ok);
+            const int i0 = fast ? in0 : ke, i1 = fast ? in1 : ke;
+            if (sub == 0) a = acc_boundary<METRIC>(map, job.target + gi, Qx, m, f);
             edge = a.c1;
             auto term = [&](int k, float lo, float up) {
                 const float2 x = Qx[k];
@@ -706,41 +809,74 @@ __global__ void __launch_bounds__(256, 3) k_glb_qt(Geom g, GlbJob job) {
                 dead = dead || acc_dead<METRIC>(a, f);
                 return !__any_sync(0xffffffffu, !dead);
             };
+            const float* __restrict__ cl = job.rel + (g.S * g.m_k + s * g.m_k + j);
+            const float* __restrict__ cu = cl + g.S * g.m_k;
             bool stop = false;
-            for (int k = kb; k < i0 && !stop; k += 4) {
-                if (k + 4 <= i0) {
+            if (grouped) {
+                auto some = [&](int b, int e) {  // points of [b, e), which holds no interior point or only those
+                    const bool inner = b == i0 && e == i1;
+                    for (int k = b + sub; k - sub < e && !stop; k += inner ? 64 : 16) {
+                        if (inner) {
+                            float lo[8], up[8];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) ends(k + u);
-                } else {
-                    for (int u = 0; k + u < i0; ++u) ends(k + u);
+                            for (int u = 0; u < 8; ++u) {
+                                const int kk = min(k + 8 * u, e - 1);
+                                lo[u] = cl[kk];
+                                up[u] = cu[kk];
+                            }
+#pragma unroll
+                            for (int u = 0; u < 8; ++u)
+                                if (k + 8 * u < e) term(k + 8 * u, rm.at(lo[u]), rm.at(up[u]));
+                        } else {
+#pragma unroll
+                            for (int u = 0; u < 2; ++u)
+                                if (k + 8 * u < e) ends(k + 8 * u);
+                        }
+                        Acc t = group_sum(a);
+                        dead = dead || acc_dead<METRIC>(t, f);
+                        stop = !__any_sync(0xffffffffu, !dead);
+                    }
+                };
+                some(kb, i0);
+                some(i0, i1);
+                some(i1, ke);
+                a = group_sum(a);
+                edge = __shfl_sync(0xffffffffu, edge, threadIdx.x & 24);
+            } else {
+                for (int k = kb; k < i0 && !stop; k += 4) {
+                    if (k + 4 <= i0) {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) ends(k + u);
+                    } else {
+                        for (int u = 0; k + u < i0; ++u) ends(k + u);
+                    }
+                    stop = done();
                 }
-                stop = done();
-            }
-            const double* __restrict__ cl = job.clo + gi;
-            const double* __restrict__ cu = job.cup + gi;
-            for (int k = i0; k < i1 && !stop; k += 8) {
-                if (k + 8 <= i1) {
-                    double lo[8], up[8];
+                for (int k = i0; k < i1 && !stop; k += 8) {
+                    if (k + 8 <= i1) {
+                        float lo[8], up[8];
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) { lo[u] = cl[k + u]; up[u] = cu[k + u]; }
+                        for (int u = 0; u < 8; ++u) { lo[u] = cl[k + u]; up[u] = cu[k + u]; }
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) term(k + u, map.at_checked(lo[u]), map.at_checked(up[u]));
-                } else {
-                    for (int u = 0; k + u < i1; ++u) term(k + u, map.at_checked(cl[k + u]), map.at_checked(cu[k + u]));
+                        for (int u = 0; u < 8; ++u) term(k + u, rm.at(lo[u]), rm.at(up[u]));
+                    } else {
+                        for (int u = 0; k + u < i1; ++u) term(k + u, rm.at(cl[k + u]), rm.at(cu[k + u]));
+                    }
+                    stop = done();
                 }
-                stop = done();
-            }
-            for (int k = i1; k < ke && !stop; k += 4) {
-                if (k + 4 <= ke) {
+                for (int k = i1; k < ke && !stop; k += 4) {
+                    if (k + 4 <= ke) {
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) ends(k + u);
-                } else {
-                    for (int u = 0; k + u < ke; ++u) ends(k + u);
+                        for (int u = 0; u < 4; ++u) ends(k + u);
+                    } else {
+                        for (int u = 0; k + u < ke; ++u) ends(k + u);
+                    }
+                    stop = done();
                 }
-                stop = done();
             }
             dead = dead || acc_dead<METRIC>(a, f);
         }
+        active = active && sub == 0;  // the first lane decides
         // what the abandon tests of the exact distances take: a lower bound of
         // the Q->T sum (LCSS: an upper bound of the count), the T->Q count
         double os, ot = tq;

@@ -33,8 +33,8 @@ struct GlbJob {
     const double* target;
     const double* lraw;         // forward windows min / max(t[p .. p+w]) of the raw target
     const double* uraw;
-    const double* clo;          // optional: centred windows min / max(t[p-w .. p+w])
-    const double* cup;
+    const float* rel;           // optional: [3][S m_k] FP32 relative to the segment (k_rel)
+    const double2* rseg;        // [S] what it is relative to, and how far a point is off at most
     const double* MU;
     const double* SIG;
     const long long* in;
@@ -152,8 +152,11 @@ __global__ void k_glb_qt(Geom g, GlbJob job);
 constexpr int kFwdThreads = 256;
 constexpr int kFwdTile = 2048;
 __global__ void k_fwd_env(const double* __restrict__ t, long long n, int w, double* __restrict__ lo,
-                          double* __restrict__ up, double* __restrict__ clo, double* __restrict__ cup);
-size_t fwd_env_smem_bytes(int w, bool centred);
+                          double* __restrict__ up);
+size_t fwd_env_smem_bytes(int w);
+// FP32 points and centred windows by segment, relative to its middle (GLB)
+__global__ void k_rel(const double* __restrict__ t, const double* __restrict__ lraw, const double* __restrict__ uraw,
+                      Geom g, int w, float* __restrict__ rel, double2* __restrict__ seg);
 template <int METRIC, bool GW>
 __global__ void k_dp(Geom g, DpJob job);
 // the DP kernel for a metric, with its band in shared memory or in job.gwork

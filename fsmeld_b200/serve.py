@@ -65,7 +65,7 @@ def footprint(n: int, m: int, mode: str, concurrent: int = 1) -> int:
     shared = 16 * S * kml      # window means and sigmas
     shared += 16 * S * mk      # segment envelopes U/L_normal
     shared += 16 * n           # forward windows min/max of the raw target
-    # (the centred windows, 16 n more, are given up when they do not fit)
+    # (the FP32 rows, 12 S mk more, are given up when they do not fit)
     q = 40 * tsn               # GLB stage lists (index, boundary, T->Q, survivors, Q->T)
     q += 24 * tsn              # survivors and the (index, distance) result list
     q += 16 * tsn              # sort buffers of the results

@@ -224,3 +224,34 @@ def test_lbgemm_groups(api, m, w):  # noqa: F811
             assert g["counters"]["valid"] == r["counters"]["valid"]
             assert g["counters"]["matches"] == r["counters"]["matches"]
             assert g["counters"]["after_lb"] == full["counters"]["after_lb"] >= r["counters"]["matches"]
+
+
+# GLB on FP32 rows (2^18 points and more): segments whose range dwarfs the
+# windows' sigma (FP64 points there), flat stretches, non-finite points, windows
+# without interior points, lists short enough for 8 lanes a candidate and longer
+# ones; the survivor counts are the oracle's
+@pytest.mark.parametrize("m,w,raw", [(24, 0, False), (33, 2, False), (40, 19, False), (130, 6, False), (24, 2, True)])
+@pytest.mark.parametrize("metric,arg", [("dtw", 0.0), ("erp", 0.4), ("edr", 0.25), ("lcss", 0.25), ("msm", 0.5)])
+def test_glb_fp32_rows(api, oracle, metric, arg, m, w, raw):  # noqa: F811
+    n = (1 << 18) + 77
+    t = random_walk(n, [22, m])
+    t[5000:5300] *= 1e4
+    t[9000:9400] = t[9000]
+    t[12_000:14_000] = t[12_000] + 1e-3 * np.random.default_rng(3).normal(size=2000)
+    t[13_000] += 1e6
+    t[[100, 20_000, n - 50]] = [np.nan, np.inf, np.nan]
+    q, _ = query_from(t[30_000:60_000], m, np.random.default_rng([23, m]))
+    mode = "raw" if raw else "zscore"
+    oracle.set_normalization(mode)
+    try:
+        with api.Engine(t) as e:
+            e.set_normalization(mode)
+            _, d, _ = e.cutoff(q, m, 20, metric, w, arg)
+            for cut in (float(d[-1]) * 1.001, float(d[-1]) * 1.6):
+                idx, c = e.search(q, m, cut, metric, w, arg)
+                oidx, oc = oracle.search(t, q, m, cut, metric, w, arg)
+                assert list(idx) == list(oidx)
+                assert c["after_lb"] == oc["after_lb"]
+                assert c["after_glb"] == oc["after_glb"]
+    finally:
+        oracle.set_normalization("zscore")
