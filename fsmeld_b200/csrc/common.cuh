@@ -217,6 +217,7 @@ struct QueryDev {
     double arg;
     double cutoff;
     double qlo, qhi;       // smallest and largest point of qn
+    double step;           // MSM: mean distance of neighbouring points of qn
     const double* qn;      // normalised query, original order [m]
     const double* LQ;      // query envelope (radius w) [m]
     const double* UQ;

@@ -570,6 +570,7 @@ static int upload_query(fsmeld_ctx* c, const HostQuery& hq, const std::string& s
     qd->cutoff = 0.0;
     qd->qlo = hq.qs.front();
     qd->qhi = hq.qs.back();
+    qd->step = mean_step(hq.qn.data(), hq.m);
     qd->qn = D + o_qn; qd->LQ = D + o_LQ; qd->UQ = D + o_UQ; qd->qs = D + o_qs;
     qd->pw = D + o_pw; qd->Dq = D + o_Dq; qd->tlq = D + o_tlq; qd->tuq = D + o_tuq;
     qd->opw = D + o_opw; qd->oD = D + o_oD; qd->otl = D + o_otl; qd->otu = D + o_otu;

@@ -12,6 +12,13 @@
 // on a path of at most 2m + 2 cells: the factor G.
 //   MSM: a path of true cost D costs at most (D + (2m+2) delta_c) G here
 //     (delta_c = delta + 2^-23 c).
+//     Where the query's points lie close together against c (on average within
+//     c/2), a first pass takes c alone for the steps up and left: at most the
+//     true cost, so what it drops is dropped for certain, and what it keeps runs
+//     through the second pass with the intervals.  Its slots hold a cell plus c;
+//     the two roundings of a cell's sums stay relative, that of |x-y| - c and c's
+//     share of the slot's (2^-24 (|x-y| + 2 c)) lie in delta, which has twice
+//     what the difference needs.
 //   DTW, ERP: at most (sqrt(D) + delta sqrt(2m+2))^2 G (Cauchy-Schwarz over
 //     the path's differences); for D <= R <= s^2 that is at most
 //     (R + 2 e s + e^2) G with e = delta sqrt(2m+2).
@@ -31,12 +38,16 @@
 // each point once and writes one cell for two computed, and two chains of
 // dependent operations interleave.
 //
-// What bounds it: instruction issue (DTW about 6, MSM 13 instructions per
-// cell; the exact DP spends 30 to 110 on FP64 selects and compares).  Measured
-// on the five-metric workload (2^24 points, m = 256, w = 13): MSM 82 ms by the
-// exact DP alone, 36 ms screen + 0.2 ms exact; ERP 2.6 -> 1.2 + 0.2 ms.  A warp
-// steps until its last candidate is dropped: 1.5 (MSM) to 1.9 (ERP, DTW) lane
-// rows per useful one.
+// What bounds it: instruction issue (about 6 instructions per cell for DTW, 7 and
+// 13 for MSM without and with the intervals; the exact DP spends 30 to 110 on
+// FP64 selects and compares).  Measured on the five-metric workload (2^24 points,
+// m = 256, w = 13), a query with 16 million candidates: MSM 82 ms by the exact DP
+// alone, 36 ms screen + 0.2 ms exact with intervals only, 29 + 0.2 ms with the
+// first pass (which steps 95 rows of a candidate instead of 77); ERP 2.6 -> 1.1 +
+// 0.1 ms.  A warp steps until its last candidate is dropped: 1.5 (MSM) to 1.9
+// (ERP, DTW) lane rows per useful one.
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -76,12 +87,21 @@ __device__ __forceinline__ Col make_col(float y, float yprev, float arg) {
     return c;
 }
 
-// one cell from the cells above (up), diagonal and left
-template <int METRIC>
+// What a band slot holds of a cell: its value, or (MSM without the intervals)
+// its value plus the cost of a step, which up and left moves read as it is and
+// a diagonal move takes off again under |x - y|.
+template <bool FULL>
+__device__ __forceinline__ float slot(float v, float arg) {
+    return FULL ? v : v + arg;
+}
+
+// one cell from the slots above (up), diagonal and left
+template <int METRIC, bool FULL>
 __device__ __forceinline__ float cell(float up, float diag, float left, const Row& r, const Col& c, float arg) {
     const float d = r.x - c.y;
     if (METRIC == DTW) return fmaf(d, d, min3(up, diag, left));
     if (METRIC == ERP) return min3(fmaf(d, d, diag), left + c.gy, up + r.c0);
+    if (!FULL) return min3(up, left, diag + (fabsf(d) - arg));
     // MSM: C(x, x', y) = c + the distance of x to [x', y], C(y, x, y') likewise
     const float e2 = fmaxf(arg, fminf(r.c0, fmaf(r.s, d, arg)));
     const float e3 = fmaxf(0.f, fminf(c.ady, __uint_as_float(__float_as_uint(d) ^ c.flip)));
@@ -90,10 +110,16 @@ __device__ __forceinline__ float cell(float up, float diag, float left, const Ro
 
 }  // namespace
 
+double mean_step(const double* x, int m) {
+    double s = 0.0;
+    for (int i = 1; i < m; ++i) s += fabs(x[i] - x[i - 1]);
+    return m > 1 ? s / (m - 1) : 0.0;
+}
+
 size_t screen_warp_bytes(int w) { return (size_t)(2 * w + 2 + 2 * w + 2) * 32 * sizeof(float); }
 
 template <int METRIC>
-__global__ void __launch_bounds__(kScreenThreads) k_screen(Geom g, DpJob job, long long* __restrict__ out,
+__global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_screen(Geom g, DpJob job, long long* __restrict__ out,
                                                            unsigned long long* __restrict__ n_out, long long few) {
     extern __shared__ __align__(16) float scr_smem[];
     const QueryDev& q = job.q;
@@ -130,6 +156,9 @@ __global__ void __launch_bounds__(kScreenThreads) k_screen(Geom g, DpJob job, lo
     const float ylim = (float)ymax, narrow = (float)(0x1p-21 * ymax);
     const float grow = (float)(1.0 + (m + 16.0) * 0x1p-23);
 
+    // MSM: the intervals add at most |x - x'| to a step's cost c; a mean of c/2
+    // keeps the first pass's cells within about a half of the second's
+    const bool rough = METRIC == MSM && q.step <= 0.5 * q.arg;
     unsigned long long valid_count = 0, cells = 0;
     const int erp = METRIC == ERP ? 1 : 0;
     // first row of the first pair: row 0 (ERP: -1, the empty prefix), one
@@ -160,8 +189,9 @@ __global__ void __launch_bounds__(kScreenThreads) k_screen(Geom g, DpJob job, lo
             }
         }
         if (!active) gi = 0;
-        bool keep = active;
-        if (!pass && __any_sync(kAll, active)) {
+        bool keep = active, over = false;
+        auto run = [&](auto full_c) {
+            constexpr bool FULL = decltype(full_c)::value;
             const double inv = 1.0 / sg;
             const double* __restrict__ tp = job.target + gi;
             const double* __restrict__ lr = job.lraw + gi;
@@ -170,7 +200,6 @@ __global__ void __launch_bounds__(kScreenThreads) k_screen(Geom g, DpJob job, lo
             // (R - S + Pre + E) G: the part known before the first row, rounded up
             const float lim0 = (float)((R - (casc ? S : 0.0) + Eb) * G + 0x1p-20 * lim_all);
             const float limg = (float)(G * (1.0 + 0x1p-22)) * grow;
-            bool over = false;
             float pre = 0.f;
             // ring: point k0 - w in slot 1, so a pair's columns d = 1, 2 start on an even slot
             auto point = [&](int p, double raw) {
@@ -183,7 +212,7 @@ __global__ void __launch_bounds__(kScreenThreads) k_screen(Geom g, DpJob job, lo
             };
             for (int d = 0; d < NR; ++d) A[d * 32] = kBlock;
             // the cell that the first row grows from (see the rows above the matrix below)
-            A[(w + (erp ? -k0 : 0)) * 32] = 0.f;
+            A[(w + (erp ? -k0 : 0)) * 32] = slot<FULL>(0.f, arg);
             for (int i = 0; i < NR; ++i) {
                 const int p = k0 - w + i;
                 const double raw = (active && p >= 0 && p < m) ? tp[p] : 0.0;
@@ -257,36 +286,37 @@ __global__ void __launch_bounds__(kScreenThreads) k_screen(Geom g, DpJob job, lo
                 float ext = kBlock, left2 = kBlock;
                 Col c = make_col<METRIC>(Yr[b * 32], yl0, arg);
                 float pd = A[0], pn = A[32];
-                float v1 = cell<METRIC>(pn, pd, kBlock, r1, c, arg);
+                float v1 = slot<FULL>(cell<METRIC, FULL>(pn, pd, kBlock, r1, c, arg), arg);
                 float yp = c.y;
-                int slot = b + 1 == NR ? 0 : b + 1, d = 1;
+                int sl = b + 1 == NR ? 0 : b + 1, d = 1;
                 // columns d = 1 .. 2w, two at a time (even slots: no wrap inside a two)
-                const int first = min(w, (NR - slot) >> 1);
+                const int first = min(w, (NR - sl) >> 1);
 #pragma unroll 1
                 for (int part = 0; part < 2; ++part) {
                     const int cnt = part ? w - first : first;
-                    const float* yptr = Yr + slot * 32;
+                    const float* yptr = Yr + sl * 32;
                     float* aptr = A + d * 32;
 #pragma unroll 2
                     for (int t = 0; t < cnt; ++t) {
                         const float ya = yptr[0], yb = yptr[32];
                         const float pna = aptr[32], pnb = aptr[64];
                         Col ca = make_col<METRIC>(ya, yp, arg);
-                        const float va = cell<METRIC>(pna, pn, v1, r1, ca, arg);
-                        left2 = cell<METRIC>(va, v1, left2, r2, ca, arg);
+                        const float va = slot<FULL>(cell<METRIC, FULL>(pna, pn, v1, r1, ca, arg), arg);
+                        const float l1 = cell<METRIC, FULL>(va, v1, left2, r2, ca, arg);
+                        left2 = slot<FULL>(l1, arg);
                         aptr[-32] = left2;
-                        const float l1 = left2;
                         Col cb = make_col<METRIC>(yb, ya, arg);
-                        v1 = cell<METRIC>(pnb, pna, va, r1, cb, arg);
-                        left2 = cell<METRIC>(v1, va, left2, r2, cb, arg);
+                        v1 = slot<FULL>(cell<METRIC, FULL>(pnb, pna, va, r1, cb, arg), arg);
+                        const float l2 = cell<METRIC, FULL>(v1, va, left2, r2, cb, arg);
+                        left2 = slot<FULL>(l2, arg);
                         aptr[0] = left2;
-                        ext = min3(ext, l1, left2);
+                        ext = min3(ext, l1, l2);
                         pn = pnb;
                         yp = yb;
                         yptr += 64;
                         aptr += 64;
                     }
-                    slot = 0;
+                    sl = 0;
                     d += 2 * cnt;
                 }
                 // column 2w+1: the second row's last cell only
@@ -294,9 +324,9 @@ __global__ void __launch_bounds__(kScreenThreads) k_screen(Geom g, DpJob job, lo
                     int ls = b + 2 * w + 1;
                     if (ls >= NR) ls -= NR;
                     c = make_col<METRIC>(Yr[ls * 32], yp, arg);
-                    left2 = cell<METRIC>(kBlock, v1, left2, r2, c, arg);
-                    A[2 * w * 32] = left2;
-                    ext = fminf(ext, left2);
+                    const float l1 = cell<METRIC, FULL>(kBlock, v1, left2, r2, c, arg);
+                    A[2 * w * 32] = slot<FULL>(l1, arg);
+                    ext = fminf(ext, l1);
                 }
                 cells += active ? (unsigned long long)(2 * w + 1) * 2 : 0ull;
                 // the next pair starts two columns on: the slots of this pair's
@@ -317,7 +347,16 @@ __global__ void __launch_bounds__(kScreenThreads) k_screen(Geom g, DpJob job, lo
                 if (!__any_sync(kAll, active)) break;
             }
             // the last row's cell (m-1, m-1)
-            if (active && A[w * 32] > (float)lim_all) keep = false;
+            const double last = FULL ? (double)A[w * 32] : (double)A[w * 32] * (1.0 - 0x1p-22) - (double)arg;
+            if (active && last > lim_all) keep = false;
+        };
+        if (!pass && __any_sync(kAll, active)) {
+            if (METRIC == MSM && rough) {
+                run(std::false_type{});
+                active = keep && !over;
+                __syncwarp();
+            }
+            if (__any_sync(kAll, active)) run(std::true_type{});
         }
         const unsigned mask = __ballot_sync(kAll, keep);
         if (mask) {

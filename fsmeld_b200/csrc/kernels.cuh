@@ -197,6 +197,7 @@ __global__ void k_screen(Geom g, DpJob job, long long* __restrict__ out, unsigne
                          long long few);
 const void* screen_kernel(int metric);
 size_t screen_warp_bytes(int w);
+double mean_step(const double* x, int m);  // QueryDev::step
 __global__ void k_lb_filter(Geom g, const double* __restrict__ z, const double* __restrict__ SIG,
                             const double* __restrict__ cutoff, int metric, long long* out,
                             unsigned long long* n_out, long long cap);

@@ -216,6 +216,7 @@ static int exact_noalloc(int device, const double* device_target, int64_t n, con
     qd.m = m; qd.w = w; qd.metric = metric; qd.arg = arg; qd.cutoff = cutoff; qd.qn = qn;
     qd.qlo = *std::min_element(t_qn, t_qn + m);
     qd.qhi = *std::max_element(t_qn, t_qn + m);
+    qd.step = mean_step(t_qn, m);
     DpJob dj{};
     dj.q = qd; dj.target = device_target; dj.MU = MU; dj.SIG = SIG;
     dj.list = nullptr; dj.n_windows = g.tsn; dj.mode = 0; dj.cutoff = cutoff;

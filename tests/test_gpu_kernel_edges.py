@@ -255,3 +255,24 @@ def test_glb_fp32_rows(api, oracle, metric, arg, m, w, raw):  # noqa: F811
                 assert c["after_glb"] == oc["after_glb"]
     finally:
         oracle.set_normalization("zscore")
+
+
+# k_screen, MSM: the first pass without intervals (a step's cost of at least
+# twice the mean step of the query: here for the larger costs) and the second
+# pass alone, zero cost, smooth and jumpy targets; every decision is the oracle's
+@pytest.mark.parametrize("m,w", [(16, 2), (41, 6), (96, 40), (150, 8)])
+@pytest.mark.parametrize("arg", [0.0, 0.05, 0.6, 2.0, 40.0])
+def test_screen_msm_costs(api, oracle, arg, m, w):  # noqa: F811
+    n = 5800 + m
+    t = random_walk(n, [24, m])
+    t[3000:4500] += np.random.default_rng([25, m]).normal(0.0, 20.0, 1500)
+    t[2000:2010] += 500.0
+    q, _ = query_from(t, m, np.random.default_rng([26, m]))
+    oi, od, _ = oracle.exact(t, q, m, 1e300, "msm", w, arg)
+    ranked = np.sort(od)
+    with api.Engine(t) as e:
+        for cut in (ranked[20], 0.5 * (ranked[200] + ranked[201]), ranked[len(ranked) // 2], ranked[-1]):
+            keep = od <= cut
+            gi, gd, _ = e.exact(q, m, float(cut), "msm", w, arg)
+            assert list(gi) == list(oi[keep]), cut
+            assert bits_equal(gd, od[keep]), cut
