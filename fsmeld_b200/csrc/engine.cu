@@ -919,7 +919,7 @@ static int run_screen(fsmeld_ctx* c, const Geom& g, DpJob* job) {
     const void* kf = screen_kernel(job->q.metric);
     const size_t per_warp = screen_warp_bytes(job->q.w);
     const int warps = per_warp * 4 <= 64 * 1024 ? 4 : per_warp * 2 <= 96 * 1024 ? 2 : 1;
-    const size_t smem = per_warp * warps;
+    const size_t smem = screen_smem_bytes(job->q.w, job->q.m, warps);
     int r;
     if ((r = allow_smem(c, kf, smem))) return r;
     int per_sm = 0;
@@ -1122,7 +1122,7 @@ static int search_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     double* od = l.d(L_OUTD);
     DpJob dj{};
     dj.q = qd; dj.target = c->d_target; dj.MU = st.MU; dj.SIG = st.SIG;
-    dj.lraw = st.Lraw; dj.uraw = st.Uraw;
+    dj.lraw = st.Lraw; dj.uraw = st.Uraw; dj.rel = st.rel; dj.rseg = st.rseg;
     dj.list = g2; dj.list_s = g2t; dj.list_t = g2q; dj.n_list = cnt + C_G2; dj.list_cap = cap; dj.mode = 0; dj.cutoff = qr.cutoff;
     dj.screened = surv; dj.n_screened = cnt + C_SCREEN;  // the LB_IP survivors are done with
     dj.out_idx = oi; dj.out_dist = od; dj.n_out = cnt + C_OUT; dj.n_cells = cnt + C_CELLS; dj.out_cap = cap; dj.n_valid = nullptr;
@@ -1246,7 +1246,7 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     double* od = l.d(L_OUTD);
     DpJob dj{};
     dj.q = qt; dj.target = c->d_target; dj.MU = st.MU; dj.SIG = st.SIG;
-    dj.lraw = st.Lraw; dj.uraw = st.Uraw;
+    dj.lraw = st.Lraw; dj.uraw = st.Uraw; dj.rel = st.rel; dj.rseg = st.rseg;
     dj.list = g2; dj.list_s = g2t; dj.list_t = g2q; dj.n_list = cnt + C_G2; dj.list_cap = cap; dj.mode = 1; dj.cutoff = DBL_MAX;
     dj.cutoff_ptr = tau_dev;
     if (nslot >= qr.k) { dj.screened = f1; dj.n_screened = cnt + C_SCREEN; }  // fewer seeds than k: tau is no bound

@@ -30,6 +30,10 @@
 // Points outside the matrix are +-1e15: every path through them costs at least
 // about 1e15, and the screen is skipped unless (R + E) G < 1e12.
 //
+// Points and centred windows come in FP32 relative to the segment (k_rel) where
+// there are such rows and the warp's windows allow it, else in FP64: two loads and
+// conversions less a row; the query's points in FP32 from shared memory.
+//
 // One lane per candidate, the band row and the candidate points in shared
 // memory [slot][lane].  A warp takes 32 consecutive list entries and steps
 // them together, so every index is uniform and neighbours read neighbouring
@@ -43,8 +47,10 @@
 // FP64 selects and compares).  Measured on the five-metric workload (2^24 points,
 // m = 256, w = 13), a query with 16 million candidates: MSM 82 ms by the exact DP
 // alone, 36 ms screen + 0.2 ms exact with intervals only, 29 + 0.2 ms with the
-// first pass (which steps 95 rows of a candidate instead of 77); ERP 2.6 -> 1.1 +
-// 0.1 ms.  A warp steps until its last candidate is dropped: 1.5 (MSM) to 1.9
+// first pass (which steps 95 rows of a candidate instead of 77), 28 with FP32
+// points; ERP 2.6 -> 1.1 + 0.1 ms; 8 top-k queries (m = 512) 3.9 ms with FP64
+// points, 3.6 with FP32.  DTW and ERP run best with 118 registers (8% slower at
+// 80), MSM with 72 and seven blocks an SM (4% slower at 91).  A warp steps until its last candidate is dropped: 1.5 (MSM) to 1.9
 // (ERP, DTW) lane rows per useful one.
 #include <type_traits>
 
@@ -116,6 +122,8 @@ double mean_step(const double* x, int m) {
     return m > 1 ? s / (m - 1) : 0.0;
 }
 
+size_t screen_smem_bytes(int w, int m, int warps) { return screen_warp_bytes(w) * warps + (size_t)m * sizeof(float); }
+
 size_t screen_warp_bytes(int w) { return (size_t)(2 * w + 2 + 2 * w + 2) * 32 * sizeof(float); }
 
 template <int METRIC>
@@ -128,7 +136,7 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
     constexpr unsigned kAll = 0xffffffffu;
     float* const A = scr_smem + (size_t)warp * 2 * NR * 32 + lane;  // band row A[d * 32], d in [0, 2w+1]
     float* const Yr = A + NR * 32;                                  // points, slot p - (k0-w) + 1 (mod NR)
-    const double* __restrict__ X = q.qn;
+    float* const X = scr_smem + (size_t)(blockDim.x >> 5) * 2 * NR * 32;  // [m] query points
     const unsigned long long n_all = job.list ? *job.n_list : (unsigned long long)job.n_windows;
     const unsigned long long n =
         (job.list && n_all > (unsigned long long)job.list_cap) ? job.list_cap : n_all;
@@ -138,7 +146,9 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
     const double xm = fmax(-q.qlo, q.qhi);
     const double ymax = 2.0 * xm + 8.0;
     const double cut_s = cut + 1e-9 * (1.0 + fabs(cut));
-    const double delta = 0x1p-22 * (xm + ymax + fabs(q.arg)) * 1.01;
+    // FP32 points (RelMap's range test below): off by 2^-17 + 2^-23 Y more
+    const double rel_err = job.rel ? 0x1.02p-17 + 0x1p-23 * ymax : 0.0;
+    const double delta = 0x1p-22 * (xm + ymax + fabs(q.arg)) * 1.01 + rel_err;
     const double G = 1.0 + (2.0 * m + 16.0) * 0x1p-23 * 1.01;
     double R, Eb;
     if (METRIC == MSM) {
@@ -153,12 +163,16 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
     // nothing to gain (a short list: the exact DP runs it in one wave) or no
     // proof possible: every valid candidate goes on
     const bool pass = n <= (unsigned long long)few || !(lim_all < 1e12) || !(xm + ymax + fabs(q.arg) < 1e9);
-    const float ylim = (float)ymax, narrow = (float)(0x1p-21 * ymax);
+    const float ylim = (float)ymax, narrow = (float)(0x1p-21 * ymax + 1.01 * rel_err);
     const float grow = (float)(1.0 + (m + 16.0) * 0x1p-23);
 
     // MSM: the intervals add at most |x - x'| to a step's cost c; a mean of c/2
     // keeps the first pass's cells within about a half of the second's
     const bool rough = METRIC == MSM && q.step <= 0.5 * q.arg;
+    if (!pass) {
+        for (int i = threadIdx.x; i < m; i += blockDim.x) X[i] = (float)q.qn[i];
+        __syncthreads();
+    }
     unsigned long long valid_count = 0, cells = 0;
     const int erp = METRIC == ERP ? 1 : 0;
     // first row of the first pair: row 0 (ERP: -1, the empty prefix), one
@@ -171,13 +185,12 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
         if (base >= n) break;
         const unsigned long long item = base + lane;
         bool active = item < n;
-        long long gi = 0;
+        long long gi = 0, s = 0;
+        int j = 0;
         double mu = 0.0, sg = 1.0, S = 0.0;
         bool casc = false;
         if (active) {
             gi = job.list ? job.list[item] : (long long)item;
-            long long s;
-            int j;
             g.locate(gi, &s, &j);
             mu = job.MU[s * g.kml + j];
             sg = job.SIG[s * g.kml + j];
@@ -197,6 +210,26 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
             const double* __restrict__ lr = job.lraw + gi;
             const double* __restrict__ ur = job.uraw + gi;
             const bool warp_casc = __any_sync(kAll, casc);
+            // FP32 points relative to the segment while its half range and the
+            // mean's place in it stay below 64 sigma
+            float ra = 0.f, rb = 0.f;
+            bool rel_ok = !active;
+            const float* rp = nullptr;
+            if (job.rel) {
+                rp = job.rel + (s * g.m_k + j);
+                if (active) {
+                    const double2 sr = job.rseg[s];
+                    ra = (float)inv;
+                    const double p = (sr.x - mu) * (double)ra;
+                    rb = (float)p;
+                    rel_ok = inv > 1e-30 && inv < 1e30 && sr.y < 1e30 && sr.y * inv <= 64.0 && fabs(p) <= 64.0;
+                }
+            }
+            const bool fast = job.rel && __all_sync(kAll, rel_ok);
+            const long long N = g.S * g.m_k;
+            auto pack = [](float v) { return __hiloint2double(0, __float_as_int(v)); };
+            auto unpack = [&](double v) { return fmaf(__int_as_float(__double2loint(v)), ra, rb); };
+            auto inner = [&](int k) { return fast && k >= max(w, 1) && k + 1 <= min(m - 1 - w, m - 2); };
             // (R - S + Pre + E) G: the part known before the first row, rounded up
             const float lim0 = (float)((R - (casc ? S : 0.0) + Eb) * G + 0x1p-20 * lim_all);
             const float limg = (float)(G * (1.0 + 0x1p-22)) * grow;
@@ -205,7 +238,7 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
             auto point = [&](int p, double raw) {
                 float y = p < 0 ? -kOut : kOut;
                 if (p >= 0 && p < m) {
-                    y = (float)((raw - mu) * inv);
+                    y = fast ? unpack(raw) : (float)((raw - mu) * inv);
                     over = over || !(fabsf(y) <= ylim);
                 }
                 return y;
@@ -215,7 +248,8 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
             A[(w + (erp ? -k0 : 0)) * 32] = slot<FULL>(0.f, arg);
             for (int i = 0; i < NR; ++i) {
                 const int p = k0 - w + i;
-                const double raw = (active && p >= 0 && p < m) ? tp[p] : 0.0;
+                const bool in = active && p >= 0 && p < m;
+                const double raw = !in ? 0.0 : fast ? pack(rp[p]) : tp[p];
                 Yr[((i + 1) % NR) * 32] = point(p, raw);
             }
             int b = 1;  // slot of the pair's first column
@@ -223,10 +257,24 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
             double n0 = 0.0, n1 = 0.0, ea[4], eb[4];
             auto load = [&](int k) {  // the last two points of the pair (k, k+1)
                 const int p = k + w;
-                n0 = (active && p >= 0 && p < m) ? tp[p] : 0.0;
-                n1 = (active && p + 1 >= 0 && p + 1 < m) ? tp[p + 1] : 0.0;
+                const bool i0 = active && p >= 0 && p < m, i1 = active && p + 1 >= 0 && p + 1 < m;
+                if (fast) {
+                    n0 = i0 ? pack(rp[p]) : 0.0;
+                    n1 = i1 ? pack(rp[p + 1]) : 0.0;
+                } else {
+                    n0 = i0 ? tp[p] : 0.0;
+                    n1 = i1 ? tp[p + 1] : 0.0;
+                }
             };
-            auto load_env = [&](int k) {  // its rows' forward windows
+            auto load_env = [&](int k) {  // its rows' centred (FP32) or forward windows
+                if (inner(k)) {
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        ea[2 * u] = casc ? pack(rp[N + k + u]) : 0.0;
+                        eb[2 * u] = casc ? pack(rp[2 * N + k + u]) : 0.0;
+                    }
+                    return;
+                }
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                     const int kk = k + u;
@@ -246,14 +294,14 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
                 // diagonal (DTW, MSM) or straight down (ERP, whose row -1 then
                 // gathers the deletions of the prefix) to the first real row
                 Row r1, r2;
-                r1.x = k >= 0 ? (float)X[k] : -kOut;
-                r2.x = k + 1 >= 0 ? (float)X[k + 1] : -kOut;
+                r1.x = k >= 0 ? X[k] : -kOut;
+                r2.x = k + 1 >= 0 ? X[k + 1] : -kOut;
                 if (METRIC == ERP) {
                     r1.c0 = k >= 0 ? (r1.x - arg) * (r1.x - arg) : 0.f;
                     r2.c0 = k + 1 >= 0 ? (r2.x - arg) * (r2.x - arg) : 0.f;
                     r1.s = r2.s = 0.f;
                 } else if (METRIC == MSM) {
-                    const float xp = k >= 1 ? (float)X[k - 1] : -kOut;
+                    const float xp = k >= 1 ? X[k - 1] : -kOut;
                     r1.c0 = fabsf(r1.x - xp) + arg;
                     r1.s = r1.x >= xp ? 1.f : -1.f;
                     r2.c0 = fabsf(r2.x - r1.x) + arg;
@@ -267,9 +315,18 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
                     float e2[2];
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
-                        const double a = ea[2 * u] < ea[2 * u + 1] ? ea[2 * u] : ea[2 * u + 1];
-                        const double c = eb[2 * u] > eb[2 * u + 1] ? eb[2 * u] : eb[2 * u + 1];
-                        const float lo = (float)((a - mu) * inv) + narrow, up = (float)((c - mu) * inv) - narrow;
+                        float lo, up;
+                        if (inner(k)) {
+                            lo = unpack(ea[2 * u]);
+                            up = unpack(eb[2 * u]);
+                        } else {
+                            const double a = ea[2 * u] < ea[2 * u + 1] ? ea[2 * u] : ea[2 * u + 1];
+                            const double c = eb[2 * u] > eb[2 * u + 1] ? eb[2 * u] : eb[2 * u + 1];
+                            lo = (float)((a - mu) * inv);
+                            up = (float)((c - mu) * inv);
+                        }
+                        lo += narrow;
+                        up -= narrow;
                         const float x = u ? r2.x : r1.x;
                         const float e = fmaxf(fmaxf(lo - x, x - up), 0.f);
                         float t;

@@ -56,6 +56,8 @@ struct DpJob {
     const double* target;
     const double* lraw;         // forward windows of the raw target (cascading abandon terms)
     const double* uraw;
+    const float* rel;           // optional: FP32 points and windows by segment (k_screen)
+    const double2* rseg;
     const double* MU;
     const double* SIG;
     const long long* list;      // candidates, or null for windows [0, n_windows)
@@ -197,6 +199,7 @@ __global__ void k_screen(Geom g, DpJob job, long long* __restrict__ out, unsigne
                          long long few);
 const void* screen_kernel(int metric);
 size_t screen_warp_bytes(int w);
+size_t screen_smem_bytes(int w, int m, int warps);
 double mean_step(const double* x, int m);  // QueryDev::step
 __global__ void k_lb_filter(Geom g, const double* __restrict__ z, const double* __restrict__ SIG,
                             const double* __restrict__ cutoff, int metric, long long* out,

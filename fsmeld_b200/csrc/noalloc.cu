@@ -279,7 +279,7 @@ static int exact_noalloc(int device, const double* device_target, int64_t n, con
         long long* list = (long long*)win;
         unsigned long long* n_list = cnt + 4;
         void* args[] = {&g, &dj, &list, &n_list, &few};
-        if ((r = launch(screen_kernel(metric), args, nw * 32, per_warp * nw, "k_screen"))) return r;
+        if ((r = launch(screen_kernel(metric), args, nw * 32, screen_smem_bytes(w, m, nw), "k_screen"))) return r;
         dj.list = list; dj.n_list = n_list; dj.list_cap = kMaxWin; dj.n_valid = nullptr; dj.next = cnt + 5;
         void* args2[] = {&g, &dj};
         if ((r = launch(dpw_kernel(metric, w), args2, kDpwThreads, dpw_smem_bytes(m, kDpwThreads / 32), "k_dpw")))
