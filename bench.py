@@ -156,27 +156,35 @@ def load_peaks():
 # three; MSM |x - y| + add, two split/merge costs (4 compares, 2 subs, 2 abs,
 # min, add) + adds, min of three.
 FLOPS_PER_CELL = {"dtw": 5, "erp": 11, "edr": 8, "lcss": 6, "msm": 27}
+SCREEN_OPS_PER_CELL = {"dtw": 5, "erp": 7, "msm": 6}  # k_screen
 # B200 FP64 issue rate: 148 SMs x 64 FP64 lanes x 1.965 GHz (the datasheet's
 # 37 TFLOP/s counts a fused multiply-add as two operations)
 FP64_PEAK_TOPS = 148 * 64 * 1.965e9 / 1e12
+FP32_PEAK_TOPS = 148 * 128 * 1.965e9 / 1e12
 
 
 def roofline(stages, cells, peaks):
-    """The dominant kernel, the exact DP, is FP64-bound: algorithmic work =
-    band cells it computed (device counter; early abandon skips the rest) x
-    FP64 operations per cell of the reference's recurrence, over its average
-    launch time.  The lane DP (k_dp) and the wavefront (k_dpw, where the
-    tuning table selects it) share the counter, so their launches are taken
-    together."""
-    ms_lane, n_lane = stages.get("k_dp", (0.0, 0))
-    ms_wave, n_wave = stages.get("k_dpw", (0.0, 0))
-    ms, launches = ms_lane + ms_wave, n_lane + n_wave
+    """The elastic distances of DTW, ERP and MSM: the FP32 screen (k_screen) drops
+    candidates, the exact DP (k_dpw, k_dp where the screen does not apply)
+    decides what is left.  Algorithmic work = band cells computed (one device
+    counter for both; early abandon skips the rest) x operations per cell, over
+    the average launch time of the screen and the exact DP behind it.  With a
+    screen, which computes nearly all of the cells, those are the additions,
+    multiplications and minima of its own cells (MSM: without the intervals)
+    against the FP32 issue rate; otherwise those of the reference's recurrence
+    against FP64's."""
+    screen = stages.get("k_screen", (0.0, 0))
+    exact = [stages.get(k, (0.0, 0)) for k in ("k_dp", "k_dpw")]
+    launches = screen[1] or sum(n for _, n in exact)
+    ms = screen[0] + sum(t for t, _ in exact)
     if launches == 0 or ms <= 0.0:
         return None
-    kernel = "k_dp" if n_wave == 0 else ("k_dpw" if n_lane == 0 else "k_dp+k_dpw")
-    # EDR and LCSS run as bit vectors (k_bitdp): no FP64 cells
+    kernel = "k_screen+k_dpw" if screen[1] else "k_dp" if exact[1][1] == 0 else "k_dpw" if exact[0][1] == 0 else "k_dp+k_dpw"
+    bound, peak = ("fp32", FP32_PEAK_TOPS) if screen[1] else ("fp64", FP64_PEAK_TOPS)
+    # EDR and LCSS run as bit vectors (k_bitdp): no cells of their own
     cells = {mt: c for mt, c in cells.items() if mt not in ("edr", "lcss")}
-    flops = sum(cells[mt] * FLOPS_PER_CELL[mt] for mt in cells)
+    ops = SCREEN_OPS_PER_CELL if screen[1] else FLOPS_PER_CELL
+    flops = sum(cells[mt] * ops[mt] for mt in cells)
     avg_s = ms / launches / 1e3
     achieved = flops / launches / avg_s / 1e12
     traffic = None
@@ -185,12 +193,12 @@ def roofline(stages, cells, peaks):
             traffic = json.load(f).get(kernel, {}).get("bytes_per_launch")
     except Exception:
         pass
-    return {"bound": "fp64", "kernel": kernel, "achieved": round(achieved, 3), "peak": round(FP64_PEAK_TOPS, 2),
-            "unit": "TFLOP/s", "frac": round(achieved / FP64_PEAK_TOPS, 4), "traffic": traffic,
+    return {"bound": bound, "kernel": kernel, "achieved": round(achieved, 3), "peak": round(peak, 2),
+            "unit": "TFLOP/s", "frac": round(achieved / peak, 4), "traffic": traffic,
             "algorithmic_flops_per_launch": flops / launches, "avg_launch_ms": round(avg_s * 1e3, 4),
-            "dp_cells_per_launch": sum(cells.values()) / launches, "flops_per_cell": FLOPS_PER_CELL,
-            "peak_source": "nominal FP64 issue rate of B200 (148 SMs x 64 lanes x 1.965 GHz); "
-                           "MEASURED_PEAKS.json holds no FP64 figure"}
+            "dp_cells_per_launch": sum(cells.values()) / launches, "flops_per_cell": ops,
+            "peak_source": "nominal issue rate of B200 (148 SMs x 128 FP32 or 64 FP64 lanes x 1.965 GHz); "
+                           "MEASURED_PEAKS.json holds neither"}
 
 
 def roofline_hbm(stages, geom, peaks):
@@ -221,12 +229,13 @@ def stage_rooflines(stages, geom, n, peaks):
     per launch and its average CUDA-event launch time:
       k_mvmean   8 B per segment point read (halo included) + 16 B per window
       k_envelope 8 B per segment point + 16 B per window read, 16 B per point written
-      k_fwd_env  8 B per target point read, 16 B written
+      k_fwd_env  8 B per target point read, 16 B written; from 2^18 points on as
+                 many launches of k_rel, 24 B read and 12 B written per segment point
       k_seed / k_lb_filter (k_select): 8 B per window (top-k only)"""
     S, m_k, kml = geom["S"], geom["m_k"], geom["kml"]
     per_launch = {"k_mvmean": 8.0 * S * m_k + 16.0 * S * kml,
                   "k_envelope": 8.0 * S * m_k + 16.0 * S * kml + 16.0 * S * m_k,
-                  "k_fwd_env": 24.0 * n}
+                  "k_fwd_env": 24.0 * n if n < 1 << 18 else 0.5 * (24.0 * n + 36.0 * S * m_k)}
     out = {}
     for k, b in per_launch.items():
         if k not in stages or stages[k][1] == 0:

@@ -2,8 +2,10 @@
 // include/fsmeld_cuda.h.
 //
 // Per query: window statistics (k_mvmean) -> envelopes (k_envelope) ->
-// thresholds (k_threshold) -> LB_IP + compaction (k_lbip) -> GLB
-// (k_glb_tq, k_glb_qt) -> exact DP (k_dp) -> ordered results.  Statistics
+// thresholds (k_threshold) -> LB_IP + compaction (k_lbip_runs, k_lbip or, for a
+// group, k_lbgemm) -> GLB (k_glb_tq, k_glb_qt) -> the distances: EDR and LCSS as
+// bit vectors (k_bitdp), DTW, ERP and MSM through an FP32 screen (k_screen) and
+// the exact DP (k_dpw, k_dp) -> ordered results (k_finish).  Statistics
 // and envelopes depend only on (target, m, w), so a batch computes them once
 // per distinct (m, w).  All candidate lists stay on the device; the host
 // reads back counters and the final (small) result lists.

@@ -64,7 +64,8 @@ typedef struct {
     int64_t segments;     /* full macro segments */
     int64_t tail;         /* windows in the EOF-aligned tail segment */
     double device_ms;     /* device time of the call (CUDA events) */
-    int64_t dp_cells;     /* band cells the exact DP computed (rows done x (2w+1)) */
+    int64_t dp_cells;     /* band cells computed (rows done x (2w+1)) by the FP32 screen, the
+                             bit-vector DP and the exact DP together */
 } fsmeld_counters;
 
 /* one query of a batched call */
@@ -137,7 +138,8 @@ int fsmeld_normalization(const fsmeld_ctx* ctx);
 /* LB_IP form of batched searches and top-k queries (fsmeld_batch, modes 0
  * and 1) whose queries share (m, w) and metric (no reference counterpart; the reference computes LB_IP
  * per query with FFTs, src/sip.cpp:16-52).  FSMELD_LB_FFT: per query and
- * segment, the reference's threshold selection and an FP64 FFT.
+ * segment, the reference's threshold selection and FP64 sums over the mask
+ * changes (an FP64 FFT for narrow bands, 100 (w + 1) < m).
  * FSMELD_LB_GEMM: one threshold pair for the group and the sliding inner
  * products of all its queries as one tensor-core product (BF16x3 split, FP32
  * accumulation, each bound lowered by its rounding-error margin).  Match
@@ -156,8 +158,11 @@ int fsmeld_set_lb_form(fsmeld_ctx* ctx, int form);
  *   dpx <metric> <m_k> <w_max> lane|wave   the same for the exact scan
  *   lb <metric> <m_k> <q_min>  fft|gemm    LB_IP form for groups of >= q_min searches
  *   lbk <metric> <m_k> <q_min> fft|gemm    the same for groups of top-k queries
- * Shapes no rule covers keep the built-in choice (the lane DP while its band
- * fits shared memory; the FFT LB_IP).  fsmeld_b200/tune.py measures the
+ * Shapes no rule covers keep the built-in choice (the per-query LB_IP; the lane
+ * DP while its band fits shared memory).  dp and dpx rules reach only what the
+ * FP32 screen and the bit vectors leave: lists of DTW, ERP and MSM with w < 2,
+ * a cutoff of 1e12 or more, or a band too wide for the screen; EDR and LCSS
+ * with bands past 16 words of bits.  fsmeld_b200/tune.py measures the
  * rules on the GPU and writes fsmeld_b200/tune_table.txt, which the Python
  * binding loads into every context. */
 int fsmeld_set_tuning(fsmeld_ctx* ctx, const char* table);
