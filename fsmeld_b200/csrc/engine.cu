@@ -912,16 +912,16 @@ static int run_bitdp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected
 // band and points take at most a third of an SM's shared memory; a cutoff no
 // bound can reach (every window is asked for) is not screened.
 static bool use_screen(const fsmeld_ctx* c, const DpJob& job) {
-    return job.screened && c->dp_form == 0 && !c->dp_exact && screen_kernel(job.q.metric) && job.q.w >= 2 &&
-           3 * screen_warp_bytes(job.q.w) <= (size_t)c->smem_optin && (job.cutoff_ptr || job.cutoff < 1e12) &&
+    return job.screened && c->dp_form == 0 && !c->dp_exact && screen_kernel(job.q.metric, job.q.w) && job.q.w >= 2 &&
+           3 * screen_warp_bytes(job.q.metric, job.q.w) <= (size_t)c->smem_optin && (job.cutoff_ptr || job.cutoff < 1e12) &&
            dpw_kernel(job.q.metric, job.q.w);
 }
 
 static int run_screen(fsmeld_ctx* c, const Geom& g, DpJob* job) {
-    const void* kf = screen_kernel(job->q.metric);
-    const size_t per_warp = screen_warp_bytes(job->q.w);
+    const void* kf = screen_kernel(job->q.metric, job->q.w);
+    const size_t per_warp = screen_warp_bytes(job->q.metric, job->q.w);
     const int warps = per_warp * 4 <= 64 * 1024 ? 4 : per_warp * 2 <= 96 * 1024 ? 2 : 1;
-    const size_t smem = screen_smem_bytes(job->q.w, job->q.m, warps);
+    const size_t smem = screen_smem_bytes(job->q.metric, job->q.w, job->q.m, warps);
     int r;
     if ((r = allow_smem(c, kf, smem))) return r;
     int per_sm = 0;

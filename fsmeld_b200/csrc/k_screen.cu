@@ -37,21 +37,22 @@
 // One lane per candidate, the band row and the candidate points in shared
 // memory [slot][lane].  A warp takes 32 consecutive list entries and steps
 // them together, so every index is uniform and neighbours read neighbouring
-// points.  Two rows are computed per pass: cell d of the first and cell d-1 of
-// the second row lie in the same column, so a pass reads each band cell and
-// each point once and writes one cell for two computed, and two chains of
-// dependent operations interleave.
+// points.  R rows (2, 4 or 8) are computed per pass: cell d of the first and cell
+// d-u of row u lie in the same column, so a pass reads each band cell and each
+// point once and writes one cell for R computed, tests and loads once for R rows,
+// and R chains of dependent operations interleave.
 //
-// What bounds it: instruction issue (about 6 instructions per cell for DTW, 7 and
-// 13 for MSM without and with the intervals; the exact DP spends 30 to 110 on
-// FP64 selects and compares).  Measured on the five-metric workload (2^24 points,
-// m = 256, w = 13), a query with 16 million candidates: MSM 82 ms by the exact DP
-// alone, 36 ms screen + 0.2 ms exact with intervals only, 29 + 0.2 ms with the
-// first pass (which steps 95 rows of a candidate instead of 77), 28 with FP32
-// points; ERP 2.6 -> 1.1 + 0.1 ms; 8 top-k queries (m = 512) 3.9 ms with FP64
-// points, 3.6 with FP32.  DTW and ERP run best with 118 registers (8% slower at
-// 80), MSM with 72 and seven blocks an SM (4% slower at 91).  A warp steps until its last candidate is dropped: 1.5 (MSM) to 1.9
-// (ERP, DTW) lane rows per useful one.
+// What bounds it: instruction issue (a cell takes 3 operations for DTW, 5 and 12
+// for MSM without and with the intervals, and a share of the pass; the exact DP
+// spends 30 to 110 on FP64 selects and compares).  Measured on the five-metric
+// workload (2^24 points, m = 256, w = 13), a query with 16 million candidates: MSM
+// 82 ms by the exact DP alone; screen 36 ms with intervals only, 29 with the first
+// pass (which steps 95 rows of a candidate instead of 77), 28 with FP32 points, 22
+// with four rows a pass instead of two, and 0.2 ms exact; ERP 2.6 -> 0.95 + 0.1 ms;
+// 8 top-k queries (DTW, m = 512) 3.9 ms with two rows and FP64 points, 2.1 now.
+// DTW and ERP run best with 120 registers (8% slower at 80), MSM with 80 and six
+// blocks an SM (3% slower at 72).  A warp steps until its last candidate is
+// dropped: 1.5 (MSM) to 1.9 (ERP, DTW) lane rows per useful one.
 #include <type_traits>
 
 #include "common.cuh"
@@ -122,21 +123,35 @@ double mean_step(const double* x, int m) {
     return m > 1 ? s / (m - 1) : 0.0;
 }
 
-size_t screen_smem_bytes(int w, int m, int warps) { return screen_warp_bytes(w) * warps + (size_t)m * sizeof(float); }
+// Rows a pass: four from w = 4 on (ERP's row -4 lies inside the band), DTW eight
+// from w = 12.  A pass of R rows has R - 1 columns more than the band at half
+// their work.  Measured with two, four and eight rows: DTW w = 13 0.20, 0.148,
+// 0.119 ms, w = 26 (8 queries) 3.6, 2.46, 2.07; ERP w = 13 1.13, 0.95, 1.01; MSM
+// w = 13 27.9, 21.9, 24.0 (registers).  The widest bands keep two rows, whose
+// points still fit a third of an SM's shared memory (up to w = 150).
+static int screen_rows(int metric, int w) {
+    return w < 4 || w > 149 ? 2 : metric == DTW && w >= 12 && w <= 128 ? 8 : 4;
+}
 
-size_t screen_warp_bytes(int w) { return (size_t)(2 * w + 2 + 2 * w + 2) * 32 * sizeof(float); }
+size_t screen_warp_bytes(int metric, int w) {
+    return (size_t)(2 * w + 2 + 2 * w + screen_rows(metric, w)) * 32 * sizeof(float);
+}
 
-template <int METRIC>
-__global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_screen(Geom g, DpJob job, long long* __restrict__ out,
+size_t screen_smem_bytes(int metric, int w, int m, int warps) {
+    return screen_warp_bytes(metric, w) * warps + (size_t)m * sizeof(float);
+}
+
+template <int METRIC, int R>
+__global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 6 : 1) k_screen(Geom g, DpJob job, long long* __restrict__ out,
                                                            unsigned long long* __restrict__ n_out, long long few) {
     extern __shared__ __align__(16) float scr_smem[];
     const QueryDev& q = job.q;
-    const int m = q.m, w = q.w, NR = 2 * w + 2;
+    const int m = q.m, w = q.w, NR = 2 * w + R;  // points of a pass's columns
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr unsigned kAll = 0xffffffffu;
-    float* const A = scr_smem + (size_t)warp * 2 * NR * 32 + lane;  // band row A[d * 32], d in [0, 2w+1]
-    float* const Yr = A + NR * 32;                                  // points, slot p - (k0-w) + 1 (mod NR)
-    float* const X = scr_smem + (size_t)(blockDim.x >> 5) * 2 * NR * 32;  // [m] query points
+    float* const A = scr_smem + (size_t)warp * (2 * w + 2 + NR) * 32 + lane;  // band row A[d * 32], d in [0, 2w+1]
+    float* const Yr = A + (2 * w + 2) * 32;                                   // points, slot p - (k0-w) + 1 (mod NR)
+    float* const X = scr_smem + (size_t)(blockDim.x >> 5) * (2 * w + 2 + NR) * 32;  // [m] query points
     const unsigned long long n_all = job.list ? *job.n_list : (unsigned long long)job.n_windows;
     const unsigned long long n =
         (job.list && n_all > (unsigned long long)job.list_cap) ? job.list_cap : n_all;
@@ -150,16 +165,16 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
     const double rel_err = job.rel ? 0x1.02p-17 + 0x1p-23 * ymax : 0.0;
     const double delta = 0x1p-22 * (xm + ymax + fabs(q.arg)) * 1.01 + rel_err;
     const double G = 1.0 + (2.0 * m + 16.0) * 0x1p-23 * 1.01;
-    double R, Eb;
+    double Rc, Eb;
     if (METRIC == MSM) {
-        R = cut_s;
+        Rc = cut_s;
         Eb = (2.0 * m + 2.0) * (delta + 0x1p-23 * fabs(q.arg));
     } else {
         const double e = delta * sqrt(2.0 * m + 2.0);
-        R = cut_s * cut_s * (1.0 + 0x1p-50);
+        Rc = cut_s * cut_s * (1.0 + 0x1p-50);
         Eb = 2.0 * e * cut_s + e * e;
     }
-    const double lim_all = (R + Eb) * G * (1.0 + 0x1p-20);
+    const double lim_all = (Rc + Eb) * G * (1.0 + 0x1p-20);
     // nothing to gain (a short list: the exact DP runs it in one wave) or no
     // proof possible: every valid candidate goes on
     const bool pass = n <= (unsigned long long)few || !(lim_all < 1e12) || !(xm + ymax + fabs(q.arg) < 1e9);
@@ -175,9 +190,9 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
     }
     unsigned long long valid_count = 0, cells = 0;
     const int erp = METRIC == ERP ? 1 : 0;
-    // first row of the first pair: row 0 (ERP: -1, the empty prefix), one
-    // earlier when that makes the number of rows even
-    const int k0 = ((m + erp) & 1) ? -1 - erp : -erp;
+    // first row of the first pass: row 0 (ERP: -1, the empty prefix), earlier when
+    // that makes the number of rows a multiple of R
+    const int k0 = -erp - (R - (m + erp) % R) % R;
     for (;;) {
         unsigned long long base = 0;
         if (lane == 0) base = atomicAdd(job.next, 32ull);
@@ -229,12 +244,12 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
             const long long N = g.S * g.m_k;
             auto pack = [](float v) { return __hiloint2double(0, __float_as_int(v)); };
             auto unpack = [&](double v) { return fmaf(__int_as_float(__double2loint(v)), ra, rb); };
-            auto inner = [&](int k) { return fast && k >= max(w, 1) && k + 1 <= min(m - 1 - w, m - 2); };
+            auto inner = [&](int k) { return fast && k >= max(w, 1) && k + R - 1 <= min(m - 1 - w, m - 2); };
             // (R - S + Pre + E) G: the part known before the first row, rounded up
-            const float lim0 = (float)((R - (casc ? S : 0.0) + Eb) * G + 0x1p-20 * lim_all);
+            const float lim0 = (float)((Rc - (casc ? S : 0.0) + Eb) * G + 0x1p-20 * lim_all);
             const float limg = (float)(G * (1.0 + 0x1p-22)) * grow;
             float pre = 0.f;
-            // ring: point k0 - w in slot 1, so a pair's columns d = 1, 2 start on an even slot
+            // ring: point k0 - w in slot 1, so a pass's columns R-1, R start on an even slot
             auto point = [&](int p, double raw) {
                 float y = p < 0 ? -kOut : kOut;
                 if (p >= 0 && p < m) {
@@ -243,7 +258,7 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
                 }
                 return y;
             };
-            for (int d = 0; d < NR; ++d) A[d * 32] = kBlock;
+            for (int d = 0; d < 2 * w + 2; ++d) A[d * 32] = kBlock;
             // the cell that the first row grows from (see the rows above the matrix below)
             A[(w + (erp ? -k0 : 0)) * 32] = slot<FULL>(0.f, arg);
             for (int i = 0; i < NR; ++i) {
@@ -252,149 +267,140 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
                 const double raw = !in ? 0.0 : fast ? pack(rp[p]) : tp[p];
                 Yr[((i + 1) % NR) * 32] = point(p, raw);
             }
-            int b = 1;  // slot of the pair's first column
-            // inputs of the next pair, loaded a pair ahead
-            double n0 = 0.0, n1 = 0.0, ea[4], eb[4];
-            auto load = [&](int k) {  // the last two points of the pair (k, k+1)
-                const int p = k + w;
-                const bool i0 = active && p >= 0 && p < m, i1 = active && p + 1 >= 0 && p + 1 < m;
-                if (fast) {
-                    n0 = i0 ? pack(rp[p]) : 0.0;
-                    n1 = i1 ? pack(rp[p + 1]) : 0.0;
-                } else {
-                    n0 = i0 ? tp[p] : 0.0;
-                    n1 = i1 ? tp[p + 1] : 0.0;
+            int b = 1;  // slot of the pass's first column
+            auto ring = [&](int i) { return b + i >= NR ? b + i - NR : b + i; };
+            // points of the next pass, loaded a pass ahead
+            double nx[R];
+            auto load = [&](int k) {
+#pragma unroll
+                for (int u = 0; u < R; ++u) {
+                    const int p = k + w + u;
+                    const bool in = active && p >= 0 && p < m;
+                    nx[u] = !in ? 0.0 : fast ? pack(rp[p]) : tp[p];
                 }
             };
-            auto load_env = [&](int k) {  // its rows' centred (FP32) or forward windows
-                if (inner(k)) {
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        ea[2 * u] = casc ? pack(rp[N + k + u]) : 0.0;
-                        eb[2 * u] = casc ? pack(rp[2 * N + k + u]) : 0.0;
-                    }
-                    return;
-                }
-#pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const int kk = k + u;
-                    const bool in = casc && active && kk >= 1 && kk <= m - 2;
-                    const int p0 = in ? qt_p0(kk, w) : 0, p1 = in ? qt_p1(kk, m, w) : 0;
-                    ea[2 * u] = in ? lr[p0] : 0.0;
-                    ea[2 * u + 1] = in ? lr[p1] : 0.0;
-                    eb[2 * u] = in ? ur[p0] : 0.0;
-                    eb[2 * u + 1] = in ? ur[p1] : 0.0;
-                }
+            // the term of row k on its narrowed window
+            auto term = [&](float lo, float up, float x) {
+                const float e = fmaxf(fmaxf((lo + narrow) - x, x - (up - narrow)), 0.f);
+                if (METRIC == MSM) return fminf(e, arg * (1.f + 0x1p-22f));
+                if (METRIC == ERP) return fminf(e * e, (fabsf(x - arg) + narrow) * (fabsf(x - arg) + narrow));
+                return e * e;
             };
-            float yl0 = -kOut;  // the point left of the pair's first column (MSM)
-            if (warp_casc) load_env(k0);
-            for (int k = k0; k < m; k += 2) {
+            float yl0 = -kOut;  // the point left of the pass's first column (MSM)
+            for (int k = k0; k < m; k += R) {
                 // rows above the matrix: x = -1e15 matches the padding left of it
                 // at no cost and nothing else, so the zero travels down the
                 // diagonal (DTW, MSM) or straight down (ERP, whose row -1 then
                 // gathers the deletions of the prefix) to the first real row
-                Row r1, r2;
-                r1.x = k >= 0 ? X[k] : -kOut;
-                r2.x = k + 1 >= 0 ? X[k + 1] : -kOut;
-                if (METRIC == ERP) {
-                    r1.c0 = k >= 0 ? (r1.x - arg) * (r1.x - arg) : 0.f;
-                    r2.c0 = k + 1 >= 0 ? (r2.x - arg) * (r2.x - arg) : 0.f;
-                    r1.s = r2.s = 0.f;
-                } else if (METRIC == MSM) {
-                    const float xp = k >= 1 ? X[k - 1] : -kOut;
-                    r1.c0 = fabsf(r1.x - xp) + arg;
-                    r1.s = r1.x >= xp ? 1.f : -1.f;
-                    r2.c0 = fabsf(r2.x - r1.x) + arg;
-                    r2.s = r2.x >= r1.x ? 1.f : -1.f;
-                } else {
-                    r1.c0 = r2.c0 = r1.s = r2.s = 0.f;
-                }
-                if (k + 2 < m) load(k + 2);
-                // terms of the pair's rows on the narrowed envelope
-                if (warp_casc) {
-                    float e2[2];
+                Row r[R];
 #pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        float lo, up;
-                        if (inner(k)) {
-                            lo = unpack(ea[2 * u]);
-                            up = unpack(eb[2 * u]);
-                        } else {
-                            const double a = ea[2 * u] < ea[2 * u + 1] ? ea[2 * u] : ea[2 * u + 1];
-                            const double c = eb[2 * u] > eb[2 * u + 1] ? eb[2 * u] : eb[2 * u + 1];
-                            lo = (float)((a - mu) * inv);
-                            up = (float)((c - mu) * inv);
-                        }
-                        lo += narrow;
-                        up -= narrow;
-                        const float x = u ? r2.x : r1.x;
-                        const float e = fmaxf(fmaxf(lo - x, x - up), 0.f);
-                        float t;
-                        if (METRIC == MSM) t = fminf(e, arg * (1.f + 0x1p-22f));
-                        else if (METRIC == ERP) t = fminf(e * e, (fabsf(x - arg) + narrow) * (fabsf(x - arg) + narrow));
-                        else t = e * e;
-                        e2[u] = (casc && k + u >= 1 && k + u <= m - 2) ? t : 0.f;
+                for (int u = 0; u < R; ++u) {
+                    const int kk = k + u;
+                    const float x = kk >= 0 ? X[kk] : -kOut;
+                    r[u].x = x;
+                    r[u].c0 = r[u].s = 0.f;
+                    if (METRIC == ERP) r[u].c0 = kk >= 0 ? (x - arg) * (x - arg) : 0.f;
+                    if (METRIC == MSM && FULL) {
+                        const float xp = kk >= 1 ? X[kk - 1] : -kOut;
+                        r[u].c0 = fabsf(x - xp) + arg;
+                        r[u].s = x >= xp ? 1.f : -1.f;
                     }
-                    pre += e2[0];
-                    pre += e2[1];
-                    if (k + 2 < m) load_env(k + 2);
                 }
-                // the pair
-                float ext = kBlock, left2 = kBlock;
-                Col c = make_col<METRIC>(Yr[b * 32], yl0, arg);
-                float pd = A[0], pn = A[32];
-                float v1 = slot<FULL>(cell<METRIC, FULL>(pn, pd, kBlock, r1, c, arg), arg);
-                float yp = c.y;
-                int sl = b + 1 == NR ? 0 : b + 1, d = 1;
-                // columns d = 1 .. 2w, two at a time (even slots: no wrap inside a two)
-                const int first = min(w, (NR - sl) >> 1);
+                if (k + R < m) load(k + R);
+                float el[R], eu[R];  // the rows' centred windows, for the test at the pass's end
+                const bool mid = warp_casc && inner(k);
+                if (mid) {
+#pragma unroll
+                    for (int u = 0; u < R; ++u) {
+                        el[u] = casc ? rp[N + k + u] : 0.f;
+                        eu[u] = casc ? rp[2 * N + k + u] : 0.f;
+                    }
+                }
+                // the pass, column by column: row u's cell there is band cell c - u
+                float ext = kBlock, pv[R];
+#pragma unroll
+                for (int u = 0; u < R; ++u) pv[u] = kBlock;
+                float yp = yl0, pd = A[0];
+                auto column = [&](float y, float diag0, float up0, int lo, int hi) {  // rows lo .. hi
+                    const Col c = make_col<METRIC>(y, yp, arg);
+                    float diag = diag0, up = up0, last = kBlock;
+#pragma unroll
+                    for (int u = 0; u < R; ++u) {
+                        if (u < lo || u > hi) {
+                            diag = pv[u];
+                            pv[u] = up = kBlock;
+                            continue;
+                        }
+                        const float v = cell<METRIC, FULL>(up, diag, pv[u], r[u], c, arg);
+                        diag = pv[u];
+                        pv[u] = up = slot<FULL>(v, arg);
+                        last = v;
+                    }
+                    yp = y;
+                    return last;
+                };
+                // columns 0 .. R-2: the upper rows only
+#pragma unroll
+                for (int c = 0; c < R - 1; ++c) {
+                    const float pn = A[(c + 1) * 32];
+                    column(Yr[ring(c) * 32], pd, pn, 0, c);
+                    pd = pn;
+                }
+                // columns R-1 .. 2w, two at a time (even slots: no wrap inside a two)
+                const int all = w - R / 2 + 1;
+                int sl = ring(R - 1), d = R - 1;
+                const int first = min(all, (NR - sl) >> 1);
 #pragma unroll 1
                 for (int part = 0; part < 2; ++part) {
-                    const int cnt = part ? w - first : first;
+                    const int cnt = part ? all - first : first;
                     const float* yptr = Yr + sl * 32;
                     float* aptr = A + d * 32;
 #pragma unroll 2
                     for (int t = 0; t < cnt; ++t) {
                         const float ya = yptr[0], yb = yptr[32];
                         const float pna = aptr[32], pnb = aptr[64];
-                        Col ca = make_col<METRIC>(ya, yp, arg);
-                        const float va = slot<FULL>(cell<METRIC, FULL>(pna, pn, v1, r1, ca, arg), arg);
-                        const float l1 = cell<METRIC, FULL>(va, v1, left2, r2, ca, arg);
-                        left2 = slot<FULL>(l1, arg);
-                        aptr[-32] = left2;
-                        Col cb = make_col<METRIC>(yb, ya, arg);
-                        v1 = slot<FULL>(cell<METRIC, FULL>(pnb, pna, va, r1, cb, arg), arg);
-                        const float l2 = cell<METRIC, FULL>(v1, va, left2, r2, cb, arg);
-                        left2 = slot<FULL>(l2, arg);
-                        aptr[0] = left2;
+                        const float l1 = column(ya, pd, pna, 0, R - 1);
+                        aptr[-32 * (R - 1)] = pv[R - 1];
+                        const float l2 = column(yb, pna, pnb, 0, R - 1);
+                        aptr[-32 * (R - 2)] = pv[R - 1];
                         ext = min3(ext, l1, l2);
-                        pn = pnb;
-                        yp = yb;
+                        pd = pnb;
                         yptr += 64;
                         aptr += 64;
                     }
                     sl = 0;
                     d += 2 * cnt;
                 }
-                // column 2w+1: the second row's last cell only
-                {
-                    int ls = b + 2 * w + 1;
-                    if (ls >= NR) ls -= NR;
-                    c = make_col<METRIC>(Yr[ls * 32], yp, arg);
-                    const float l1 = cell<METRIC, FULL>(kBlock, v1, left2, r2, c, arg);
-                    A[2 * w * 32] = slot<FULL>(l1, arg);
+                // columns 2w+1 .. 2w+R-1: the lower rows only
+#pragma unroll
+                for (int c = 1; c < R; ++c) {
+                    const float l1 = column(Yr[ring(2 * w + c) * 32], kBlock, kBlock, c, R - 1);
+                    A[(2 * w + c - R + 1) * 32] = pv[R - 1];
                     ext = fminf(ext, l1);
                 }
-                cells += active ? (unsigned long long)(2 * w + 1) * 2 : 0ull;
-                // the next pair starts two columns on: the slots of this pair's
-                // first two columns take its last two points
-                if (METRIC == MSM) yl0 = Yr[(b + 1 == NR ? 0 : b + 1) * 32];
-                if (k + 2 < m) {
-                    const int p = k + 2 + w;
-                    Yr[b * 32] = point(p, n0);
-                    Yr[(b + 1 == NR ? 0 : b + 1) * 32] = point(p + 1, n1);
-                    b += 2;
+                cells += active ? (unsigned long long)(2 * w + 1) * R : 0ull;
+                // the next pass starts R columns on: the slots of this pass's
+                // first R columns take its last R points
+                if (METRIC == MSM && FULL) yl0 = Yr[ring(R - 1) * 32];
+                if (k + R < m) {
+#pragma unroll
+                    for (int u = 0; u < R; ++u) Yr[ring(u) * 32] = point(k + R + w + u, nx[u]);
+                    b += R;
                     if (b >= NR) b -= NR;
+                }
+                // terms of the pass's rows
+                if (mid) {
+#pragma unroll
+                    for (int u = 0; u < R; ++u)
+                        pre += casc ? term(fmaf(el[u], ra, rb), fmaf(eu[u], ra, rb), r[u].x) : 0.f;
+                } else if (warp_casc) {
+                    for (int u = 0; u < R; ++u) {
+                        const int kk = k + u;
+                        if (!(casc && active && kk >= 1 && kk <= m - 2)) continue;
+                        const int p0 = qt_p0(kk, w), p1 = qt_p1(kk, m, w);
+                        const double a = lr[p0] < lr[p1] ? lr[p0] : lr[p1], c = ur[p0] > ur[p1] ? ur[p0] : ur[p1];
+                        pre += term((float)((a - mu) * inv), (float)((c - mu) * inv), X[kk]);
+                    }
                 }
                 if (over) {  // keep: the bound does not cover it
                     active = false;
@@ -434,15 +440,14 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 7 : 1) k_scree
     }
 }
 
-template __global__ void k_screen<DTW>(Geom, DpJob, long long*, unsigned long long*, long long);
-template __global__ void k_screen<ERP>(Geom, DpJob, long long*, unsigned long long*, long long);
-template __global__ void k_screen<MSM>(Geom, DpJob, long long*, unsigned long long*, long long);
-
-const void* screen_kernel(int metric) {
+const void* screen_kernel(int metric, int w) {
+    const int rows = screen_rows(metric, w);
     switch (metric) {
-        case DTW: return (const void*)k_screen<DTW>;
-        case ERP: return (const void*)k_screen<ERP>;
-        case MSM: return (const void*)k_screen<MSM>;
+        case DTW:
+            return rows == 8 ? (const void*)k_screen<DTW, 8>
+                 : rows == 4 ? (const void*)k_screen<DTW, 4> : (const void*)k_screen<DTW, 2>;
+        case ERP: return rows == 4 ? (const void*)k_screen<ERP, 4> : (const void*)k_screen<ERP, 2>;
+        case MSM: return rows == 4 ? (const void*)k_screen<MSM, 4> : (const void*)k_screen<MSM, 2>;
         default: return nullptr;
     }
 }

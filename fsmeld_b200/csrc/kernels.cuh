@@ -194,12 +194,12 @@ __host__ __device__ inline size_t bit_table_offset(int m) {
 // FP32 screen before the exact DP (DTW, ERP, MSM): the candidates it cannot
 // drop, to out; lists of at most `few` entries go on whole
 constexpr int kScreenThreads = 128;
-template <int METRIC>
+template <int METRIC, int R>
 __global__ void k_screen(Geom g, DpJob job, long long* __restrict__ out, unsigned long long* __restrict__ n_out,
                          long long few);
-const void* screen_kernel(int metric);
-size_t screen_warp_bytes(int w);
-size_t screen_smem_bytes(int w, int m, int warps);
+const void* screen_kernel(int metric, int w);
+size_t screen_warp_bytes(int metric, int w);
+size_t screen_smem_bytes(int metric, int w, int m, int warps);
 double mean_step(const double* x, int m);  // QueryDev::step
 __global__ void k_lb_filter(Geom g, const double* __restrict__ z, const double* __restrict__ SIG,
                             const double* __restrict__ cutoff, int metric, long long* out,

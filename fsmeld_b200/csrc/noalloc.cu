@@ -273,13 +273,13 @@ static int exact_noalloc(int device, const double* device_target, int64_t n, con
         }
     } else if (w >= 2 && cutoff < 1e12 && dpw_kernel(metric, w) &&
                dpw_smem_bytes(m, kDpwThreads / 32) + 1024 <= (size_t)dev_optin) {
-        const size_t per_warp = screen_warp_bytes(w);
+        const size_t per_warp = screen_warp_bytes(metric, w);
         const int nw = per_warp * 4 <= 64 * 1024 ? 4 : per_warp * 2 <= 96 * 1024 ? 2 : 1;
         long long few = 32LL * sms;
         long long* list = (long long*)win;
         unsigned long long* n_list = cnt + 4;
         void* args[] = {&g, &dj, &list, &n_list, &few};
-        if ((r = launch(screen_kernel(metric), args, nw * 32, screen_smem_bytes(w, m, nw), "k_screen"))) return r;
+        if ((r = launch(screen_kernel(metric, w), args, nw * 32, screen_smem_bytes(metric, w, m, nw), "k_screen"))) return r;
         dj.list = list; dj.n_list = n_list; dj.list_cap = kMaxWin; dj.n_valid = nullptr; dj.next = cnt + 5;
         void* args2[] = {&g, &dj};
         if ((r = launch(dpw_kernel(metric, w), args2, kDpwThreads, dpw_smem_bytes(m, kDpwThreads / 32), "k_dpw")))

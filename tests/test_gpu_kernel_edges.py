@@ -276,3 +276,23 @@ def test_screen_msm_costs(api, oracle, arg, m, w):  # noqa: F811
             gi, gd, _ = e.exact(q, m, float(cut), "msm", w, arg)
             assert list(gi) == list(oi[keep]), cut
             assert bits_equal(gd, od[keep]), cut
+
+
+# k_screen's rows a pass (2, 4, 8 by metric and band): band widths on both sides
+# of each rule, every remainder of the row count; every decision is the oracle's
+@pytest.mark.parametrize("m", [25, 26, 27, 28, 29, 30, 31, 32])
+@pytest.mark.parametrize("w", [3, 4, 11, 12, 24])
+@pytest.mark.parametrize("metric,arg", [("dtw", 0.0), ("erp", 0.4), ("msm", 0.5)])
+def test_screen_rows_a_pass(api, oracle, metric, arg, m, w):  # noqa: F811
+    n = 5700 + m
+    t = random_walk(n, [27, m])
+    t[4100] = np.nan
+    q, _ = query_from(t, m, np.random.default_rng([28, m]))
+    oi, od, _ = oracle.exact(t, q, m, 1e300, metric, w, arg)
+    ranked = np.sort(od)
+    with api.Engine(t) as e:
+        for cut in (ranked[20], 0.5 * (ranked[300] + ranked[301]), ranked[len(ranked) // 2]):
+            keep = od <= cut
+            gi, gd, _ = e.exact(q, m, float(cut), metric, w, arg)
+            assert list(gi) == list(oi[keep]), cut
+            assert bits_equal(gd, od[keep]), cut
