@@ -298,8 +298,7 @@ constexpr int kWarpExact = 6;  // candidates of a warp decided one after another
 
 // ------------------------------------------------ fixed point and FP32 sums
 
-constexpr float kF0 = 12582912.0f;                 // 1.5 * 2^23
-constexpr double kM = 6755399441055744.0 + (double)0x4b400000;  // 1.5 * 2^52 + the bits of kF0
+constexpr double kM = 6755399441055744.0 + (double)0x4b400000;  // 1.5 * 2^52 + the bits of the float 1.5 * 2^23
 constexpr unsigned kMHi = 0x43380000u;             // upper word of every in-range v
 
 // Scale and limits of one query at one cutoff, in units of 2^-K.

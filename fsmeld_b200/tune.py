@@ -10,12 +10,12 @@ Two choices depend on the shape and are settled by measurement:
   walk), `dpx` rules for the exact scan of every window (timed at the
   rank-20 distance on a random walk).
 * the LB_IP form of batched searches (`lb` rules) and top-k queries (`lbk`):
-  per-query thresholds and FP64 FFTs, or one tensor-core product for the
+  per-query thresholds and FP64 sums, or one tensor-core product for the
   group, per metric, m_k and group size.  Timed as one batched `search` of
   the group at each query's rank-10 distance, and one batched `cutoff` k=10,
   on a 2^22-point random walk.
 
-A rule departs from the built-in choice (lane DP, FFT LB_IP) only where the
+A rule departs from the built-in choice (lane DP, per-query LB_IP) only where the
 other form measured at least MARGIN (5%) faster, so timing noise between two
 nearly equal forms does not flip a shape back and forth.  Shapes where the
 lane DP's band does not fit shared memory need no measurement (the wavefront
