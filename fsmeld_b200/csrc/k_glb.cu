@@ -503,8 +503,11 @@ __device__ __forceinline__ float fix_units(double x, const Fix& f) {
 
 }  // namespace
 
+// Five blocks an SM (48 registers, the exact path spills): a list of a few hundred
+// thousand candidates is as much latency as issue.  32 DTW queries (m = 128, 2^22
+// points) 2.75, 2.40, 2.27 ms at three, four and five, 2.23 at six, where MSM loses 2%.
 template <int METRIC>
-__global__ void __launch_bounds__(256, 4) k_glb_tq(Geom g, GlbJob job) {
+__global__ void __launch_bounds__(256, 5) k_glb_tq(Geom g, GlbJob job) {
     extern __shared__ __align__(16) float2 gtq_smem[];
     const QueryDev& q = job.q;
     const int m = q.m;
