@@ -46,9 +46,9 @@
 // FP64 points) and 11 (Q->T; 18, with the L1 path 84% busy) where the FP64 sums
 // took 45 and 90 issue slots.  Measured on the five-metric workload (2^24 points,
 // m = 256, w = 13), T->Q and Q->T of all five queries: 19.3 and 14.6 ms with FP64
-// sums, 10.1 and 6.5 ms with fixed point, 8.0 and 5.2 ms with FP32 points (and
+// sums, 10.1 and 6.5 ms with fixed point, 7.9 and 5.2 ms with FP32 points (and
 // 0.1 ms for k_rel); 8 top-k queries (m = 512, 2^23 points) 18.6 and 7.6, 4.5 and
-// 1.4, 3.5 and 1.3 ms.  Q->T of 20 queries of mixed length with some thousand
+// 1.4, 3.4 and 1.2 ms.  Q->T of 20 queries of mixed length with some thousand
 // candidates each: 1.5 ms a lane per candidate, 1.05 ms 8 lanes.
 #include "common.cuh"
 #include "kernels.cuh"
