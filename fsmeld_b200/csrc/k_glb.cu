@@ -395,7 +395,7 @@ struct FixMap {
         badl |= l ^ 0x4b000000u;
         return __uint_as_float(l);
     }
-    __device__ __forceinline__ float at_checked(double t) const {  // a point already checked
+    __device__ __forceinline__ float at_checked(double t) const {  // T->Q has checked every point of the window
         return __uint_as_float((unsigned)__double2loint(fma(t, A, B)));
     }
     __device__ __forceinline__ bool bad() const { return (badh | (badl & 0xff800000u)) != 0u; }
@@ -451,6 +451,9 @@ __device__ __forceinline__ Acc acc_boundary(FixMap& map, const double* __restric
     Acc a;
     if (METRIC == LCSS) return a;
     const float TL = map.at(tp[m - 1]), ql = Qx[m - 1].x;
+    // EDR and ERP have no term of point 0, but Q->T's envelopes hold it: its range
+    // is checked with the others'
+    if (METRIC == EDR || METRIC == ERP) map.at(tp[0]);
     if (METRIC == EDR) {
         const float e = fabsf(ql - TL);
         a.c1 = e > f.e1 ? 1 : 0;

@@ -1,0 +1,43 @@
+"""Pruning decisions that hang on a single point, against the oracle (needs a
+B200)."""
+import numpy as np
+import pytest
+
+from tests.test_gpu_parity import api, bits_equal  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+# GLB in raw mode: a window that matches but for one point far outside the
+# fixed-point range (the first, the last, one inside).  The spikes' fixed-point
+# words are NaN, negative and tiny floats; below 2^18 points the sums run on FP64
+# points, above on FP32 rows where a segment's range allows it.
+@pytest.mark.parametrize("n,spike", [(6000, 1e4), (6000, -1e4), (6000, 3e4), (6000, 1e5), (6000, 1e6), (6000, -1e6),
+                                     (6000, 1e12), ((1 << 18) + 500, 1e6), ((1 << 18) + 500, 1e12)])
+@pytest.mark.parametrize("metric,arg,w", [("edr", 0.25, 10), ("lcss", 0.25, 10), ("erp", 0.0, 10), ("erp", 40.0, 3),
+                                          ("dtw", 0.0, 10), ("msm", 0.5, 10)])
+def test_one_point_out_of_range(api, oracle, metric, arg, w, spike, n):  # noqa: F811
+    m = 64
+    rng = np.random.default_rng(41)
+    q = np.arange(m - 1.0, -1.0, -1.0)
+    t = 500.0 + rng.normal(0.0, 1.0, n)
+    starts = (1000, 2000, 3000, 4000)
+    for s, p in zip(starts, (0, m - 1, m // 2, 5)):
+        t[s:s + m] = q - 2.0
+        t[s + p] = spike
+    oracle.set_normalization("raw")
+    try:
+        d = min(oracle.distance(metric, q, t[s:s + m].copy(), w, arg) for s in starts)
+        far = max(oracle.distance(metric, q, t[s:s + m].copy(), w, arg) for s in starts)
+        with api.Engine(t) as e:
+            e.set_normalization("raw")
+            for cut in (d, 1.5 * d, far):
+                idx, c = e.search(q, m, cut, metric, w, arg)
+                oidx, oc = oracle.search(t, q, m, cut, metric, w, arg)
+                assert list(idx) == list(oidx), cut
+                assert c["after_glb"] == oc["after_glb"], cut
+            ci, cd, _ = e.cutoff(q, m, 4, metric, w, arg)
+            oi, od, _ = oracle.cutoff(t, q, m, 4, metric, w, arg)
+            assert list(ci) == list(oi) and bits_equal(cd, od)
+    finally:
+        oracle.set_normalization("zscore")
