@@ -19,7 +19,10 @@
 //     candidates;
 //  3. every valid window whose LB does not exceed tau (k_lb_filter) goes
 //     through GLB at tau and then the exact DP; any window whose distance is
-//     at most the true k-th distance survives both admissible bounds;
+//     at most the true k-th distance survives both admissible bounds.  Where
+//     a bound equals the distance (narrow bands, flat runs) its sum, taken in
+//     another order, can round above it, so tau is the k-th distance and a
+//     little more (raise);
 //  4. a lexicographic sort of the surviving (distance, index) pairs gives the
 //     ranking and the threshold.
 #include <cfloat>
@@ -186,6 +189,11 @@ __device__ void sort_pairs(Pair* __restrict__ v, int n, PairSort::TempStorage& t
     __syncthreads();
 }
 
+// A bound for the filters from a distance: more than the roundings that a lower
+// bound's sum of up to 2 m terms may lie above the distance's by (2^-30 is over a
+// hundred times that at m = 16384; the absolute term covers squares that underflow).
+__device__ double raise(double d) { return d < 1e300 ? d * (1.0 + 0x1p-30) + 1e-150 : d; }
+
 }  // namespace
 
 // The end of a query in one block: up to kFinishSort results in their order (by
@@ -257,7 +265,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_order(const unsigned long lo
     }
 }
 
-// The bound tau (the k-th smallest seed distance, DBL_MAX with fewer than k
+// The bound tau (the k-th smallest seed distance, raised; DBL_MAX with fewer than k
 // seeds) and the windows to refine it with.  Seeds lie at the smallest bound of
 // their stretch; the windows next to a good match are good matches too, and
 // most of the ranking usually, so the kRefineReach windows on either side of
@@ -282,7 +290,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_tau_block(const double* __re
     if (threadIdx.x == 0) s_np = s_n = 0;
     __syncthreads();
     if (!sorted) sort_pairs(v, n, tmp);
-    if (threadIdx.x == 0) *tau = k <= n_all ? (k <= n ? v[k - 1].d : dist[k - 1]) : DBL_MAX;
+    if (threadIdx.x == 0) *tau = k <= n_all ? raise(k <= n ? v[k - 1].d : dist[k - 1]) : DBL_MAX;
     if (!picks) return;
     if (threadIdx.x < 32) {
         // best first, 32 seeds at a time: those that clash with no pick so far,
@@ -329,7 +337,7 @@ __global__ void __launch_bounds__(kFinishThreads) k_tau_refine(const double* __r
     for (int i = threadIdx.x; i < n; i += blockDim.x) v[i] = Pair{dist[i], i};
     __syncthreads();
     sort_pairs(v, n, tmp);
-    if (threadIdx.x == 0 && v[k - 1].d < *tau) *tau = v[k - 1].d;
+    if (threadIdx.x == 0) *tau = fmin(*tau, raise(v[k - 1].d));
 }
 
 size_t finish_smem_bytes() { return sizeof(Pair) * kFinishSort + sizeof(PairSort::TempStorage) + 16; }

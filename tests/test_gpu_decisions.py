@@ -1,8 +1,9 @@
-"""Pruning decisions that hang on a single point, against the oracle (needs a
-B200)."""
+"""Pruning decisions that hang on a single point or on the last bit of a
+distance, against the oracle (needs a B200)."""
 import numpy as np
 import pytest
 
+from fsmeld_b200.synth import query_from, random_walk, walk_with_structure
 from tests.test_gpu_parity import api, bits_equal  # noqa: F401
 
 pytestmark = pytest.mark.gpu
@@ -39,5 +40,34 @@ def test_one_point_out_of_range(api, oracle, metric, arg, w, spike, n):  # noqa:
             ci, cd, _ = e.cutoff(q, m, 4, metric, w, arg)
             oi, od, _ = oracle.cutoff(t, q, m, 4, metric, w, arg)
             assert list(ci) == list(oi) and bits_equal(cd, od)
+    finally:
+        oracle.set_normalization("zscore")
+
+
+# Top-k where GLB equals the distance in exact arithmetic and exceeds it by its
+# rounding: bands of radius 0 (the envelopes are the points), and flat runs beside
+# each other in raw mode (many windows at the k-th distance).
+@pytest.mark.parametrize("seed", range(6))
+@pytest.mark.parametrize("metric,arg", [("dtw", 0.0), ("erp", 0.4), ("msm", 0.5), ("edr", 0.25), ("lcss", 0.25)])
+def test_ranking_at_equal_bounds(api, oracle, metric, arg, seed):  # noqa: F811
+    m = (17, 38, 40, 64, 101, 200)[seed]
+    t = random_walk(5000 + m, [42, seed])
+    q, _ = query_from(t, m, np.random.default_rng([43, seed]))
+    with api.Engine(t) as e:
+        for k in (1, 2, 3, 5, 10, 20):
+            ci, cd, _ = e.cutoff(q, m, k, metric, 0, arg)
+            oi, od, _ = oracle.cutoff(t, q, m, k, metric, 0, arg)
+            assert list(ci) == list(oi) and bits_equal(cd, od), k
+    scale, shift = 10.0 ** (seed - 4), (0.0, 833.0, 1e4)[seed % 3]
+    t = walk_with_structure(6800, m, seed=[44, seed], nan_fraction=1e-3, flat_runs=4) * scale + shift
+    q, _ = query_from(np.where(np.isfinite(t), t, shift), m, np.random.default_rng([45, seed]))
+    oracle.set_normalization("raw")
+    try:
+        with api.Engine(t) as e:
+            e.set_normalization("raw")
+            for k in (1, 10, 60):
+                ci, cd, _ = e.cutoff(q, m, k, metric, 8, arg * scale)
+                oi, od, _ = oracle.cutoff(t, q, m, k, metric, 8, arg * scale)
+                assert list(ci) == list(oi) and bits_equal(cd, od), k
     finally:
         oracle.set_normalization("zscore")
