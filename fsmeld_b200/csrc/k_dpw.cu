@@ -24,7 +24,13 @@
 // instructions of its K chunks, one warp against a full-length candidate of
 // 2m steps; the lists it gets are short.  Away from the matrix's corners a pair
 // of steps runs without index arithmetic or tests; blocks of one warp spread
-// a short list over the SMs.
+// a short list over the SMs.  On long lists MSM's wide bands are bound by the
+// instruction cache and the registers as well: with the corner steps twice in the
+// code (before and after the interior) and 128 to 254 registers, 65,536 candidates
+// took 11.8 ms (m = 200, w = 100), 32.5 (m = 400, w = 150), 58.8 (m = 728, w = 161)
+// and 134 (m = 700, w = 250).  So from four chunks on MSM has them once: 9.3, 24.6,
+// 49.4 and 81 ms.  At five and six chunks it reads the points before its own again
+// from shared memory instead of holding them, at six it is held to 168 registers.
 // Cells outside the band or outside the matrix hold the reference's
 // out-of-band value (MAX_VAL = 1e18, 0 for LCSS), which is exactly what the
 // reference reads for such neighbours; row 0 and column 0 of ERP, EDR and
@@ -159,12 +165,13 @@ size_t dpw_smem_bytes(int m, int warps) {
 }
 
 template <int METRIC, int K>
-__global__ void __launch_bounds__(kDpwThreads) k_dpw(Geom g, DpJob job) {
+__global__ void __launch_bounds__(kDpwThreads, METRIC == MSM && K == 6 ? 12 : 0) k_dpw(Geom g, DpJob job) {
     extern __shared__ __align__(16) double dpw_smem[];
     const QueryDev& q = job.q;
     const int m = q.m, w = q.w;
     constexpr bool ONE_BASED = (METRIC == ERP || METRIC == EDR);
     constexpr double SENT = (METRIC == LCSS) ? 0.0 : kDpMax;
+    constexpr bool kOneCopy = METRIC == MSM && K >= 4, kReload = METRIC == MSM && (K == 5 || K == 6);
     const int R = ONE_BASED ? m : m - 1;  // last grid row and column
     const int W2 = 2 * w + 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -322,8 +329,7 @@ __global__ void __launch_bounds__(kDpwThreads) k_dpw(Geom g, DpJob job) {
         // row and column, for w < h < R.
         constexpr int SH = ONE_BASED ? 1 : 0;  // grid (i, j) reads points i - 1, j - 1
         const int hlo = w + 1, hhi = R;        // interior: hlo <= h < hhi
-        edge_steps(hhi > hlo ? 2 * hlo - w : 2 * R + 1);
-        if (!stop && hhi > hlo) {
+        auto interior = [&] {
             // lanes past the band in the last chunk read the band's last points
             const int dlast = 64 * (K - 1) + 2 * lane;
             const bool oke = dlast < W2, oko = dlast + 1 < W2;
@@ -346,6 +352,11 @@ __global__ void __launch_bounds__(kDpwThreads) k_dpw(Geom g, DpJob job) {
                     const int o = (c == K - 1 ? ll : lane) + 32 * c;
                     xq[c] = px[-o];
                     yn[c] = py[o + 1];
+                    if (kReload) {
+                        xp[c] = px[-o - 1];
+                        yp[c] = py[o - 1];
+                        yq[c] = py[o];
+                    }
                 }
 #pragma unroll
                 for (int c = 0; c < K; ++c) rot[c] = __shfl_sync(0xffffffffu, O[c], (lane + 31) & 31);
@@ -373,7 +384,7 @@ __global__ void __launch_bounds__(kDpwThreads) k_dpw(Geom g, DpJob job) {
                     if (stop) break;
                 }
 #pragma unroll
-                for (int c = 0; c < K; ++c) {
+                for (int c = 0; c < K && !kReload; ++c) {
                     yp[c] = yq[c];
                     yq[c] = yn[c];
                     xp[c] = xq[c];
@@ -381,9 +392,23 @@ __global__ void __launch_bounds__(kDpwThreads) k_dpw(Geom g, DpJob job) {
                 ++px;
                 ++py;
             }
-            if (!stop) {
-                a = 2 * hhi - w;
-                edge_steps(2 * R + 1);
+            if (!stop) a = 2 * hhi - w;
+        };
+        bool before = hhi > hlo;
+        if (kOneCopy) {
+#pragma unroll 1
+            for (;;) {
+                edge_steps(before ? 2 * hlo - w : 2 * R + 1);
+                if (stop || !before) break;
+                before = false;
+                interior();
+                if (stop) break;
+            }
+        } else {
+            edge_steps(before ? 2 * hlo - w : 2 * R + 1);
+            if (before && !stop) {
+                interior();
+                if (!stop) edge_steps(2 * R + 1);
             }
         }
         if (stop) {
