@@ -573,6 +573,8 @@ static int upload_query(fsmeld_ctx* c, const HostQuery& hq, const std::string& s
     qd->qlo = hq.qs.front();
     qd->qhi = hq.qs.back();
     qd->step = mean_step(hq.qn.data(), hq.m);
+    qd->spread = query_spread(hq.metric, hq.qn.data(), hq.m);
+    qd->loose = screen_loose(hq.metric, qd->spread, c->raw);
     qd->qn = D + o_qn; qd->LQ = D + o_LQ; qd->UQ = D + o_UQ; qd->qs = D + o_qs;
     qd->pw = D + o_pw; qd->Dq = D + o_Dq; qd->tlq = D + o_tlq; qd->tuq = D + o_tuq;
     qd->opw = D + o_opw; qd->oD = D + o_oD; qd->otl = D + o_otl; qd->otu = D + o_otu;
@@ -907,14 +909,15 @@ static int run_bitdp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected
     return FSMELD_OK;
 }
 
-// DTW, ERP, MSM: the FP32 screen, then `job` is the exact DP over what it left.
+// DTW, ERP, MSM: the FP32 screen, then `job` is the exact DP over what it left (by
+// the wavefront, or for long lists long_dp).
 // Bands from w = 2 (the kernel's row -2 lies inside the band) while a warp's
 // band and points take at most a third of an SM's shared memory; a cutoff no
 // bound can reach (every window is asked for) is not screened.
 static bool use_screen(const fsmeld_ctx* c, const DpJob& job) {
     return job.screened && c->dp_form == 0 && !c->dp_exact && screen_kernel(job.q.metric, job.q.w) && job.q.w >= 2 &&
            3 * screen_warp_bytes(job.q.metric, job.q.w) <= (size_t)c->smem_optin && (job.cutoff_ptr || job.cutoff < 1e12) &&
-           dpw_kernel(job.q.metric, job.q.w);
+           dpw_kernel(job.q.metric, job.q.w) && dpw_smem_bytes(job.q.m, kDpwThreads / 32) + 1024 <= (size_t)c->smem_optin;
 }
 
 static int run_screen(fsmeld_ctx* c, const Geom& g, DpJob* job) {
@@ -944,8 +947,9 @@ static int run_screen(fsmeld_ctx* c, const Geom& g, DpJob* job) {
 }
 
 // the query's counters, all zero, and behind them the work counters of its DP
-// launches (the seeds' and the survivors', a screen and an exact DP each)
-constexpr int kNexts = 4;
+// launches (the seeds', the refining windows', and the survivors' screen and two
+// exact DPs)
+constexpr int kNexts = 5;
 static int zero_counters(fsmeld_ctx* c, unsigned long long** cnt) {
     int r;
     if ((r = bufT(c, "counters", C_N + kNexts, cnt))) return r;
@@ -968,6 +972,7 @@ static int run_dp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
     unsigned grid;
     if (use_bitdp(c, job.q)) return run_bitdp(c, g, job, expected);
     const bool screened = use_screen(c, job);
+    const long long list_max = job.list ? job.list_cap : job.n_windows;
     if (screened) {
         if ((r = run_screen(c, g, &job))) return r;
         next_counter(c);
@@ -989,9 +994,25 @@ static int run_dp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
         grid = (unsigned)std::max<long long>(1, std::min<long long>(want, (long long)std::max(1, per_sm) * c->sm_count));
         prof_begin(c, ST_DPW);
         Geom ga = g;
+        // a screened list's length stays on the device: both kernels are launched
+        // where it may be long, and one of them finds nothing to do (2 us)
+        LongDp ld{};
+        if (screened) ld = long_dp(job, c->sm_count);
+        const bool two = ld.kernel && list_max > ld.from;
+        if (two) job.run_to = ld.from;
         void* args[] = {&ga, &job};
-        const cudaError_t le = cudaLaunchKernel(wk, dim3(grid), dim3(kDpwThreads), args, wsm, c->stream);
+        cudaError_t le = cudaLaunchKernel(wk, dim3(grid), dim3(kDpwThreads), args, wsm, c->stream);
         if (le != cudaSuccess) return cuda_fail(le, "k_dpw launch", __FILE__, __LINE__);
+        LAUNCH_CHECK(c);
+        if (!two) return FSMELD_OK;
+        job.run_from = ld.from;
+        job.run_to = 0;
+        job.next = next_counter(c);
+        if ((r = allow_smem(c, ld.kernel, ld.smem))) return r;
+        prof_begin(c, ld.lane ? ST_DP : ST_DPW);
+        le = cudaLaunchKernel(ld.kernel, dim3((unsigned)(ld.blocks * c->sm_count)), dim3(ld.threads), args, ld.smem,
+                              c->stream);
+        if (le != cudaSuccess) return cuda_fail(le, "exact DP launch", __FILE__, __LINE__);
         LAUNCH_CHECK(c);
         return FSMELD_OK;
     }
@@ -1252,6 +1273,7 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     dj.list = g2; dj.list_s = g2t; dj.list_t = g2q; dj.n_list = cnt + C_G2; dj.list_cap = cap; dj.mode = 1; dj.cutoff = DBL_MAX;
     dj.cutoff_ptr = tau_dev;
     if (nslot >= qr.k) { dj.screened = f1; dj.n_screened = cnt + C_SCREEN; }  // fewer seeds than k: tau is no bound
+    dj.few = picks > 0;
     dj.out_idx = oi; dj.out_dist = od; dj.n_out = cnt + C_OUT; dj.n_cells = cnt + C_CELLS; dj.out_cap = cap;
     if ((r = run_dp(c, g, dj, (long long)c->sm_count * 16 * 128))) return r;
     std::vector<int64_t> ki(qr.k);

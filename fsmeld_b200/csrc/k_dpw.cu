@@ -164,8 +164,13 @@ size_t dpw_smem_bytes(int m, int warps) {
     return sizeof(double) * (xq + (size_t)warps * dpw_warp_doubles(m));
 }
 
-template <int METRIC, int K>
-__global__ void __launch_bounds__(kDpwThreads, METRIC == MSM && K == 6 ? 12 : 0) k_dpw(Geom g, DpJob job) {
+// blocks an SM the registers are held to (0: as many registers as it takes)
+constexpr int dpw_blocks(int metric, int k, bool inner) {
+    return metric != MSM ? 0 : inner ? (k == 6 ? 12 : 0) : k < 7 ? 28 : 0;
+}
+
+template <int METRIC, int K, bool INNER>
+__global__ void __launch_bounds__(kDpwThreads, dpw_blocks(METRIC, K, INNER)) k_dpw(Geom g, DpJob job) {
     extern __shared__ __align__(16) double dpw_smem[];
     const QueryDev& q = job.q;
     const int m = q.m, w = q.w;
@@ -184,7 +189,8 @@ __global__ void __launch_bounds__(kDpwThreads, METRIC == MSM && K == 6 ? 12 : 0)
 
     const unsigned long long n_all = job.list ? *job.n_list : (unsigned long long)job.n_windows;
     const unsigned long long n =
-        (job.list && n_all > (unsigned long long)job.list_cap) ? job.list_cap : n_all;
+        other_length(job, n_all) ? 0ull
+        : (job.list && n_all > (unsigned long long)job.list_cap) ? job.list_cap : n_all;
     const double cut = job.cutoff_ptr ? *job.cutoff_ptr : job.cutoff;
     const double arg = q.arg;
     const double cut_s = wslack(cut);
@@ -394,14 +400,14 @@ __global__ void __launch_bounds__(kDpwThreads, METRIC == MSM && K == 6 ? 12 : 0)
             }
             if (!stop) a = 2 * hhi - w;
         };
-        bool before = hhi > hlo;
+        bool before = INNER && hhi > hlo;
         if (kOneCopy) {
 #pragma unroll 1
             for (;;) {
                 edge_steps(before ? 2 * hlo - w : 2 * R + 1);
                 if (stop || !before) break;
                 before = false;
-                interior();
+                if (INNER) interior();
                 if (stop) break;
             }
         } else {
@@ -448,32 +454,36 @@ __host__ __device__ size_t dpw_warp_doubles(int m) {
     return y + s4;
 }
 
-#define FSM_DPW_INST(M)                                     \
-    template __global__ void k_dpw<M, 1>(Geom, DpJob);      \
-    template __global__ void k_dpw<M, 2>(Geom, DpJob);      \
-    template __global__ void k_dpw<M, 3>(Geom, DpJob);      \
-    template __global__ void k_dpw<M, 4>(Geom, DpJob);      \
-    template __global__ void k_dpw<M, 5>(Geom, DpJob);      \
-    template __global__ void k_dpw<M, 6>(Geom, DpJob);      \
-    template __global__ void k_dpw<M, 7>(Geom, DpJob);      \
-    template __global__ void k_dpw<M, 8>(Geom, DpJob);
+#define FSM_DPW_INST(M)                                           \
+    template __global__ void k_dpw<M, 1, true>(Geom, DpJob);      \
+    template __global__ void k_dpw<M, 2, true>(Geom, DpJob);      \
+    template __global__ void k_dpw<M, 3, true>(Geom, DpJob);      \
+    template __global__ void k_dpw<M, 4, true>(Geom, DpJob);      \
+    template __global__ void k_dpw<M, 5, true>(Geom, DpJob);      \
+    template __global__ void k_dpw<M, 6, true>(Geom, DpJob);      \
+    template __global__ void k_dpw<M, 7, true>(Geom, DpJob);      \
+    template __global__ void k_dpw<M, 8, true>(Geom, DpJob);
 FSM_DPW_INST(DTW)
 FSM_DPW_INST(ERP)
 FSM_DPW_INST(EDR)
 FSM_DPW_INST(LCSS)
 FSM_DPW_INST(MSM)
+template __global__ void k_dpw<MSM, 5, false>(Geom, DpJob);
+template __global__ void k_dpw<MSM, 6, false>(Geom, DpJob);
+template __global__ void k_dpw<MSM, 7, false>(Geom, DpJob);
+template __global__ void k_dpw<MSM, 8, false>(Geom, DpJob);
 
 template <int M>
 static const void* dpw_for(int k) {
     switch (k) {
-        case 1: return (const void*)k_dpw<M, 1>;
-        case 2: return (const void*)k_dpw<M, 2>;
-        case 3: return (const void*)k_dpw<M, 3>;
-        case 4: return (const void*)k_dpw<M, 4>;
-        case 5: return (const void*)k_dpw<M, 5>;
-        case 6: return (const void*)k_dpw<M, 6>;
-        case 7: return (const void*)k_dpw<M, 7>;
-        case 8: return (const void*)k_dpw<M, 8>;
+        case 1: return (const void*)k_dpw<M, 1, true>;
+        case 2: return (const void*)k_dpw<M, 2, true>;
+        case 3: return (const void*)k_dpw<M, 3, true>;
+        case 4: return (const void*)k_dpw<M, 4, true>;
+        case 5: return (const void*)k_dpw<M, 5, true>;
+        case 6: return (const void*)k_dpw<M, 6, true>;
+        case 7: return (const void*)k_dpw<M, 7, true>;
+        case 8: return (const void*)k_dpw<M, 8, true>;
         default: return nullptr;
     }
 }
@@ -488,6 +498,46 @@ const void* dpw_kernel(int metric, int w) {
         case LCSS: return dpw_for<LCSS>(k);
         default: return dpw_for<MSM>(k);
     }
+}
+
+// Long lists.  What the screen leaves runs to its last row mostly, so the lanes of
+// the lane-per-candidate DP stay together, and it computes a band of 2w+1 cells
+// where the wavefront's warp computes 64: 131,072 candidates of m = 256 take (ms,
+// lane / wavefront), DTW w = 2 0.54 / 2.57, w = 13 1.19 / 2.66, w = 20 2.38 / 2.71,
+// w = 26 3.55 / 2.76; MSM w = 6 1.24 / 5.44, w = 20 4.45 / 5.69, w = 26 6.9 / 5.8; the
+// line lies where four of its blocks still fit an SM.  A short list takes it the
+// time of one candidate, which the wavefront needs for (m = 256, DTW and MSM) 11,300
+// and 6700 candidates at w = 2, 14,700 and 10,200 at w = 6, 20,400 and 16,100 at
+// w = 13, 26,500 and 22,000 at w = 20; m = 64 up to a fifth more, m = 1000 a third less.
+// MSM's widest bands, where 2w comes near m: the kernel without interior steps runs
+// two to three times the warps (65,536 candidates, m = 400, w = 200: 35.3 against
+// 47.4 ms, m = 500, w = 250 53 against 65; 4000 of them 2.75 against 3.12; one wave
+// of the other kernel 0.25 against 0.40).
+// The launch that finds nothing to do costs a call 3 to 5 us, so it is left out
+// where few candidates can be expected: a ranking at a refined bound, a cutoff below
+// 0.35 of the query's distance from its mean (random walks of m = 64 to 600 have less
+// than one window in 5000 there).
+LongDp long_dp(const DpJob& job, int sm_count) {
+    LongDp d{nullptr, 0, 0, 0, 0, false};
+    const int metric = job.q.metric, w = job.q.w, m = job.q.m;
+    if (job.few || job.cutoff < 0.35 * job.q.spread) return d;
+    const int k = (2 * w + 1 + 63) / 64;
+    if (w <= 20) {
+        d.kernel = dp_kernel(metric, false);
+        d.from = 2LL * sm_count * (34 + 3 * w) * (metric == MSM ? 3 : 4) / 4;
+        d.threads = kDpThreads;
+        d.smem = sizeof(double) * dp_warp_doubles(w) * (kDpThreads / 32);
+        d.blocks = (int)(size_t(220) * 1024 / (d.smem + 1024) < 16 ? size_t(220) * 1024 / (d.smem + 1024) : 16);
+        d.lane = true;
+    } else if (metric == MSM && k >= 5 && k <= kDpwMaxChunks && m <= (k == 5 ? 5 : 7) * w / 2) {
+        d.kernel = k == 5 ? (const void*)k_dpw<MSM, 5, false> : k == 6 ? (const void*)k_dpw<MSM, 6, false>
+                 : k == 7 ? (const void*)k_dpw<MSM, 7, false> : (const void*)k_dpw<MSM, 8, false>;
+        d.from = 12LL * sm_count;
+        d.threads = kDpwThreads;
+        d.smem = dpw_smem_bytes(m, kDpwThreads / 32);
+        d.blocks = 28;
+    }
+    return d;
 }
 
 }  // namespace fsm

@@ -53,6 +53,7 @@
 // DTW and ERP run best with 120 registers (8% slower at 80), MSM with 80 and six
 // blocks an SM (3% slower at 72).  A warp steps until its last candidate is
 // dropped: 1.5 (MSM) to 1.9 (ERP, DTW) lane rows per useful one.
+#include <cfloat>
 #include <type_traits>
 
 #include "common.cuh"
@@ -123,6 +124,24 @@ double mean_step(const double* x, int m) {
     return m > 1 ? s / (m - 1) : 0.0;
 }
 
+// The screen costs a fifth to a quarter (DTW, ERP) or two fifths (MSM, two passes)
+// of the lane-per-candidate DP on a list it drops nothing of, so it loses from
+// about 75% (60%) of the list kept on.  In units of the query's distance from its
+// mean (QueryDev::spread), random walks of m = 64 to 600, z-scored, have their 80th percentile at 1.07 to 1.73 (DTW), 0.81 to 1.33 (ERP), 0.82 to
+// 1.03 (MSM), rankings of a few of a million below 0.5, and no DTW or ERP distance
+// lies above 2.  Raw series have no such scale.  131,072 windows of m = 200, w = 6 at
+// a cutoff that keeps all: MSM 1.38 ms with the screen, 0.97 without.
+double screen_loose(int metric, double spread, bool raw) {
+    return raw ? DBL_MAX : (metric == DTW ? 1.3 : metric == ERP ? 1.15 : 0.9) * spread;
+}
+
+double query_spread(int metric, const double* x, int m) {
+    double mean = 0.0, s = 0.0;
+    for (int i = 0; i < m; ++i) mean += x[i] / m;
+    for (int i = 0; i < m; ++i) s += metric == MSM ? fabs(x[i] - mean) : (x[i] - mean) * (x[i] - mean);
+    return metric == MSM ? s : sqrt(s);
+}
+
 // Rows a pass: four from w = 4 on (ERP's row -4 lies inside the band), DTW eight
 // from w = 12.  A pass of R rows has R - 1 columns more than the band at half
 // their work.  Measured with two, four and eight rows: DTW w = 13 0.20, 0.148,
@@ -175,9 +194,9 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 6 : 1) k_scree
         Eb = 2.0 * e * cut_s + e * e;
     }
     const double lim_all = (Rc + Eb) * G * (1.0 + 0x1p-20);
-    // nothing to gain (a short list: the exact DP runs it in one wave) or no
-    // proof possible: every valid candidate goes on
-    const bool pass = n <= (unsigned long long)few || !(lim_all < 1e12) || !(xm + ymax + fabs(q.arg) < 1e9);
+    // nothing to gain (a short list: the exact DP runs it in one wave; a loose
+    // cutoff) or no proof possible: every valid candidate goes on
+    const bool pass = n <= (unsigned long long)few || cut >= q.loose || !(lim_all < 1e12) || !(xm + ymax + fabs(q.arg) < 1e9);
     const float ylim = (float)ymax, narrow = (float)(0x1p-21 * ymax + 1.01 * rel_err);
     const float grow = (float)(1.0 + (m + 16.0) * 0x1p-23);
 

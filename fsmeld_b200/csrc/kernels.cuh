@@ -80,6 +80,8 @@ struct DpJob {
     const double* cutoff_ptr;   // when set: the cutoff in device memory (read at kernel start)
     long long* screened;        // when set: room for the candidates an FP32 screen leaves
     unsigned long long* n_screened;
+    int few;                    // the screen will leave few (a ranking at a refined bound)
+    long long run_from, run_to; // runs on lists of [run_from, run_to) candidates only (run_to 0: no upper limit)
 };
 
 // LB_IP of a group of queries of equal (m, w) with shared thresholds as one
@@ -165,7 +167,8 @@ __global__ void k_dp(Geom g, DpJob job);
 const void* dp_kernel(int metric, bool gw);
 // wide-band DP: one warp per candidate, one anti-diagonal per step, the band
 // in registers (K chunks of 64 band offsets per warp, 2w+1 <= 64 K)
-template <int METRIC, int K>
+// INNER: with the fast steps away from the matrix's corners
+template <int METRIC, int K, bool INNER>
 __global__ void k_dpw(Geom g, DpJob job);
 constexpr int kDpwThreads = 32;  // one warp: a short list spreads over the SMs
 constexpr int kDpwMaxChunks = 8;  // w <= 255
@@ -175,6 +178,20 @@ const void* dpw_kernel(int metric, int w);
 // suffix sums of the abandon bound
 __host__ __device__ size_t dpw_warp_doubles(int m);
 size_t dpw_smem_bytes(int m, int warps);
+// the exact DP for lists of `from` candidates and more behind the screen (kernel
+// null: the wavefront kernel for every length)
+struct LongDp {
+    const void* kernel;
+    long long from;
+    int threads, blocks;  // threads a block, blocks an SM
+    size_t smem;
+    bool lane;
+};
+LongDp long_dp(const DpJob& job, int sm_count);
+// whether a list of n candidates is outside job's lengths
+__host__ __device__ inline bool other_length(const DpJob& job, unsigned long long n) {
+    return n < (unsigned long long)job.run_from || (job.run_to && n >= (unsigned long long)job.run_to);
+}
 // EDR and LCSS as bit vectors: the query's matching table (BitTab in
 // common.cuh), one lane per candidate
 constexpr int kBitThreads = 256;
@@ -201,6 +218,8 @@ const void* screen_kernel(int metric, int w);
 size_t screen_warp_bytes(int metric, int w);
 size_t screen_smem_bytes(int metric, int w, int m, int warps);
 double mean_step(const double* x, int m);  // QueryDev::step
+double query_spread(int metric, const double* x, int m);       // QueryDev::spread
+double screen_loose(int metric, double spread, bool raw);      // QueryDev::loose
 __global__ void k_lb_filter(Geom g, const double* __restrict__ z, const double* __restrict__ SIG,
                             const double* __restrict__ cutoff, int metric, long long* out,
                             unsigned long long* n_out, long long cap);

@@ -13,9 +13,9 @@
 // loads the library holds until the process exits.
 //
 // The DPs are those of the allocating path: DTW, ERP and MSM go through the
-// FP32 screen and the wavefront DP, EDR and LCSS through the bit vectors, a
-// cutoff that no bound can reach and bands below 2 through the lane DP.  Up to
-// kFinishSort matches are put in window order by one block; more are marked at
+// FP32 screen and the wavefront DP (long lists: long_dp), EDR and LCSS through the
+// bit vectors, a cutoff that no bound can reach and bands below 2 through the lane
+// DP.  Up to kFinishSort matches are put in window order by one block; more are marked at
 // their windows and compacted.  120,000 points, DTW, m = 200, w = 10: 0.47 ms
 // with the lane DP on every window and a serial compaction, 0.24 ms now.
 //
@@ -217,17 +217,18 @@ static int exact_noalloc(int device, const double* device_target, int64_t n, con
     qd.qlo = *std::min_element(t_qn, t_qn + m);
     qd.qhi = *std::max_element(t_qn, t_qn + m);
     qd.step = mean_step(t_qn, m);
+    qd.spread = query_spread(metric, t_qn, m);
+    qd.loose = screen_loose(metric, qd.spread, false);
     DpJob dj{};
     dj.q = qd; dj.target = device_target; dj.MU = MU; dj.SIG = SIG;
     dj.list = nullptr; dj.n_windows = g.tsn; dj.mode = 0; dj.cutoff = cutoff;
     dj.out_idx = li; dj.out_dist = ld; dj.n_out = cnt + 0; dj.out_cap = kMaxWin;
     dj.n_valid = cnt + 1; dj.next = cnt + 2; dj.gwork = nullptr;
-    auto launch = [&](const void* kf, void** args, int threads, size_t bytes, const char* what) -> int {
+    auto launch = [&](const void* kf, void** args, int threads, size_t bytes, const char* what, int per_sm = 0) -> int {
         cudaError_t le;
         if ((le = raise_smem_limit(kf, device, bytes)) != cudaSuccess)
             return cuda_fail(le, "cudaFuncSetAttribute", __FILE__, __LINE__);
-        int per_sm = 0;
-        if ((le = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kf, threads, bytes)) != cudaSuccess)
+        if (!per_sm && (le = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kf, threads, bytes)) != cudaSuccess)
             return cuda_fail(le, "occupancy", __FILE__, __LINE__);
         const unsigned grid = (unsigned)std::max(1, per_sm) * (unsigned)sms;
         if ((le = cudaLaunchKernel(kf, dim3(grid), dim3(threads), args, bytes, st)) != cudaSuccess)
@@ -282,8 +283,15 @@ static int exact_noalloc(int device, const double* device_target, int64_t n, con
         if ((r = launch(screen_kernel(metric, w), args, nw * 32, screen_smem_bytes(metric, w, m, nw), "k_screen"))) return r;
         dj.list = list; dj.n_list = n_list; dj.list_cap = kMaxWin; dj.n_valid = nullptr; dj.next = cnt + 5;
         void* args2[] = {&g, &dj};
+        const LongDp ld = long_dp(dj, sms);
+        const bool two = ld.kernel && g.tsn > ld.from;
+        if (two) dj.run_to = ld.from;
         if ((r = launch(dpw_kernel(metric, w), args2, kDpwThreads, dpw_smem_bytes(m, kDpwThreads / 32), "k_dpw")))
             return r;
+        dj.run_from = ld.from;
+        dj.run_to = 0;
+        dj.next = cnt + 6;
+        if (two && (r = launch(ld.kernel, args2, ld.threads, ld.smem, "exact DP", ld.blocks))) return r;
         done = true;
     }
     if (!done) {

@@ -71,3 +71,42 @@ def test_ranking_at_equal_bounds(api, oracle, metric, arg, seed):  # noqa: F811
                 assert list(ci) == list(oi) and bits_equal(cd, od), k
     finally:
         oracle.set_normalization("zscore")
+
+
+# The exact DP by the length of the list that the screen leaves (long_dp): lists on
+# both sides of the line, for the lane-per-candidate DP (w <= 20) and for MSM's
+# widest bands (five to eight register chunks, m near 2w); cutoffs that the
+# screen is used at and that it is not.  Long lists run on the kernel for them:
+# the wavefront's launch finds nothing to do.
+@pytest.mark.parametrize("metric,arg,m,w,n", [
+    ("dtw", 0.0, 24, 2, 30_000), ("erp", 0.4, 24, 6, 30_000), ("msm", 0.5, 24, 6, 30_000), ("dtw", 0.0, 40, 20, 48_000),
+    ("msm", 0.5, 24, 20, 48_000), ("dtw", 0.0, 24, 21, 12_000), ("msm", 0.5, 300, 140, 2600),
+    ("msm", 0.5, 300, 165, 2600), ("msm", 0.5, 300, 200, 2600), ("msm", 0.5, 300, 240, 2600)])
+def test_lists_behind_the_screen(api, oracle, metric, arg, m, w, n):  # noqa: F811
+    import torch
+
+    t = random_walk(n, [46, m, w])
+    t[700] = np.nan
+    q, _ = query_from(t, m, np.random.default_rng([47, m, w]))
+    oi, od, oc = oracle.exact(t, q, m, 1e300, metric, w, arg)
+    ranked = np.sort(od)
+    d_t = torch.from_numpy(t).cuda()
+    idx = torch.zeros(n, dtype=torch.int64, device="cuda")
+    dist = torch.zeros(n, dtype=torch.float64, device="cuda")
+    with api.Engine(t) as e:
+        for cut in (ranked[20], ranked[len(ranked) // 2], ranked[-1], 1e6):
+            keep = od <= cut
+            e.exact(q, m, float(cut), metric, w, arg)
+            e.set_profiling(True)
+            gi, gd, gc = e.exact(q, m, float(cut), metric, w, arg)
+            st = e.stage_times()
+            e.set_profiling(False)
+            assert list(gi) == list(oi[keep]) and gc["valid"] == oc["valid"], cut
+            assert bits_equal(gd, od[keep]), cut
+            if w > 94:  # fsmeld_exact_noalloc takes no wider band
+                continue
+            c = api.exact_noalloc(d_t.data_ptr(), n, q, m, float(cut), metric, w, arg, idx.data_ptr(), dist.data_ptr(), n)
+            assert c == keep.sum()
+            assert np.array_equal(idx[:c].cpu().numpy(), oi[keep]) and bits_equal(dist[:c].cpu().numpy(), od[keep])
+        if w <= 20:  # the last list holds every window
+            assert st["k_dp"][0] > 2 * st["k_dpw"][0]
