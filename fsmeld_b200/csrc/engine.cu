@@ -930,8 +930,7 @@ static int run_screen(fsmeld_ctx* c, const Geom& g, DpJob* job) {
     int per_sm = 0;
     FSM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kf, warps * 32, smem));
     const unsigned grid = (unsigned)(std::max(1, per_sm) * c->sm_count);
-    // the exact DP runs this many candidates in one wave of warps
-    long long few = 32LL * c->sm_count;
+    long long few = screen_few(*job, c->sm_count);
     Geom ga = g;
     void* args[] = {&ga, job, &job->screened, &job->n_screened, &few};
     prof_begin(c, ST_SCREEN);
@@ -947,9 +946,9 @@ static int run_screen(fsmeld_ctx* c, const Geom& g, DpJob* job) {
 }
 
 // the query's counters, all zero, and behind them the work counters of its DP
-// launches (the seeds', the refining windows', and the survivors' screen and two
-// exact DPs)
-constexpr int kNexts = 5;
+// launches (two for the seeds, two for the refining windows, the survivors' screen
+// and two exact DPs)
+constexpr int kNexts = 7;
 static int zero_counters(fsmeld_ctx* c, unsigned long long** cnt) {
     int r;
     if ((r = bufT(c, "counters", C_N + kNexts, cnt))) return r;
@@ -992,19 +991,21 @@ static int run_dp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
         FSM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wk, kDpwThreads, wsm));
         const long long want = (expected + kDpwThreads / 32 - 1) / (kDpwThreads / 32);
         grid = (unsigned)std::max<long long>(1, std::min<long long>(want, (long long)std::max(1, per_sm) * c->sm_count));
-        prof_begin(c, ST_DPW);
         Geom ga = g;
-        // a screened list's length stays on the device: both kernels are launched
-        // where it may be long, and one of them finds nothing to do (2 us)
-        LongDp ld{};
-        if (screened) ld = long_dp(job, c->sm_count);
-        const bool two = ld.kernel && list_max > ld.from;
-        if (two) job.run_to = ld.from;
+        // a list's length stays on the device: both kernels are launched where it may
+        // be long, and one of them finds nothing to do
+        const LongDp ld = long_dp(job, screened, c->sm_count);
+        const bool may_be_long = ld.kernel && list_max >= ld.from;
+        if (may_be_long) job.run_to = ld.from;
         void* args[] = {&ga, &job};
-        cudaError_t le = cudaLaunchKernel(wk, dim3(grid), dim3(kDpwThreads), args, wsm, c->stream);
-        if (le != cudaSuccess) return cuda_fail(le, "k_dpw launch", __FILE__, __LINE__);
-        LAUNCH_CHECK(c);
-        if (!two) return FSMELD_OK;
+        cudaError_t le = cudaSuccess;
+        if (job.list || !may_be_long) {
+            prof_begin(c, ST_DPW);
+            le = cudaLaunchKernel(wk, dim3(grid), dim3(kDpwThreads), args, wsm, c->stream);
+            if (le != cudaSuccess) return cuda_fail(le, "k_dpw launch", __FILE__, __LINE__);
+            LAUNCH_CHECK(c);
+        }
+        if (!may_be_long) return FSMELD_OK;
         job.run_from = ld.from;
         job.run_to = 0;
         job.next = next_counter(c);

@@ -509,27 +509,34 @@ const void* dpw_kernel(int metric, int w) {
 // time of one candidate, which the wavefront needs for (m = 256, DTW and MSM) 11,300
 // and 6700 candidates at w = 2, 14,700 and 10,200 at w = 6, 20,400 and 16,100 at
 // w = 13, 26,500 and 22,000 at w = 20; m = 64 up to a fifth more, m = 1000 a third less.
-// MSM's widest bands, where 2w comes near m: the kernel without interior steps runs
-// two to three times the warps (65,536 candidates, m = 400, w = 200: 35.3 against
-// 47.4 ms, m = 500, w = 250 53 against 65; 4000 of them 2.75 against 3.12; one wave
-// of the other kernel 0.25 against 0.40).
+// Lists that the screen hands on whole stay with the wavefront, whose abandon test
+// ends them early.
+// MSM's widest bands, where the steps near the corners outweigh the interior: the
+// kernel without interior steps runs two to three times the warps (65,536
+// candidates, m = 400, w = 200: 35.3 against 47.4 ms, m = 500, w = 250 53 against 65;
+// 4000 of them 2.75 against 3.12; one wave of the other kernel 0.25 against 0.40).
+// An unscreened GLB list ends within the first half of the rows mostly, so there
+// the line lies at twice the m: 45,013 candidates, m = 728, w = 161 8.4 and 10.6 ms.
 // The launch that finds nothing to do costs a call 3 to 5 us, so it is left out
 // where few candidates can be expected: a ranking at a refined bound, a cutoff below
 // 0.35 of the query's distance from its mean (random walks of m = 64 to 600 have less
 // than one window in 5000 there).
-LongDp long_dp(const DpJob& job, int sm_count) {
+LongDp long_dp(const DpJob& job, bool screened, int sm_count) {
     LongDp d{nullptr, 0, 0, 0, 0, false};
     const int metric = job.q.metric, w = job.q.w, m = job.q.m;
-    if (job.few || job.cutoff < 0.35 * job.q.spread) return d;
     const int k = (2 * w + 1 + 63) / 64;
-    if (w <= 20) {
+    const bool edges = metric == MSM && k >= 5 && k <= kDpwMaxChunks &&
+                       m <= (k == 5 ? 5 : 7) * w / (!screened && job.list ? 1 : 2);
+    if (screened && (job.few || job.cutoff < 0.35 * job.q.spread)) return d;
+    if (screened && w <= 20) {
+        const long long from = 2LL * sm_count * (34 + 3 * w) * (metric == MSM ? 3 : 4) / 4, few = screen_few(job, sm_count);
         d.kernel = dp_kernel(metric, false);
-        d.from = 2LL * sm_count * (34 + 3 * w) * (metric == MSM ? 3 : 4) / 4;
+        d.from = from > few ? from : few + 1;
         d.threads = kDpThreads;
         d.smem = sizeof(double) * dp_warp_doubles(w) * (kDpThreads / 32);
         d.blocks = (int)(size_t(220) * 1024 / (d.smem + 1024) < 16 ? size_t(220) * 1024 / (d.smem + 1024) : 16);
         d.lane = true;
-    } else if (metric == MSM && k >= 5 && k <= kDpwMaxChunks && m <= (k == 5 ? 5 : 7) * w / 2) {
+    } else if (edges) {
         d.kernel = k == 5 ? (const void*)k_dpw<MSM, 5, false> : k == 6 ? (const void*)k_dpw<MSM, 6, false>
                  : k == 7 ? (const void*)k_dpw<MSM, 7, false> : (const void*)k_dpw<MSM, 8, false>;
         d.from = 12LL * sm_count;

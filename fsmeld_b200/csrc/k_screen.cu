@@ -142,6 +142,24 @@ double query_spread(int metric, const double* x, int m) {
     return metric == MSM ? s : sqrt(s);
 }
 
+// Lists that go on whole.  A warp of the screen steps its 32 candidates one row after
+// another, so one with a match in it takes (2w+1) m cells however short the list is,
+// while the wavefront's abandon test ends most candidates of a GLB list early.  On
+// searches of random walks (rank 10 and 300; m = 2.6 w to 21 w) the two are even at lists of
+// 15,000 to 20,000 (w = 6), 16,000 to 30,000 (w = 13), 20,000 to 45,000 (w = 31), 30,000
+// to 60,000 (w = 67), 20,000 to 115,000 (w = 96), 30,000 to 180,000 (w = 129; DTW over
+// 200,000): MSM, m = 676, w = 129, 21,748 candidates 6.6 ms screened, 1.5 whole;
+// 64,861 of a looser cutoff 15 and 25; 973,569 91 and 224.  A scan of every window has no such test:
+// there the wavefront takes a list only when all of it fits one wave.
+long long screen_few(const DpJob& job, int sm_count) {
+    const int metric = job.q.metric, w = job.q.w;
+    const long long wave = 32LL * sm_count;
+    if (!job.list) return wave;
+    // DTW past w = 128: four rows a pass instead of eight
+    const double waves = metric == MSM ? 4.0 + w / 15.0 : (2.5 + w / 16.0) * (metric == DTW && w > 128 ? 4.0 : 1.0);
+    return (long long)(waves * (double)wave);
+}
+
 // Rows a pass: four from w = 4 on (ERP's row -4 lies inside the band), DTW eight
 // from w = 12.  A pass of R rows has R - 1 columns more than the band at half
 // their work.  Measured with two, four and eight rows: DTW w = 13 0.20, 0.148,

@@ -187,7 +187,7 @@ struct LongDp {
     size_t smem;
     bool lane;
 };
-LongDp long_dp(const DpJob& job, int sm_count);
+LongDp long_dp(const DpJob& job, bool screened, int sm_count);
 // whether a list of n candidates is outside job's lengths
 __host__ __device__ inline bool other_length(const DpJob& job, unsigned long long n) {
     return n < (unsigned long long)job.run_from || (job.run_to && n >= (unsigned long long)job.run_to);
@@ -215,6 +215,7 @@ template <int METRIC, int R>
 __global__ void k_screen(Geom g, DpJob job, long long* __restrict__ out, unsigned long long* __restrict__ n_out,
                          long long few);
 const void* screen_kernel(int metric, int w);
+long long screen_few(const DpJob& job, int sm_count);
 size_t screen_warp_bytes(int metric, int w);
 size_t screen_smem_bytes(int metric, int w, int m, int warps);
 double mean_step(const double* x, int m);  // QueryDev::step

@@ -276,14 +276,14 @@ static int exact_noalloc(int device, const double* device_target, int64_t n, con
                dpw_smem_bytes(m, kDpwThreads / 32) + 1024 <= (size_t)dev_optin) {
         const size_t per_warp = screen_warp_bytes(metric, w);
         const int nw = per_warp * 4 <= 64 * 1024 ? 4 : per_warp * 2 <= 96 * 1024 ? 2 : 1;
-        long long few = 32LL * sms;
+        long long few = screen_few(dj, sms);
         long long* list = (long long*)win;
         unsigned long long* n_list = cnt + 4;
         void* args[] = {&g, &dj, &list, &n_list, &few};
         if ((r = launch(screen_kernel(metric, w), args, nw * 32, screen_smem_bytes(metric, w, m, nw), "k_screen"))) return r;
         dj.list = list; dj.n_list = n_list; dj.list_cap = kMaxWin; dj.n_valid = nullptr; dj.next = cnt + 5;
         void* args2[] = {&g, &dj};
-        const LongDp ld = long_dp(dj, sms);
+        const LongDp ld = long_dp(dj, true, sms);
         const bool two = ld.kernel && g.tsn > ld.from;
         if (two) dj.run_to = ld.from;
         if ((r = launch(dpw_kernel(metric, w), args2, kDpwThreads, dpw_smem_bytes(m, kDpwThreads / 32), "k_dpw")))

@@ -73,8 +73,8 @@ def test_ranking_at_equal_bounds(api, oracle, metric, arg, seed):  # noqa: F811
         oracle.set_normalization("zscore")
 
 
-# The exact DP by the length of the list that the screen leaves (long_dp): lists on
-# both sides of the line, for the lane-per-candidate DP (w <= 20) and for MSM's
+# The screen and the exact DP by the length of the list (screen_few, long_dp): lists
+# on both sides of the lines, for the lane-per-candidate DP (w <= 20) and for MSM's
 # widest bands (five to eight register chunks, m near 2w); cutoffs that the
 # screen is used at and that it is not.  Long lists run on the kernel for them:
 # the wavefront's launch finds nothing to do.
@@ -103,6 +103,9 @@ def test_lists_behind_the_screen(api, oracle, metric, arg, m, w, n):  # noqa: F8
             e.set_profiling(False)
             assert list(gi) == list(oi[keep]) and gc["valid"] == oc["valid"], cut
             assert bits_equal(gd, od[keep]), cut
+            si, sc = e.search(q, m, float(cut), metric, w, arg)
+            yi, yc = oracle.search(t, q, m, float(cut), metric, w, arg)
+            assert list(si) == list(yi) and sc["after_glb"] == yc["after_glb"], cut
             if w > 94:  # fsmeld_exact_noalloc takes no wider band
                 continue
             c = api.exact_noalloc(d_t.data_ptr(), n, q, m, float(cut), metric, w, arg, idx.data_ptr(), dist.data_ptr(), n)
