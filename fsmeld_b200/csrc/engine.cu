@@ -398,9 +398,18 @@ static int buf(fsmeld_ctx* c, const std::string& name, size_t bytes, void** out)
     return FSMELD_OK;
 }
 
-// a buffer the caller can do without: false (and no error) when it does not fit
+// a buffer the caller can do without: false (and no error) when it does not fit;
+// a smaller one that is there already then stays
 static bool buf_optional(fsmeld_ctx* c, const std::string& name, size_t bytes, double** out) {
     void* p = nullptr;
+    {
+        fsmeld_ctx* root = ws_root(c);
+        std::lock_guard<std::mutex> lk(root->ws_mu);
+        const size_t own = c->bufs[name].bytes;
+        if (own < bytes && root->ws_limit > 0 &&
+            (long long)(ws_family_total(root) - own + bytes + bytes / 8) > root->ws_limit)
+            return false;
+    }
     if (buf(c, name, bytes, &p) == FSMELD_OK) { *out = (double*)p; return true; }
     cudaGetLastError();
     g_last_error.clear();
@@ -787,9 +796,9 @@ static int run_lbip(fsmeld_ctx* c, const Geom& g, LbJob job) {
 }
 
 // A query's lists of up to `cap` windows, in one buffer (an allocation takes the
-// driver as long as a small query): the LB_IP survivors, later what the screen
-// leaves; the results; and, where GLB runs, its two stages.
-enum { L_SURV, L_OUTI, L_OUTD, L_EXACT, L_G1 = L_EXACT, L_G1B, L_G1T, L_G2, L_G2T, L_ALL };
+// driver as long as a small query): the results; the LB_IP survivors, later what
+// the screen leaves; and, where GLB runs, its two stages.
+enum { L_OUTI, L_OUTD, L_RESULTS, L_SURV = L_RESULTS, L_EXACT, L_G1 = L_EXACT, L_G1B, L_G1T, L_G2, L_G2T, L_ALL };
 struct Lists {
     double* p = nullptr;
     size_t cap = 0;
@@ -915,7 +924,7 @@ static int run_bitdp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected
 // band and points take at most a third of an SM's shared memory; a cutoff no
 // bound can reach (every window is asked for) is not screened.
 static bool use_screen(const fsmeld_ctx* c, const DpJob& job) {
-    return job.screened && c->dp_form == 0 && !c->dp_exact && screen_kernel(job.q.metric, job.q.w) && job.q.w >= 2 &&
+    return c->dp_form == 0 && !c->dp_exact && screen_kernel(job.q.metric, job.q.w) && job.q.w >= 2 &&
            3 * screen_warp_bytes(job.q.metric, job.q.w) <= (size_t)c->smem_optin && (job.cutoff_ptr || job.cutoff < 1e12) &&
            dpw_kernel(job.q.metric, job.q.w) && dpw_smem_bytes(job.q.m, kDpwThreads / 32) + 1024 <= (size_t)c->smem_optin;
 }
@@ -970,7 +979,7 @@ static int run_dp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
     job.force_exact = c->dp_exact ? 1 : 0;
     unsigned grid;
     if (use_bitdp(c, job.q)) return run_bitdp(c, g, job, expected);
-    const bool screened = use_screen(c, job);
+    const bool screened = job.screened && use_screen(c, job);
     const long long list_max = job.list ? job.list_cap : job.n_windows;
     if (screened) {
         if ((r = run_screen(c, g, &job))) return r;
@@ -1318,16 +1327,21 @@ static int run_query(fsmeld_ctx* c, const QueryRun& qr, const Geom& g0, Stats& s
     out.tail = g.tsn % g.kml;
 
     if (qr.mode == 2) {  // exact: every valid window through the DP
-        Lists l;
-        if ((r = lists(c, cap, L_EXACT, &l))) return r;
-        long long* oi = l.i(L_OUTI);
-        double* od = l.d(L_OUTD);
         qd.cutoff = qr.cutoff;
         DpJob dj{};
         dj.q = qd; dj.target = c->d_target; dj.MU = st.MU; dj.SIG = st.SIG;
         dj.list = nullptr; dj.n_windows = g.tsn; dj.list_cap = cap; dj.mode = 0; dj.cutoff = qr.cutoff;
-        dj.screened = l.i(L_SURV);
-        dj.n_screened = cnt + C_SCREEN;
+        // the screen's list only where there is a screen and room for it
+        Lists l;
+        if (use_screen(c, dj) && buf_optional(c, "lists", sizeof(double) * L_EXACT * (size_t)cap, &l.p)) {
+            l.cap = (size_t)cap;
+            dj.screened = l.i(L_SURV);
+            dj.n_screened = cnt + C_SCREEN;
+        } else if ((r = lists(c, cap, L_RESULTS, &l))) {
+            return r;
+        }
+        long long* oi = l.i(L_OUTI);
+        double* od = l.d(L_OUTD);
         dj.out_idx = oi; dj.out_dist = od; dj.n_out = cnt + C_OUT; dj.n_cells = cnt + C_CELLS; dj.out_cap = cap; dj.n_valid = cnt + C_VALID;
         if ((r = run_dp(c, g, dj, g.tsn))) return r;
         if ((r = finish(c, cnt, cap, false, oi, od, qr.cap, qr.out_idx, qr.out_dist, h))) return r;
