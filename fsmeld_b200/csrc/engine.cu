@@ -321,6 +321,11 @@ struct fsmeld_ctx {
     bool raw = false;
     // workspace is short: envelopes without the buffers a query can do without
     bool lean = false;
+    // under a workspace limit: the bytes that the call's queries will still ask for
+    // after the envelopes (GLB's FP32 rows leave them room), and the contexts that
+    // share the limit with this one, each with its own statistics and envelopes
+    size_t rows_after = 0;
+    int rows_share = 1;
     double last_ms = 0.0;
     std::string err;
     struct Buf { void* p = nullptr; size_t bytes = 0; };
@@ -637,13 +642,31 @@ static int launch_env(fsmeld_ctx* c, const Geom& g, int w, Stats* st) {
     return FSMELD_OK;
 }
 
+// Whether the workspace limit has room for `bytes` of GLB's FP32 rows beside what
+// the queries will ask for; rows of an earlier call are given back where not.
+static bool rows_fit(fsmeld_ctx* c, const std::string& name, size_t bytes) {
+    fsmeld_ctx* root = ws_root(c);
+    if (root->ws_limit <= 0) return true;
+    bool fit, there;
+    {
+        std::lock_guard<std::mutex> lk(root->ws_mu);
+        const size_t own = c->bufs[name].bytes, want = std::max(own, bytes + bytes / 8);
+        const size_t held = c == root ? ws_family_total(root) : ws_total(c);
+        fit = (long long)(held - own + want + c->rows_after) <= root->ws_limit / c->rows_share;
+        there = own > 0;
+    }
+    if (!fit && there) release_buf(c, name);
+    return fit;
+}
+
 // GLB's FP32 rows: from 2^18 points on; below, the launch costs what they save
 static int run_rel(fsmeld_ctx* c, const Geom& g, int w, Stats* st, const std::string& tag) {
     st->rel = nullptr;
     st->rseg = nullptr;
     const size_t N = (size_t)g.S * g.m_k;
     double* p;
-    if (c->lean || g.n < (1 << 18) || !buf_optional(c, "rel" + tag, sizeof(double2) * g.S + sizeof(float) * 3 * N, &p))
+    const size_t bytes = sizeof(double2) * g.S + sizeof(float) * 3 * N;
+    if (c->lean || g.n < (1 << 18) || !rows_fit(c, "rel" + tag, bytes) || !buf_optional(c, "rel" + tag, bytes, &p))
         return FSMELD_OK;
     st->rseg = (double2*)p;
     st->rel = (float*)(st->rseg + g.S);
@@ -808,6 +831,19 @@ struct Lists {
 static int lists(fsmeld_ctx* c, long long cap, int slots, Lists* l) {
     l->cap = (size_t)cap;
     return bufT(c, "lists", (size_t)slots * (size_t)cap, &l->p);
+}
+
+// What a search or top-k query asks for after the envelopes, at most, less what the
+// context (null: not there yet) holds of it.
+static size_t query_buffers(const fsmeld_ctx* c, const Geom& g, bool topk) {
+    size_t need = sizeof(double) * ((size_t)L_ALL * g.tsn + 10 * (size_t)g.S + (topk ? (size_t)g.S * g.kml : 0));
+    need += need / 8 + (2 << 20);
+    for (const char* name : {"lists", "zbuf"}) {
+        if (!c) break;
+        const auto it = c->bufs.find(name);
+        if (it != c->bufs.end()) need -= std::min(need, it->second.bytes);
+    }
+    return need;
 }
 
 // counters slot layout
@@ -1813,7 +1849,14 @@ static int run_tasks_parallel(fsmeld_ctx* c, std::vector<QueryRun>& runs, const 
                 any = any || wanted(k);
             }
             if (!any) { gi = gj; continue; }
-            if (need_env && (q = run_env(wk, g, w, &st, ""))) { mark(gi, gj, q); gi = gj; continue; }
+            bool topk = false;
+            for (size_t k = gi; k < gj; ++k) topk = topk || runs[order[k]].mode == 1;
+            wk->rows_after = query_buffers(wk, g, topk);
+            wk->rows_share = conc;
+            if (need_env) q = run_env(wk, g, w, &st, "");
+            wk->rows_after = 0;
+            wk->rows_share = 1;
+            if (q) { mark(gi, gj, q); gi = gj; continue; }
             std::vector<char> done(hi, 0);
             for (size_t k = gi; k < gj; ++k) done[k] = !wanted(k);
             if ((q = group_gemm(wk, g, st, runs, order, gi, gj, status, &done, false)) == FSMELD_E_CUDA) {
@@ -1928,7 +1971,19 @@ int run_batch(fsmeld_ctx* c, std::vector<QueryRun>& runs, std::vector<int>* stat
         bool need_env = false;
         for (size_t k = oi; k < oj; ++k) need_env = need_env || runs[order[k]].mode != 2;
         if (!r && need_env && w != cur_w) {
+            bool topk = false;
+            int n_glb = 0;
+            for (size_t k = oi; k < oj; ++k) {
+                topk = topk || runs[order[k]].mode == 1;
+                n_glb += runs[order[k]].mode != 2;
+            }
+            c->rows_after = 0;
+            if (std::min(std::max(1, c->concurrency), n_glb) <= 1) c->rows_after = query_buffers(c, g, topk);
+            else
+                for (int t = 0; t < std::min(c->concurrency, n_glb); ++t)
+                    c->rows_after += query_buffers(t < (int)c->workers.size() ? c->workers[t] : nullptr, g, topk);
             r = run_env(c, g, w, &st, "");
+            c->rows_after = 0;
             cur_w = r ? -1 : w;
             have_env = !r;
         }

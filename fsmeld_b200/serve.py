@@ -65,7 +65,7 @@ def footprint(n: int, m: int, mode: str, concurrent: int = 1) -> int:
     shared = 16 * S * kml      # window means and sigmas
     shared += 16 * S * mk      # segment envelopes U/L_normal
     shared += 16 * n           # forward windows min/max of the raw target
-    # (the FP32 rows, 12 S mk more, are given up when they do not fit)
+    # (GLB's FP32 rows are in `rows_bytes`: used where there is room)
     q = 40 * tsn               # GLB stage lists (index, boundary, T->Q, survivors, Q->T)
     q += 24 * tsn              # survivors and the (index, distance) result list
     q += 16 * tsn              # sort buffers of the results
@@ -74,6 +74,16 @@ def footprint(n: int, m: int, mode: str, concurrent: int = 1) -> int:
         q += 8 * S * kml + 24 * S  # LB values of every window, seed distances
     per_query = int(q * 1.05) + (64 << 20)  # kernel scratch (sort temporaries, work areas)
     return int(shared * 1.05) + max(1, concurrent) * per_query
+
+
+def rows_bytes(n: int, m: int) -> int:
+    """GLB's FP32 rows of a search or top-k on a target of n points: what a
+    request gains speed from but does not need."""
+    if n < 1 << 18:
+        return 0
+    mk = macro_length(m, n)
+    S = -(-(n - m + 1) // (mk - m + 1))
+    return int((12 * S * mk + 16 * S) * 1.13)
 
 
 class ServerError(RuntimeError):
@@ -283,9 +293,14 @@ class Server:
                 batch, fps = [r for r, _ in keep], [fp for _, fp in keep]
             for r in batch:
                 self._queue.remove(r)
-            # grant enough for the engine's concurrent queries, within the room
-            want = sum(sorted(fps)[-CONCURRENCY:])
-            grant = min(room, max(self._held(eng), want))
+            # grant enough for the engine's concurrent queries, within the room, and
+            # the FP32 rows unless they take the room of another such batch
+            want = max(self._held(eng), sum(sorted(fps)[-CONCURRENCY:]))
+            if head.mode != "exact":
+                rows = max(rows_bytes(tgt.n, r.spec["m"]) if r.spec["m"] <= tgt.n else 0 for r in batch)
+                if not room - want - rows < max(fps) <= room - want:
+                    want += rows
+            grant = min(room, want)
             self._granted[id(eng)] = grant
             self._busy.add(id(eng))
             return batch, fps, eng, grant

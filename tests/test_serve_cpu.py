@@ -10,7 +10,7 @@ import time
 import numpy as np
 import pytest
 
-from fsmeld_b200.serve import E_NOMEM, Server, ServerError, footprint
+from fsmeld_b200.serve import E_NOMEM, Server, ServerError, footprint, rows_bytes
 
 
 class FakeEngine:
@@ -224,5 +224,25 @@ def test_large_result_alone_after_release():
         idx, cnt = srv.submit("a", "search", _q(3), 32, "dtw", 3, cutoff=99.0).result(timeout=10)
         assert list(idx) == [0, 1, 2, 3, 4]
         assert engines[0].released == 1
+    finally:
+        srv.close()
+
+
+@pytest.mark.parametrize("extra", ["plenty", "none", "one_more"])
+def test_grant_leaves_room_for_the_rows(extra):
+    """A batch is granted GLB's FP32 rows beside its footprint where there is
+    room, and not where they would take the room of another request."""
+    log, engines = [], []
+    n, m = 1 << 20, 64
+    fp, rows = footprint(n, m, "search"), rows_bytes(n, m)
+    assert rows > 12 * n
+    budget = 8 * n + fp + {"plenty": 4 * fp, "none": 0, "one_more": fp + rows // 2}[extra]
+    srv = Server(budget_bytes=budget, slots=1, engine_factory=lambda t: engines.append(FakeEngine(t, log)) or engines[-1])
+    try:
+        srv.add_target("a", np.zeros(n))
+        srv.submit("a", "search", _q(1, m), m, "dtw", 3, cutoff=1.0).result(timeout=10)
+        assert engines[0].limit == fp + (rows if extra == "plenty" else 0)
+        srv.submit("a", "exact", _q(1, m), m, "dtw", 3, cutoff=1.0).result(timeout=10)
+        assert engines[0].limit < fp + rows
     finally:
         srv.close()
