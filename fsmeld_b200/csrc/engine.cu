@@ -342,6 +342,7 @@ struct fsmeld_ctx {
     unsigned long long* next = nullptr;
     int next_used = 0;
     bool prof = false;
+    bool prof_open = false;  // the last record has no end yet
     struct ProfRec { int stage; cudaEvent_t a, b; };
     std::vector<ProfRec> pending;
     std::vector<cudaEvent_t> pool;
@@ -463,10 +464,12 @@ static void prof_begin(fsmeld_ctx* c, int stage) {
     fsmeld_ctx::ProfRec r{stage, prof_event(c), prof_event(c)};
     cudaEventRecord(r.a, c->stream);
     c->pending.push_back(r);
+    c->prof_open = true;
 }
 static void prof_end(fsmeld_ctx* c) {
-    if (!c->prof || c->pending.empty()) return;
+    if (!c->prof || c->pending.empty() || !c->prof_open) return;
     cudaEventRecord(c->pending.back().b, c->stream);
+    c->prof_open = false;
 }
 static void prof_collect(fsmeld_ctx* c) {
     if (c->pending.empty()) return;
@@ -577,6 +580,7 @@ static int upload_query(fsmeld_ctx* c, const HostQuery& hq, const std::string& s
         if ((r = bufT(c, "bit" + slot, words, &tab))) return r;
         bt.table = tab;
         const unsigned grid = (unsigned)std::min<size_t>((words + 255) / 256, (size_t)c->sm_count * 8);
+        prof_begin(c, ST_BIT);
         k_bit_table<<<grid, 256, 0, c->stream>>>(pa, pa + m, m, bt.pad, bt.rs, tab);
         LAUNCH_CHECK(c);
     }

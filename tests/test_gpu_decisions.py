@@ -113,3 +113,23 @@ def test_lists_behind_the_screen(api, oracle, metric, arg, m, w, n):  # noqa: F8
             assert np.array_equal(idx[:c].cpu().numpy(), oi[keep]) and bits_equal(dist[:c].cpu().numpy(), od[keep])
         if w <= 20:  # the last list holds every window
             assert st["k_dp"][0] > 2 * st["k_dpw"][0]
+
+
+# Stage times: every launch has a record of its own (the matching table of EDR and
+# LCSS counts with its DP), so no stage takes the time up to another's launch.
+@pytest.mark.parametrize("metric", ["edr", "lcss", "dtw"])
+def test_stage_records(api, metric):  # noqa: F811
+    t = random_walk(20_000, 48)
+    q, _ = query_from(t, 64, np.random.default_rng(49))
+    spec = [dict(query=q, m=64, metric=metric, w=3, arg=0.25 if metric != "dtw" else 0.0, cutoff=0.5)] * 3
+    with api.Engine(t) as e:
+        e.set_concurrency(1)
+        e.set_lb_form("fft")
+        e.batch("search", spec)
+        before = e.launches
+        e.set_profiling(True)
+        e.batch("search", spec)
+        st = e.stage_times()
+        e.set_profiling(False)
+        assert sum(v[1] for v in st.values()) == e.launches - before
+        assert st["k_bitdp"][1] == (0 if metric == "dtw" else 6)
