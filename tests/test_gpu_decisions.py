@@ -133,3 +133,49 @@ def test_stage_records(api, metric):  # noqa: F811
         e.set_profiling(False)
         assert sum(v[1] for v in st.values()) == e.launches - before
         assert st["k_bitdp"][1] == (0 if metric == "dtw" else 6)
+
+
+# LB_IP by the changes of the masks, against the products in extended precision:
+# off by the fixed-point rounding of each penalty (m/2 units of 2^-60 m h_max a
+# side), the two conversions and, squared again here, the root.  Noise (a change at
+# nearly every position), walks, raw series of large values and with spikes that
+# become thresholds.
+@pytest.mark.parametrize("kind", ["walk", "noise", "raw", "spikes"])
+@pytest.mark.parametrize("m,w", [(16, 0), (100, 0), (200, 1), (1000, 9), (512, 26)])
+@pytest.mark.parametrize("metric,arg", [("dtw", 0.0), ("erp", 0.4), ("msm", 0.5)])
+def test_mask_changes_in_extended_precision(api, oracle, metric, arg, m, w, kind):  # noqa: F811
+    mk = 1
+    while mk < 8 * m:
+        mk *= 2
+    kml = mk - m + 1
+    t = np.random.default_rng([50, m]).normal(size=2 * kml + m) if kind == "noise" else random_walk(2 * kml + m, [50, m])
+    raw = kind in ("raw", "spikes")
+    q, _ = query_from(t, m, np.random.default_rng([51, m]))
+    if kind == "raw":
+        t, q = t * 1e4 + 1e5, q * 1e4 + 1e5
+    if kind == "spikes":
+        t[[kml // 3, kml + kml // 2]] += [1e12, -1e12]
+    x = np.asarray(q) if raw else oracle.normalize_query(q)
+    with api.Engine(t) as e:
+        e.set_normalization("raw" if raw else "zscore")
+        z = e.inspect(q, m, metric, w, arg, 5).reshape(-1, kml)
+        thr = e.inspect(q, m, metric, w, arg, 4).reshape(-1, 2)
+        un = e.inspect(q, m, metric, w, arg, 2).reshape(-1, mk)
+        ln = e.inspect(q, m, metric, w, arg, 3).reshape(-1, mk)
+    for s in range(2):
+        tl, tu = thr[s]
+        h = [oracle.q_to_h(u, metric, x, thr[s, u], arg).astype(np.longdouble) for u in (0, 1)]
+        g = [ln[s] >= tl, un[s] <= tu]
+        ref = np.zeros(kml, dtype=np.longdouble)
+        for u in (0, 1):
+            for k in range(m):
+                ref += h[u][k] * g[u][k:k + kml]
+        far = [max(0.0, tl - x.min()), max(0.0, x.max() - tu)]
+        hmax = [min(f, arg) if metric == "msm" else f * f for f in far]
+        if metric == "erp":
+            hmax = [min(v, max((x.min() - arg) ** 2, (x.max() - arg) ** 2)) for v in hmax]
+        tol = sum(0.5 * m * 2.0 ** -60 * m * v for v in hmax) + 2.0 ** -50 * ref
+        got = z[s].astype(np.longdouble)
+        ok = ~np.isnan(got)
+        err = np.abs((got if metric == "msm" else got * got) - ref)
+        assert ok.any() and np.all(err[ok] <= tol[ok]), (s, float((err[ok] / tol[ok]).max()))
