@@ -200,12 +200,14 @@ __device__ __forceinline__ double qt_term(int metric, double x, int k, int m, in
 // +inf; grid[b] is the number of ends in buckets below b; table has a row of
 // rs words for each of the 2m + 1 ranges between ends.
 constexpr int kBitBuckets = 2048;
+constexpr int kBitDeep = 12;
 struct BitTab {
     const double* E = nullptr;
     const unsigned short* grid = nullptr;
     const unsigned* table = nullptr;
     int rs = 0, pad = 0;  // words per row, zero words in front of query point 0
     int in_smem = 0;
+    int most = 0;         // the most ends in one bucket
     double e0 = 0.0, elast = 0.0, scale = 0.0;
 };
 

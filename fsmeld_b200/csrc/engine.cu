@@ -191,6 +191,7 @@ void match_table(HostQuery* hq) {
         memcpy(&u, &v, 8);
         ++cnt[(int)(u & 0xffffffff) + 1];
     }
+    hq->bit_most = *std::max_element(cnt.begin(), cnt.end());
     for (int b = 1; b <= kBitBuckets; ++b) cnt[b] += cnt[b - 1];
     for (int b = 0; b <= kBitBuckets; ++b) hq->bitGrid[b] = (unsigned short)cnt[b];
 }
@@ -571,6 +572,7 @@ static int upload_query(fsmeld_ctx* c, const HostQuery& hq, const std::string& s
         bt.e0 = hq.bit_e0;
         bt.elast = hq.bit_elast;
         bt.scale = hq.bit_scale;
+        bt.most = hq.bit_most;
         const unsigned char* b = (const unsigned char*)dev + bytes0;
         bt.E = (const double*)b;
         const int* pa = (const int*)(b + hq.bitE.size() * 8);

@@ -19,6 +19,7 @@ struct HostQuery {
     std::vector<unsigned short> bitGrid;
     std::vector<int> bitA, bitB;
     double bit_e0 = 0.0, bit_elast = 0.0, bit_scale = 0.0;
+    int bit_most = 0;
 };
 
 // raw: the query is used as given (no z-normalisation; raw mode)

@@ -264,7 +264,7 @@ static int exact_noalloc(int device, const double* device_target, int64_t n, con
             k_bit_table<<<(unsigned)sms, 256, 0, st>>>(pa, pa + m, m, bt.pad, bt.rs, dt);
             if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_bit_table", __FILE__, __LINE__);
             bt.E = dE; bt.grid = dg; bt.table = dt;
-            bt.e0 = hq.bit_e0; bt.elast = hq.bit_elast; bt.scale = hq.bit_scale;
+            bt.e0 = hq.bit_e0; bt.elast = hq.bit_elast; bt.scale = hq.bit_scale; bt.most = hq.bit_most;
             size_t bytes = bit_table_offset(m);
             bt.in_smem = bytes + tab <= 54 * 1024;
             if (bt.in_smem) bytes += tab;

@@ -179,3 +179,41 @@ def test_mask_changes_in_extended_precision(api, oracle, metric, arg, m, w, kind
         ok = ~np.isnan(got)
         err = np.abs((got if metric == "msm" else got * got) - ref)
         assert ok.any() and np.all(err[ok] <= tol[ok]), (s, float((err[ok] / tol[ok]).max()))
+
+
+# The bit vectors with outliers among the query's points: nearly all ends of the
+# matching intervals in one bucket of the lookup (bisected there), windows with
+# and without the outlier, points on and beside the ends.  On its time: 30 times
+# that of the same query without the outlier when the bucket was stepped through.
+@pytest.mark.parametrize("spike", [50.0, -1e3, 1e9])
+@pytest.mark.parametrize("metric,arg", [("edr", 0.25), ("lcss", 0.25), ("edr", 0.0), ("lcss", 2.0)])
+def test_bit_vectors_with_outliers(api, oracle, metric, arg, spike):  # noqa: F811
+    m, w = 700, 9
+    t = np.round(random_walk(3500, 55), 2)
+    t[900] += spike
+    q = t[800:800 + m].copy()
+    q[::7] += 0.25
+    oracle.set_normalization("raw")
+    try:
+        with api.Engine(t) as e:
+            e.set_normalization("raw")
+            for cut in (1e300, 0.6 if metric == "lcss" else 300.0):
+                gi, gd, gc = e.exact(q, m, cut, metric, w, arg)
+                oi, od, oc = oracle.exact(t, q, m, cut, metric, w, arg)
+                assert list(gi) == list(oi) and bits_equal(gd, od) and gc["valid"] == oc["valid"]
+            ci, cd, _ = e.cutoff(q, m, 20, metric, w, arg)
+            oi, od, _ = oracle.cutoff(t, q, m, 20, metric, w, arg)
+            assert list(ci) == list(oi) and bits_equal(cd, od)
+
+            def scan(query):
+                times = []
+                for _ in range(5):
+                    e.exact(query, m, 1e300, metric, w, arg)
+                    times.append(e.last_call_ms)
+                return min(times)
+
+            plain = q.copy()
+            plain[100] = plain[99]
+            assert scan(q) < 4.0 * scan(plain)
+    finally:
+        oracle.set_normalization("zscore")
