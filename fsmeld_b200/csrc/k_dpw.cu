@@ -508,9 +508,11 @@ const void* dpw_kernel(int metric, int w) {
 // line lies where four of its blocks still fit an SM.  A short list takes it the
 // time of one candidate, which the wavefront needs for (m = 256, DTW and MSM) 11,300
 // and 6700 candidates at w = 2, 14,700 and 10,200 at w = 6, 20,400 and 16,100 at
-// w = 13, 26,500 and 22,000 at w = 20; m = 64 up to a fifth more, m = 1000 a third less.
-// Lists that the screen hands on whole stay with the wavefront, whose abandon test
-// ends them early.
+// w = 13, 26,500 and 22,000 at w = 20; m = 64 up to a fifth more.  From m = 700 on
+// shared memory holds fewer than 18 of the wavefront's warps an SM and the line falls
+// with them: m = 1000, w = 6 9400 and 8500, m = 2000, w = 10 6400.
+// GLB lists that the screen hands on whole stay with the wavefront, whose abandon
+// test ends them early.
 // MSM's widest bands, where the steps near the corners outweigh the interior: the
 // kernel without interior steps runs two to three times the warps (65,536
 // candidates, m = 400, w = 200: 35.3 against 47.4 ms, m = 500, w = 250 53 against 65;
@@ -529,7 +531,10 @@ LongDp long_dp(const DpJob& job, bool screened, int sm_count) {
                        m <= (k == 5 ? 5 : 7) * w / (!screened && job.list ? 1 : 2);
     if (screened && (job.few || job.cutoff < 0.35 * job.q.spread)) return d;
     if (screened && w <= 20) {
-        const long long from = 2LL * sm_count * (34 + 3 * w) * (metric == MSM ? 3 : 4) / 4, few = screen_few(job, sm_count);
+        // warps of the wavefront an SM: its candidate, query and suffix sums in shared memory
+        const long long warps = (long long)(size_t(220) * 1024 / dpw_smem_bytes(m, 1));
+        const long long from = 2LL * sm_count * (34 + 3 * w) * (metric == MSM ? 3 : 4) / 4 * (warps < 18 ? warps : 18) / 18;
+        const long long few = job.lraw ? screen_few(job, sm_count) : 0;
         d.kernel = dp_kernel(metric, false);
         d.from = from > few ? from : few + 1;
         d.threads = kDpThreads;
