@@ -26,7 +26,8 @@
 // the cutoff (squared for DTW, ERP; with the 1e-9 slack of the exact DP's
 // abandon test) less what the rows to come must still add: GLB's Q->T sum
 // less an upper bound of the terms of the rows done (FP32 on an envelope
-// narrowed by 2^-21 Y).  A candidate with a point beyond Y = 2A + 8 is kept.
+// narrowed by 2^-21 Y).  A candidate with a point beyond Y = 2A + 8 is kept (raw
+// series of values below 1: Y = 10A).
 // Points outside the matrix are +-1e15: every path through them costs at least
 // about 1e15, and the screen is skipped unless (R + E) G < 1e12.
 //
@@ -154,8 +155,8 @@ double query_spread(int metric, const double* x, int m) {
 long long screen_few(const DpJob& job, int sm_count) {
     const int metric = job.q.metric, w = job.q.w;
     const long long wave = 32LL * sm_count;
-    if (!job.list) return wave;
     // DTW past w = 128: four rows a pass instead of eight
+    if (!job.list) return wave;
     const double waves = metric == MSM ? 4.0 + w / 15.0 : (2.5 + w / 16.0) * (metric == DTW && w > 128 ? 4.0 : 1.0);
     return (long long)(waves * (double)wave);
 }
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 6 : 1) k_scree
     const float arg = (float)q.arg;
 
     const double xm = fmax(-q.qlo, q.qhi);
-    const double ymax = 2.0 * xm + 8.0;
+    const double ymax = 2.0 * xm + (g.raw ? fmin(8.0, 8.0 * xm) : 8.0);
     const double cut_s = cut + 1e-9 * (1.0 + fabs(cut));
     // FP32 points (RelMap's range test below): off by 2^-17 + 2^-23 Y more
     const double rel_err = job.rel ? 0x1.02p-17 + 0x1p-23 * ymax : 0.0;
@@ -212,9 +213,11 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 6 : 1) k_scree
         Eb = 2.0 * e * cut_s + e * e;
     }
     const double lim_all = (Rc + Eb) * G * (1.0 + 0x1p-20);
-    // nothing to gain (a short list: the exact DP runs it in one wave; a loose
-    // cutoff) or no proof possible: every valid candidate goes on
-    const bool pass = n <= (unsigned long long)few || cut >= q.loose || !(lim_all < 1e12) || !(xm + ymax + fabs(q.arg) < 1e9);
+    // nothing to gain (a short list, a loose cutoff) or no proof possible (distances
+    // past FP32's exact range; points far from zero that lie closer together than
+    // FP32 tells apart): every valid candidate goes on
+    const bool pass = n <= (unsigned long long)few || cut >= q.loose || !(lim_all < 1e12) ||
+                      !(xm + ymax + fabs(q.arg) < 1e9) || !(Eb < (METRIC == MSM ? q.spread : q.spread * q.spread));
     const float ylim = (float)ymax, narrow = (float)(0x1p-21 * ymax + 1.01 * rel_err);
     const float grow = (float)(1.0 + (m + 16.0) * 0x1p-23);
 
