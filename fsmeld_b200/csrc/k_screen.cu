@@ -150,14 +150,17 @@ double query_spread(int metric, const double* x, int m) {
 // 15,000 to 20,000 (w = 6), 16,000 to 30,000 (w = 13), 20,000 to 45,000 (w = 31), 30,000
 // to 60,000 (w = 67), 20,000 to 115,000 (w = 96), 30,000 to 180,000 (w = 129; DTW over
 // 200,000): MSM, m = 676, w = 129, 21,748 candidates 6.6 ms screened, 1.5 whole;
-// 64,861 of a looser cutoff 15 and 25; 973,569 91 and 224.  A scan of every window has no such test:
-// there the wavefront takes a list only when all of it fits one wave.
+// 64,861 of a looser cutoff 15 and 25; 973,569 91 and 224.  A scan of every window at
+// a tight cutoff ends early too (rank 25, m = 200 and 800: even at 46,000 to 230,000 windows for
+// DTW, 60,000 to 124,000 ERP, 20,000 to 114,000 MSM); at a looser one the
+// wavefront takes what it runs in the screen's time for one candidate (5000 to
+// 11,000 of full length).
 long long screen_few(const DpJob& job, int sm_count) {
     const int metric = job.q.metric, w = job.q.w;
     const long long wave = 32LL * sm_count;
     // DTW past w = 128: four rows a pass instead of eight
-    if (!job.list) return wave;
-    const double waves = metric == MSM ? 4.0 + w / 15.0 : (2.5 + w / 16.0) * (metric == DTW && w > 128 ? 4.0 : 1.0);
+    double waves = metric == MSM ? 4.0 + w / 15.0 : (2.5 + w / 16.0) * (metric == DTW && w > 128 ? 4.0 : 1.0);
+    if (!job.lraw) waves = job.cutoff < 0.35 * job.q.spread ? waves * (metric == MSM ? 2.0 : 3.0) : w >= 13 ? 2.0 : 1.0;
     return (long long)(waves * (double)wave);
 }
 
