@@ -217,3 +217,26 @@ def test_bit_vectors_with_outliers(api, oracle, metric, arg, spike):  # noqa: F8
             assert scan(q) < 4.0 * scan(plain)
     finally:
         oracle.set_normalization("zscore")
+
+
+# Raw series on which FP32 proves nothing (values far from zero against their
+# differences) are not screened, those of tiny values are: either way the scan does
+# less than the cells of one full band a window.
+@pytest.mark.parametrize("scale,shift", [(1e-9, 5.0), (1e-9, 0.0), (1.0, 1e7)])
+@pytest.mark.parametrize("metric,arg,w", [("dtw", 0.0, 25), ("erp", 0.0, 25), ("msm", 0.1, 25), ("dtw", 0.0, 5)])
+def test_raw_series_beyond_fp32(api, oracle, metric, arg, w, scale, shift):  # noqa: F811
+    n, m = 30_000, 120
+    t = random_walk(n, 56) * scale + shift
+    q = t[700:700 + m] + np.random.default_rng(57).normal(0.0, 0.1, m) * scale
+    oracle.set_normalization("raw")
+    try:
+        with api.Engine(t) as e:
+            e.set_normalization("raw")
+            _, d, _ = e.cutoff(q, m, 20, metric, w, arg * scale)
+            gi, gd, c = e.exact(q, m, float(d[-1]), metric, w, arg * scale)
+            oi, od, _ = oracle.exact(t, q, m, float(d[-1]), metric, w, arg * scale)
+            assert list(gi) == list(oi) and bits_equal(gd, od)
+            _, _, c = e.exact(q, m, 0.0, metric, w, arg * scale)
+            assert c["dp_cells"] < (n - m) * m * (2 * w + 1)
+    finally:
+        oracle.set_normalization("zscore")
