@@ -150,17 +150,21 @@ double query_spread(int metric, const double* x, int m) {
 // 15,000 to 20,000 (w = 6), 16,000 to 30,000 (w = 13), 20,000 to 45,000 (w = 31), 30,000
 // to 60,000 (w = 67), 20,000 to 115,000 (w = 96), 30,000 to 180,000 (w = 129; DTW over
 // 200,000): MSM, m = 676, w = 129, 21,748 candidates 6.6 ms screened, 1.5 whole;
-// 64,861 of a looser cutoff 15 and 25; 973,569 91 and 224.  A scan of every window at
-// a tight cutoff ends early too (rank 25, m = 200 and 800: even at 46,000 to 230,000 windows for
-// DTW, 60,000 to 124,000 ERP, 20,000 to 114,000 MSM); at a looser one the
-// wavefront takes what it runs in the screen's time for one candidate (5000 to
-// 11,000 of full length).
+// 64,861 of a looser cutoff 15 and 25; 973,569 91 and 224.  A scan of every window ends
+// early too, in proportion to the cutoff: even at 5000 to 11,000 windows of full
+// length and, at rank 25 (0.05 to 0.3 of the query's spread), at 46,000 to 230,000 for
+// DTW, 60,000 to 124,000 ERP, 20,000 to 114,000 MSM (m = 200, 800).  MSM, m = 800,
+// w = 31, 65,536 windows at rank 25: 2.1 ms screened, 1.1 whole.
 long long screen_few(const DpJob& job, int sm_count) {
     const int metric = job.q.metric, w = job.q.w;
     const long long wave = 32LL * sm_count;
     // DTW past w = 128: four rows a pass instead of eight
     double waves = metric == MSM ? 4.0 + w / 15.0 : (2.5 + w / 16.0) * (metric == DTW && w > 128 ? 4.0 : 1.0);
-    if (!job.lraw) waves = job.cutoff < 0.35 * job.q.spread ? waves * (metric == MSM ? 2.0 : 3.0) : w >= 13 ? 2.0 : 1.0;
+    if (!job.lraw) {
+        const double most = waves * (metric == MSM ? 2.0 : 3.0), full = w >= 13 ? 2.0 : 1.2;
+        const double by_cut = job.cutoff * most <= full * job.q.spread ? most : full * job.q.spread / job.cutoff;
+        waves = by_cut > full ? by_cut : full;
+    }
     return (long long)(waves * (double)wave);
 }
 
