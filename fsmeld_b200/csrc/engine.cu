@@ -960,6 +960,11 @@ static int run_bitdp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected
     return FSMELD_OK;
 }
 
+// the wavefront's band in registers and its candidate in shared memory
+static bool use_wave(const fsmeld_ctx* c, const QueryDev& q) {
+    return dpw_kernel(q.metric, q.w) && dpw_smem_bytes(q.m, kDpwThreads / 32) + 1024 <= (size_t)c->smem_optin;
+}
+
 // DTW, ERP, MSM: the FP32 screen, then `job` is the exact DP over what it left (by
 // the wavefront, or for long lists long_dp).
 // Bands from w = 2 (the kernel's row -2 lies inside the band) while a warp's
@@ -968,7 +973,7 @@ static int run_bitdp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected
 static bool use_screen(const fsmeld_ctx* c, const DpJob& job) {
     return c->dp_form == 0 && !c->dp_exact && screen_kernel(job.q.metric, job.q.w) && job.q.w >= 2 &&
            3 * screen_warp_bytes(job.q.metric, job.q.w) <= (size_t)c->smem_optin && (job.cutoff_ptr || job.cutoff < 1e12) &&
-           dpw_kernel(job.q.metric, job.q.w) && dpw_smem_bytes(job.q.m, kDpwThreads / 32) + 1024 <= (size_t)c->smem_optin;
+           use_wave(c, job.q);
 }
 
 static int run_screen(fsmeld_ctx* c, const Geom& g, DpJob* job) {
@@ -1149,7 +1154,7 @@ static int finish(fsmeld_ctx* c, const unsigned long long* cnt, long long cap, b
     memcpy(h, c->pin_out->cnt, sizeof(unsigned long long) * C_N);
     const long long nout = std::min<long long>((long long)h[C_OUT], cap);
     const long long n = std::min(nout, want);
-    if (n <= 0) return FSMELD_OK;
+    if (n <= 0 || (lex && nout < want)) return FSMELD_OK;  // a ranking with too few is refused
     if (nout <= kFinishSort && n <= kFinishOut) {
         if (out_idx) memcpy(out_idx, c->pin_out->idx, sizeof(long long) * n);
         if (out_dist) memcpy(out_dist, c->pin_out->dist, sizeof(double) * n);
@@ -1235,7 +1240,10 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     // seeds
     // seeds per segment: enough for k of them (2k over all segments), eight on
     // short targets (the seeds' DP is one wave up to some thousands), at most 32
-    const long long few_seg = std::min<long long>(8, (1024 + g.S - 1) / g.S);
+    // (one a segment where a window's distance takes one lane the time of the whole
+    // list: bands past the wavefront's and the bit vectors')
+    const bool slow = !use_bitdp(c, qd) && !use_wave(c, qd);
+    const long long few_seg = slow ? 1 : std::min<long long>(8, (1024 + g.S - 1) / g.S);
     const int per_seg =
         (int)std::min<long long>(32, std::max<long long>(std::max<long long>(1, few_seg), (2 * qr.k + g.S - 1) / g.S));
     const long long nslot = g.S * per_seg;
@@ -1260,10 +1268,10 @@ static int cutoff_tail(fsmeld_ctx* c, const Geom& g, const QueryDev& qd, const S
     // the query reads it from device memory, so the host waits only once
     long long *rl = (long long*)(sd + nslot), *ri = rl + kFinishSort;
     double *rd = (double*)(ri + kFinishSort), *tau_dev = rd + kFinishSort;
-    // refining windows: about 1024 of them or 2k; large k and seeds that give no
-    // bound go without
+    // refining windows: about 1024 of them or 2k; large k, seeds that give no bound
+    // and slow distances go without (m = 700, w = 699: 730 ms with them, 526 without)
     const long long span = 2 * kRefineReach + 1;
-    const int picks = qr.k <= 2048 && nslot >= qr.k
+    const int picks = qr.k <= 2048 && nslot >= qr.k && !slow
                           ? (int)std::min<long long>(kRefinePicks, (std::max<long long>(1024, 2 * qr.k) + span - 1) / span)
                           : 0;
     const double* sdist = sd;

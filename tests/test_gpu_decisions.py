@@ -240,3 +240,21 @@ def test_raw_series_beyond_fp32(api, oracle, metric, arg, w, scale, shift):  # n
             assert c["dp_cells"] < (n - m) * m * (2 * w + 1)
     finally:
         oracle.set_normalization("zscore")
+
+
+
+# Top-k past the wavefront's and the bit vectors' bands: the seeds' distances and the
+# survivors', no refining windows between (a launch more of one lane a window)
+@pytest.mark.parametrize("metric,arg", [("dtw", 0.0), ("msm", 0.5), ("lcss", 0.25)])
+def test_widest_bands_are_not_refined(api, oracle, metric, arg):  # noqa: F811
+    m, w = 280, 260
+    t = random_walk(1500, 58)
+    q, _ = query_from(t, m, np.random.default_rng(59))
+    with api.Engine(t) as e:
+        e.set_profiling(True)
+        ci, cd, _ = e.cutoff(q, m, 5, metric, w, arg)
+        st = e.stage_times()
+        e.set_profiling(False)
+    oi, od, _ = oracle.cutoff(t, q, m, 5, metric, w, arg)
+    assert list(ci) == list(oi) and bits_equal(cd, od)
+    assert st["k_dp"][1] == 2
