@@ -199,7 +199,7 @@ __device__ __noinline__ bool exact_tq(const double* __restrict__ Q, const double
         }
         if (alive) {
             for (; k < m - 1; ++k) tq = dadd(tq, tq_term<METRIC>(TN(k), LQ[k], UQ[k], arg));
-            if (dadd(boundary, tq) > lim) alive = false;
+            if (m > 2 && dadd(boundary, tq) > lim) alive = false;  // m = 2 has no inner point to test at
         }
     }
 #undef TN
@@ -270,7 +270,7 @@ __device__ __noinline__ bool warp_tq(const double* __restrict__ Q, const double*
     }
     if (METRIC == LCSS) {
         if (dmax0(dsub(1.0, ddiv(tq, (double)m))) > bsf) alive = false;
-    } else if (dadd(boundary, tq) > lim) {
+    } else if (m > 2 && dadd(boundary, tq) > lim) {
         alive = false;
     }
     boundary_out = boundary;
@@ -937,9 +937,9 @@ __global__ void __launch_bounds__(256, 3) k_glb_qt(Geom g, GlbJob job) {
                 } else {
                     const double tot = dadd(boundary, qt);
                     if (METRIC == DTW || METRIC == ERP)
-                        glb = (tot > dmul(bsf, bsf)) ? kGlbMax : dsqrt(dmax0(dadd(boundary, dmaxv(tq, qt))));
+                        glb = (m > 2 && tot > dmul(bsf, bsf)) ? kGlbMax : dsqrt(dmax0(dadd(boundary, dmaxv(tq, qt))));
                     else
-                        glb = (tot > bsf) ? kGlbMax : dadd(boundary, dmaxv(tq, qt));
+                        glb = (m > 2 && tot > bsf) ? kGlbMax : dadd(boundary, dmaxv(tq, qt));
                 }
                 keep = glb <= bsf;
                 os = boundary == -1.0 ? -1.0 : qt;

@@ -258,3 +258,24 @@ def test_widest_bands_are_not_refined(api, oracle, metric, arg):  # noqa: F811
     oi, od, _ = oracle.cutoff(t, q, m, 5, metric, w, arg)
     assert list(ci) == list(oi) and bits_equal(cd, od)
     assert st["k_dp"][1] == 2
+
+
+# m = 2: GLB is its boundary alone, and the reference abandons at inner points only;
+# cutoffs at the distances themselves, where the square's rounding decides
+@pytest.mark.parametrize("metric,arg", [("dtw", 0.0), ("erp", 0.4), ("msm", 0.5), ("edr", 0.25), ("lcss", 0.25)])
+@pytest.mark.parametrize("seed", range(4))
+def test_two_points(api, oracle, metric, arg, seed):  # noqa: F811
+    t = np.round(random_walk(400, [60, seed])) if seed < 2 else random_walk(400, [60, seed])
+    q = np.array([0.3, -1.1]) if seed % 2 else t[50:52] + np.array([0.01, -0.02])
+    raw = seed >= 2
+    oracle.set_normalization("raw" if raw else "zscore")
+    try:
+        with api.Engine(t) as e:
+            e.set_normalization("raw" if raw else "zscore")
+            _, od, _ = oracle.exact(t, q, 2, 1e300, metric, 0, arg)
+            for cut in np.unique(od)[:12]:
+                si, sc = e.search(q, 2, float(cut), metric, 0, arg)
+                oi, oc = oracle.search(t, q, 2, float(cut), metric, 0, arg)
+                assert list(si) == list(oi) and sc["after_glb"] == oc["after_glb"], cut
+    finally:
+        oracle.set_normalization("zscore")
