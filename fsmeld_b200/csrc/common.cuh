@@ -221,7 +221,7 @@ struct QueryDev {
     double qlo, qhi;       // smallest and largest point of qn
     double step;           // MSM: mean distance of neighbouring points of qn
     double spread;         // distance of qn from its mean: root of the squares' sum, MSM the sum of |x|
-    double loose;          // cutoffs from which on the FP32 screen drops too little
+    double loose;          // a scan's cutoffs from which on the FP32 screen drops nothing
     const double* qn;      // normalised query, original order [m]
     const double* LQ;      // query envelope (radius w) [m]
     const double* UQ;

@@ -853,7 +853,7 @@ static size_t query_buffers(const fsmeld_ctx* c, const Geom& g, bool topk) {
 }
 
 // counters slot layout
-enum { C_SURV, C_G1, C_G2, C_OUT, C_VALID, C_SEED, C_SEEDOUT, C_DPNEXT, C_CELLS, C_SCREEN, C_REF, C_REFOUT, C_N };
+enum { C_SURV, C_G1, C_G2, C_OUT, C_VALID, C_SEED, C_SEEDOUT, C_DPNEXT, C_CELLS, C_SCREEN, C_REF, C_REFOUT, C_SAMPLE, C_SAMPLEKEPT, C_N };
 
 static bool use_bitdp(const fsmeld_ctx* c, const QueryDev& q) { return q.bit.E && c->dp_form == 0 && !c->dp_exact; }
 
@@ -976,6 +976,8 @@ static bool use_screen(const fsmeld_ctx* c, const DpJob& job) {
            use_wave(c, job.q);
 }
 
+static unsigned long long* next_counter(fsmeld_ctx* c) { return c->next + c->next_used++; }
+
 static int run_screen(fsmeld_ctx* c, const Geom& g, DpJob* job) {
     const void* kf = screen_kernel(job->q.metric, job->q.w);
     const size_t per_warp = screen_warp_bytes(job->q.metric, job->q.w);
@@ -988,6 +990,24 @@ static int run_screen(fsmeld_ctx* c, const Geom& g, DpJob* job) {
     const unsigned grid = (unsigned)(std::max(1, per_sm) * c->sm_count);
     long long few = screen_few(*job, c->sm_count);
     Geom ga = g;
+    if (screen_sampled(*job, c->sm_count)) {
+        unsigned long long* two = c->next - C_N + C_SAMPLE;  // the query's counters lie before its work counters
+        DpJob js = *job;
+        js.n_windows = kScreenSample;
+        js.stride = job->n_windows / kScreenSample;
+        js.n_valid = two;
+        js.n_cells = nullptr;
+        js.next = next_counter(c);
+        unsigned long long* kept = two + 1;
+        long long none = 0;
+        void* args[] = {&ga, &js, &js.screened, &kept, &none};
+        prof_begin(c, ST_SCREEN);
+        const unsigned blocks = (unsigned)((kScreenSample / 32 + warps - 1) / warps);
+        const cudaError_t le = cudaLaunchKernel(kf, dim3(blocks), dim3(warps * 32), args, smem, c->stream);
+        if (le != cudaSuccess) return cuda_fail(le, "k_screen launch", __FILE__, __LINE__);
+        LAUNCH_CHECK(c);
+        job->sample = two;
+    }
     void* args[] = {&ga, job, &job->screened, &job->n_screened, &few};
     prof_begin(c, ST_SCREEN);
     const cudaError_t le = cudaLaunchKernel(kf, dim3(grid), dim3(warps * 32), args, smem, c->stream);
@@ -997,14 +1017,14 @@ static int run_screen(fsmeld_ctx* c, const Geom& g, DpJob* job) {
     job->n_list = job->n_screened;
     job->list_s = nullptr;
     job->n_valid = nullptr;
-    job->next = job->next + 1;  // its own counter (run_dp takes it off the list)
+    job->next = next_counter(c);
     return FSMELD_OK;
 }
 
 // the query's counters, all zero, and behind them the work counters of its DP
-// launches (two for the seeds, two for the refining windows, the survivors' screen
-// and two exact DPs)
-constexpr int kNexts = 7;
+// launches (two for the seeds, two for the refining windows, the survivors' sample,
+// screen and two exact DPs)
+constexpr int kNexts = 8;
 static int zero_counters(fsmeld_ctx* c, unsigned long long** cnt) {
     int r;
     if ((r = bufT(c, "counters", C_N + kNexts, cnt))) return r;
@@ -1013,7 +1033,6 @@ static int zero_counters(fsmeld_ctx* c, unsigned long long** cnt) {
     c->next_used = 0;
     return FSMELD_OK;
 }
-static unsigned long long* next_counter(fsmeld_ctx* c) { return c->next + c->next_used++; }
 
 static int run_dp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
     const int w = job.q.w;
@@ -1030,7 +1049,6 @@ static int run_dp(fsmeld_ctx* c, const Geom& g, DpJob job, long long expected) {
     const long long list_max = job.list ? job.list_cap : job.n_windows;
     if (screened) {
         if ((r = run_screen(c, g, &job))) return r;
-        next_counter(c);
         expected = (long long)c->sm_count * 16 * 128;
     }
     const bool gw_path = smem > (size_t)c->smem_optin - 4096;

@@ -126,14 +126,20 @@ double mean_step(const double* x, int m) {
 }
 
 // The screen costs a fifth to a quarter (DTW, ERP) or two fifths (MSM, two passes)
-// of the lane-per-candidate DP on a list it drops nothing of, so it loses from
-// about 75% (60%) of the list kept on.  In units of the query's distance from its
-// mean (QueryDev::spread), random walks of m = 64 to 600, z-scored, have their 80th percentile at 1.07 to 1.73 (DTW), 0.81 to 1.33 (ERP), 0.82 to
-// 1.03 (MSM), rankings of a few of a million below 0.5, and no DTW or ERP distance
-// lies above 2.  Raw series have no such scale.  131,072 windows of m = 200, w = 6 at
-// a cutoff that keeps all: MSM 1.38 ms with the screen, 0.97 without.
-double screen_loose(int metric, double spread, bool raw) {
-    return raw ? DBL_MAX : (metric == DTW ? 1.3 : metric == ERP ? 1.15 : 0.9) * spread;
+// of the lane-per-candidate DP on windows it drops none of, so a scan that keeps
+// over 75% (60%) of its windows does better without.  No z-scored DTW or ERP distance
+// lies above twice the query's spread, hardly an MSM distance above 1.5 times; below
+// that and from about the spread on a strided sample of the windows is screened
+// first (screen_sampled): random walks, z-scored, m = 64 to 600, have their median
+// at 0.8 to 1.5 of the spread (DTW), 0.7 to 1.2 (ERP, MSM), their 80th percentile at
+// 1.07 to 1.73 and 0.81 to 1.33.  131,072 windows of m = 200, w = 6 at a cutoff that keeps
+// all: MSM 1.38 ms with the screen, 0.97 without.
+double screen_loose(int metric, double spread, bool raw) { return raw ? DBL_MAX : (metric == MSM ? 1.5 : 2.0) * spread; }
+
+// A sample takes the time of one candidate's full band: scans of seven waves at least.
+bool screen_sampled(const DpJob& job, int sm_count) {
+    return !job.list && job.n_windows >= 7 * 32LL * sm_count &&
+           job.cutoff >= (job.q.metric == DTW ? 1.0 : 0.78) * job.q.spread && job.cutoff < job.q.loose;
 }
 
 double query_spread(int metric, const double* x, int m) {
@@ -150,7 +156,9 @@ double query_spread(int metric, const double* x, int m) {
 // 15,000 to 20,000 (w = 6), 16,000 to 30,000 (w = 13), 20,000 to 45,000 (w = 31), 30,000
 // to 60,000 (w = 67), 20,000 to 115,000 (w = 96), 30,000 to 180,000 (w = 129; DTW over
 // 200,000): MSM, m = 676, w = 129, 21,748 candidates 6.6 ms screened, 1.5 whole;
-// 64,861 of a looser cutoff 15 and 25; 973,569 91 and 224.  A scan of every window ends
+// 64,861 of a looser cutoff 15 and 25; 973,569 91 and 224.  Past 0.4 of the spread the
+// cutoff ends them later and the line falls with it (19,793 windows, m = 126, w = 3, MSM,
+// all near the cutoff: 0.26 ms screened, 0.41 whole).  A scan of every window ends
 // early too, in proportion to the cutoff: even at 5000 to 11,000 windows of full
 // length and, at rank 25 (0.05 to 0.3 of the query's spread), at 46,000 to 230,000 for
 // DTW, 60,000 to 124,000 ERP, 20,000 to 114,000 MSM (m = 200, 800).  MSM, m = 800,
@@ -159,7 +167,7 @@ long long screen_few(const DpJob& job, int sm_count) {
     const int metric = job.q.metric, w = job.q.w;
     const long long wave = 32LL * sm_count;
     // DTW past w = 128: four rows a pass instead of eight
-    double waves = metric == MSM ? 4.0 + w / 15.0 : (2.5 + w / 16.0) * (metric == DTW && w > 128 ? 4.0 : 1.0);
+    double waves = metric == MSM ? 4.0 + w / 15.0 : (1.8 + w / 20.0) * (metric == DTW && w > 128 ? 4.0 : 1.0);
     if (!job.lraw) {
         const double most = waves * (metric == MSM ? 2.0 : 3.0), full = w >= 13 ? 2.0 : 1.2;
         const double by_cut = job.cutoff * most <= full * job.q.spread ? most : full * job.q.spread / job.cutoff;
@@ -223,8 +231,11 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 6 : 1) k_scree
     // nothing to gain (a short list, a loose cutoff) or no proof possible (distances
     // past FP32's exact range; points far from zero that lie closer together than
     // FP32 tells apart): every valid candidate goes on
-    const bool pass = n <= (unsigned long long)few || cut >= q.loose || !(lim_all < 1e12) ||
+    // (few: for lists that the wavefront ends early, less so at cutoffs near the spread)
+    const double whole = job.lraw && cut > 0.4 * q.spread ? (double)few * (0.4 * q.spread / cut) : (double)few;
+    bool pass = (double)n <= whole || (!job.list && cut >= q.loose) || !(lim_all < 1e12) ||
                       !(xm + ymax + fabs(q.arg) < 1e9) || !(Eb < (METRIC == MSM ? q.spread : q.spread * q.spread));
+    if (job.sample) pass = pass || (double)job.sample[1] >= (METRIC == MSM ? 0.6 : 0.75) * (double)job.sample[0];
     const float ylim = (float)ymax, narrow = (float)(0x1p-21 * ymax + 1.01 * rel_err);
     const float grow = (float)(1.0 + (m + 16.0) * 0x1p-23);
 
@@ -252,7 +263,7 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 6 : 1) k_scree
         double mu = 0.0, sg = 1.0, S = 0.0;
         bool casc = false;
         if (active) {
-            gi = job.list ? job.list[item] : (long long)item;
+            gi = job.list ? job.list[item] : (long long)item * (job.stride ? job.stride : 1);
             g.locate(gi, &s, &j);
             mu = job.MU[s * g.kml + j];
             sg = job.SIG[s * g.kml + j];

@@ -81,6 +81,8 @@ struct DpJob {
     long long* screened;        // when set: room for the candidates an FP32 screen leaves
     unsigned long long* n_screened;
     int few;                    // the screen will leave few (a ranking at a refined bound)
+    long long stride;           // without a list: window of item i (0: i itself)
+    const unsigned long long* sample;  // optional: valid and kept windows of a sample that was screened before
     long long run_from, run_to; // runs on lists of [run_from, run_to) candidates only (run_to 0: no upper limit)
 };
 
@@ -216,6 +218,8 @@ __global__ void k_screen(Geom g, DpJob job, long long* __restrict__ out, unsigne
                          long long few);
 const void* screen_kernel(int metric, int w);
 long long screen_few(const DpJob& job, int sm_count);
+constexpr long long kScreenSample = 2048;
+bool screen_sampled(const DpJob& job, int sm_count);
 size_t screen_warp_bytes(int metric, int w);
 size_t screen_smem_bytes(int metric, int w, int m, int warps);
 double mean_step(const double* x, int m);  // QueryDev::step

@@ -54,7 +54,7 @@ constexpr int kMaxM = FSMELD_NOALLOC_MAX_M;
 constexpr long long kMaxKml = 8LL * kMaxM;  // kml < m_k <= 2^ceil(log2 8m) <= 8 * kMaxM
 // scratch layout (bytes, 256-aligned pieces)
 constexpr size_t kOffQuery = 0;                                        // qn [kMaxM]
-constexpr size_t kOffCnt = kOffQuery + sizeof(double) * kMaxM;         // counters [8]
+constexpr size_t kOffCnt = kOffQuery + sizeof(double) * kMaxM;         // counters [10]
 constexpr size_t kOffMu = kOffCnt + 256;                               // window means
 constexpr size_t kStatN = (size_t)(kMaxWin + kMaxKml);                 // [S][kml] covers tail padding
 constexpr size_t kOffSig = kOffMu + sizeof(double) * kStatN;           // window sigmas
@@ -278,6 +278,19 @@ static int exact_noalloc(int device, const double* device_target, int64_t n, con
         const int nw = per_warp * 4 <= 64 * 1024 ? 4 : per_warp * 2 <= 96 * 1024 ? 2 : 1;
         long long few = screen_few(dj, sms);
         long long* list = (long long*)win;
+        if (screen_sampled(dj, sms)) {
+            DpJob js = dj;
+            js.n_windows = kScreenSample;
+            js.stride = dj.n_windows / kScreenSample;
+            js.n_valid = cnt + 7;
+            js.next = cnt + 9;
+            unsigned long long* kept = cnt + 8;
+            long long none = 0;
+            void* sargs[] = {&g, &js, &list, &kept, &none};
+            if ((r = launch(screen_kernel(metric, w), sargs, nw * 32, screen_smem_bytes(metric, w, m, nw), "k_screen", 1)))
+                return r;
+            dj.sample = cnt + 7;
+        }
         unsigned long long* n_list = cnt + 4;
         void* args[] = {&g, &dj, &list, &n_list, &few};
         if ((r = launch(screen_kernel(metric, w), args, nw * 32, screen_smem_bytes(metric, w, m, nw), "k_screen"))) return r;
