@@ -624,7 +624,7 @@ static int run_stats(fsmeld_ctx* c, const Geom& g, Stats* st, const std::string&
     const int seg = mvmean_segments(g.S, c->sm_count);
     const unsigned blocks = (unsigned)((g.S + seg - 1) / seg);
     prof_begin(c, ST_STATS);
-    k_mvmean<<<blocks, kMvmeanThreads, smem, c->stream>>>(c->d_target, g, st->MU, st->SIG, seg);
+    k_mvmean<<<blocks, kMvmeanThreads, smem, c->stream>>>(c->d_target, g, st->MU, st->SIG, seg, c->sm_count);
     LAUNCH_CHECK(c);
     return FSMELD_OK;
 }

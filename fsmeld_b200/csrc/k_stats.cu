@@ -29,7 +29,7 @@
 // (mvmean_segments), so that their windows' divisions spread over more SMs.
 // Measured against one warp that loads, chains and stages: m_k = 16384 2.39 ->
 // 0.33 ms, 2^20 points with m_k = 1024 0.162 -> 0.046 ms, 2^24 points with
-// m_k = 2048 (585 blocks) 0.320 -> 0.165 ms = 2.6 TB/s.
+// m_k = 2048 (585 blocks) 0.320 -> 0.165 to 0.18 ms = 2.3 to 2.6 TB/s.
 //
 // Raw (non-normalised) mode (g.raw): a window is valid iff its points are all
 // finite, and its statistics are mean 0 and sigma 1, so every later stage
@@ -51,7 +51,7 @@ static_assert(2 * kHelpers == kRows, "helpers take rows h and h + kHelpers");
 
 __global__ void __launch_bounds__(kMvmeanThreads, 4) k_mvmean(const double* __restrict__ target, Geom g,
                                                               double* __restrict__ mu, double* __restrict__ sig,
-                                                              int seg) {
+                                                              int seg, int sms) {
     extern __shared__ __align__(16) double sm[];
     double* tin = sm;                                     // [2][kRows][kPitch] incoming points t[k], by tile parity
     double* tout = tin + 2 * kTileDoubles;                // [2][kRows][kPitch] outgoing points t[k-m]
@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(kMvmeanThreads, 4) k_mvmean(const double* __re
     const int lane = threadIdx.x & 31;
     // the chain warps of the blocks resident on one SM sit on different
     // sub-partitions (blocks are handed out to the SMs in turn)
-    const int id = threadIdx.x >> 5, cw = (int)(blockIdx.x / 148) & 3;
+    const int id = threadIdx.x >> 5, cw = (int)(blockIdx.x / (unsigned)sms) & 3;
     const bool chain = id == cw;
     const int h = id - (id > cw ? 1 : 0);  // helper: rows h and h + kHelpers
     const long long s0 = (long long)blockIdx.x * seg;  // seg <= kRows segments

@@ -132,7 +132,7 @@ constexpr int kLbGemmKChunk = 64;
 // and eight load the points and derive mean and sigma
 constexpr int kMvmeanThreads = 288;
 __global__ void k_mvmean(const double* __restrict__ target, Geom g, double* __restrict__ mu,
-                         double* __restrict__ sig, int seg);
+                         double* __restrict__ sig, int seg, int sms);
 int mvmean_segments(long long S, int sm_count);
 // one block per tile of T * OPT outputs of a segment
 template <int T, int OPT>

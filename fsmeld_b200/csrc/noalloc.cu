@@ -209,7 +209,7 @@ static int exact_noalloc(int device, const double* device_target, int64_t n, con
     if ((e = raise_smem_limit((const void*)k_mvmean, device, sm_stats)) != cudaSuccess)
         return cuda_fail(e, "cudaFuncSetAttribute", __FILE__, __LINE__);
     const int seg = mvmean_segments(g.S, sms);
-    k_mvmean<<<(unsigned)((g.S + seg - 1) / seg), kMvmeanThreads, sm_stats, st>>>(device_target, g, MU, SIG, seg);
+    k_mvmean<<<(unsigned)((g.S + seg - 1) / seg), kMvmeanThreads, sm_stats, st>>>(device_target, g, MU, SIG, seg, sms);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "k_mvmean", __FILE__, __LINE__);
 
     QueryDev qd{};
