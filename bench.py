@@ -156,7 +156,10 @@ def load_peaks():
 # three; MSM |x - y| + add, two split/merge costs (4 compares, 2 subs, 2 abs,
 # min, add) + adds, min of three.
 FLOPS_PER_CELL = {"dtw": 5, "erp": 11, "edr": 8, "lcss": 6, "msm": 27}
-SCREEN_OPS_PER_CELL = {"dtw": 5, "erp": 7, "msm": 6}  # k_screen
+# operations k_screen issues per cell (a fused multiply-add and a minimum of three are
+# one each); MSM's are those of its first pass, its second takes 12, which the
+# counter of cells does not tell apart
+SCREEN_OPS_PER_CELL = {"dtw": 3, "erp": 5, "msm": 5}
 # B200 FP64 issue rate: 148 SMs x 64 FP64 lanes x 1.965 GHz (the datasheet's
 # 37 TFLOP/s counts a fused multiply-add as two operations)
 FP64_PEAK_TOPS = 148 * 64 * 1.965e9 / 1e12
@@ -169,8 +172,8 @@ def roofline(stages, cells, peaks):
     decides what is left.  Algorithmic work = band cells computed (one device
     counter for both; early abandon skips the rest) x operations per cell, over
     the average launch time of the screen and the exact DP behind it.  With a
-    screen, which computes nearly all of the cells, those are the additions,
-    multiplications and minima of its own cells (MSM: without the intervals)
+    screen, which computes nearly all of the cells, those are the operations it
+    issues per cell (MSM: of the first pass, so its fraction is a lower bound)
     against the FP32 issue rate; otherwise those of the reference's recurrence
     against FP64's."""
     screen = stages.get("k_screen", (0.0, 0))

@@ -5,10 +5,11 @@ Two choices depend on the shape and are settled by measurement:
 * the exact DP kernel: the lane-per-candidate DP (band and candidate ring
   per lane in shared memory) or the anti-diagonal wavefront (one warp per
   candidate, band in registers), per metric, macro-segment length m_k and
-  radius w; `dp` rules for the DP over the GLB survivors of a search or
-  top-k query (timed as a search at the rank-50 distance on a structured
-  walk), `dpx` rules for the exact scan of every window (timed at the
-  rank-20 distance on a random walk).
+  radius w, where neither the FP32 screen (DTW, ERP and MSM with w >= 2 and a
+  cutoff below 1e12) nor the bit vectors (EDR and LCSS) run first: `dp` rules
+  for the candidate lists of a search or top-k query with w < 2 (timed as a
+  search at the rank-50 distance on a structured walk), `dpx` rules for the
+  scan at a cutoff past every distance (timed on a random walk).
 * the LB_IP form of batched searches (`lb` rules) and top-k queries (`lbk`):
   per-query thresholds and FP64 sums, or one tensor-core product for the
   group, per metric, m_k and group size.  Timed as one batched `search` of
@@ -38,6 +39,7 @@ from fsmeld_b200 import api
 from fsmeld_b200.synth import query_from, random_walk, walk_with_structure
 
 METRIC_ARGS = {"dtw": 0.0, "erp": 0.0, "edr": 0.25, "lcss": 0.25, "msm": 0.5}
+DP_METRICS = ("dtw", "erp", "msm")
 DP_SHAPES = {64: (2, 3, 6, 13, 31), 128: (3, 6, 13, 26, 51), 256: (6, 13, 26, 51, 94),
              512: (13, 26, 51, 94), 1024: (26, 51, 94), 2048: (51, 94)}
 LB_SHAPES = {128: (8, 32), 256: (8, 32), 512: (8, 32)}
@@ -76,10 +78,10 @@ def timed(eng, fn, reps=2):
 
 
 def tune_dp(metrics, shapes, log):
-    """dp: the DP over a candidate list (search and top-k), timed as a search
-    at the query's rank-50 distance on a structured walk of 2^20 points (the
-    search's other stages are the same for both forms); dpx: the exact scan
-    (every window), timed at the rank-20 distance on 2^16-2^17 points."""
+    """dp: the DP over a candidate list (search and top-k, w < 2), timed as a
+    search at the query's rank-50 distance on a structured walk of 2^20 points
+    (the search's other stages are the same for both forms); dpx: the scan that
+    keeps every window (cutoff 1e13), timed on 2^16-2^17 points."""
     rules = []
     for m, ws in shapes.items():
         n = (1 << 17) if m <= 256 else (1 << 16)
@@ -88,12 +90,14 @@ def tune_dp(metrics, shapes, log):
         ts = walk_with_structure(1 << 20, m, seed=9002 + m, motifs=40, nan_fraction=1e-3, flat_runs=8)
         qs, _ = query_from(ts, m, np.random.default_rng(9003 + m))
         for metric in metrics:
+            if metric not in DP_METRICS:
+                continue
             arg = METRIC_ARGS[metric]
-            for w in ws:
+            for w in (0, 1) + ws:
                 if w >= m or not lane_fits(w):
                     continue
                 mk = macro_length(m)
-                for kind in ("dp", "dpx"):
+                for kind in ("dp",) if w < 2 else ("dpx",):
                     times = {}
                     for form in ("lane", "wave"):
                         table = f"{kind} {metric} {mk} 1000 {form}\n"
@@ -104,9 +108,7 @@ def tune_dp(metrics, shapes, log):
                                 times[form] = timed(e, lambda: e.search(qs, m, cut, metric, w, arg))
                         else:
                             with api.Engine(t, tuning=table) as e:
-                                _, d, _ = e.cutoff(q, m, 20, metric, w, arg)
-                                cut = float(d[-1])
-                                times[form] = timed(e, lambda: e.exact(q, m, cut, metric, w, arg))
+                                times[form] = timed(e, lambda: e.exact(q, m, 1e13, metric, w, arg))
                     choice = choose(kind, times)
                     log(f"{kind} {metric} m={m} w={w}: lane {times['lane']:.2f} ms, wave {times['wave']:.2f} ms "
                         f"-> {choice}")

@@ -159,10 +159,12 @@ int fsmeld_set_lb_form(fsmeld_ctx* ctx, int form);
  *   lb <metric> <m_k> <q_min>  fft|gemm    LB_IP form for groups of >= q_min searches
  *   lbk <metric> <m_k> <q_min> fft|gemm    the same for groups of top-k queries
  * Shapes no rule covers keep the built-in choice (the per-query LB_IP; the lane
- * DP while its band fits shared memory).  dp and dpx rules reach only what the
- * FP32 screen and the bit vectors leave: lists of DTW, ERP and MSM with w < 2,
- * a cutoff of 1e12 or more, or a band too wide for the screen; EDR and LCSS
- * with bands past 16 words of bits.  fsmeld_b200/tune.py measures the
+ * DP while its band fits shared memory).  dp and dpx rules reach only what
+ * neither the FP32 screen nor the bit vectors take, in bands that the lane DP
+ * holds in shared memory: DTW, ERP and MSM with w < 2, at a cutoff of 1e12 or
+ * more, top-k seed lists of over 32 windows an SM and rankings without a bound
+ * (k over 32 per macro segment), and scans whose workspace has no room for the
+ * screen's list.  fsmeld_b200/tune.py measures the
  * rules on the GPU and writes fsmeld_b200/tune_table.txt, which the Python
  * binding loads into every context. */
 int fsmeld_set_tuning(fsmeld_ctx* ctx, const char* table);
