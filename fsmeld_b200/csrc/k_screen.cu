@@ -228,12 +228,13 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 6 : 1) k_scree
         Eb = 2.0 * e * cut_s + e * e;
     }
     const double lim_all = (Rc + Eb) * G * (1.0 + 0x1p-20);
-    // nothing to gain (a short list, a loose cutoff) or no proof possible (distances
-    // past FP32's exact range; points far from zero that lie closer together than
-    // FP32 tells apart): every valid candidate goes on
-    // (few: for lists that the wavefront ends early, less so at cutoffs near the spread)
-    bool pass = (n <= (unsigned long long)few && !(job.lraw && (double)n * cut > 0.4 * q.spread * (double)few)) || (!job.list && cut >= q.loose) || !(lim_all < 1e12) ||
-                      !(xm + ymax + fabs(q.arg) < 1e9) || !(Eb < (METRIC == MSM ? q.spread : q.spread * q.spread));
+    // nothing to gain (a short list, shorter at cutoffs past 0.4 of the spread, where
+    // the wavefront ends a GLB list later; a scan's loose cutoff, a sample that stayed)
+    // or no proof possible (distances past FP32's exact range; points far from zero
+    // that lie closer together than FP32 tells apart): every valid candidate goes on
+    bool pass = (n <= (unsigned long long)few && !(job.lraw && (double)n * cut > 0.4 * q.spread * (double)few)) ||
+                (!job.list && cut >= q.loose) || !(lim_all < 1e12) || !(xm + ymax + fabs(q.arg) < 1e9) ||
+                !(Eb < (METRIC == MSM ? q.spread : q.spread * q.spread));
     if (job.sample) pass = pass || 20 * job.sample[1] >= (METRIC == MSM ? 12 : 15) * job.sample[0];
     const float ylim = (float)ymax, narrow = (float)(0x1p-21 * ymax + 1.01 * rel_err);
     const float grow = (float)(1.0 + (m + 16.0) * 0x1p-23);
