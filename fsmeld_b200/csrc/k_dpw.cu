@@ -56,6 +56,8 @@
 // count is at most the maximum over the pair plus one possible match per
 // remaining row after the pair's smallest row.  A candidate whose bound
 // exceeds the cutoff (1e-9 relative slack) cannot be a match and stops.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -166,11 +168,12 @@ size_t dpw_smem_bytes(int m, int warps) {
 
 // blocks an SM the registers are held to (0: as many registers as it takes)
 constexpr int dpw_blocks(int metric, int k, bool inner) {
-    return metric != MSM ? 0 : inner ? (k == 6 ? 12 : 0) : k < 7 ? 28 : 0;
+    return metric != MSM ? 0 : inner ? (k == 6 ? 12 : 0) : k < 7 ? 7 : 0;
 }
+constexpr int kEdgeThreads = 128;  // at most, without interior steps
 
 template <int METRIC, int K, bool INNER>
-__global__ void __launch_bounds__(kDpwThreads, dpw_blocks(METRIC, K, INNER)) k_dpw(Geom g, DpJob job) {
+__global__ void __launch_bounds__(INNER ? kDpwThreads : kEdgeThreads, dpw_blocks(METRIC, K, INNER)) k_dpw(Geom g, DpJob job) {
     extern __shared__ __align__(16) double dpw_smem[];
     const QueryDev& q = job.q;
     const int m = q.m, w = q.w;
@@ -517,8 +520,17 @@ const void* dpw_kernel(int metric, int w) {
 // kernel without interior steps runs two to three times the warps (65,536
 // candidates, m = 400, w = 200: 35.3 against 47.4 ms, m = 500, w = 250 53 against 65;
 // 4000 of them 2.75 against 3.12; one wave of the other kernel 0.25 against 0.40).
-// An unscreened GLB list ends within the first half of the rows mostly, so there
-// the line lies at twice the m: 45,013 candidates, m = 728, w = 161 8.4 and 10.6 ms.
+// From m = 400 (five and six chunks) to 760 (eight) on, a block of four warps, which
+// share the query, fits more warps into an SM's shared memory than blocks of one
+// (m = 1368: 12 against 8): m = 1368, w = 255, 325,318 candidates that end early 134 ms
+// by blocks of one, 105 by blocks of four.
+// Unscreened candidates that end early, in a GLB list or at a small cutoff, hardly
+// get past the corner, so there the line lies higher for seven and eight chunks:
+// 40,000 windows, without and with interior steps, m = 1368, w = 255 16.9 and 22.1 ms
+// where 14% of the rows are stepped, 44.6 and 42.7 at 36%, 122 and 83 at all;
+// m = 1000, w = 200 9.4 and 14.7, 25.8 and 27.0, 65 and 53; m = 1368, w = 200 14.8 and
+// 17.5, 39 and 31, 109 and 68.  MSM abandons after 14% of the rows at a cutoff of a
+// tenth of the query's distance from its mean, after 36% at a quarter of it.
 // The launch that finds nothing to do costs a call 3 to 5 us, so it is left out
 // where few candidates can be expected: a ranking at a refined bound, a cutoff below
 // 0.35 of the query's distance from its mean (random walks of m = 64 to 600 have less
@@ -527,8 +539,9 @@ LongDp long_dp(const DpJob& job, bool screened, int sm_count) {
     LongDp d{nullptr, 0, 0, 0, 0, false};
     const int metric = job.q.metric, w = job.q.w, m = job.q.m;
     const int k = (2 * w + 1 + 63) / 64;
+    const bool early = !screened && (job.cutoff_ptr ? job.list != nullptr : job.cutoff < 0.3 * job.q.spread);
     const bool edges = metric == MSM && k >= 5 && k <= kDpwMaxChunks &&
-                       m <= (k == 5 ? 5 : 7) * w / (!screened && job.list ? 1 : 2);
+                       2 * m <= (k == 5 ? 5 : k == 6 || !early ? 7 : 11) * w;
     if (screened && (job.few || job.cutoff < 0.35 * job.q.spread)) return d;
     if (screened && w <= 20) {
         // warps of the wavefront an SM: its candidate, query and suffix sums in shared memory
@@ -545,9 +558,14 @@ LongDp long_dp(const DpJob& job, bool screened, int sm_count) {
         d.kernel = k == 5 ? (const void*)k_dpw<MSM, 5, false> : k == 6 ? (const void*)k_dpw<MSM, 6, false>
                  : k == 7 ? (const void*)k_dpw<MSM, 7, false> : (const void*)k_dpw<MSM, 8, false>;
         d.from = 12LL * sm_count;
-        d.threads = kDpwThreads;
-        d.smem = dpw_smem_bytes(m, kDpwThreads / 32);
-        d.blocks = 28;
+        // warps an SM by shared memory and by registers (72, 96 and 109 a thread)
+        const size_t room = size_t(220) * 1024;
+        const int one = (int)std::min<size_t>(k < 7 ? 28 : k == 7 ? 21 : 18, room / (dpw_smem_bytes(m, 1) + 1024));
+        const int four = (int)std::min<size_t>(k < 7 ? 7 : k == 7 ? 5 : 4, room / (dpw_smem_bytes(m, 4) + 1024));
+        const bool wide = 4 * four > one;
+        d.threads = wide ? kEdgeThreads : kDpwThreads;
+        d.smem = dpw_smem_bytes(m, d.threads / 32);
+        d.blocks = wide ? four : one;
     }
     return d;
 }

@@ -115,6 +115,28 @@ def test_lists_behind_the_screen(api, oracle, metric, arg, m, w, n):  # noqa: F8
             assert st["k_dp"][1] == 1
 
 
+# MSM's widest bands on long lists, by the kernel without interior steps in blocks of
+# four warps (m large for the shared memory), on both sides of the lines for
+# candidates that end early (m up to 3.5 w, 5.5 w); each chunk count from five on
+@pytest.mark.parametrize("m,w", [(396, 159), (460, 165), (760, 200), (800, 240)])
+def test_widest_bands_in_wide_blocks(api, oracle, m, w):  # noqa: F811
+    n = m + 1900
+    t = random_walk(n, [52, m, w])
+    t[700] = np.nan
+    q, _ = query_from(t, m, np.random.default_rng([53, m, w]))
+    oi, od, oc = oracle.exact(t, q, m, 1e300, "msm", w, 0.5)
+    ranked = np.sort(od)
+    with api.Engine(t) as e:
+        for cut in (0.5 * ranked[0], ranked[0], ranked[20], ranked[-1]):
+            keep = od <= cut
+            gi, gd, gc = e.exact(q, m, float(cut), "msm", w, 0.5)
+            assert list(gi) == list(oi[keep]) and gc["valid"] == oc["valid"], cut
+            assert bits_equal(gd, od[keep]), cut
+            si, sc = e.search(q, m, float(cut), "msm", w, 0.5)
+            yi, yc = oracle.search(t, q, m, float(cut), "msm", w, 0.5)
+            assert list(si) == list(yi) and sc["after_glb"] == yc["after_glb"], cut
+
+
 # Stage times: every launch has a record of its own (the matching table of EDR and
 # LCSS counts with its DP), so no stage takes the time up to another's launch.
 @pytest.mark.parametrize("metric", ["edr", "lcss", "dtw"])
