@@ -137,6 +137,33 @@ def test_widest_bands_in_wide_blocks(api, oracle, m, w):  # noqa: F811
             assert list(si) == list(yi) and sc["after_glb"] == yc["after_glb"], cut
 
 
+# Raw windows far off the query are dropped by the screen, four rows (ERP, MSM) or
+# eight (DTW) into the band, and not handed on; ERP with a gap value further out than
+# the points that the screen's bound covers
+@pytest.mark.parametrize("metric,arg,w", [("dtw", 0.0, 12), ("erp", 0.4, 6), ("erp", 500.0, 6), ("msm", 0.0, 6), ("msm", 0.5, 6)])
+def test_raw_windows_far_off(api, oracle, metric, arg, w):  # noqa: F811
+    n, m = 300_000, 40
+    rng = np.random.default_rng(54)
+    t = np.where(np.arange(n) // 5000 % 2, 1.0, -1.0) * (300.0 + rng.normal(size=n))
+    t[150_000:151_000] = random_walk(1000, 55)
+    t[150_100] = 90.0  # one point out of range, and in a window that matches without it
+    q = np.ascontiguousarray(t[150_300:150_340] + rng.normal(size=m) * 0.1)
+    oracle.set_normalization("raw")
+    try:
+        oi, od, _ = oracle.exact(t[149_000:152_000], q, m, 1e300, metric, w, arg)
+        with api.Engine(t) as e:
+            e.set_normalization("raw")
+            for cut in (np.sort(od)[0], np.sort(od)[30]):
+                gi, gd, gc = e.exact(q, m, float(cut), metric, w, arg)
+                keep = od <= cut
+                assert list(gi) == list(oi[keep] + 149_000) and bits_equal(gd, od[keep]), cut
+                rows = 8 if metric == "dtw" else 4
+                if arg < 100:
+                    assert gc["dp_cells"] < 1.5 * n * rows * (2 * w + 1), cut
+    finally:
+        oracle.set_normalization("zscore")
+
+
 # Stage times: every launch has a record of its own (the matching table of EDR and
 # LCSS counts with its DP), so no stage takes the time up to another's launch.
 @pytest.mark.parametrize("metric", ["edr", "lcss", "dtw"])
