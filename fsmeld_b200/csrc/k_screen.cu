@@ -283,8 +283,8 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 6 : 1) k_scree
             }
         }
         if (!active) gi = 0;
-        bool keep = active, over = false, nan = false;
-        float far = 0.f;
+        bool keep = active;
+        float far = 0.f;  // the furthest of the points so far (a NaN stays)
         auto run = [&](auto full_c) {
             constexpr bool FULL = decltype(full_c)::value;
             const double inv = 1.0 / sg;
@@ -321,9 +321,7 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 6 : 1) k_scree
                 float y = p < 0 ? -kOut : kOut;
                 if (p >= 0 && p < m) {
                     y = fast ? unpack(raw) : (float)((raw - mu) * inv);
-                    over = over || !(fabsf(y) <= ylim);
-                    far = fmaxf(far, fabsf(y));
-                    nan = nan || !(fabsf(y) <= FLT_MAX);
+                    asm("max.NaN.f32 %0, %0, %1;" : "+f"(far) : "f"(fabsf(y)));
                 }
                 return y;
             };
@@ -471,8 +469,8 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 6 : 1) k_scree
                         pre += term((float)((a - mu) * inv), (float)((c - mu) * inv), X[kk]);
                     }
                 }
-                if (over) {  // the rows' bound does not cover it
-                    if (far > far_lim && !nan) keep = false;
+                if (!(far <= ylim)) {  // the rows' bound does not cover it
+                    if (far > far_lim && far <= FLT_MAX) keep = false;
                     active = false;
                 } else if (active && ext > fmaf(pre, limg, lim0)) {
                     active = keep = false;
@@ -486,7 +484,7 @@ __global__ void __launch_bounds__(kScreenThreads, METRIC == MSM ? 6 : 1) k_scree
         if (!pass && __any_sync(kAll, active)) {
             if (METRIC == MSM && rough) {
                 run(std::false_type{});
-                active = keep && !over;
+                active = keep && far <= ylim;
                 __syncwarp();
             }
             if (__any_sync(kAll, active)) run(std::true_type{});
